@@ -89,7 +89,7 @@ def draw(rng):
             pz = rng.choice([32, 64, 128])
             if what == "green":
                 bx, by = [n if n != 96 else 64 for n in (bx, by)]
-        layer = pz // 4 if tiles else rng.randint(3, pz // 3)
+        layer = pz // 4 if tiles and what != "green" else rng.randint(3, pz // 3)
         nz = pz - 2 * layer
         radius = rng.uniform(2.0, min(16.0, bx / 6, by / 6, nz / 5))
         if radius < 1.0 or nz < 8:
