@@ -205,7 +205,7 @@ void fm_plan_destroy(fm_plan* P) {
   DevBuf* bufs[] = {&P->twx, &P->twy, &P->twz, &P->twz2, &P->rz, &P->rxp, &P->rxm, &P->ryp, &P->rym, &P->rzp,
                     &P->rzm, &P->V, &P->t1, &P->t2, &P->t3, &P->bbuf, &P->xbuf, &P->ebuf, &P->sbuf, &P->basis,
                     &P->gbuf2, &P->red_part, &P->red_out, &P->red_cnt, &P->active, &P->scale, &P->coef,
-                    &P->hbuf, &P->eps_dev, &P->fx, &P->fy, &P->fz, &P->maxpart, &P->maxout, &P->wt_x,
+                    &P->hbuf, &P->mgsT, &P->eps_dev, &P->fx, &P->fy, &P->fz, &P->maxpart, &P->maxout, &P->wt_x,
                     &P->wt_y, &P->wt_z, &P->wt_pe, &P->wt_ph, &P->wt_first, &P->Eo, &P->Ho, &P->errbuf,
                     &P->shifts, &P->yblk, &P->V64, &P->gtw[0], &P->gtw[1], &P->gtw[2], &P->gch[0][0],
                     &P->gch[0][1], &P->gch[1][0], &P->gch[1][1], &P->gch[2][0], &P->gch[2][1], &P->gkn[0][0],

@@ -44,4 +44,23 @@ template <typename T> __device__ __forceinline__ T from_d(double2 a);
 template <> __device__ __forceinline__ float2 from_d<float2>(double2 a) { return make_float2((float)a.x, (float)a.y); }
 template <> __device__ __forceinline__ double2 from_d<double2>(double2 a) { return a; }
 
+// ---- FP32 -> FP64 without the conversion unit ----
+// The conversion instruction issues about one lane per clock and scheduler on sm_100a, which caps a kernel that
+// widens every value it reads near 5 TB/s of FP32 data.  Moving the fields of the float into those of a double with
+// three integer instructions gives the value times WIDEN_SCALE = 2^-896 exactly, for zeros and subnormal numbers too
+// (the exponent field is kept unbiased and a double's smallest exponents take it).  The factor is taken out again by
+// exact powers of two.  Infinities and NaNs would come out finite, so the users add nonfinite_mark() of the values.
+constexpr double WIDEN_HALF = 0x1p448;  // WIDEN_HALF^2 * WIDEN_SCALE = 1
+__device__ __forceinline__ double widen(float x) {
+  const int i = __float_as_int(x);
+  return __hiloint2double((i >> 3) & 0x8fffffff, i << 29);
+}
+__device__ __forceinline__ double2 widen(float2 a) { return make_double2(widen(a.x), widen(a.y)); }
+__device__ __forceinline__ double2 widen(double2 a) { return a; }
+// accumulates zero for finite values and NaN otherwise
+__device__ __forceinline__ void nonfinite_mark(float& t, float2 a) { t = fmaf(a.x, 0.0f, fmaf(a.y, 0.0f, t)); }
+__device__ __forceinline__ void nonfinite_mark(float&, double2) {}
+// the mark as a double: 0 or NaN (the hardware's NaN result is 0x7fffffff, whose bits are a double's NaN too)
+__device__ __forceinline__ double mark_d(float t) { return __hiloint2double(__float_as_int(t), 0); }
+
 }  // namespace fm

@@ -593,19 +593,13 @@ static fm_status engine_step_t(fm_engine* E) {
       FM_TRY(green_op<R>(P, S, U, PRO_V_SCALE, (const double*)E->scale.p, EPI_PREC_OP, U, nullptr, ep, U, act,
                          (int)run.size(), &rcx));
       // classical Gram-Schmidt (optionally twice) against each slot's own basis, FP64 coefficients
-      const int nblk_d = kv_blocks(P, k_multidot<R, false>, S);
-      const int nblk_u = kv_blocks(P, k_update<R, true>, S);
       const int passes = E->ortho == FM_ORTHO_CGS2 ? 2 : 1;
       std::vector<double2> htot((size_t)S * kmax, make_double2(0, 0)), hr((size_t)S * kmax);
       FM_CK(cudaMemcpyAsync(P->scale.p, E->sch.data(), (size_t)(kmax + 1) * S * sizeof(double), cudaMemcpyHostToDevice,
                             P->st));
       for (int pass = 0; pass < passes; ++pass) {
-        const double fbA = (double)run.size() * M * sizeof(T);
-        FM_TRACK(P, KC_DOT, (kmax + 1) * fbA,
-                 (k_multidot<R, false><<<dim3(nblk_d, S), KV_THREADS, 0, P->st>>>(
-                     P->M, S, kmax, U, nullptr, (double2*)P->red_part.p, (double2*)P->red_out.p,
-                     (unsigned*)P->red_cnt.p, act, (const T* const*)(dt + S), (const int*)E->kb.p)));
-        FM_CK(cudaGetLastError());
+        FM_CK((gs_dot<R>(P, S, kmax, U, nullptr, false, act, (int)run.size(), (const void* const*)(dt + S),
+                         (const int*)E->kb.p)));
         FM_CK(cudaMemcpyAsync(hr.data(), P->red_out.p, hr.size() * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
         FM_CK(cudaStreamSynchronize(P->st));
         for (int s : run)
@@ -616,11 +610,7 @@ static fm_status engine_step_t(fm_engine* E) {
           }
         FM_CK(cudaMemcpyAsync(P->coef.p, hr.data(), hr.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
         Coef cf{(const double2*)P->coef.p, kmax, (const double*)P->scale.p, S, -1.0, 0};
-        FM_TRACK(P, KC_UPD, (kmax + 2) * fbA,
-                 (k_update<R, true><<<dim3(nblk_u, S), KV_THREADS, 0, P->st>>>(
-                     P->M, S, kmax, U, cf, nullptr, nullptr, (double2*)P->red_part.p, (double2*)P->red_out.p,
-                     (unsigned*)P->red_cnt.p, act, (T* const*)(dt + S), (const int*)E->kb.p)));
-        FM_CK(cudaGetLastError());
+        FM_CK((gs_update<R>(P, S, kmax, U, cf, nullptr, true, act, (int)run.size(), dt + S, (const int*)E->kb.p)));
       }
       std::vector<double2> nn(S);
       FM_CK(cudaMemcpyAsync(nn.data(), P->red_out.p, S * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
@@ -726,11 +716,7 @@ static fm_status engine_step_t(fm_engine* E) {
       FM_CK(cudaMemcpyAsync(P->scale.p, E->sch.data(), (size_t)(kmax + 1) * S * sizeof(double), cudaMemcpyHostToDevice,
                             P->st));
       Coef cf{(const double2*)P->coef.p, KV_KMAX + 1, (const double*)P->scale.p, S, 1.0, 1};
-      FM_TRACK(P, KC_UPD, (double)(kmax + 2) * upd.size() * M * sizeof(T),
-               (k_update<R, false><<<dim3(kv_blocks(P, k_update<R, false>, S), S), KV_THREADS, 0, P->st>>>(
-                   P->M, S, kmax, U, cf, (T*)E->X.p, nullptr, nullptr, nullptr, nullptr, act, nullptr,
-                   (const int*)E->kb.p)));
-      FM_CK(cudaGetLastError());
+      FM_CK((gs_update<R>(P, S, kmax, U, cf, E->X.p, false, act, (int)upd.size(), nullptr, (const int*)E->kb.p)));
     }
     for (int s : upd)
       if (E->slots[s].state == SL_RESTART) E->slots[s].state = SL_RESIDUAL;

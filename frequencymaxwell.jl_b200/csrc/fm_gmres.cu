@@ -8,24 +8,35 @@
 // Krylov helpers
 // ---------------------------------------------------------------------------
 template <typename R>
+cudaError_t gs_dot(fm_plan* P, int nb, int K, const void* U, const void* w, bool wnorm, const int* act, int nact,
+                   const void* const* wtab, const int* Kb) {
+  using T = cplx<R>;
+  auto kern = wnorm ? k_gsdot<R, true, false> : k_gsdot<R, false, false>;
+  FM_TRACK(P, KC_DOT, (double)(K + 1) * nact * P->M * sizeof(T),
+           (kern<<<dim3(gs_blocks<R>(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
+               P->M, nb, K, (const T*)U, (const T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
+               (unsigned*)P->red_cnt.p, act, (const T* const*)wtab, Kb, MgsTail{})));
+  return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t gs_update(fm_plan* P, int nb, int K, const void* U, const Coef& cf, void* w, bool norm, const int* act,
+                      int nact, void* const* wtab, const int* Kb) {
+  using T = cplx<R>;
+  auto kern = norm ? k_gsupdate<R, true> : k_gsupdate<R, false>;
+  FM_TRACK(P, KC_UPD, (double)(K + 2) * nact * P->M * sizeof(T),
+           (kern<<<dim3(gs_blocks<R>(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
+               P->M, nb, K, (const T*)U, cf, (T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
+               (unsigned*)P->red_cnt.p, act, (T* const*)wtab, Kb)));
+  return cudaGetLastError();
+}
+
+template <typename R>
 fm_status multidot(fm_plan* P, int nb, int K, const void* U, const void* w, bool wnorm, const int* act,
                    std::vector<double2>& host_out, int nact) {
   FM_TRY(ensure_reduce(P, nb, K));
   if (nact < 0) nact = nb;
-  const int nblk = wnorm ? kv_blocks(P, k_multidot<R, true>, nb) : kv_blocks(P, k_multidot<R, false>, nb);
-  dim3 g(nblk, nb);
-  const double bytes = (double)(K + 1) * nact * P->M * sizeof(cplx<R>);
-  if (wnorm)
-    FM_TRACK(P, KC_DOT, bytes,
-             (k_multidot<R, true><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, K, (const cplx<R>*)U, (const cplx<R>*)w,
-                                                               (double2*)P->red_part.p, (double2*)P->red_out.p,
-                                                               (unsigned*)P->red_cnt.p, act)));
-  else
-    FM_TRACK(P, KC_DOT, bytes,
-             (k_multidot<R, false><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, K, (const cplx<R>*)U, (const cplx<R>*)w,
-                                                                (double2*)P->red_part.p, (double2*)P->red_out.p,
-                                                                (unsigned*)P->red_cnt.p, act)));
-  FM_CK(cudaGetLastError());
+  FM_CK((gs_dot<R>(P, nb, K, U, w, wnorm, act, nact)));
   const int KK = K + (wnorm ? 1 : 0);
   host_out.resize((size_t)nb * KK);
   FM_CK(cudaMemcpyAsync(host_out.data(), P->red_out.p, host_out.size() * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
@@ -122,7 +133,10 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
   if (mem + 1 > KV_KMAX) return fail(FM_ERR_UNSUPPORTED, "Krylov basis larger than 127 vectors");
   FM_CK(P->basis.ensure((size_t)(mem + 1) * fbytes));
   FM_CK(P->scale.ensure((size_t)(KV_KMAX + 1) * nb * sizeof(double)));
-  FM_CK(P->hbuf.ensure((size_t)nb * (KV_KMAX + 2) * sizeof(double2)));
+  if (o.ortho == FM_ORTHO_MGS) {
+    FM_CK(P->hbuf.ensure((size_t)nb * (KV_KMAX + 2) * sizeof(double2)));
+    FM_CK(P->mgsT.ensure((size_t)nb * KV_KMAX * KV_KMAX * sizeof(double2)));
+  }
   FM_CK(P->active.ensure((size_t)nb * sizeof(int)));
   FM_TRY(ensure_reduce(P, nb, mem + 1));
   T* U = (T*)P->basis.p;
@@ -195,22 +209,26 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
       const int K = j + 1;
       std::vector<double2> hcol((size_t)nb * (K + 1));
       if (o.ortho == FM_ORTHO_MGS) {
+        // one sweep for the coefficients (k_gsdot's MGS tail leaves them on the device), one for the subtraction:
+        // two reads of the basis per iteration, where projecting vector by vector reads it twice and w K times
         double2* hd = (double2*)P->hbuf.p;
         const int hs = KV_KMAX + 2;
-        dim3 g(kv_blocks(P, k_mgs<R>, nb), nb);
-        for (int i = 0; i <= K; ++i) {
-          const double mb = fbA * ((i > 0 ? 1 : 0) + (i < K ? 1 : 0) + 1 + (i > 0 ? 1 : 0));
-          FM_TRACK(P, KC_MGS, mb,
-                   (k_mgs<R><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, i, K, U, sc, nb, Uw, hd, hs,
-                                                          (double2*)P->red_part.p, (unsigned*)P->red_cnt.p, act)));
-        }
+        auto kern = k_gsdot<R, false, true>;
+        FM_TRACK(P, KC_DOT, (K + 1) * fbA,
+                 (kern<<<dim3(gs_blocks<R>(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
+                     P->M, nb, K, U, Uw, (double2*)P->red_part.p, nullptr, (unsigned*)P->red_cnt.p, act, nullptr,
+                     nullptr, MgsTail{(double2*)P->mgsT.p, sc, nb, hd, hs})));
         FM_CK(cudaGetLastError());
-        std::vector<double2> hh((size_t)nb * hs);
+        FM_CK((gs_update<R>(P, nb, K, U, Coef{hd, hs, sc, nb, -1.0, 1}, Uw, true, act, nact)));
+        std::vector<double2> hh((size_t)nb * hs), nn(nb);
         FM_CK(cudaMemcpyAsync(hh.data(), hd, hh.size() * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
+        FM_CK(cudaMemcpyAsync(nn.data(), P->red_out.p, nb * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
         FM_CK(cudaStreamSynchronize(P->st));
         tk_resolve(P);
-        for (int b = 0; b < nb; ++b)
-          for (int i = 0; i <= K; ++i) hcol[(size_t)b * (K + 1) + i] = hh[(size_t)b * hs + i];
+        for (int b = 0; b < nb; ++b) {
+          for (int i = 0; i < K; ++i) hcol[(size_t)b * (K + 1) + i] = hh[(size_t)b * hs + i];
+          hcol[(size_t)b * (K + 1) + K] = nn[b];
+        }
       } else {
         // classical Gram-Schmidt (optionally twice), FP64 coefficients
         std::vector<double2> hr;
@@ -228,18 +246,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
           FM_CK(P->coef.ensure((size_t)nb * K * sizeof(double2)));
           FM_CK(cudaMemcpyAsync(P->coef.p, hr.data(), hr.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
           Coef cf{(const double2*)P->coef.p, K, sc, nb, -1.0, 0};
-          const double ub = (K + 2) * fbA;
-          dim3 g(last ? kv_blocks(P, k_update<R, true>, nb) : kv_blocks(P, k_update<R, false>, nb), nb);
-          if (last)
-            FM_TRACK(P, KC_UPD, ub,
-                     (k_update<R, true><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, K, U, cf, Uw, nullptr,
-                                                                     (double2*)P->red_part.p, (double2*)P->red_out.p,
-                                                                     (unsigned*)P->red_cnt.p, act)));
-          else
-            FM_TRACK(P, KC_UPD, ub,
-                     (k_update<R, false><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, K, U, cf, Uw, nullptr, nullptr, nullptr,
-                                                                      nullptr, act)));
-          FM_CK(cudaGetLastError());
+          FM_CK((gs_update<R>(P, nb, K, U, cf, Uw, last, act, nact)));
           if (!last) {
             FM_TRY(multidot<R>(P, nb, K, U, Uw, false, act, hr, nact));
             for (int b = 0; b < nb; ++b)
@@ -334,11 +341,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
       FM_CK(cudaMemcpyAsync(P->coef.p, yh.data(), yh.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
       FM_CK(cudaMemcpyAsync(sc, sch.data(), (size_t)(KV_KMAX + 1) * nb * sizeof(double), cudaMemcpyHostToDevice, P->st));
       Coef cf{(const double2*)P->coef.p, KV_KMAX + 1, sc, nb, 1.0, 1};
-      dim3 g(kv_blocks(P, k_update<R, false>, nb), nb);
-      FM_TRACK(P, KC_UPD, (double)(Kmax + 2) * nb * fe * sizeof(T),
-               (k_update<R, false><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, Kmax, U, cf, (T*)P->xbuf.p, nullptr, nullptr,
-                                                                nullptr, nullptr, nullptr)));
-      FM_CK(cudaGetLastError());
+      FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, nullptr, nb)));
     }
     any = false;
     for (int b = 0; b < nb; ++b) {
@@ -590,11 +593,7 @@ static fm_status gmres_block(fm_plan* P, int nb, const fm_solve_opts& o, std::ve
       if (acth[b]) blk_cgs_coefs(St[b], m, hr.data() + (size_t)b * K, cf.data() + (size_t)b * K);
     FM_CK(cudaMemcpyAsync(P->coef.p, cf.data(), cf.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
     Coef c{(const double2*)P->coef.p, K, nullptr, nb, -1.0, 0};
-    dim3 g(kv_blocks(P, k_update<R, true>, nb), nb);
-    FM_TRACK(P, KC_UPD, (double)(K + 2) * nact * fe * sizeof(T),
-             (k_update<R, true><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, K, U, c, Uw, nullptr, (double2*)P->red_part.p,
-                                                             (double2*)P->red_out.p, (unsigned*)P->red_cnt.p, act)));
-    FM_CK(cudaGetLastError());
+    FM_CK((gs_update<R>(P, nb, K, U, c, Uw, true, act, nact)));
     std::vector<double2> nn(nb);
     FM_CK(cudaMemcpyAsync(nn.data(), P->red_out.p, nb * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
     FM_CK(cudaStreamSynchronize(P->st));
@@ -689,11 +688,7 @@ static fm_status gmres_block(fm_plan* P, int nb, const fm_solve_opts& o, std::ve
   if (Kmax > 0) {
     FM_CK(cudaMemcpyAsync(P->coef.p, yh.data(), yh.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
     Coef cf{(const double2*)P->coef.p, KV_KMAX, nullptr, nb, 1.0, 1};
-    dim3 g(kv_blocks(P, k_update<R, false>, nb), nb);
-    FM_TRACK(P, KC_UPD, (double)(Kmax + 2) * nb * fe * sizeof(T),
-             (k_update<R, false><<<g, KV_THREADS, 0, P->st>>>(P->M, nb, Kmax, U, cf, (T*)P->xbuf.p, nullptr, nullptr,
-                                                              nullptr, nullptr, nullptr)));
-    FM_CK(cudaGetLastError());
+    FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, nullptr, nb)));
   }
   for (int b = 0; b < nb; ++b) {
     info[b].iterations = St[b].iters;
@@ -895,6 +890,14 @@ fm_status solve_core(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<fm_
   return check_device_error(P);
 }
 
+template cudaError_t gs_dot<float>(fm_plan*, int, int, const void*, const void*, bool, const int*, int,
+                                   const void* const*, const int*);
+template cudaError_t gs_dot<double>(fm_plan*, int, int, const void*, const void*, bool, const int*, int,
+                                    const void* const*, const int*);
+template cudaError_t gs_update<float>(fm_plan*, int, int, const void*, const Coef&, void*, bool, const int*, int,
+                                      void* const*, const int*);
+template cudaError_t gs_update<double>(fm_plan*, int, int, const void*, const Coef&, void*, bool, const int*, int,
+                                       void* const*, const int*);
 template fm_status multidot<float>(fm_plan*, int, int, const void*, const void*, bool, const int*,
                                    std::vector<double2>&, int);
 template fm_status multidot<double>(fm_plan*, int, int, const void*, const void*, bool, const int*,

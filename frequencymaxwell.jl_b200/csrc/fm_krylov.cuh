@@ -50,65 +50,264 @@ __device__ __forceinline__ void finish_reduce(double2* part, double2* out, unsig
   if (threadIdx.x == 0) counter[b] = 0;
 }
 
+// The same tail for one real value per block (part[b*nblk + blk].x): the first warp sums the partials.
+__device__ __forceinline__ void finish_norm(double2* part, double2* out, unsigned* counter, int nblk, int b) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&counter[b], 1u) == (unsigned)(nblk - 1);
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  __threadfence();
+  double2 s = make_double2(0.0, 0.0);
+  for (int k = threadIdx.x; k < nblk; k += 32) s.x += __ldcg(&part[(size_t)b * nblk + k]).x;
+  s = warp_sum(s);
+  if (threadIdx.x == 0) {
+    out[b] = s;
+    counter[b] = 0;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Gram-Schmidt passes against a stored basis: k_gsdot (inner products) and k_gsupdate (combination).
+//
+// Both stream the basis once from HBM and do little with each value, so bytes in flight decide.  A warp owns one
+// contiguous range of elements and takes GS_GROUP basis vectors at a time, GsCfg::EPT elements a lane from each (192
+// or 256 bytes in flight per thread, no prefetch registers, two CTAs of 8 warps an SM).  k_gsupdate walks its ranges
+// backwards, so its first reads are the elements that k_gsdot read last and L2 still holds.
+//
+// Measured on 50 basis vectors of one 128^3 right-hand side (3 x 128^3 values): FP64 6.6 (dot) and 6.5 TB/s (update);
+// FP32 6.2 and 6.2 TB/s with widen(), 4.2 and 4.8 TB/s at best with the conversion instruction.  Smaller groups, fewer
+// elements a lane, or three CTAs an SM with spills were 5-30 % slower in FP32 (EPT 4: 5.6, 8: 5.9, 6 in pairs: 5.6).
+// ---------------------------------------------------------------------------
+constexpr int GS_GROUP = 4;
+template <typename R> struct GsCfg {
+  static constexpr bool F32 = sizeof(R) == 4;  // basis values go through widen() (fm_complex.cuh)
+  static constexpr int EPT = F32 ? 6 : 4;
+  static constexpr int STEP = 32 * EPT;  // elements of one warp step
+};
+
+// element range [lo, hi) of this warp (multiples of 4, so FP32 ranges start on 32-byte sectors)
+__device__ __forceinline__ void gs_range(long long M, int nblk, long long& lo, long long& hi) {
+  const long long nw = (long long)nblk * KV_WARPS;
+  const long long per = ((M + nw - 1) / nw + 3) / 4 * 4;
+  lo = ((long long)blockIdx.x * KV_WARPS + (threadIdx.x >> 5)) * per;
+  hi = min(M, lo + per);
+}
+
+// Sums NV values over the warp with NV + 1 or fewer exchanges instead of 5 NV: each halving step sends half of
+// the values to the partner and keeps the sums of the other half.  The sum of value (lane / (32 / NV)) comes back.
+template <int NV>
+__device__ __forceinline__ double warp_transpose_sum(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int n = NV; n > 1; n >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < n / 2; ++q) {
+      const double send = up ? v[q] : v[q + n / 2];
+      const double keep = up ? v[q + n / 2] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  double s = v[0];
+  for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// Modified Gram-Schmidt of the newest vector from one sweep of inner products.  MGS applies
+// (I - v_j v_j^H) ... (I - v_0 v_0^H) to w; its coefficients h solve (I + L) h = V^H w with the strictly lower
+// triangular L_ik = <v_i, v_k> (A. Bjorck, "Numerics of Gram-Schmidt orthogonalization", 1994, section 3; used for
+// GMRES by K. Swirydowicz, J. Langou, S. Ananthan, U. Yang, S. Thomas, "Low synchronization Gram-Schmidt and
+// generalized minimal residual algorithms", 2020).  So h = T V^H w with T = (I + L)^{-1}, which grows by one row
+// per step.  The sweep that reads the basis for V^H w also forms <v_k, v_j>, the new row of L.
+struct MgsTail {
+  double2* T;         // [b][KV_KMAX][KV_KMAX], row-major, unit lower triangular
+  const double* sc;   // v_i = sc[i*ss + b] * U_i
+  int ss;
+  double2* h;         // out: h[b*hs + i], i < K
+  int hs;
+};
+
 // out[b][i] = sum_e conj(U_i[b][e]) * w[b][e]   (i < K), plus out[b][K] = ||w||^2 when WNORM.
 // Optional per-RHS arguments: wtab[b] replaces w + b*M, Kb[b] (<= K) the number of basis vectors.
-template <typename R, bool WNORM>
-__global__ void __launch_bounds__(KV_THREADS) k_multidot(long long M, int B, int K, const cplx<R>* __restrict__ U,
-                                                         const cplx<R>* __restrict__ w, double2* __restrict__ part,
-                                                         double2* __restrict__ out, unsigned* __restrict__ counter,
-                                                         const int* __restrict__ active,
-                                                         const cplx<R>* const* __restrict__ wtab = nullptr,
-                                                         const int* __restrict__ Kb = nullptr) {
+// MGS: U_{K-1} is the newest basis vector; mt.h gets the modified Gram-Schmidt coefficients of w against
+// v_0 .. v_{K-1} and row K-1 of mt.T is formed (no `out`).
+// Bound by HBM (MGS in FP64 6.4 TB/s at the size above; in FP32 4.9, where twice the sums per value bind it).
+// Against one launch per basis vector (three field accesses each, 3.8 TB/s), the MGS form and k_gsupdate took one
+// FP64 solve of 100 iterations on 128^3 from 574 to 220 ms, and on 64^3 from 154 to 38 ms.
+template <typename R, bool WNORM, bool MGS>
+__global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int K, const cplx<R>* __restrict__ U,
+                                                      const cplx<R>* __restrict__ w, double2* __restrict__ part,
+                                                      double2* __restrict__ out, unsigned* __restrict__ counter,
+                                                      const int* __restrict__ active,
+                                                      const cplx<R>* const* __restrict__ wtab,
+                                                      const int* __restrict__ Kb, MgsTail mt) {
   using T = cplx<R>;
-  __shared__ double2 acc[KV_WARPS][KV_KMAX + 1];
+  constexpr int EPT = GsCfg<R>::EPT, G = GS_GROUP, NV = MGS ? 2 : 1;  // NV right-hand vectors: w (and U_{K-1})
+  constexpr bool F32 = GsCfg<R>::F32;
+  constexpr int NQ = G * NV * 2;
+  static_assert(!(WNORM && MGS), "the norm belongs to the plain dot");
+  __shared__ double acc[KV_WARPS][(KV_KMAX + G) * NV * 2];
+  __shared__ double nacc[KV_WARPS];
+  __shared__ bool last;
   const int b = blockIdx.y, nblk = gridDim.x;
-  const int KK = K + (WNORM ? 1 : 0);
   if (active && !active[b]) return;  // uniform per block; no reduction is issued for inactive RHS
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  for (int i = lane; i < KK; i += 32) acc[wi][i] = make_double2(0.0, 0.0);
+  for (int i = lane; i < (K + G - 1) / G * NQ; i += 32) acc[wi][i] = 0.0;
   __syncwarp();
-  const long long chunk = (long long)KV_THREADS * KV_EPT;
-  const long long per = ((M + nblk - 1) / nblk + chunk - 1) / chunk * chunk;
-  const long long lo = (long long)blockIdx.x * per, hi = min(M, lo + per);
+  long long lo, hi;
+  gs_range(M, nblk, lo, hi);
   const T* wb = wtab ? wtab[b] : w + (size_t)b * M;
   const int Kr = Kb ? Kb[b] : K;
-  for (long long c0 = lo; c0 < hi; c0 += chunk) {
-    double2 wv[KV_EPT];
+  const size_t us = (size_t)B * M;
+  const T* ub = U + (size_t)b * M;
+  double nrm = 0.0;
+  for (long long c0 = lo; c0 < hi; c0 += GsCfg<R>::STEP) {
+    double2 wv[NV][EPT];
+    bool in[EPT];
 #pragma unroll
-    for (int k = 0; k < KV_EPT; ++k) {
-      long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
-      wv[k] = e < hi ? to_d(wb[e]) : make_double2(0.0, 0.0);
-    }
-    for (int i = 0; i < Kr; ++i) {
-      const T* ub = U + ((size_t)i * B + b) * M;
-      double2 s = make_double2(0.0, 0.0);
+    for (int k = 0; k < EPT; ++k) {
+      const long long e = c0 + 32 * k + lane;
+      in[k] = e < hi;
+      wv[0][k] = in[k] ? to_d(wb[e]) : make_double2(0.0, 0.0);
+      if constexpr (MGS) wv[1][k] = in[k] ? to_d(ub[(size_t)(K - 1) * us + e]) : make_double2(0.0, 0.0);
+      if constexpr (WNORM) nrm = fma(wv[0][k].x, wv[0][k].x, fma(wv[0][k].y, wv[0][k].y, nrm));
+      if constexpr (F32) {
 #pragma unroll
-      for (int k = 0; k < KV_EPT; ++k) {
-        long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
-        if (e < hi) {
-          double2 u = to_d(ub[e]);
-          s.x = fma(u.x, wv[k].x, fma(u.y, wv[k].y, s.x));
-          s.y = fma(u.x, wv[k].y, fma(-u.y, wv[k].x, s.y));
-        }
+        for (int v = 0; v < NV; ++v) wv[v][k] = cscale(wv[v][k], WIDEN_HALF);
       }
-      s = warp_sum(s);
-      if (lane == 0) { acc[wi][i].x += s.x; acc[wi][i].y += s.y; }
     }
-    if constexpr (WNORM) {
-      double2 s = make_double2(0.0, 0.0);
+    for (int i0 = 0; i0 < Kr; i0 += G) {
+      T u[G][EPT];
 #pragma unroll
-      for (int k = 0; k < KV_EPT; ++k) s.x = fma(wv[k].x, wv[k].x, fma(wv[k].y, wv[k].y, s.x));
-      s = warp_sum(s);
-      if (lane == 0) acc[wi][K].x += s.x;
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int k = 0; k < EPT; ++k) {
+          u[g][k].x = 0;
+          u[g][k].y = 0;
+          if (i0 + g < Kr && in[k]) u[g][k] = ub[(size_t)(i0 + g) * us + c0 + 32 * k + lane];
+        }
+      double s[NQ];
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          double sx = 0.0, sy = 0.0;
+          if constexpr (F32) {
+            float bad = 0.0f;
+#pragma unroll
+            for (int k = 0; k < EPT; ++k) nonfinite_mark(bad, u[g][k]);
+            sx = mark_d(bad);
+          }
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            const double2 x = widen(u[g][k]);
+            sx = fma(x.x, wv[v][k].x, fma(x.y, wv[v][k].y, sx));
+            sy = fma(x.x, wv[v][k].y, fma(-x.y, wv[v][k].x, sy));
+          }
+          s[(g * NV + v) * 2] = sx;
+          s[(g * NV + v) * 2 + 1] = sy;
+        }
+      const double t = warp_transpose_sum<NQ>(s);
+      constexpr int LPV = 32 / NQ;  // lanes per value
+      if ((lane & (LPV - 1)) == 0) acc[wi][i0 * NV * 2 + lane / LPV] += t;
     }
+  }
+  if constexpr (WNORM) {
+    const double2 s = warp_sum(make_double2(nrm, 0.0));
+    if (lane == 0) nacc[wi] = s.x;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < KK; i += blockDim.x) {
+  // partial sums of the block, block index fastest so that the last block's warps read them coalesced
+  const int NO = K * NV + (WNORM ? 1 : 0);
+  for (int o = threadIdx.x; o < NO; o += blockDim.x) {
     double2 s = make_double2(0.0, 0.0);
-    for (int q = 0; q < KV_WARPS; ++q) { s.x += acc[q][i].x; s.y += acc[q][i].y; }
-    part[((size_t)b * nblk + blockIdx.x) * KK + i] = s;
+    for (int q = 0; q < KV_WARPS; ++q) {
+      if (WNORM && o == K) {
+        s.x += nacc[q];
+      } else {
+        s.x += acc[q][2 * o];
+        s.y += acc[q][2 * o + 1];
+      }
+    }
+    if (F32 && !(WNORM && o == K)) s = cscale(s, WIDEN_HALF);
+    part[((size_t)b * NO + o) * nblk + blockIdx.x] = s;
   }
-  finish_reduce(part, out, counter, KK, nblk, b);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&counter[b], 1u) == (unsigned)(nblk - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // grid sums: a warp per value (fixed order, so the result does not depend on the schedule)
+  double2* rs = reinterpret_cast<double2*>(&acc[0][0]);
+  for (int o = wi; o < NO; o += KV_WARPS) {
+    double2 s = make_double2(0.0, 0.0);
+    for (int k = lane; k < nblk; k += 32) {
+      const double2 v = __ldcg(&part[((size_t)b * NO + o) * nblk + k]);
+      s.x += v.x;
+      s.y += v.y;
+    }
+    s = warp_sum(s);
+    if (lane == 0) {
+      if constexpr (MGS) rs[o] = s;
+      else out[(size_t)b * NO + o] = s;
+    }
+  }
+  if (threadIdx.x == 0) counter[b] = 0;
+  if constexpr (MGS) {
+    // rs[2m] = <U_m, w>, rs[2m+1] = <U_m, U_j>, j = K - 1.  L_jm = <v_j, v_m>;  T_j = e_j - L_j T;  h = T V^H w.
+    __shared__ double2 r[KV_KMAX], trow[2][KV_KMAX];
+    __syncthreads();
+    const int j = K - 1;
+    double2* Tb = mt.T + (size_t)b * KV_KMAX * KV_KMAX;
+    const double scj = mt.sc[(size_t)j * mt.ss + b];
+    double2 lj = make_double2(0.0, 0.0);
+    if (threadIdx.x < K) {
+      const double sm = mt.sc[(size_t)threadIdx.x * mt.ss + b];
+      const double2 a = rs[2 * threadIdx.x], c = rs[2 * threadIdx.x + 1];
+      r[threadIdx.x] = make_double2(a.x * sm, a.y * sm);
+      lj = make_double2(c.x * sm * scj, -c.y * sm * scj);  // conj(<v_m, v_j>)
+    }
+    __syncthreads();  // rs is read: its storage takes L_j
+    if (threadIdx.x < K) rs[threadIdx.x] = lj;
+    __syncthreads();
+    {
+      static_assert(KV_THREADS == 2 * KV_KMAX, "two threads per column of T");
+      const int k = threadIdx.x & (KV_KMAX - 1), half = threadIdx.x / KV_KMAX;
+      double2 s = make_double2(0.0, 0.0);
+      if (k < j) {
+#pragma unroll 4
+        for (int m = k + half; m < j; m += 2) {
+          const double2 l = rs[m], t = __ldcg(&Tb[(size_t)m * KV_KMAX + k]);
+          s.x = fma(-l.x, t.x, fma(l.y, t.y, s.x));
+          s.y = fma(-l.x, t.y, fma(-l.y, t.x, s.y));
+        }
+      }
+      trow[half][k] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < K) {
+      double2 t = make_double2(trow[0][threadIdx.x].x + trow[1][threadIdx.x].x,
+                               trow[0][threadIdx.x].y + trow[1][threadIdx.x].y);
+      if (threadIdx.x == j) t = make_double2(1.0, 0.0);
+      trow[0][threadIdx.x] = t;
+      Tb[(size_t)j * KV_KMAX + threadIdx.x] = t;
+    }
+    __syncthreads();
+    for (int i = wi; i < K; i += KV_WARPS) {
+      double2 s = make_double2(0.0, 0.0);
+      for (int k = lane; k <= i; k += 32) {
+        const double2 t = i == j ? trow[0][k] : __ldcg(&Tb[(size_t)i * KV_KMAX + k]);
+        s.x = fma(t.x, r[k].x, fma(-t.y, r[k].y, s.x));
+        s.y = fma(t.x, r[k].y, fma(t.y, r[k].x, s.y));
+      }
+      s = warp_sum(s);
+      if (lane == 0) mt.h[(size_t)b * mt.hs + i] = s;
+    }
+  }
 }
 
 // Coefficient source for the update kernels.  For RHS b and vector i the
@@ -133,59 +332,80 @@ struct Coef {
   }
 };
 
-// w[b] = a0[b]*w[b] + sum_i coef(b,i) * U_i[b]   (FP64 accumulation); optional ||w'||^2.
-// a0 scale (real) is taken from w_scale[b] when given, else 1.
+// w[b] += sum_i coef(b,i) * U_i[b]   (FP64 accumulation); optional out[b] = ||w'||^2 (of the stored values).
+// Optional per-RHS arguments as in k_gsdot.
 template <typename R, bool NORM>
-__global__ void __launch_bounds__(KV_THREADS) k_update(long long M, int B, int K, const cplx<R>* __restrict__ U,
-                                                       Coef cf, cplx<R>* __restrict__ w, const double* __restrict__ w_scale,
-                                                       double2* __restrict__ part, double2* __restrict__ out,
-                                                       unsigned* __restrict__ counter, const int* __restrict__ active,
-                                                       cplx<R>* const* __restrict__ wtab = nullptr,
-                                                       const int* __restrict__ Kb = nullptr) {
+__global__ void __launch_bounds__(KV_THREADS, 2) k_gsupdate(long long M, int B, int K, const cplx<R>* __restrict__ U,
+                                                         Coef cf, cplx<R>* __restrict__ w,
+                                                         double2* __restrict__ part, double2* __restrict__ out,
+                                                         unsigned* __restrict__ counter, const int* __restrict__ active,
+                                                         cplx<R>* const* __restrict__ wtab,
+                                                         const int* __restrict__ Kb) {
   using T = cplx<R>;
-  __shared__ double2 cs[KV_KMAX];
+  constexpr int EPT = GsCfg<R>::EPT, G = GS_GROUP, STEP = GsCfg<R>::STEP;
+  constexpr bool F32 = GsCfg<R>::F32;
+  __shared__ double2 cs[KV_KMAX + G];
   __shared__ double red[KV_WARPS];
   const int b = blockIdx.y, nblk = gridDim.x;
   if (active && !active[b]) return;
   const int Kr = Kb ? Kb[b] : K;
-  for (int i = threadIdx.x; i < Kr; i += blockDim.x) cs[i] = cf.get(b, i);
+  for (int i = threadIdx.x; i < Kr; i += blockDim.x) cs[i] = F32 ? cscale(cf.get(b, i), WIDEN_HALF) : cf.get(b, i);
   __syncthreads();
-  const double a0 = w_scale ? w_scale[b] : 1.0;
-  const long long chunk = (long long)KV_THREADS * KV_EPT;
-  const long long per = ((M + nblk - 1) / nblk + chunk - 1) / chunk * chunk;
-  const long long lo = (long long)blockIdx.x * per, hi = min(M, lo + per);
+  const int lane = threadIdx.x & 31;
+  long long lo, hi;
+  gs_range(M, nblk, lo, hi);
+  const size_t us = (size_t)B * M;
+  const T* ub = U + (size_t)b * M;
   T* wb = wtab ? wtab[b] : w + (size_t)b * M;
   double nrm = 0.0;
-  for (long long c0 = lo; c0 < hi; c0 += chunk) {
-    double2 acc[KV_EPT];
+  if (lo < hi) {
+    for (long long c0 = lo + (hi - lo - 1) / STEP * STEP; c0 >= lo; c0 -= STEP) {
+      double2 acc[EPT];
+      bool in[EPT];
 #pragma unroll
-    for (int k = 0; k < KV_EPT; ++k) {
-      long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
-      double2 v = e < hi ? to_d(wb[e]) : make_double2(0.0, 0.0);
-      acc[k] = make_double2(v.x * a0, v.y * a0);
-    }
-    for (int i = 0; i < Kr; ++i) {
-      const T* ub = U + ((size_t)i * B + b) * M;
-      const double2 c = cs[i];
+      for (int k = 0; k < EPT; ++k) {
+        const long long e = c0 + 32 * k + lane;
+        in[k] = e < hi;
+        acc[k] = in[k] ? to_d(wb[e]) : make_double2(0.0, 0.0);
+        if constexpr (F32) acc[k] = cscale(acc[k], 1.0 / WIDEN_HALF);
+      }
+      float bad[EPT];
 #pragma unroll
-      for (int k = 0; k < KV_EPT; ++k) {
-        long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
-        if (e < hi) {
-          double2 u = to_d(ub[e]);
-          acc[k].x = fma(c.x, u.x, fma(-c.y, u.y, acc[k].x));
-          acc[k].y = fma(c.x, u.y, fma(c.y, u.x, acc[k].y));
+      for (int k = 0; k < EPT; ++k) bad[k] = 0.0f;
+      for (int i0 = 0; i0 < Kr; i0 += G) {
+        T u[G][EPT];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            u[g][k].x = 0;
+            u[g][k].y = 0;
+            if (i0 + g < Kr && in[k]) u[g][k] = ub[(size_t)(i0 + g) * us + c0 + 32 * k + lane];
+          }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          if (i0 + g >= Kr) break;  // uniform
+          const double2 c = cs[i0 + g];
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            nonfinite_mark(bad[k], u[g][k]);
+            const double2 x = widen(u[g][k]);
+            acc[k].x = fma(c.x, x.x, fma(-c.y, x.y, acc[k].x));
+            acc[k].y = fma(c.x, x.y, fma(c.y, x.x, acc[k].y));
+          }
         }
       }
-    }
 #pragma unroll
-    for (int k = 0; k < KV_EPT; ++k) {
-      long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
-      if (e < hi) {
-        T r = from_d<T>(acc[k]);
-        wb[e] = r;
-        if constexpr (NORM) {
-          double2 rd = to_d(r);
-          nrm = fma(rd.x, rd.x, fma(rd.y, rd.y, nrm));
+      for (int k = 0; k < EPT; ++k) {
+        if (in[k]) {
+          if constexpr (F32) acc[k] = make_double2(fma(acc[k].x, WIDEN_HALF, mark_d(bad[k])),
+                                                   fma(acc[k].y, WIDEN_HALF, mark_d(bad[k])));
+          const T r = from_d<T>(acc[k]);
+          wb[c0 + 32 * k + lane] = r;
+          if constexpr (NORM) {
+            const double2 rd = to_d(r);
+            nrm = fma(rd.x, rd.x, fma(rd.y, rd.y, nrm));
+          }
         }
       }
     }
@@ -199,88 +419,7 @@ __global__ void __launch_bounds__(KV_THREADS) k_update(long long M, int B, int K
       for (int q = 0; q < KV_WARPS; ++q) t += red[q];
       part[(size_t)b * nblk + blockIdx.x] = make_double2(t, 0.0);
     }
-    finish_reduce(part, out, counter, 1, nblk, b);
-  }
-}
-
-// One step of modified Gram-Schmidt as Krylov.jl runs it (sc[i*ss + b] scales U_i):
-//   if i > 0:  w -= h_{i-1} * v_{i-1}        (h read from device, v = sc*U)
-//   if i < K:  h_i = <v_i, w>                (reduced into hout[b*hs + i])
-//   else:      hout[b*hs + K] = ||w||^2
-template <typename R>
-__global__ void __launch_bounds__(KV_THREADS) k_mgs(long long M, int B, int i, int K, const cplx<R>* __restrict__ U,
-                                                    const double* __restrict__ sc, int ss, cplx<R>* __restrict__ w,
-                                                    double2* __restrict__ hout, int hs, double2* __restrict__ part,
-                                                    unsigned* __restrict__ counter, const int* __restrict__ active) {
-  using T = cplx<R>;
-  __shared__ double2 red[KV_WARPS];
-  const int b = blockIdx.y, nblk = gridDim.x;
-  if (active && !active[b]) return;
-  const long long chunk = (long long)KV_THREADS * KV_EPT;
-  const long long per = ((M + nblk - 1) / nblk + chunk - 1) / chunk * chunk;
-  const long long lo = (long long)blockIdx.x * per, hi = min(M, lo + per);
-  T* wb = w + (size_t)b * M;
-  double2 cprev = make_double2(0.0, 0.0);
-  const T* up = nullptr;
-  if (i > 0) {
-    double2 h = hout[(size_t)b * hs + (i - 1)];
-    double s = sc ? sc[(size_t)(i - 1) * ss + b] : 1.0;
-    cprev = make_double2(-h.x * s, -h.y * s);
-    up = U + ((size_t)(i - 1) * B + b) * M;
-  }
-  const T* ui = (i < K) ? U + ((size_t)i * B + b) * M : nullptr;
-  const double si = (i < K && sc) ? sc[(size_t)i * ss + b] : 1.0;
-  double2 acc = make_double2(0.0, 0.0);
-  for (long long c0 = lo; c0 < hi; c0 += chunk) {
-#pragma unroll
-    for (int k = 0; k < KV_EPT; ++k) {
-      long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
-      if (e < hi) {
-        double2 wv = to_d(wb[e]);
-        if (up) {
-          double2 u = to_d(up[e]);
-          wv.x = fma(cprev.x, u.x, fma(-cprev.y, u.y, wv.x));
-          wv.y = fma(cprev.x, u.y, fma(cprev.y, u.x, wv.y));
-          T r = from_d<T>(wv);
-          wb[e] = r;
-          wv = to_d(r);
-        }
-        if (ui) {
-          double2 u = to_d(ui[e]);
-          acc.x = fma(u.x, wv.x, fma(u.y, wv.y, acc.x));
-          acc.y = fma(u.x, wv.y, fma(-u.y, wv.x, acc.y));
-        } else {
-          acc.x = fma(wv.x, wv.x, fma(wv.y, wv.y, acc.x));
-        }
-      }
-    }
-  }
-  acc = warp_sum(acc);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double2 t = make_double2(0.0, 0.0);
-    for (int q = 0; q < KV_WARPS; ++q) { t.x += red[q].x; t.y += red[q].y; }
-    if (ui) { t.x *= si; t.y *= si; }
-    part[(size_t)b * nblk + blockIdx.x] = t;
-  }
-  // reduce into hout[b*hs + i]
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(&counter[b], 1u) == (unsigned)(nblk - 1));
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  if (threadIdx.x == 0) {
-    double2 s = make_double2(0.0, 0.0);
-    for (int k = 0; k < nblk; ++k) {
-      double2 v = __ldcg(&part[(size_t)b * nblk + k]);
-      s.x += v.x;
-      s.y += v.y;
-    }
-    hout[(size_t)b * hs + i] = s;
-    counter[b] = 0;
+    finish_norm(part, out, counter, nblk, b);
   }
 }
 
@@ -793,7 +932,7 @@ __global__ void __launch_bounds__(KV_THREADS) k_axpby3(long long M, const cplx<R
       for (int q = 0; q < KV_WARPS; ++q) t += red[q];
       part[(size_t)b * nblk + blockIdx.x] = make_double2(t, 0.0);
     }
-    finish_reduce(part, out, counter, 1, nblk, b);
+    finish_norm(part, out, counter, nblk, b);
   }
 }
 

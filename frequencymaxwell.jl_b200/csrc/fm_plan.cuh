@@ -104,7 +104,7 @@ struct fm_plan {
   DevBuf V;
   // workspace
   DevBuf t1, t2, t3, bbuf, xbuf, ebuf, sbuf, basis, gbuf2;  // t3: first branch of a two-branch average
-  DevBuf red_part, red_out, red_cnt, active, scale, coef, hbuf, shifts, yblk, V64;
+  DevBuf red_part, red_out, red_cnt, active, scale, coef, hbuf, mgsT, shifts, yblk, V64;
   DevBuf eps_dev, fx, fy, fz, maxpart, maxout;
   bool eps_phantom = false;  // eps_dev holds the permittivity fm_phantom_fill painted (fm_build_potential eps = NULL)
   DevBuf shapes;             // fm_phantom_fill's shape table
@@ -332,16 +332,25 @@ static int kv_blocks(const fm_plan* P, Kern kern, int nb) {
   const long long maxb = (P->M + chunk - 1) / chunk;
   return (int)std::max(1LL, std::min<long long>(maxb, cap / nb));
 }
+// The same for the Gram-Schmidt passes, whose smallest share is one warp step per warp.
+template <typename R, typename Kern>
+static int gs_blocks(const fm_plan* P, Kern kern, int nb) {
+  int bps = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, KV_THREADS, 0) != cudaSuccess || bps < 1) bps = 1;
+  const long long cap = (long long)P->sms * std::min(bps, 8);
+  const long long maxb = (P->M + KV_WARPS * GsCfg<R>::STEP - 1) / (KV_WARPS * GsCfg<R>::STEP);
+  return (int)std::max(1LL, std::min<long long>(maxb, cap / nb));
+}
 inline int red_blocks_max(const fm_plan* P, int nb) {
-  // upper bound of kv_blocks over all kernels (at most 8 blocks of 256 threads per SM)
-  const long long chunk = (long long)KV_THREADS * KV_EPT;
+  // upper bound of kv_blocks and gs_blocks over all kernels (at most 8 blocks of 256 threads per SM)
+  const long long chunk = KV_WARPS * GsCfg<double>::STEP;
   const long long maxb = (P->M + chunk - 1) / chunk;
   return (int)std::max(1LL, std::min<long long>(maxb, (long long)P->sms * 8 / nb));
 }
 
 inline fm_status ensure_reduce(fm_plan* P, int nb, int K) {
   const int nblk = red_blocks_max(P, nb);
-  FM_CK(P->red_part.ensure((size_t)nb * nblk * (KV_KMAX + 2) * sizeof(double2)));
+  FM_CK(P->red_part.ensure((size_t)nb * nblk * (2 * KV_KMAX + 2) * sizeof(double2)));  // two dots per vector (MGS)
   FM_CK(P->red_out.ensure((size_t)nb * (KV_KMAX + 2) * sizeof(double2)));
   if (P->red_cnt.cap < (size_t)nb * sizeof(unsigned)) {
     FM_CK(P->red_cnt.ensure((size_t)nb * sizeof(unsigned)));
@@ -382,6 +391,14 @@ template <typename R>
 fm_status curl_batch(fm_plan* P, int nb, const void* in, void* out, const int* act);
 
 // ---- Krylov drivers (fm_gmres.cu) ----
+// Launches of the Gram-Schmidt passes (fm_krylov.cuh) on the plan's stream, results in P->red_out: `out` of
+// k_gsdot, and the norms of k_gsupdate when norm is set.  nact: right-hand sides that are active (accounting).
+template <typename R>
+cudaError_t gs_dot(fm_plan* P, int nb, int K, const void* U, const void* w, bool wnorm, const int* act, int nact,
+                   const void* const* wtab = nullptr, const int* Kb = nullptr);
+template <typename R>
+cudaError_t gs_update(fm_plan* P, int nb, int K, const void* U, const Coef& cf, void* w, bool norm, const int* act,
+                      int nact, void* const* wtab = nullptr, const int* Kb = nullptr);
 template <typename R>
 fm_status multidot(fm_plan* P, int nb, int K, const void* U, const void* w, bool wnorm, const int* act,
                    std::vector<double2>& host_out, int nact = -1);
