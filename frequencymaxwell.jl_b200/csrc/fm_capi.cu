@@ -80,7 +80,7 @@ static fm_status plan_wave_size(fm_plan* P, int nrhs, const fm_solve_opts& o, in
   // basis + b + x + s + e + t1 + t2 + fp64 staging and outputs
   // (the output term also covers the second output slot of host-output solves: 2 * 3g * 16 <= 2 * M * 16)
   // (+ t3 when the Green average runs as two branches: absorbing x or y)
-  const size_t two_branch = (P->avg && !P->zonly && !P->zsplit) ? 1 : 0;  // (the general passes use t1 and t3)
+  const size_t two_branch = (P->avg && !P->zonly && !P->zsplit) ? 1 : 0;
   const size_t per = fb * (size_t)(vecs + 6 + two_branch) + (size_t)P->M * sizeof(double2) * 5 + extra;
   const size_t held = P->basis.cap + P->bbuf.cap + P->xbuf.cap + P->sbuf.cap + P->ebuf.cap + P->t1.cap + P->t2.cap +
                       P->t3.cap +
@@ -134,29 +134,18 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   if (desc->device < 0 || desc->device >= nd) return fail(FM_ERR_INVALID, "device ordinal out of range");
   const int n3[3] = {desc->grid[0] + 2 * desc->pad[0], desc->grid[1] + 2 * desc->pad[1], desc->grid[2] + 2 * desc->pad[2]};
   bool avg = desc->absorbing[0] || desc->absorbing[1] || desc->absorbing[2];
-  bool zonly = desc->absorbing[2] && !desc->absorbing[0] && !desc->absorbing[1];
+  const bool zonly = desc->absorbing[2] && !desc->absorbing[0] && !desc->absorbing[1];
   const int prec = desc->precision == FM_PREC_F64 ? FM_PREC_F64 : FM_PREC_F32;  // storage
   const bool c64 = desc->precision != FM_PREC_F32;                                   // arithmetic
-  // The fused passes take axes of 96 or powers of two in [8, 512] (an averaged z axis a power of two) that
-  // tile the warps; every other grid runs the general passes (fm_generic.cuh).
-  bool generic = false;
+  // Fused passes take an axis of 96 or a power of two in [8, 512]; any other length up to 256 runs Bluestein passes
+  // on that axis (fm_generic.cuh).
   for (int a = 0; a < 3; ++a)
-    if (!axis_supported(n3[a])) generic = true;
-  if (zonly && (n3[2] > AXIS_MAX || (n3[2] & (n3[2] - 1)))) generic = true;
-  // padded z above 256: the two shifted branches run as two z passes (the second adds to the first)
-  bool zsplit = zonly && n3[2] > AXIS_MAX_AVG2;
-  if (!generic) {
-    const int pwy = c64 ? pencils_per_warp<double>(n3[1]) : pencils_per_warp<float>(n3[1]);
-    const int lz = (zonly && !zsplit) ? 2 * n3[2] : n3[2];
-    const int pwz = c64 ? pencils_per_warp<double>(lz) : pencils_per_warp<float>(lz);
-    if (pwy <= 0 || pwz <= 0 || n3[0] % pwy || n3[0] % pwz) generic = true;
-  }
-  if (generic) {
-    for (int a = 0; a < 3; ++a)
-      if (!gen_axis_supported(n3[a]))
-        return fail(FM_ERR_UNSUPPORTED, "padded axis sizes must be at most 256, or powers of two up to 512");
-    zonly = zsplit = false;
-  }
+    if (!axis_supported(n3[a]) && !blue_axis_supported(n3[a]))
+      return fail(FM_ERR_UNSUPPORTED, "padded axis sizes must be at most 256, or powers of two up to 512");
+  // shifts on z only: both branches in one length-2L z pass where the length has one, else two z passes (the second
+  // adds to the first)
+  const bool avg2 = axis_supported(n3[2]) && n3[2] <= AXIS_MAX_AVG2 && (n3[2] & (n3[2] - 1)) == 0;
+  const bool zsplit = zonly && !avg2;
   if (cudaSetDevice(desc->device) != cudaSuccess) return fail(FM_ERR_CUDA, "cudaSetDevice failed");
   fm_plan* P = new fm_plan();
   P->desc = *desc;
@@ -171,7 +160,6 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   P->avg = avg;
   P->zonly = zonly && !zsplit;
   P->zsplit = zsplit;
-  P->generic = generic;
   for (int a = 0; a < 3; ++a) P->shift[a] = desc->absorbing[a] ? 0.25 : 0.0;
   {
     cudaDeviceProp prop;

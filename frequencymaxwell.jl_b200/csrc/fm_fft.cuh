@@ -76,10 +76,9 @@ __device__ __forceinline__ T tw16(T a) {
   }
 }
 
+// second half of the radix-8 butterfly: twiddles and radix-2 combinations of the even and odd radix-4 results
 template <int DIR, typename T>
-__device__ __forceinline__ void bf8(T* v) {
-  bf4<DIR>(v[0], v[2], v[4], v[6]);
-  bf4<DIR>(v[1], v[3], v[5], v[7]);
+__device__ __forceinline__ void bf8_tail(T* v) {
   T o1 = tw16<DIR, 2>(v[3]), o2 = tw16<DIR, 4>(v[5]), o3 = tw16<DIR, 6>(v[7]);
   T e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
   v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
@@ -89,10 +88,15 @@ __device__ __forceinline__ void bf8(T* v) {
 }
 
 template <int DIR, typename T>
-__device__ __forceinline__ void bf16(T* v) {
-  // n = 4*n1 + n2 ; k = k1 + 4*k2
-#pragma unroll
-  for (int n2 = 0; n2 < 4; ++n2) bf4<DIR>(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
+__device__ __forceinline__ void bf8(T* v) {
+  bf4<DIR>(v[0], v[2], v[4], v[6]);
+  bf4<DIR>(v[1], v[3], v[5], v[7]);
+  bf8_tail<DIR>(v);
+}
+
+// second half of the radix-16 butterfly (n = 4*n1 + n2, k = k1 + 4*k2)
+template <int DIR, typename T>
+__device__ __forceinline__ void bf16_tail(T* v) {
   // v[n2 + 4*k1] *= w16^(n2*k1)
   v[5] = tw16<DIR, 1>(v[5]);  v[9] = tw16<DIR, 2>(v[9]);   v[13] = tw16<DIR, 3>(v[13]);
   v[6] = tw16<DIR, 2>(v[6]);  v[10] = tw16<DIR, 4>(v[10]); v[14] = tw16<DIR, 6>(v[14]);
@@ -109,6 +113,13 @@ __device__ __forceinline__ void bf16(T* v) {
     for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = t[4 * k1 + k2];
 }
 
+template <int DIR, typename T>
+__device__ __forceinline__ void bf16(T* v) {
+#pragma unroll
+  for (int n2 = 0; n2 < 4; ++n2) bf4<DIR>(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
+  bf16_tail<DIR>(v);
+}
+
 template <int DIR, int RAD, typename T>
 __device__ __forceinline__ void bfly(T* v) {
   if constexpr (RAD == 2) bf2<DIR>(v[0], v[1]);
@@ -117,6 +128,34 @@ __device__ __forceinline__ void bfly(T* v) {
   else if constexpr (RAD == 8) bf8<DIR>(v);
   else if constexpr (RAD == 16) bf16<DIR>(v);
   else static_assert(RAD == 2, "unsupported radix");
+}
+
+// The same butterflies when the upper half of the inputs is zero (the first stage of a zero-padded transform):
+// the additions with zeros are left out, the results are the same.
+template <int DIR, typename T>
+__device__ __forceinline__ void bf4_lo(T& v0, T& v1, T& v2, T& v3) {
+  const T a = v0, b = v1, ib = cmul_i<DIR>(v1);
+  v0 = cadd(a, b);
+  v2 = csub(a, b);
+  v1 = cadd(a, ib);
+  v3 = csub(a, ib);
+}
+template <int DIR, int RAD, typename T>
+__device__ __forceinline__ void bfly_lo(T* v) {
+  if constexpr (RAD == 2) {
+    v[1] = v[0];
+  } else if constexpr (RAD == 4) {
+    bf4_lo<DIR>(v[0], v[1], v[2], v[3]);
+  } else if constexpr (RAD == 8) {
+    bf4_lo<DIR>(v[0], v[2], v[4], v[6]);
+    bf4_lo<DIR>(v[1], v[3], v[5], v[7]);
+    bf8_tail<DIR>(v);
+  } else {
+    static_assert(RAD == 16, "unsupported radix");
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) bf4_lo<DIR>(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
+    bf16_tail<DIR>(v);
+  }
 }
 
 // ---- shared-memory exchange: one padding slot every 128 bytes of data ----
@@ -132,7 +171,8 @@ __device__ __forceinline__ int sm_phys(int i) {
 // prior product NS, entry (NS - 1) + (q - 1)*NS + k holds exp(-2*pi*i*k*q/(NS*RAD)),
 // k in [0, NS), q in [1, RAD).  Consecutive lanes (consecutive k) read consecutive
 // entries, and the stages together need exactly L - 1 entries.
-template <int DIR, int L, int E, int RAD, int NS, bool LAST, typename T>
+// LO: the upper half of the pencil is zero (first stage only).
+template <int DIR, int L, int E, int RAD, int NS, bool LAST, bool LO = false, typename T>
 __device__ __forceinline__ void fft_stage(T (&v)[E], T* sm, const T* tw, int t) {
   constexpr int TP = L / E;
   constexpr int NB = E / RAD;
@@ -149,7 +189,8 @@ __device__ __forceinline__ void fft_stage(T (&v)[E], T* sm, const T* tw, int t) 
         v[m * RAD + q] = cmul(v[m * RAD + q], w);
       }
     }
-    bfly<DIR, RAD>(&v[m * RAD]);
+    if constexpr (LO) bfly_lo<DIR, RAD>(&v[m * RAD]);
+    else bfly<DIR, RAD>(&v[m * RAD]);
     if constexpr (!LAST) {
       const int base = (j / NS) * NS * RAD + k;
 #pragma unroll
@@ -168,19 +209,19 @@ __device__ __forceinline__ void fft_gather(T (&v)[E], const T* sm, int t) {
 }
 
 // Full FFT of one pencil with the radix sequence (R0, R1, R2) (zeros = unused).
-template <int DIR, int L, int E, int R0, int R1, int R2, typename T>
+template <int DIR, int L, int E, int R0, int R1, int R2, bool LO = false, typename T>
 __device__ __forceinline__ void fft_run(T (&v)[E], T* sm, const T* tw, int t) {
   static_assert(R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) == L, "radices must multiply to L");
   if constexpr (R1 == 0) {
-    fft_stage<DIR, L, E, R0, 1, true>(v, sm, tw, t);
+    fft_stage<DIR, L, E, R0, 1, true, LO>(v, sm, tw, t);
   } else if constexpr (R2 == 0) {
-    fft_stage<DIR, L, E, R0, 1, false>(v, sm, tw, t);
+    fft_stage<DIR, L, E, R0, 1, false, LO>(v, sm, tw, t);
     __syncwarp();
     fft_gather<L, E, R1>(v, sm, t);
     __syncwarp();
     fft_stage<DIR, L, E, R1, R0, true>(v, sm, tw, t);
   } else {
-    fft_stage<DIR, L, E, R0, 1, false>(v, sm, tw, t);
+    fft_stage<DIR, L, E, R0, 1, false, LO>(v, sm, tw, t);
     __syncwarp();
     fft_gather<L, E, R1>(v, sm, t);
     __syncwarp();
@@ -196,7 +237,7 @@ __device__ __forceinline__ void fft_run(T (&v)[E], T* sm, const T* tw, int t) {
 // Pencil c exchanges through its own buffer sm + c*SMS, so between two __syncwarp the loads and butterflies of
 // all NC pencils are independent and one pencil's exchange latency overlaps the others' arithmetic.  The stage
 // twiddles are loaded once, before any store of the stage, and shared by the NC pencils.
-template <int DIR, int L, int E, int RAD, int NS, bool LAST, int NC, int SMS, typename T>
+template <int DIR, int L, int E, int RAD, int NS, bool LAST, int NC, int SMS, bool LO = false, typename T>
 __device__ __forceinline__ void fft_stage_n(T (&v)[NC][E], T* sm, const T* tw, int t) {
   constexpr int TP = L / E;
   constexpr int NB = E / RAD;
@@ -222,7 +263,8 @@ __device__ __forceinline__ void fft_stage_n(T (&v)[NC][E], T* sm, const T* tw, i
 #pragma unroll
         for (int q = 1; q < RAD; ++q) v[c][m * RAD + q] = cmul(v[c][m * RAD + q], w[m][q - 1]);
       }
-      bfly<DIR, RAD>(&v[c][m * RAD]);
+      if constexpr (LO) bfly_lo<DIR, RAD>(&v[c][m * RAD]);
+      else bfly<DIR, RAD>(&v[c][m * RAD]);
       if constexpr (!LAST) {
         const int base = (j / NS) * NS * RAD + k;
 #pragma unroll
@@ -238,19 +280,19 @@ __device__ __forceinline__ void fft_gather_n(T (&v)[NC][E], const T* sm, int t) 
   for (int c = 0; c < NC; ++c) fft_gather<L, E, RAD>(v[c], sm + c * SMS, t);
 }
 
-template <int DIR, int L, int E, int R0, int R1, int R2, int NC, int SMS, typename T>
+template <int DIR, int L, int E, int R0, int R1, int R2, int NC, int SMS, bool LO = false, typename T>
 __device__ __forceinline__ void fft_run_n(T (&v)[NC][E], T* sm, const T* tw, int t) {
   static_assert(R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) == L, "radices must multiply to L");
   if constexpr (R1 == 0) {
-    fft_stage_n<DIR, L, E, R0, 1, true, NC, SMS>(v, sm, tw, t);
+    fft_stage_n<DIR, L, E, R0, 1, true, NC, SMS, LO>(v, sm, tw, t);
   } else if constexpr (R2 == 0) {
-    fft_stage_n<DIR, L, E, R0, 1, false, NC, SMS>(v, sm, tw, t);
+    fft_stage_n<DIR, L, E, R0, 1, false, NC, SMS, LO>(v, sm, tw, t);
     __syncwarp();
     fft_gather_n<L, E, R1, NC, SMS>(v, sm, t);
     __syncwarp();
     fft_stage_n<DIR, L, E, R1, R0, true, NC, SMS>(v, sm, tw, t);
   } else {
-    fft_stage_n<DIR, L, E, R0, 1, false, NC, SMS>(v, sm, tw, t);
+    fft_stage_n<DIR, L, E, R0, 1, false, NC, SMS, LO>(v, sm, tw, t);
     __syncwarp();
     fft_gather_n<L, E, R1, NC, SMS>(v, sm, t);
     __syncwarp();
@@ -291,9 +333,10 @@ FM_PLAN(96, double, 24, 8, 4, 3)
 #undef FM_PLAN
 
 // forward-order run (radices R0, R1, R2) with its stage-twiddle table
-template <int DIR, typename P, typename T>
+// (LO: the elements at and above L/2 are zero and are not read from v)
+template <int DIR, typename P, bool LO = false, typename T>
 __device__ __forceinline__ void fft_fwd_plan(T (&v)[P::E], T* sm, const T* tw_fwd, int t) {
-  fft_run<DIR, P::L, P::E, P::R0, P::R1, P::R2>(v, sm, tw_fwd, t);
+  fft_run<DIR, P::L, P::E, P::R0, P::R1, P::R2, LO>(v, sm, tw_fwd, t);
 }
 // reversed-order run (consumes the RL-layout, returns the R0-layout) with its own table
 template <int DIR, typename P, typename T>
@@ -304,9 +347,9 @@ __device__ __forceinline__ void fft_rev_plan(T (&v)[P::E], T* sm, const T* tw_re
 }
 
 // NC pencils at once (exchange buffers SMS elements apart)
-template <int DIR, typename P, int NC, int SMS, typename T>
+template <int DIR, typename P, int NC, int SMS, bool LO = false, typename T>
 __device__ __forceinline__ void fft_fwd_plan_n(T (&v)[NC][P::E], T* sm, const T* tw_fwd, int t) {
-  fft_run_n<DIR, P::L, P::E, P::R0, P::R1, P::R2, NC, SMS>(v, sm, tw_fwd, t);
+  fft_run_n<DIR, P::L, P::E, P::R0, P::R1, P::R2, NC, SMS, LO>(v, sm, tw_fwd, t);
 }
 template <int DIR, typename P, int NC, int SMS, typename T>
 __device__ __forceinline__ void fft_rev_plan_n(T (&v)[NC][P::E], T* sm, const T* tw_rev, int t) {

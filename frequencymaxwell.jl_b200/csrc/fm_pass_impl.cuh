@@ -24,7 +24,7 @@ static cudaError_t xf_L(const Dims& d, const void* in, const void* V, const doub
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
   const long long rows = (long long)d.ny * d.nz * d.nb;
-  const long long warps = rows / PW;
+  const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(L + W * PW * PencilStride<L, T, P_::TP, true>::v) * sizeof(T);
   allow_smem(k_xf<S, R, L, PRO>, smem);
@@ -43,7 +43,7 @@ static cudaError_t xi_L(const Dims& d, const void* in, const void* V, const void
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
   const long long rows = (long long)d.ny * d.nz * d.nb;
-  const long long warps = rows / PW;
+  const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(L + W * PW * PencilStride<L, T, P_::TP, true>::v) * sizeof(T);
   allow_smem(k_xi<S, R, L, EPI>, smem);
@@ -61,7 +61,7 @@ static cudaError_t xi_xf_L(const Dims& d, const void* in, const void* V, const v
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
   const long long rows = (long long)d.ny * d.nz * d.nb;
-  const long long warps = rows / PW;
+  const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(2 * L + W * PW * PencilStride<L, T, P_::TP, true>::v) * sizeof(T);
   allow_smem(k_xi_xf<S, R, L>, smem);
@@ -78,7 +78,7 @@ static cudaError_t y_L(const Dims& d, const void* in, const void* tw, const void
   using P_ = Plan<L, R>;
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
-  const long long warps = (long long)(d.nx / PW) * d.nz * 3 * d.nb;
+  const long long warps = (long long)((d.nx + PW - 1) / PW) * d.nz * 3 * d.nb;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   // one pencil per warp and FP32 storage: four x-consecutive pencils per CTA, staged for coalesced rows
   if constexpr (PW == 1 && std::is_same<S, float>::value) {
@@ -106,7 +106,7 @@ static cudaError_t zg_L(const Dims& d, const void* in, const GreenParams& gp, co
   constexpr int LF = (MODE == ZMODE_AVG2) ? 2 * L : L;
   using P_ = Plan<LF, R>;
   constexpr int PW = 32 / P_::TP, W = ZG_THREADS / 32;
-  const long long warps = (long long)(d.nx / PW) * d.ny * d.nb;
+  const long long warps = (long long)((d.nx + PW - 1) / PW) * d.ny * d.nb;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(2 * LF + L + W * PW * PencilStride<LF, T, P_::TP, false>::v) * sizeof(T);
   // one pencil per warp and FP32 storage: stage the CTA's column block for coalesced loads and stores

@@ -137,10 +137,10 @@ __global__ void __launch_bounds__(256) k_y(Dims d, const cplx<S>* __restrict__ i
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane % PW, t = lane / PW;
   const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + wic;
-  const int xg = d.nx / PW;
+  const int xg = (d.nx + PW - 1) / PW;
   const long long total = (long long)xg * d.nz * 3 * d.nb;
   if (gw >= total) return;
-  const int x = (int)(gw % xg) * PW + p;
+  const int xl = (int)(gw % xg) * PW + p, x = min(xl, d.nx - 1);  // a ragged last group repeats the last column
   const long long zcb = gw / xg;  // z + nz*(c + 3b)
   const int b = (int)(zcb / (3LL * d.nz));
   if (active && !active[b]) return;
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(256) k_y(Dims d, const cplx<S>* __restrict__ i
   };
   auto st = [&](int y, T a) {
     if constexpr (STG) tile[tix(y, wic)] = cv<TS>(a);
-    else out[base + (long long)y * d.nx] = cv<TS>(a);
+    else if (xl < d.nx) out[base + (long long)y * d.nx] = cv<TS>(a);
   };
   T v[E];
   if constexpr (DIR < 0) {
@@ -233,6 +233,55 @@ __device__ __forceinline__ R kidx_curl(int i, int n) {
   return (R)(i < (n >> 1) ? i : i - n);
 }
 
+// The per-bin 3x3 operators between the forward and inverse z transforms, on the components (e1, e2, e3) at k.
+template <typename R>
+struct GreenBin {
+  using T = cplx<R>;
+  R ksr, ksi;
+  T sc, iks;  // folded normalisation; 1/k_square
+  __device__ __forceinline__ GreenBin(const GreenParams& gp, int b) {
+    ksr = (R)gp.ksq_re;
+    ksi = gp.ksq_im_b ? (R)gp.ksq_im_b[b] : (R)gp.ksq_im;
+    sc = mk((R)gp.scale_re, (R)gp.scale_im);
+    const R kden = ksr * ksr + ksi * ksi;
+    iks = mk(ksr / kden, -ksi / kden);
+  }
+  // (E - k (k.E)/k_square) / (|k|^2 - k_square)
+  __device__ __forceinline__ void green(T& e1, T& e2, T& e3, R kx, R ky, R kz) const {
+    const T kE = cmul(cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz)), iks);
+    const R dr = kx * kx + ky * ky + kz * kz - ksr, di = -ksi;
+    const R dd = dr * dr + di * di;
+    const R rdd = R(1) / dd;  // one division for both parts of 1 / (k^2 - ks)
+    const T f = cmul(sc, mk(dr * rdd, -di * rdd));
+    e1 = cmul(csub(e1, cscale(kE, kx)), f);
+    e2 = cmul(csub(e2, cscale(kE, ky)), f);
+    e3 = cmul(csub(e3, cscale(kE, kz)), f);
+  }
+  // i k x E
+  __device__ __forceinline__ void curl(T& e1, T& e2, T& e3, R kx, R ky, R kz) const {
+    const T isc = cmul_i<1>(sc);
+    const T c1 = csub(cscale(e3, ky), cscale(e2, kz));
+    const T c2 = csub(cscale(e1, kz), cscale(e3, kx));
+    const T c3 = csub(cscale(e2, kx), cscale(e1, ky));
+    e1 = cmul(c1, isc);
+    e2 = cmul(c2, isc);
+    e3 = cmul(c3, isc);
+  }
+};
+
+// wave number of z bin m (MODE_AVG2: bin 2k is the +s spectrum at k, bin 2k - 1 the -s spectrum)
+template <int MODE, int L, typename R>
+__device__ __forceinline__ R z_wavenumber(const GreenParams& gp, int m) {
+  if constexpr (MODE == ZMODE_AVG2) {
+    if ((m & 1) == 0) return (R)gp.dk[2] * (kidx_green<R>(m >> 1, L) + (R)gp.shift[2]);
+    return (R)gp.dk[2] * (kidx_green<R>(((m + 1) >> 1) % L, L) - (R)gp.shift[2]);
+  } else if constexpr (MODE == ZMODE_ONE) {
+    return (R)gp.dk[2] * (kidx_green<R>(m, L) + (R)gp.shift[2]);
+  } else {
+    return (R)gp.dk[2] * kidx_curl<R>(m, L);
+  }
+}
+
 constexpr int ZG_WARPS = 4;  // warps per CTA of the register z pass
 
 // STG (one pencil per warp only): the CTA's warps take x-consecutive pencils at the same (y, b), and the CTA stages
@@ -260,10 +309,10 @@ __global__ void __launch_bounds__(256) k_zg(Dims d, const cplx<S>* __restrict__ 
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane % PW, t = lane / PW;
   const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + wic;
-  const int xg = d.nx / PW;
+  const int xg = (d.nx + PW - 1) / PW;
   const long long total = (long long)xg * d.ny * d.nb;
   if (gw >= total) return;
-  const int x = (int)(gw % xg) * PW + p;
+  const int xl = (int)(gw % xg) * PW + p, x = min(xl, d.nx - 1);  // a ragged last group repeats the last column
   const long long yb = gw / xg;
   const int y = (int)(yb % d.ny);
   const int b = (int)(yb / d.ny);
@@ -300,60 +349,27 @@ __global__ void __launch_bounds__(256) k_zg(Dims d, const cplx<S>* __restrict__ 
       }
       v[c][e] = a;
     }
-    fft_fwd_plan<-1, P_>(v[c], sm, tw, t);
+    fft_fwd_plan<-1, P_, MODE == ZMODE_AVG2>(v[c], sm, tw, t);
     __syncwarp();
   }
 
   // per-bin 3x3 operator
   {
-    int kxi = x, kyi = y;
+    const GreenBin<R> gb(gp, b);
     R kx, ky;
     if (MODE == ZMODE_CURL) {
-      kx = (R)gp.dk[0] * kidx_curl<R>(kxi, d.nx);
-      ky = (R)gp.dk[1] * kidx_curl<R>(kyi, d.ny);
+      kx = (R)gp.dk[0] * kidx_curl<R>(x, d.nx);
+      ky = (R)gp.dk[1] * kidx_curl<R>(y, d.ny);
     } else {
-      kx = (R)gp.dk[0] * (kidx_green<R>(kxi, d.nx) + (R)gp.shift[0]);
-      ky = (R)gp.dk[1] * (kidx_green<R>(kyi, d.ny) + (R)gp.shift[1]);
+      kx = (R)gp.dk[0] * (kidx_green<R>(x, d.nx) + (R)gp.shift[0]);
+      ky = (R)gp.dk[1] * (kidx_green<R>(y, d.ny) + (R)gp.shift[1]);
     }
-    const R ksr = (R)gp.ksq_re, ksi = gp.ksq_im_b ? (R)gp.ksq_im_b[b] : (R)gp.ksq_im;
-    const T sc = mk((R)gp.scale_re, (R)gp.scale_im);
-    // 1/k_square
-    const R kden = ksr * ksr + ksi * ksi;
-    const T iks = mk(ksr / kden, -ksi / kden);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int m = lay_idx<LF, E, P_::RL>(t, e);
-      R kz;
-      if constexpr (MODE == ZMODE_AVG2) {
-        if ((m & 1) == 0) kz = (R)gp.dk[2] * (kidx_green<R>(m >> 1, L) + (R)gp.shift[2]);
-        else kz = (R)gp.dk[2] * (kidx_green<R>(((m + 1) >> 1) % L, L) - (R)gp.shift[2]);
-      } else if constexpr (MODE == ZMODE_ONE) {
-        kz = (R)gp.dk[2] * (kidx_green<R>(m, L) + (R)gp.shift[2]);
-      } else {
-        kz = (R)gp.dk[2] * kidx_curl<R>(m, L);
-      }
-      T e1 = v[0][e], e2 = v[1][e], e3 = v[2][e];
-      if constexpr (MODE == ZMODE_CURL) {
-        // (ik x E) * sc
-        T c1 = csub(cscale(e3, ky), cscale(e2, kz));
-        T c2 = csub(cscale(e1, kz), cscale(e3, kx));
-        T c3 = csub(cscale(e2, kx), cscale(e1, ky));
-        const T isc = cmul_i<1>(sc);
-        v[0][e] = cmul(c1, isc);
-        v[1][e] = cmul(c2, isc);
-        v[2][e] = cmul(c3, isc);
-      } else {
-        T kE = cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz));
-        kE = cmul(kE, iks);
-        const R k2 = kx * kx + ky * ky + kz * kz;
-        const R dr = k2 - ksr, di = -ksi;
-        const R dd = dr * dr + di * di;
-        const R rdd = R(1) / dd;  // one division for both parts of 1 / (k^2 - ks)
-        const T f = cmul(sc, mk(dr * rdd, -di * rdd));
-        v[0][e] = cmul(csub(e1, cscale(kE, kx)), f);
-        v[1][e] = cmul(csub(e2, cscale(kE, ky)), f);
-        v[2][e] = cmul(csub(e3, cscale(kE, kz)), f);
-      }
+      const R kz = z_wavenumber<MODE, L, R>(gp, m);
+      if constexpr (MODE == ZMODE_CURL) gb.curl(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+      else gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
     }
   }
 
@@ -369,7 +385,7 @@ __global__ void __launch_bounds__(256) k_zg(Dims d, const cplx<S>* __restrict__ 
         if (MODE != ZMODE_CURL && rz) a = cmul(a, cconj(rtab[z]));
         if constexpr (STG) {
           tile[tix(c * L + z, wic)] = cv<TS>(a);
-        } else {
+        } else if (xl < d.nx) {
           const long long o = base0 + (long long)c * d.n + (long long)z * plane;
           if (gp.accumulate) a = cadd(a, cv<T>(out[o]));
           out[o] = cv<TS>(a);

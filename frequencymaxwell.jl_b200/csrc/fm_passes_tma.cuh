@@ -232,8 +232,6 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
   const int p = lane / TP, t = lane % TP;
   constexpr int NCX = C::NCX, SMS = C::STRIDE;
   T* sm = ex + (warp * PW + p) * NCX * SMS;
-  const R ksr = (R)gp.ksq_re;
-  const T sc = mk((R)gp.scale_re, (R)gp.scale_im);
   int it = 0;
   bool ok = true;
   for (long long tile = next_active(blockIdx.x, ntiles, per_rhs, active); tile < ntiles;
@@ -245,9 +243,7 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
     const uint32_t ph = (it / NST) & 1;
     if (!mbar_wait(full + s, ph, err, 23)) { ok = false; break; }
     unsigned char* tl = tiles + s * C::TILE;
-    const R ksi = gp.ksq_im_b ? (R)gp.ksq_im_b[b] : (R)gp.ksq_im;
-    const R kden = ksr * ksr + ksi * ksi;
-    const T iks = mk(ksr / kden, -ksi / kden);
+    const GreenBin<R> gb(gp, b);
 #pragma unroll 1
     for (int rd = 0; rd < C::ROUNDS; ++rd) {
       const int xl = rd * CW * PW + warp * PW + p;
@@ -266,12 +262,12 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
           v[c][e] = a;
         }
         if constexpr (NCX == 1) {
-          fft_fwd_plan<-1, P_>(v[c], sm, tw, t);
+          fft_fwd_plan<-1, P_, MODE == ZMODE_AVG2>(v[c], sm, tw, t);
           __syncwarp();
         }
       }
       if constexpr (NCX == 3) {
-        fft_fwd_plan_n<-1, P_, 3, SMS>(v, sm, tw, t);
+        fft_fwd_plan_n<-1, P_, 3, SMS, MODE == ZMODE_AVG2>(v, sm, tw, t);
         __syncwarp();
       }
       R kx, ky;
@@ -284,33 +280,9 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
       }
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const int m = lay_idx<LF, E, P_::RL>(t, e);
-        R kz;
-        if constexpr (MODE == ZMODE_AVG2) {
-          if ((m & 1) == 0) kz = (R)gp.dk[2] * (kidx_green<R>(m >> 1, L) + (R)gp.shift[2]);
-          else kz = (R)gp.dk[2] * (kidx_green<R>(((m + 1) >> 1) % L, L) - (R)gp.shift[2]);
-        } else if constexpr (MODE == ZMODE_ONE) {
-          kz = (R)gp.dk[2] * (kidx_green<R>(m, L) + (R)gp.shift[2]);
-        } else {
-          kz = (R)gp.dk[2] * kidx_curl<R>(m, L);
-        }
-        T e1 = v[0][e], e2 = v[1][e], e3 = v[2][e];
-        if constexpr (MODE == ZMODE_CURL) {
-          const T isc = cmul_i<1>(sc);
-          v[0][e] = cmul(csub(cscale(e3, ky), cscale(e2, kz)), isc);
-          v[1][e] = cmul(csub(cscale(e1, kz), cscale(e3, kx)), isc);
-          v[2][e] = cmul(csub(cscale(e2, kx), cscale(e1, ky)), isc);
-        } else {
-          T kE = cmul(cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz)), iks);
-          const R k2 = kx * kx + ky * ky + kz * kz;
-          const R dr = k2 - ksr, di = -ksi;
-          const R dd = dr * dr + di * di;
-          const R rdd = R(1) / dd;  // one division for both parts of 1 / (k^2 - ks)
-          const T f = cmul(sc, mk(dr * rdd, -di * rdd));
-          v[0][e] = cmul(csub(e1, cscale(kE, kx)), f);
-          v[1][e] = cmul(csub(e2, cscale(kE, ky)), f);
-          v[2][e] = cmul(csub(e3, cscale(kE, kz)), f);
-        }
+        const R kz = z_wavenumber<MODE, L, R>(gp, lay_idx<LF, E, P_::RL>(t, e));
+        if constexpr (MODE == ZMODE_CURL) gb.curl(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+        else gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
       }
       if constexpr (NCX == 3) {
         fft_rev_plan_n<+1, P_, 3, SMS>(v, sm, twr, t);

@@ -90,9 +90,8 @@ struct fm_plan {
   DevBuf errbuf;        // device error code written by bounded pipeline waits
   bool avg = false;     // any absorbing axis
   bool zonly = false;   // shifts only on z -> single pass with the length-2L transform
-  bool zsplit = false;  // shifts only on z, padded z longer than the length-2L pass takes: two z passes
-  bool generic = false; // an axis without a fused pass (fm_generic.cuh): plain passes, Bluestein where needed
-  GenAxis gax[3];       // device tables of the general passes per axis
+  bool zsplit = false;  // shifts only on z, padded z of a length the length-2L pass does not take: two z passes
+  BlueAxis blue[3];     // axes without a fused pass (blue[a].n > 0): tables of their Bluestein passes (fm_generic.cuh)
   DevBuf gtw[3], gch[3][2], gkn[3][2];
   double shift[3] = {0, 0, 0};
   // potential / physics
@@ -197,6 +196,12 @@ inline void tk_end(const Tk& t) {
 template <typename S>
 static cudaError_t pass_xf(const fm_plan* P, const Dims& d, int pro, const void* in, const void* V, const double* rs,
                            const void* tw, const void* ramp, void* out, const int* act, VecTab vt = VecTab{}) {
+  if (P->blue[0].n) {
+    if constexpr (std::is_same<S, double>::value)
+      return launch_bxf<double, double>(d, pro, in, V, rs, P->blue[0], ramp, out, act, P->st, vt);
+    else return P->c64 ? launch_bxf<float, double>(d, pro, in, V, rs, P->blue[0], ramp, out, act, P->st, vt)
+                       : launch_bxf<float, float>(d, pro, in, V, rs, P->blue[0], ramp, out, act, P->st, vt);
+  }
   if constexpr (std::is_same<S, double>::value)
     return launch_xf<double, double>(d, pro, in, V, rs, tw, ramp, out, act, P->st, vt);
   else return P->c64 ? launch_xf<float, double>(d, pro, in, V, rs, tw, ramp, out, act, P->st, vt)
@@ -205,6 +210,12 @@ static cudaError_t pass_xf(const fm_plan* P, const Dims& d, int pro, const void*
 template <typename S>
 static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* in, const void* tw, const void* ramp,
                           void* out, const int* act) {
+  if (P->blue[1].n) {
+    if constexpr (std::is_same<S, double>::value)
+      return launch_by<double, double>(d, dir, in, P->blue[1], ramp, out, act, P->st);
+    else return P->c64 ? launch_by<float, double>(d, dir, in, P->blue[1], ramp, out, act, P->st)
+                       : launch_by<float, float>(d, dir, in, P->blue[1], ramp, out, act, P->st);
+  }
   if (P->use_tma && P->tma_y && !ramp) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
@@ -221,6 +232,12 @@ static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* 
 template <typename S>
 static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void* in, const GreenParams& gp,
                            const void* tw, const void* rz, void* out, const int* act) {
+  if (P->blue[2].n) {
+    if constexpr (std::is_same<S, double>::value)
+      return launch_bz<double, double>(d, mode, in, gp, P->blue[2], rz, out, act, P->st);
+    else return P->c64 ? launch_bz<float, double>(d, mode, in, gp, P->blue[2], rz, out, act, P->st)
+                       : launch_bz<float, float>(d, mode, in, gp, P->blue[2], rz, out, act, P->st);
+  }
   if (P->use_tma && P->tma_z) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
@@ -238,6 +255,12 @@ template <typename S>
 static cudaError_t pass_xi(const fm_plan* P, const Dims& d, int epi, const void* in, const void* V, const void* xv,
                            const void* bv, const double* rs, const EpiParams& ep, const void* tw, const void* ramp,
                            void* out, const int* act, VecTab vt = VecTab{}) {
+  if (P->blue[0].n) {
+    if constexpr (std::is_same<S, double>::value)
+      return launch_bxi<double, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], ramp, out, act, P->st, vt);
+    else return P->c64 ? launch_bxi<float, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], ramp, out, act, P->st, vt)
+                       : launch_bxi<float, float>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], ramp, out, act, P->st, vt);
+  }
   if constexpr (std::is_same<S, double>::value)
     return launch_xi<double, double>(d, epi, in, V, xv, bv, rs, ep, tw, ramp, out, act, P->st, vt);
   else return P->c64 ? launch_xi<float, double>(d, epi, in, V, xv, bv, rs, ep, tw, ramp, out, act, P->st, vt)
@@ -269,37 +292,26 @@ static cudaError_t upload_cplx(DevBuf& buf, const std::vector<cd>& v, cudaStream
 
 template <typename R>
 static fm_status init_tables(fm_plan* P) {
-  if (P->generic) {
-    const int n3[3] = {P->dims.nx, P->dims.ny, P->dims.nz};
-    for (int a = 0; a < 3; ++a) {
-      const GenAxisTables t = gen_axis_tables(n3[a]);
-      GenAxis& g = P->gax[a];
-      g.n = t.n;
-      g.m = t.m;
-      FM_CK(upload_cplx<R>(P->gtw[a], twiddles<R>(t.m), P->st));
-      g.tw = P->gtw[a].p;
-      if (t.m != t.n) {
-        for (int dir = 0; dir < 2; ++dir) {
-          FM_CK(upload_cplx<R>(P->gch[a][dir], t.chirp[dir], P->st));
-          FM_CK(upload_cplx<R>(P->gkn[a][dir], t.kern[dir], P->st));
-          g.chirp[dir] = P->gch[a][dir].p;
-          g.kern[dir] = P->gkn[a][dir].p;
-        }
-      }
+  const int n3[3] = {P->dims.nx, P->dims.ny, P->dims.nz};
+  DevBuf* tw[3] = {&P->twx, &P->twy, &P->twz};
+  for (int a = 0; a < 3; ++a) {
+    if (axis_supported(n3[a])) {
+      FM_CK(upload_cplx<R>(*tw[a], twiddles<R>(n3[a]), P->st));
+      continue;
     }
-    if (P->avg) {
-      FM_CK(upload_cplx<R>(P->rxp, ramp(P->dims.nx, P->shift[0], -1.0), P->st));
-      FM_CK(upload_cplx<R>(P->rxm, ramp(P->dims.nx, P->shift[0], +1.0), P->st));
-      FM_CK(upload_cplx<R>(P->ryp, ramp(P->dims.ny, P->shift[1], -1.0), P->st));
-      FM_CK(upload_cplx<R>(P->rym, ramp(P->dims.ny, P->shift[1], +1.0), P->st));
-      FM_CK(upload_cplx<R>(P->rzp, ramp(P->dims.nz, P->shift[2], -1.0), P->st));
-      FM_CK(upload_cplx<R>(P->rzm, ramp(P->dims.nz, P->shift[2], +1.0), P->st));
+    const BlueAxisTables t = blue_axis_tables(n3[a]);
+    BlueAxis& g = P->blue[a];
+    g.n = t.n;
+    g.m = t.m;
+    FM_CK(upload_cplx<R>(P->gtw[a], twiddles<R>(t.m), P->st));
+    g.tw = P->gtw[a].p;
+    for (int dir = 0; dir < 2; ++dir) {
+      FM_CK(upload_cplx<R>(P->gch[a][dir], t.chirp[dir], P->st));
+      FM_CK(upload_cplx<R>(P->gkn[a][dir], t.kern[dir], P->st));
+      g.chirp[dir] = P->gch[a][dir].p;
+      g.kern[dir] = P->gkn[a][dir].p;
     }
-    return FM_OK;
   }
-  FM_CK(upload_cplx<R>(P->twx, twiddles<R>(P->dims.nx), P->st));
-  FM_CK(upload_cplx<R>(P->twy, twiddles<R>(P->dims.ny), P->st));
-  FM_CK(upload_cplx<R>(P->twz, twiddles<R>(P->dims.nz), P->st));
   if (P->zonly) {
     FM_CK(upload_cplx<R>(P->twz2, twiddles<R>(2 * P->dims.nz), P->st));
     FM_CK(upload_cplx<R>(P->rz, ramp(P->dims.nz, P->shift[2], -1.0), P->st));
@@ -381,10 +393,10 @@ template <typename R>
 fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs, int epi, const void* xv,
                    const void* bv, const EpiParams& ep_in, void* out, const int* act, int nact = -1,
                    const RhsCtx* rc = nullptr, int chain = 0);
-// the five fused passes (no shift, or z-only shifts in one length-2L z pass), contiguous batches: where green_op
-// can chain applications
+// one sweep of the passes (no shift, or z-only shifts), fused x passes, contiguous batches: where green_op can
+// chain applications
 inline bool green_chain_ok(const fm_plan* P, const RhsCtx* rc) {
-  return !P->generic && (!P->avg || P->zonly) && !(rc && (rc->vt.in || rc->vt.out));
+  return !P->blue[0].n && (!P->avg || P->zonly || P->zsplit) && !(rc && (rc->vt.in || rc->vt.out));
 }
 // H = -i lambda/(2 pi 377) curl(E) for nb fields (in -> out, contiguous batches; act masks RHS)
 template <typename R>

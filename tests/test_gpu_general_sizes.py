@@ -112,3 +112,28 @@ def test_general_size_batch_equals_single():
     for i, x in enumerate(xs):
         assert np.array_equal(Y[..., i], plan.apply_operator(x))
     solver.release()
+
+
+# One kernel per axis: fused lengths mix with Bluestein lengths on any axis, pencil groups and shared-memory tiles
+# end inside an axis, and z-only averages run as two z passes on any length that has no length-2L pass.
+MIXED = [((21, 32, 16), "absz"), ((5, 64, 30), "absz"), ((32, 9, 8), "absz"), ((7, 8, 96), "per"), ((9, 16, 48), "absz"),
+         ((1, 3, 2), "per"), ((3, 128, 1), "per"), ((33, 8, 65), "all"), ((8, 131, 20), "per"), ((130, 8, 9), "per"),
+         ((16, 10, 128), "absz")]
+
+
+@pytest.mark.parametrize("precision", ["float64", "float32", "float32-math64"])
+@pytest.mark.parametrize("grid,kind", MIXED)
+def test_mixed_axis_kinds(precision, grid, kind):
+    ocfg, solver = configs(grid, _bcs(kind, grid), precision=precision)
+    eps = np.asfortranarray(EPS_BG + 0.3 * np.random.default_rng(7).random(grid).astype(complex))
+    pot = O.build_potential(ocfg, eps, EPS_BG, WL)
+    plan = solver.plan()
+    plan.set_potential(pot.V, pot.k_bg, pot.eps_imag, WL)
+    xs = [random_field(ocfg.padded_size + (3,), s) for s in (61, 62)]
+    X = np.asfortranarray(np.stack(xs, axis=-1))
+    G, A, H = plan.green_apply(X), plan.apply_operator(X), plan.curl_field(X)
+    for b, x in enumerate(xs):
+        assert rel(G[..., b], O.green_conv(x, ocfg, pot.k_square)) < OP_TOL[precision]
+        assert rel(A[..., b], O.cbs_operator(x, pot.V, ocfg, pot.k_square)) < OP_TOL[precision]
+        assert rel(H[..., b], O.magnetic_field(x, RES, WL)) < OP_TOL[precision]
+    solver.release()
