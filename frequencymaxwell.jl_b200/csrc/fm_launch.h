@@ -43,6 +43,14 @@ template <typename S, typename R>
 cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenParams& gp, const void* twz,
                           const void* rz, void* out, const int* active, int* err, int sms, cudaStream_t st);
 
+// z pass of the z-only average, both branches in one sweep (k_zavg): nz 128, 256 or 512, nx a multiple of the tile
+// (zavg_takes).  twz: the table of twiddles16(nz); rz: exp(-2 pi i z/(4 nz)); gp.shift[2] = 1/4.
+template <typename S, typename R>
+bool zavg_takes(const Dims& d);
+template <typename S, typename R>
+cudaError_t launch_zavg(const Dims& d, const void* in, const GreenParams& gp, const void* twz, const void* rz, void* out,
+                        const int* active, int* err, int sms, cudaStream_t st);
+
 // pencils that share one warp for an axis of length L (y/z passes need nx to be a multiple)
 template <typename R>
 int pencils_per_warp(int L);

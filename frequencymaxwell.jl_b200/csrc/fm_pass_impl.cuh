@@ -237,9 +237,11 @@ static EncodeTiledFn encode_fn() {
 }
 
 // Field batch viewed as 8-byte elements (one complex64, or half a complex128).
-// rank 3: (x, y, z*3*nb)  box (128 B, by, 1)      -- y pencils
-// rank 4: (x, y, z, 3*nb) box (128 B, 1, bz, 3)   -- z pencils, all components
-static bool make_map(CUtensorMap* m, void* base, const Dims& d, int esz, int rank, int box_y, int box_z) {
+// rank 3: (x, y, z*3*nb)  box (row_bytes, by, 1)      -- y pencils
+// rank 4: (x, y, z, 3*nb) box (row_bytes, 1, bz, 3)   -- z pencils, all components
+// row_bytes 128, 64 or 32, swizzled over as many bytes
+static bool make_map(CUtensorMap* m, void* base, const Dims& d, int esz, int rank, int box_y, int box_z,
+                     int row_bytes = 128) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const int w = esz / 8;  // 8-byte words per complex value
@@ -249,7 +251,7 @@ static bool make_map(CUtensorMap* m, void* base, const Dims& d, int esz, int ran
   dims[1] = (cuuint64_t)d.ny;
   strides[0] = (cuuint64_t)d.nx * esz;
   strides[1] = (cuuint64_t)d.nx * d.ny * esz;
-  box[0] = 16;
+  box[0] = (cuuint32_t)(row_bytes / 8);
   if (rank == 3) {
     dims[2] = (cuuint64_t)d.nz * 3 * d.nb;
     box[1] = (cuuint32_t)box_y;
@@ -263,7 +265,11 @@ static bool make_map(CUtensorMap* m, void* base, const Dims& d, int esz, int ran
     box[3] = 3;
   }
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, (cuuint32_t)rank, base, dims, strides, box, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  row_bytes == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                  : row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                    : CU_TENSOR_MAP_SWIZZLE_32B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -360,6 +366,40 @@ cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenPa
     default: return cudaErrorNotSupported;
   }
 #undef ZT
+}
+
+template <typename S, typename R, int L>
+static cudaError_t zavg_L(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz,
+                          void* out, const int* act, int* err, int sms, cudaStream_t st) {
+  using C = ZAvgCfg<S, R, L>;
+  static_assert(2 * (C::SM::total + 1024) <= 233472, "two CTAs at least share the 228 KB of an SM");
+  CUtensorMap mi, mo;
+  if (!make_map(&mi, const_cast<void*>(in), d, (int)sizeof(cplx<S>), 4, 1, C::BZ, C::ROWB) ||
+      !make_map(&mo, out, d, (int)sizeof(cplx<S>), 4, 1, C::BZ, C::ROWB))
+    return cudaErrorNotSupported;
+  const long long ntiles = (long long)(d.nx / C::TX) * d.ny * d.nb;
+  const size_t smem = C::SM::total;
+  allow_smem(k_zavg<S, R, L>, smem);
+  const unsigned grid = persistent_grid(k_zavg<S, R, L>, C::THREADS, smem, ntiles, sms, d.tma_ctas);
+  k_zavg<S, R, L><<<grid, C::THREADS, smem, st>>>(d, mi, mo, gp, (const cplx<R>*)tw, (const cplx<R>*)rz, act, err);
+  return cudaGetLastError();
+}
+
+template <typename S, typename R>
+bool zavg_takes(const Dims& d) {
+  return (d.nz == 128 && d.nx % ZAvgCfg<S, R, 128>::TX == 0) || (d.nz == 256 && d.nx % ZAvgCfg<S, R, 256>::TX == 0) ||
+         (d.nz == 512 && d.nx % ZAvgCfg<S, R, 512>::TX == 0);
+}
+
+template <typename S, typename R>
+cudaError_t launch_zavg(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz, void* out,
+                        const int* act, int* err, int sms, cudaStream_t st) {
+  switch (d.nz) {
+    case 128: return zavg_L<S, R, 128>(d, in, gp, tw, rz, out, act, err, sms, st);
+    case 256: return zavg_L<S, R, 256>(d, in, gp, tw, rz, out, act, err, sms, st);
+    case 512: return zavg_L<S, R, 512>(d, in, gp, tw, rz, out, act, err, sms, st);
+    default: return cudaErrorNotSupported;
+  }
 }
 
 template <typename R>

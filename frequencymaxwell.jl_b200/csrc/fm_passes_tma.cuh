@@ -329,4 +329,168 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
   }
 }
 
+// ---------------------------------------------------------------------------
+// z pass of the averaged Green function (shift 1/4 on z) for L = 128, 256, 512: the two shifted branches run as two
+// transforms of length L on neighbouring lane groups, sixteen values a lane and component, so all three components of
+// a branch stay in registers from the forward transform through the Green product to the inverse one.  Branch s
+// multiplies by exp(-/+ 2 pi i z/(4L)), and the groups add their results at the end (a shuffle; for L = 512, where a
+// branch fills a warp, through shared memory).
+//
+// What bounds it is shared memory: per value and branch one exchange (two at L = 512) each way, where the length-2L
+// transform in eight values a lane exchanges twice on twice the values.  192 of 255 registers hold the values, so an
+// SM has two CTAs of four warps; each has one tile, and one CTA's copies overlap the other's transforms.
+// ---------------------------------------------------------------------------
+template <typename S, typename R, int L>
+struct ZAvgCfg {
+  using T = cplx<R>;
+  using TS = cplx<S>;
+  using P = Plan16<L>;
+  static constexpr int W = 4, THREADS = 32 * W;
+  static constexpr int GROUPS = THREADS / (2 * P::TP);  // pencils in flight per CTA: 8, 4, 2
+  static constexpr int CTAS = sizeof(R) == 8 ? 2 : 4;   // per SM: 255 or 128 registers
+  // bytes of a tile row: whole rounds of pencils, and room for CTAS tiles on an SM
+  static constexpr int ROWB = sizeof(R) == 8 ? (L == 512 ? 32 : (L == 256 || sizeof(TS) == 8 ? 64 : 128))
+                                             : (L == 128 ? 64 : 32);
+  static constexpr int TX = ROWB / (int)sizeof(TS);     // pencils of a tile
+  static constexpr int ROUNDS = TX / GROUPS;
+  static_assert(TX % GROUPS == 0 && ROUNDS >= 1, "tile rows hold whole rounds");
+  static constexpr int BZ = L > 256 ? 256 : L;          // z extent of one copy
+  static constexpr int TILE = 3 * L * ROWB;
+  static constexpr int EXB = 2 * GROUPS * P::STRIDE * (int)sizeof(T);
+  using SM = TmaSmem<TILE, 1, EXB, 3 * L * (int)sizeof(T)>;
+  // element (component 0, z = t < TP, pencil x) of the tile: rows of ROWB bytes, swizzled by the copy in 16-byte chunks
+  static __device__ __forceinline__ unsigned char* at(unsigned char* tile, int t, int x) {
+    const int byte = x * (int)sizeof(TS);
+    const int sw = ROWB == 128 ? (t & 7) : ROWB == 64 ? ((t >> 1) & 3) : ((t >> 2) & 1);
+    return tile + t * ROWB + (((byte >> 4) ^ sw) << 4) + (byte & 15);
+  }
+  // byte offset of component c and z = t + e*TP from there (whole multiples of 8 rows, which the swizzle repeats over)
+  static constexpr int off(int c, int e) {
+    return ((e * P::TP / BZ) * (3 * BZ) + c * BZ + (e * P::TP) % BZ) * ROWB;
+  }
+};
+
+template <typename S, typename R, int L>
+__global__ void __launch_bounds__(128, ZAvgCfg<S, R, L>::CTAS)
+    k_zavg(Dims d, const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out, GreenParams gp,
+           const cplx<R>* __restrict__ twz, const cplx<R>* __restrict__ rz, const int* __restrict__ active,
+           int* __restrict__ err) {
+  using C = ZAvgCfg<S, R, L>;
+  using T = typename C::T;
+  using TS = typename C::TS;
+  using P_ = typename C::P;
+  constexpr int TP = P_::TP;
+  extern __shared__ unsigned char smraw_[];
+  unsigned char* sm0 = (unsigned char*)(((uintptr_t)smraw_ + 1023) & ~(uintptr_t)1023);
+  unsigned char* tl = sm0 + C::SM::tiles;
+  T* ex = reinterpret_cast<T*>(sm0 + C::SM::ex);
+  T* tw = reinterpret_cast<T*>(sm0 + C::SM::tab);
+  T* twr = tw + L;
+  T* rtab = twr + L;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm0 + C::SM::bars);
+  const int xtiles = d.nx / C::TX;
+  const long long per_rhs = (long long)xtiles * d.ny;
+  const long long ntiles = per_rhs * d.nb;
+  load_table(tw, twz, 2 * L);
+  load_table(rtab, rz, L);
+  if (threadIdx.x == 0) {
+    mbar_init(full, 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  auto issue = [&](long long tile) {
+    const int xt = (int)(tile % xtiles);
+    const long long yb = tile / xtiles;
+    mbar_expect_tx(full, C::TILE);
+    for (int k = 0; k < L / C::BZ; ++k)
+      tma_load_4d(tl + k * 3 * C::BZ * C::ROWB, &tm_in, full, xt * (C::ROWB / 8), (int)(yb % d.ny), k * C::BZ,
+                  3 * (int)(yb / d.ny));
+  };
+  long long tile = next_active(blockIdx.x, ntiles, per_rhs, active);
+  if (threadIdx.x == 0 && tile < ntiles) issue(tile);
+  // lane group of this thread: TP lanes of one branch of one pencil, the two branches of a pencil side by side
+  const int grp = threadIdx.x / TP, t = threadIdx.x % TP;
+  const int br = grp & 1, pen = grp >> 1;
+  const R sg = br ? R(-1) : R(1);
+  T* sm = ex + grp * P_::STRIDE;
+  uint32_t ph = 0;
+  for (; tile < ntiles; ph ^= 1) {
+    const int xt = (int)(tile % xtiles);
+    const long long yb = tile / xtiles;
+    const int y = (int)(yb % d.ny), b = (int)(yb / d.ny);
+    const bool ok = mbar_wait(full, ph, err, 33);
+    if (__syncthreads_or(!ok)) break;  // timed out: nothing of this CTA is in flight but the load that did not come
+    const GreenBin<R> gb(gp, b);
+    const R ky = (R)gp.dk[1] * (kidx_green<R>(y, d.ny) + (R)gp.shift[1]);
+#pragma unroll 1
+    for (int rd = 0; rd < C::ROUNDS; ++rd) {
+      const int xl = rd * C::GROUPS + pen;
+      unsigned char* tp = C::at(tl, t, xl);
+      // one component at a time between synchronisations, so that only the transform in hand needs temporaries
+      T v[3][16];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          T r = rtab[t + e * TP];
+          r.y *= sg;
+          v[c][e] = cmul(cv<T>(*reinterpret_cast<TS*>(tp + C::off(c, e))), r);
+        }
+        fft16_fwd<-1, P_>(v[c], sm, tw, t);
+        __syncwarp();
+      }
+      const R kx = (R)gp.dk[0] * (kidx_green<R>(xt * C::TX + xl, d.nx) + (R)gp.shift[0]);
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const R kz = (R)gp.dk[2] * (kidx_green<R>(lay_idx<L, 16, P_::RL>(t, e), L) + sg * (R)gp.shift[2]);
+        gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        fft16_rev<+1, P_>(v[c], sm, twr, t);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          T r = rtab[t + e * TP];
+          r.y *= -sg;
+          v[c][e] = cmul(v[c][e], r);
+        }
+        // sum of the branches: each group keeps half of the values and takes the partner's share of them.  By now both
+        // groups of the pencil have read the tile (the exchanges synchronise them), so the result may go into it.
+        if constexpr (TP < 32) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const T send = br ? v[c][e] : v[c][e + 8], keep = br ? v[c][e + 8] : v[c][e];
+            v[c][e] = mk(keep.x + __shfl_xor_sync(0xffffffffu, send.x, TP),
+                         keep.y + __shfl_xor_sync(0xffffffffu, send.y, TP));
+          }
+        } else {
+          T* other = ex + (grp ^ 1) * P_::STRIDE;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) sm[t + 32 * e] = br ? v[c][e] : v[c][e + 8];
+          named_bar(1 + pen, 64);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[c][e] = cadd(br ? v[c][e + 8] : v[c][e], other[t + 32 * e]);
+          named_bar(1 + pen, 64);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          *reinterpret_cast<TS*>(tp + C::off(c, e) + br * (C::off(0, 8) - C::off(0, 0))) = cv<TS>(v[c][e]);
+        __syncwarp();
+      }
+    }
+    fence_proxy_async();
+    __syncthreads();
+    const long long next = next_active(tile + gridDim.x, ntiles, per_rhs, active);
+    if (threadIdx.x == 0) {
+      for (int k = 0; k < L / C::BZ; ++k)
+        tma_store_4d(&tm_out, tl + k * 3 * C::BZ * C::ROWB, xt * (C::ROWB / 8), y, k * C::BZ, 3 * b);
+      bulk_commit();
+      bulk_wait_read0();
+      if (next < ntiles) issue(next);
+    }
+    tile = next;
+  }
+  if (threadIdx.x == 0) bulk_wait0();
+}
+
 }  // namespace fm

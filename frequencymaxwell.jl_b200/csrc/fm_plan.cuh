@@ -99,7 +99,7 @@ struct fm_plan {
   double k_bg = 0, eps_imag = 0, wavelength = 0, kref2 = 1;
   int bornmax = 0;
   // tables (plan precision)
-  DevBuf twx, twy, twz, twz2, rz, rxp, rxm, ryp, rym, rzp, rzm;
+  DevBuf twx, twy, twz, twz2, twz16, rz, rxp, rxm, ryp, rym, rzp, rzm;
   DevBuf V;
   // workspace
   DevBuf t1, t2, t3, bbuf, xbuf, ebuf, sbuf, basis, gbuf2;  // t3: first branch of a two-branch average
@@ -251,6 +251,23 @@ static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void
   else return P->c64 ? launch_zg<float, double>(d, mode, in, gp, tw, rz, out, act, P->st)
                      : launch_zg<float, float>(d, mode, in, gp, tw, rz, out, act, P->st);
 }
+// the z pass of a z-only average with both branches in one sweep: whether this plan's shape has it, and the pass
+template <typename S>
+static bool has_zavg(const fm_plan* P, const Dims& d) {
+  if (!P->use_tma || !P->tma_z || !(P->zonly || P->zsplit) || P->blue[2].n) return false;
+  if constexpr (std::is_same<S, double>::value) return zavg_takes<double, double>(d);
+  else return P->c64 ? zavg_takes<float, double>(d) : zavg_takes<float, float>(d);
+}
+template <typename S>
+static cudaError_t pass_zavg(const fm_plan* P, const Dims& d, const void* in, const GreenParams& gp, void* out,
+                             const int* act) {
+  const void* rz = P->zonly ? P->rz.p : P->rzp.p;
+  int* err = (int*)P->errbuf.p;
+  if constexpr (std::is_same<S, double>::value)
+    return launch_zavg<double, double>(d, in, gp, P->twz16.p, rz, out, act, err, P->sms, P->st);
+  else return P->c64 ? launch_zavg<float, double>(d, in, gp, P->twz16.p, rz, out, act, err, P->sms, P->st)
+                     : launch_zavg<float, float>(d, in, gp, P->twz16.p, rz, out, act, err, P->sms, P->st);
+}
 template <typename S>
 static cudaError_t pass_xi(const fm_plan* P, const Dims& d, int epi, const void* in, const void* V, const void* xv,
                            const void* bv, const double* rs, const EpiParams& ep, const void* tw, const void* ramp,
@@ -312,6 +329,7 @@ static fm_status init_tables(fm_plan* P) {
       g.kern[dir] = P->gkn[a][dir].p;
     }
   }
+  if (P->zonly || P->zsplit) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
   if (P->zonly) {
     FM_CK(upload_cplx<R>(P->twz2, twiddles<R>(2 * P->dims.nz), P->st));
     FM_CK(upload_cplx<R>(P->rz, ramp(P->dims.nz, P->shift[2], -1.0), P->st));
