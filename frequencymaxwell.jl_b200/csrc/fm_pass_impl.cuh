@@ -291,8 +291,8 @@ static cudaError_t y_tma_L(const Dims& d, const void* in, const void* tw, const 
   if (d.nx % C::TX) return cudaErrorNotSupported;
   CUtensorMap mi, mo;
   const int box = L > 256 ? 256 : L;
-  if (!make_map(&mi, const_cast<void*>(in), d, (int)sizeof(cplx<S>), 3, box, 1) ||
-      !make_map(&mo, out, d, (int)sizeof(cplx<S>), 3, box, 1))
+  if (!make_map(&mi, const_cast<void*>(in), d, (int)sizeof(cplx<S>), 3, box, 1, C::ROWB) ||
+      !make_map(&mo, out, d, (int)sizeof(cplx<S>), 3, box, 1, C::ROWB))
     return cudaErrorNotSupported;
   const size_t smem = C::SM::total;
   allow_smem(k_y_tma<S, R, L, DIR>, smem);
@@ -334,6 +334,7 @@ cudaError_t launch_y_tma(const Dims& d, int dir, const void* in, const void* tw,
     case 64: return YT(64);
     case 128: return YT(128);
     case 256: return YT(256);
+    case 512: return YT(512);
     default: return cudaErrorNotSupported;
   }
 #undef YT

@@ -59,8 +59,13 @@ __device__ __forceinline__ void load_table(T* dst, const T* src, int n) {
 // ---------------------------------------------------------------------------
 enum { PRO_COPY = 0, PRO_V = 1, PRO_V_SCALE = 2 };
 
+// CTAs of 256 threads per SM that a row pass is compiled for, by its length.  At 256 one CTA an SM (no bound on the
+// registers) ran the FP32-storage passes of 256^3 at 2.6 (k_xf) and 1.6 TB/s (k_xi); two and three run them at
+// 3.9 and 3.2; k_xf with three spills (3.5).  At 512 (16 values a lane) two fit.
+constexpr int row_ctas(int L, int small, int at256) { return L == 96 ? 1 : L <= 128 ? small : L == 256 ? at256 : 2; }
+
 template <typename S, typename R, int L, int PRO>
-__global__ void __launch_bounds__(256, (L <= 128 && L != 96) ? 2 : 1) k_xf(Dims d, const cplx<S>* __restrict__ in, const cplx<S>* __restrict__ V,
+__global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cplx<S>* __restrict__ in, const cplx<S>* __restrict__ V,
                                             const double* __restrict__ rhs_scale, const cplx<R>* __restrict__ twx,
                                             const cplx<R>* __restrict__ rampx, cplx<S>* __restrict__ out,
                                             const int* __restrict__ active, VecTab vt) {
@@ -82,10 +87,14 @@ __global__ void __launch_bounds__(256, (L <= 128 && L != 96) ? 2 : 1) k_xf(Dims 
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * d.ny * d.nz;
   T* sm = warp_smem<T, PencilStride<L, T, TP, true>::v>(ex, wic, PW, p);
-  T vrow[E];
-  if constexpr (PRO != PRO_COPY) {
+  // V is held across the three components, except at the long lengths: there the registers it would take decide how
+  // many CTAs fit on an SM, and it is read per component (an L1 hit after the first)
+  constexpr bool HOLD = PRO != PRO_COPY && L <= 128;
+  const cplx<S>* Vrow = V + b * d.vstride + yz * L;
+  T vrow[HOLD ? E : 1];
+  if constexpr (HOLD) {
 #pragma unroll
-    for (int e = 0; e < E; ++e) vrow[e] = cv<T>(V[b * d.vstride + yz * L + lay_idx<L, E, P_::R0>(t, e)]);
+    for (int e = 0; e < E; ++e) vrow[e] = cv<T>(Vrow[lay_idx<L, E, P_::R0>(t, e)]);
   }
   R s = R(1);
   if constexpr (PRO == PRO_V_SCALE) s = (R)rhs_scale[b];
@@ -99,7 +108,8 @@ __global__ void __launch_bounds__(256, (L <= 128 && L != 96) ? 2 : 1) k_xf(Dims 
     for (int e = 0; e < E; ++e) {
       const int x = lay_idx<L, E, P_::R0>(t, e);
       T a = cv<T>(inb[rbase + x]);
-      if constexpr (PRO != PRO_COPY) a = cmul(a, vrow[e]);
+      if constexpr (HOLD) a = cmul(a, vrow[e]);
+      else if constexpr (PRO != PRO_COPY) a = cmul(a, cv<T>(Vrow[x]));
       if constexpr (PRO == PRO_V_SCALE) a = cscale(a, s);
       if (rampx) a = cmul(a, rampx[x]);
       v[e] = a;
@@ -454,7 +464,7 @@ __device__ __forceinline__ T epi_element(T g, long long ix, const cplx<S>* xvb, 
 }
 
 template <typename S, typename R, int L, int EPI>
-__global__ void __launch_bounds__(256, (L <= 128 && L != 96) ? 3 : 1) k_xi(Dims d, const cplx<S>* __restrict__ in, const cplx<S>* __restrict__ V,
+__global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cplx<S>* __restrict__ in, const cplx<S>* __restrict__ V,
                                             const cplx<S>* __restrict__ xv, const cplx<S>* __restrict__ bv,
                                             const double* __restrict__ rhs_scale, EpiParams ep,
                                             const cplx<R>* __restrict__ twx, const cplx<R>* __restrict__ rampx,
@@ -517,7 +527,7 @@ __global__ void __launch_bounds__(256, (L <= 128 && L != 96) ? 3 : 1) k_xi(Dims 
 // application's x pass neither reads `out` nor V again.  The forward input is the stored (storage-typed) value,
 // so out2 equals k_xf's output bit for bit.  Contiguous batches and no x ramp (the z-only and periodic plans).
 template <typename S, typename R, int L>
-__global__ void __launch_bounds__(256, (L <= 128 && L != 96) ? 3 : 1) k_xi_xf(Dims d, const cplx<S>* __restrict__ in,
+__global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const cplx<S>* __restrict__ in,
                                                                           const cplx<S>* __restrict__ V,
                                                                           const cplx<S>* __restrict__ xv,
                                                                           EpiParams ep,

@@ -30,12 +30,13 @@ struct YTmaCfg {
   using T = cplx<R>;
   using TS = cplx<S>;
   using P = Plan<L, R>;
-  static constexpr int TX = 128 / (int)sizeof(TS);
+  static constexpr int ROWB = L == 512 ? 64 : 128;  // bytes of a tile row
+  static constexpr int TX = ROWB / (int)sizeof(TS);
   static constexpr int PW = 32 / P::TP;
   static constexpr int CW = (TX / PW) < 4 ? (TX / PW) : 4;
   static constexpr int ROUNDS = TX / (CW * PW);
-  static constexpr int TILE = L * 128;
-  static constexpr int NST = TILE <= 32768 ? 3 : 2;  // three stages leave room for three CTAs per SM
+  static constexpr int TILE = L * ROWB;
+  static constexpr int NST = L <= 128 ? 3 : 2;  // three stages leave room for three CTAs per SM
   static constexpr int STRIDE = PencilStride<L, T, P::TP, true>::v;
   using SM = TmaSmem<TILE, NST, CW * PW * STRIDE * (int)sizeof(T), L * (int)sizeof(T)>;
   static constexpr int THREADS = CW * 32;
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(YTmaCfg<S, R, L>::THREADS)
     const int zcb = (int)(tile / xtiles);
     mbar_expect_tx(full + s, C::TILE);
     for (int k = 0; k < L / BOX; ++k)
-      tma_load_3d(tiles + s * C::TILE + k * BOX * 128, &tm_in, full + s, xt * 16, k * BOX, zcb);
+      tma_load_3d(tiles + s * C::TILE + k * BOX * C::ROWB, &tm_in, full + s, xt * (C::ROWB / 8), k * BOX, zcb);
   };
   long long ld = next_active(blockIdx.x, ntiles, per_rhs, active);  // load cursor (thread 0)
   if (threadIdx.x == 0) {
@@ -113,17 +114,17 @@ __global__ void __launch_bounds__(YTmaCfg<S, R, L>::THREADS)
 #pragma unroll
         for (int e = 0; e < E; ++e) {
           const int y = lay_idx<L, E, P_::R0>(t, e);
-          T a = cv<T>(*tile_at<TS>(tl, y, xl));
+          T a = cv<T>(*tile_at<TS, C::ROWB>(tl, y, xl));
           if (rampy) a = cmul(a, rampy[y]);
           v[e] = a;
         }
         fft_fwd_plan<-1, P_>(v, sm, tw, t);
         __syncwarp();
 #pragma unroll
-        for (int e = 0; e < E; ++e) *tile_at<TS>(tl, lay_idx<L, E, P_::RL>(t, e), xl) = cv<TS>(v[e]);
+        for (int e = 0; e < E; ++e) *tile_at<TS, C::ROWB>(tl, lay_idx<L, E, P_::RL>(t, e), xl) = cv<TS>(v[e]);
       } else {
 #pragma unroll
-        for (int e = 0; e < E; ++e) v[e] = cv<T>(*tile_at<TS>(tl, lay_idx<L, E, P_::RL>(t, e), xl));
+        for (int e = 0; e < E; ++e) v[e] = cv<T>(*tile_at<TS, C::ROWB>(tl, lay_idx<L, E, P_::RL>(t, e), xl));
         fft_rev_plan<+1, P_>(v, sm, tw, t);
         __syncwarp();
 #pragma unroll
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(YTmaCfg<S, R, L>::THREADS)
           const int y = lay_idx<L, E, P_::R0>(t, e);
           T a = v[e];
           if (rampy) a = cmul(a, cconj(rampy[y]));
-          *tile_at<TS>(tl, y, xl) = cv<TS>(a);
+          *tile_at<TS, C::ROWB>(tl, y, xl) = cv<TS>(a);
         }
       }
       __syncwarp();
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(YTmaCfg<S, R, L>::THREADS)
     if (lane == 0) mbar_arrive(done + s);
     if (threadIdx.x == 0) {
       if (!mbar_wait(done + s, ph, err, 14)) { ok = false; break; }
-      for (int k = 0; k < L / BOX; ++k) tma_store_3d(&tm_out, tl + k * BOX * 128, xt * 16, k * BOX, zcb);
+      for (int k = 0; k < L / BOX; ++k) tma_store_3d(&tm_out, tl + k * BOX * C::ROWB, xt * (C::ROWB / 8), k * BOX, zcb);
       bulk_commit();
       bulk_wait_read0();
       if (ld < ntiles) {

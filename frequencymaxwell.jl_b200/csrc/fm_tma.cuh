@@ -111,13 +111,13 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
                : "memory");
 }
 
-// Element (row r, column x) of a 128-byte-row tile written with the 128-byte swizzle.
-template <typename TS>
+// Element (row r, column x) of a tile of ROWB-byte rows (128 or 64) written with the swizzle of that size.
+template <typename TS, int ROWB = 128>
 __device__ __forceinline__ TS* tile_at(unsigned char* tile, int r, int x) {
   constexpr int esz = (int)sizeof(TS);
   const int byte = x * esz;
-  const int chunk = (byte >> 4) ^ (r & 7);
-  return reinterpret_cast<TS*>(tile + r * 128 + (chunk << 4) + (byte & 15));
+  const int chunk = (byte >> 4) ^ (ROWB == 128 ? (r & 7) : ((r >> 1) & 3));
+  return reinterpret_cast<TS*>(tile + r * ROWB + (chunk << 4) + (byte & 15));
 }
 
 }  // namespace fm
