@@ -44,6 +44,9 @@ template <typename T> __device__ __forceinline__ T from_d(double2 a);
 template <> __device__ __forceinline__ float2 from_d<float2>(double2 a) { return make_float2((float)a.x, (float)a.y); }
 template <> __device__ __forceinline__ double2 from_d<double2>(double2 a) { return a; }
 
+// starts bringing the 128-byte line at p to L2
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ---- FP32 -> FP64 without the conversion unit ----
 // The conversion instruction issues about one lane per clock and scheduler on sm_100a, which caps a kernel that
 // widens every value it reads near 5 TB/s of FP32 data.  Moving the fields of the float into those of a double with

@@ -713,6 +713,14 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_blockupdate_mma(long long M, 
   for (long long tl = (long long)blockIdx.x * KV_WARPS + w; tl < tiles; tl += (long long)gridDim.x * KV_WARPS) {
     const long long ea = tl * TILE + QR * gid;  // A rows of this lane: elements ea .. ea + QR - 1 (wholly in or out)
     const bool ein = ea < M;
+    {
+      // the block vectors of this tile come to L2 while the basis is swept: they are read after it
+      constexpr int PY = 128 / (int)sizeof(TY), LY = (TILE + PY - 1) / PY;
+      for (int i = lane; i < S * LY; i += 32) {
+        const long long e = tl * TILE + (i % LY) * PY;
+        if (e < M) prefetch_l2(yb + (size_t)(i / LY) * us + e);
+      }
+    }
     double P[QR][NT][2], Q[QR][NT][2];
 #pragma unroll
     for (int q = 0; q < QR; ++q)
@@ -757,6 +765,16 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_blockupdate_mma(long long M, 
             mma_f64(Q[q][n][0], Q[q][n][1], x.y, bfr[n]);
           }
         }
+      }
+    }
+    {
+      // ... and the first basis vectors of the next tile while this one is written
+      const long long en = (tl + (long long)gridDim.x * KV_WARPS) * TILE;
+      constexpr int PX = 128 / (int)sizeof(T), LX = (TILE + PX - 1) / PX;
+      for (int i = lane; i < 4 * UPD_PD * LX; i += 32) {
+        const int k = i / LX;
+        const long long e = en + (i % LX) * PX;
+        if (k < K && e < M) prefetch_l2(ub + (size_t)k * us + e);
       }
     }
     // lane (gid, tig) holds C rows gid (element ea + q) and columns 2 tig, 2 tig + 1 of each tile
