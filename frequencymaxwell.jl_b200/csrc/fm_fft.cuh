@@ -379,20 +379,20 @@ __device__ __forceinline__ int lay_idx(int t, int e) {
   return t + (L / E) * (e / R) + (e % R) * (L / R);
 }
 
-// ---- sixteen values a lane: plans of L = 128, 256 (one exchange) and 512 (two), either arithmetic type ----
+// ---- sixteen values a lane: plans of L = 64, 128, 256 (one exchange) and 512 (two), either arithmetic type ----
 // A transform of length 256 in eight values a lane exchanges twice; with sixteen it exchanges once, and shared memory
 // is what binds the FP64 z pass.  The exchange is padded by one slot per 2^PS elements, PS = 4 for a first radix of
-// 16 and 3 for smaller ones, so that the strided writes of the first stage fall in distinct banks.
+// 16 and 3 or 2 for smaller ones, so that the strided writes of the first stage fall in distinct banks.
 template <int L_> struct Plan16 {
   static constexpr int L = L_, E = 16, TP = L_ / 16, R0 = 16;
-  static constexpr int R1 = L_ == 256 ? 16 : 8, R2 = L_ == 512 ? 4 : 0;
+  static constexpr int R1 = L_ == 256 ? 16 : L_ == 64 ? 4 : 8, R2 = L_ == 512 ? 4 : 0;
   static constexpr int RL = R2 ? R2 : R1;
-  static_assert(L_ == 128 || L_ == 256 || L_ == 512, "lengths of sixteen values a lane");
-  // slots per pencil: the padded length; for L = 128 in FP32 two pencils share a wavefront on disjoint halves
-  static constexpr int STRIDE = L_ + L_ / 8 + (L_ == 128 ? 8 : 0);
+  static_assert(L_ == 64 || L_ == 128 || L_ == 256 || L_ == 512, "lengths of sixteen values a lane");
+  // slots per pencil: the padded length; pencils that share a wavefront (L = 64, and 128 in FP32) on disjoint slots
+  static constexpr int STRIDE = L_ == 64 ? 84 : L_ + L_ / 8 + (L_ == 128 ? 8 : 0);
 };
 
-template <int DIR, int L, int RAD, int NS, bool LAST, int PS, typename T>
+template <int DIR, int L, int RAD, int NS, bool LAST, int PS, bool LO, typename T>
 __device__ __forceinline__ void fft16_stage(T (&v)[16], T* sm, const T* tw, int t) {
   constexpr int TP = L / 16;
 #pragma unroll
@@ -407,7 +407,8 @@ __device__ __forceinline__ void fft16_stage(T (&v)[16], T* sm, const T* tw, int 
         v[m * RAD + q] = cmul(v[m * RAD + q], w);
       }
     }
-    bfly<DIR, RAD>(&v[m * RAD]);
+    if constexpr (LO) bfly_lo<DIR, RAD>(&v[m * RAD]);
+    else bfly<DIR, RAD>(&v[m * RAD]);
     if constexpr (!LAST) {
       // the padded slot of element base + q*NS is the slot of base plus a constant: no carry crosses the pad bits
       const int base = (j / NS) * NS * RAD + k;
@@ -431,22 +432,23 @@ __device__ __forceinline__ void fft16_gather(T (&v)[16], const T* sm, int t) {
   __syncwarp();
 }
 // radix sequence (A, B, C) of length L; natural order in (layout of A) and out (layout of the last radix)
-template <int DIR, int L, int A, int B, int C, typename T>
+template <int DIR, int L, int A, int B, int C, bool LO = false, typename T>
 __device__ __forceinline__ void fft16_run(T (&v)[16], T* sm, const T* tw, int t) {
-  constexpr int PS = A == 16 ? 4 : 3;
-  fft16_stage<DIR, L, A, 1, false, PS>(v, sm, tw, t);
+  constexpr int PS = A == 16 ? 4 : L == 64 ? 2 : 3;
+  fft16_stage<DIR, L, A, 1, false, PS, LO>(v, sm, tw, t);
   fft16_gather<L, B, PS>(v, sm, t);
   if constexpr (C == 0) {
-    fft16_stage<DIR, L, B, A, true, PS>(v, sm, tw, t);
+    fft16_stage<DIR, L, B, A, true, PS, false>(v, sm, tw, t);
   } else {
-    fft16_stage<DIR, L, B, A, false, PS>(v, sm, tw, t);
+    fft16_stage<DIR, L, B, A, false, PS, false>(v, sm, tw, t);
     fft16_gather<L, C, PS>(v, sm, t);
-    fft16_stage<DIR, L, C, A * B, true, PS>(v, sm, tw, t);
+    fft16_stage<DIR, L, C, A * B, true, PS, false>(v, sm, tw, t);
   }
 }
-template <int DIR, typename P, typename T>
+// (LO: the elements at and above L/2 are zero and are not read from v)
+template <int DIR, typename P, bool LO = false, typename T>
 __device__ __forceinline__ void fft16_fwd(T (&v)[16], T* sm, const T* tw_fwd, int t) {
-  fft16_run<DIR, P::L, P::R0, P::R1, P::R2>(v, sm, tw_fwd, t);
+  fft16_run<DIR, P::L, P::R0, P::R1, P::R2, LO>(v, sm, tw_fwd, t);
 }
 template <int DIR, typename P, typename T>
 __device__ __forceinline__ void fft16_rev(T (&v)[16], T* sm, const T* tw_rev, int t) {

@@ -20,7 +20,8 @@ inline int blue_fft_length(int n) {
 }
 
 // FP64 host tables of one axis: the chirps and the transformed convolution kernels of both directions (BlueAxis).
-// The stage twiddles of length m depend on the arithmetic type's radix split: twiddles<R>(m).
+// The stage twiddles of length m: twiddles16(512), and by the arithmetic type's radix split below that,
+// twiddles<R>(m).
 struct BlueAxisTables {
   int n = 0, m = 0;
   std::vector<std::complex<double>> chirp[2], kern[2];

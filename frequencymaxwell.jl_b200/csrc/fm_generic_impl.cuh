@@ -24,12 +24,12 @@ static void blue_allow_smem(K kern, size_t bytes) {
 // grid and shared memory of the row passes
 template <typename R, int M>
 struct BlueRows {
-  static constexpr int TP = Plan<M, R>::TP, PW = 32 / TP;
+  static constexpr int TP = BluePlan<M, R>::TP, PW = 32 / TP;
   static unsigned blocks(const Dims& d) {
     return (unsigned)(((long long)d.ny * d.nz * d.nb + BX_WARPS * PW - 1) / (BX_WARPS * PW));
   }
   static constexpr size_t smem =
-      (size_t)(2 * M + BX_WARPS * PW * PencilStride<M, cplx<R>, TP, true>::v) * sizeof(cplx<R>);
+      (size_t)(2 * M + BX_WARPS * PW * BluePlan<M, R>::STRIDE) * sizeof(cplx<R>);
 };
 
 template <typename S, typename R, int M>

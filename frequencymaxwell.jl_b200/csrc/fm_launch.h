@@ -43,13 +43,14 @@ template <typename S, typename R>
 cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenParams& gp, const void* twz,
                           const void* rz, void* out, const int* active, int* err, int sms, cudaStream_t st);
 
-// z pass of the z-only average, both branches in one sweep (k_zavg): nz 128, 256 or 512, nx a multiple of the tile
-// (zavg_takes).  twz: the table of twiddles16(nz); rz: exp(-2 pi i z/(4 nz)); gp.shift[2] = 1/4.
+// z pass in sixteen values a lane (k_zreg): nz 64, 128, 256 or 512, nx a multiple of the tile (zreg_takes).
+// branches 2: the z-only average in one sweep, rz = exp(-2 pi i z/(4 nz)) and gp.shift[2] = 1/4; branches 1: one branch
+// as ZMODE_ONE (rz null without a shift).  twz: the table of twiddles16(nz).
 template <typename S, typename R>
-bool zavg_takes(const Dims& d);
+bool zreg_takes(const Dims& d, int branches);
 template <typename S, typename R>
-cudaError_t launch_zavg(const Dims& d, const void* in, const GreenParams& gp, const void* twz, const void* rz, void* out,
-                        const int* active, int* err, int sms, cudaStream_t st);
+cudaError_t launch_zreg(const Dims& d, int branches, const void* in, const GreenParams& gp, const void* twz,
+                        const void* rz, void* out, const int* active, int* err, int sms, cudaStream_t st);
 
 // pencils that share one warp for an axis of length L (y/z passes need nx to be a multiple)
 template <typename R>

@@ -369,10 +369,10 @@ cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenPa
 #undef ZT
 }
 
-template <typename S, typename R, int L>
-static cudaError_t zavg_L(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz,
+template <typename S, typename R, int L, int BR>
+static cudaError_t zreg_L(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz,
                           void* out, const int* act, int* err, int sms, cudaStream_t st) {
-  using C = ZAvgCfg<S, R, L>;
+  using C = ZRegCfg<S, R, L, BR>;
   static_assert(2 * (C::SM::total + 1024) <= 233472, "two CTAs at least share the 228 KB of an SM");
   CUtensorMap mi, mo;
   if (!make_map(&mi, const_cast<void*>(in), d, (int)sizeof(cplx<S>), 4, 1, C::BZ, C::ROWB) ||
@@ -380,27 +380,34 @@ static cudaError_t zavg_L(const Dims& d, const void* in, const GreenParams& gp, 
     return cudaErrorNotSupported;
   const long long ntiles = (long long)(d.nx / C::TX) * d.ny * d.nb;
   const size_t smem = C::SM::total;
-  allow_smem(k_zavg<S, R, L>, smem);
-  const unsigned grid = persistent_grid(k_zavg<S, R, L>, C::THREADS, smem, ntiles, sms, d.tma_ctas);
-  k_zavg<S, R, L><<<grid, C::THREADS, smem, st>>>(d, mi, mo, gp, (const cplx<R>*)tw, (const cplx<R>*)rz, act, err);
+  allow_smem(k_zreg<S, R, L, BR>, smem);
+  const unsigned grid = persistent_grid(k_zreg<S, R, L, BR>, C::THREADS, smem, ntiles, sms, d.tma_ctas);
+  k_zreg<S, R, L, BR><<<grid, C::THREADS, smem, st>>>(d, mi, mo, gp, (const cplx<R>*)tw, (const cplx<R>*)rz, act, err);
   return cudaGetLastError();
 }
 
 template <typename S, typename R>
-bool zavg_takes(const Dims& d) {
-  return (d.nz == 128 && d.nx % ZAvgCfg<S, R, 128>::TX == 0) || (d.nz == 256 && d.nx % ZAvgCfg<S, R, 256>::TX == 0) ||
-         (d.nz == 512 && d.nx % ZAvgCfg<S, R, 512>::TX == 0);
+bool zreg_takes(const Dims& d, int branches) {
+  // (in FP32 the length-2L transform of 64 points exchanges once too: 16.7 us against 18.8 on 64^3)
+  if (sizeof(R) == 4 && d.nz == 64 && branches == 2) return false;
+#define ZR(LL) (d.nx % (branches == 2 ? ZRegCfg<S, R, LL, 2>::TX : ZRegCfg<S, R, LL, 1>::TX) == 0)
+  return d.nz == 64 ? ZR(64) : d.nz == 128 ? ZR(128) : d.nz == 256 ? ZR(256) : d.nz == 512 ? ZR(512) : false;
+#undef ZR
 }
 
 template <typename S, typename R>
-cudaError_t launch_zavg(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz, void* out,
-                        const int* act, int* err, int sms, cudaStream_t st) {
+cudaError_t launch_zreg(const Dims& d, int branches, const void* in, const GreenParams& gp, const void* tw,
+                        const void* rz, void* out, const int* act, int* err, int sms, cudaStream_t st) {
+#define ZR(LL) (branches == 2 ? zreg_L<S, R, LL, 2>(d, in, gp, tw, rz, out, act, err, sms, st) \
+                              : zreg_L<S, R, LL, 1>(d, in, gp, tw, rz, out, act, err, sms, st))
   switch (d.nz) {
-    case 128: return zavg_L<S, R, 128>(d, in, gp, tw, rz, out, act, err, sms, st);
-    case 256: return zavg_L<S, R, 256>(d, in, gp, tw, rz, out, act, err, sms, st);
-    case 512: return zavg_L<S, R, 512>(d, in, gp, tw, rz, out, act, err, sms, st);
+    case 64: return ZR(64);
+    case 128: return ZR(128);
+    case 256: return ZR(256);
+    case 512: return ZR(512);
     default: return cudaErrorNotSupported;
   }
+#undef ZR
 }
 
 template <typename R>

@@ -331,33 +331,35 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
 }
 
 // ---------------------------------------------------------------------------
-// z pass of the averaged Green function (shift 1/4 on z) for L = 128, 256, 512: the two shifted branches run as two
-// transforms of length L on neighbouring lane groups, sixteen values a lane and component, so all three components of
-// a branch stay in registers from the forward transform through the Green product to the inverse one.  Branch s
+// z pass in sixteen values a lane and component, for L = 64, 128, 256, 512: all three components stay in registers
+// from the forward transform through the Green product to the inverse one.  BR = 2 is the averaged Green function
+// (shift 1/4 on z): the two shifted branches run as two transforms of length L on neighbouring lane groups; branch s
 // multiplies by exp(-/+ 2 pi i z/(4L)), and the groups add their results at the end (a shuffle; for L = 512, where a
-// branch fills a warp, through shared memory).
+// branch fills a warp, through shared memory).  BR = 1 is one branch with its ramp rz (none when z has no shift).
 //
 // What bounds it is shared memory: per value and branch one exchange (two at L = 512) each way, where the length-2L
-// transform in eight values a lane exchanges twice on twice the values.  192 of 255 registers hold the values, so an
-// SM has two CTAs of four warps; each has one tile, and one CTA's copies overlap the other's transforms.
+// transform in eight values a lane exchanges twice on twice the values.  In FP64 192 of 255 registers hold the values,
+// so an SM has eight warps, in CTAs of one tile each; one CTA's copies overlap the others' transforms.
 // ---------------------------------------------------------------------------
-template <typename S, typename R, int L>
-struct ZAvgCfg {
+template <typename S, typename R, int L, int BR>
+struct ZRegCfg {
   using T = cplx<R>;
   using TS = cplx<S>;
   using P = Plan16<L>;
-  static constexpr int W = 4, THREADS = 32 * W;
-  static constexpr int GROUPS = THREADS / (2 * P::TP);  // pencils in flight per CTA: 8, 4, 2
-  static constexpr int CTAS = sizeof(R) == 8 ? 2 : 4;   // per SM: 255 or 128 registers
-  // bytes of a tile row: whole rounds of pencils, and room for CTAS tiles on an SM
-  static constexpr int ROWB = sizeof(R) == 8 ? (L == 512 ? 32 : (L == 256 || sizeof(TS) == 8 ? 64 : 128))
-                                             : (L == 128 ? 64 : 32);
-  static constexpr int TX = ROWB / (int)sizeof(TS);     // pencils of a tile
+  static constexpr bool F64 = sizeof(R) == 8;
+  // bytes of a tile row: what lets a CTA's lane groups take whole rows, and the SM its CTAs
+  static constexpr int ROWB = L <= 128 ? (F64 && sizeof(TS) == 16 ? 128 : 64)
+                              : L == 256 ? (F64 || BR == 1 ? 64 : 32) : 32;
+  static constexpr int TX = ROWB / (int)sizeof(TS);  // pencils of a tile
+  static constexpr int WMAX = TX * BR * P::TP / 32;  // warps that one round of the tile keeps busy
+  static constexpr int W = WMAX < 4 ? WMAX : 4, THREADS = 32 * W;
+  static constexpr int GROUPS = THREADS / (BR * P::TP);  // pencils in flight
   static constexpr int ROUNDS = TX / GROUPS;
-  static_assert(TX % GROUPS == 0 && ROUNDS >= 1, "tile rows hold whole rounds");
-  static constexpr int BZ = L > 256 ? 256 : L;          // z extent of one copy
+  static constexpr int CTAS = (F64 ? 8 : 16) / W;  // per SM: 255 or 128 registers
+  static_assert(W >= 1 && TX % GROUPS == 0 && ROUNDS >= 1, "tile rows hold whole rounds");
+  static constexpr int BZ = L > 256 ? 256 : L;  // z extent of one copy
   static constexpr int TILE = 3 * L * ROWB;
-  static constexpr int EXB = 2 * GROUPS * P::STRIDE * (int)sizeof(T);
+  static constexpr int EXB = BR * GROUPS * P::STRIDE * (int)sizeof(T);
   using SM = TmaSmem<TILE, 1, EXB, 3 * L * (int)sizeof(T)>;
   // element (component 0, z = t < TP, pencil x) of the tile: rows of ROWB bytes, swizzled by the copy in 16-byte chunks
   static __device__ __forceinline__ unsigned char* at(unsigned char* tile, int t, int x) {
@@ -365,18 +367,22 @@ struct ZAvgCfg {
     const int sw = ROWB == 128 ? (t & 7) : ROWB == 64 ? ((t >> 1) & 3) : ((t >> 2) & 1);
     return tile + t * ROWB + (((byte >> 4) ^ sw) << 4) + (byte & 15);
   }
-  // byte offset of component c and z = t + e*TP from there (whole multiples of 8 rows, which the swizzle repeats over)
+  // at L = 64 (TP = 4) the rows t + 4e alternate between the halves of the swizzle's 8 rows: the odd ones have this
+  // bit of the address flipped
+  static constexpr int FLIP = P::TP == 4 ? ROWB / 2 : 0;
+  // byte offset of component c and z = t + e*TP from there (multiples of 8 rows, which the swizzle repeats over, but
+  // for FLIP)
   static constexpr int off(int c, int e) {
     return ((e * P::TP / BZ) * (3 * BZ) + c * BZ + (e * P::TP) % BZ) * ROWB;
   }
 };
 
-template <typename S, typename R, int L>
-__global__ void __launch_bounds__(128, ZAvgCfg<S, R, L>::CTAS)
-    k_zavg(Dims d, const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out, GreenParams gp,
+template <typename S, typename R, int L, int BR>
+__global__ void __launch_bounds__(ZRegCfg<S, R, L, BR>::THREADS, ZRegCfg<S, R, L, BR>::CTAS)
+    k_zreg(Dims d, const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out, GreenParams gp,
            const cplx<R>* __restrict__ twz, const cplx<R>* __restrict__ rz, const int* __restrict__ active,
            int* __restrict__ err) {
-  using C = ZAvgCfg<S, R, L>;
+  using C = ZRegCfg<S, R, L, BR>;
   using T = typename C::T;
   using TS = typename C::TS;
   using P_ = typename C::P;
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(128, ZAvgCfg<S, R, L>::CTAS)
   const long long per_rhs = (long long)xtiles * d.ny;
   const long long ntiles = per_rhs * d.nb;
   load_table(tw, twz, 2 * L);
-  load_table(rtab, rz, L);
+  if (rz) load_table(rtab, rz, L);
   if (threadIdx.x == 0) {
     mbar_init(full, 1);
     fence_barrier_init();
@@ -409,9 +415,9 @@ __global__ void __launch_bounds__(128, ZAvgCfg<S, R, L>::CTAS)
   };
   long long tile = next_active(blockIdx.x, ntiles, per_rhs, active);
   if (threadIdx.x == 0 && tile < ntiles) issue(tile);
-  // lane group of this thread: TP lanes of one branch of one pencil, the two branches of a pencil side by side
+  // lane group of this thread: TP lanes of one branch of one pencil, the branches of a pencil side by side
   const int grp = threadIdx.x / TP, t = threadIdx.x % TP;
-  const int br = grp & 1, pen = grp >> 1;
+  const int br = BR == 2 ? grp & 1 : 0, pen = grp / BR;
   const R sg = br ? R(-1) : R(1);
   T* sm = ex + grp * P_::STRIDE;
   uint32_t ph = 0;
@@ -426,16 +432,21 @@ __global__ void __launch_bounds__(128, ZAvgCfg<S, R, L>::CTAS)
 #pragma unroll 1
     for (int rd = 0; rd < C::ROUNDS; ++rd) {
       const int xl = rd * C::GROUPS + pen;
-      unsigned char* tp = C::at(tl, t, xl);
+      unsigned char* const tp0 = C::at(tl, t, xl);
+      unsigned char* const tp1 = tl + ((tp0 - tl) ^ C::FLIP);
       // one component at a time between synchronisations, so that only the transform in hand needs temporaries
       T v[3][16];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          T r = rtab[t + e * TP];
-          r.y *= sg;
-          v[c][e] = cmul(cv<T>(*reinterpret_cast<TS*>(tp + C::off(c, e))), r);
+          T a = cv<T>(*reinterpret_cast<TS*>((e & 1 ? tp1 : tp0) + C::off(c, e)));
+          if (BR == 2 || rz) {
+            T r = rtab[t + e * TP];
+            r.y *= sg;
+            a = cmul(a, r);
+          }
+          v[c][e] = a;
         }
         fft16_fwd<-1, P_>(v[c], sm, tw, t);
         __syncwarp();
@@ -449,33 +460,41 @@ __global__ void __launch_bounds__(128, ZAvgCfg<S, R, L>::CTAS)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         fft16_rev<+1, P_>(v[c], sm, twr, t);
+        if (BR == 2 || rz) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          T r = rtab[t + e * TP];
-          r.y *= -sg;
-          v[c][e] = cmul(v[c][e], r);
-        }
-        // sum of the branches: each group keeps half of the values and takes the partner's share of them.  By now both
-        // groups of the pencil have read the tile (the exchanges synchronise them), so the result may go into it.
-        if constexpr (TP < 32) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const T send = br ? v[c][e] : v[c][e + 8], keep = br ? v[c][e + 8] : v[c][e];
-            v[c][e] = mk(keep.x + __shfl_xor_sync(0xffffffffu, send.x, TP),
-                         keep.y + __shfl_xor_sync(0xffffffffu, send.y, TP));
+          for (int e = 0; e < 16; ++e) {
+            T r = rtab[t + e * TP];
+            r.y *= -sg;
+            v[c][e] = cmul(v[c][e], r);
           }
-        } else {
-          T* other = ex + (grp ^ 1) * P_::STRIDE;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) sm[t + 32 * e] = br ? v[c][e] : v[c][e + 8];
-          named_bar(1 + pen, 64);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[c][e] = cadd(br ? v[c][e + 8] : v[c][e], other[t + 32 * e]);
-          named_bar(1 + pen, 64);
         }
+        if constexpr (BR == 1) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          *reinterpret_cast<TS*>(tp + C::off(c, e) + br * (C::off(0, 8) - C::off(0, 0))) = cv<TS>(v[c][e]);
+          for (int e = 0; e < 16; ++e) *reinterpret_cast<TS*>((e & 1 ? tp1 : tp0) + C::off(c, e)) = cv<TS>(v[c][e]);
+        } else {
+          // sum of the branches: each group keeps half of the values and takes the partner's share of them.  By now
+          // both groups of the pencil have read the tile (the exchanges synchronise them): the result may go into it.
+          if constexpr (TP < 32) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const T send = br ? v[c][e] : v[c][e + 8], keep = br ? v[c][e + 8] : v[c][e];
+              v[c][e] = mk(keep.x + __shfl_xor_sync(0xffffffffu, send.x, TP),
+                           keep.y + __shfl_xor_sync(0xffffffffu, send.y, TP));
+            }
+          } else {
+            T* other = ex + (grp ^ 1) * P_::STRIDE;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sm[t + 32 * e] = br ? v[c][e] : v[c][e + 8];
+            named_bar(1 + pen, 64);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[c][e] = cadd(br ? v[c][e + 8] : v[c][e], other[t + 32 * e]);
+            named_bar(1 + pen, 64);
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            *reinterpret_cast<TS*>((e & 1 ? tp1 : tp0) + C::off(c, e) + br * (C::off(0, 8) - C::off(0, 0))) =
+                cv<TS>(v[c][e]);
+        }
         __syncwarp();
       }
     }

@@ -216,7 +216,7 @@ static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* 
     else return P->c64 ? launch_by<float, double>(d, dir, in, P->blue[1], ramp, out, act, P->st)
                        : launch_by<float, float>(d, dir, in, P->blue[1], ramp, out, act, P->st);
   }
-  if (P->use_tma && P->tma_y && !ramp) {
+  if (P->use_tma && P->tma_y) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
       e = launch_y_tma<double, double>(d, dir, in, tw, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
@@ -229,6 +229,23 @@ static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* 
   else return P->c64 ? launch_y<float, double>(d, dir, in, tw, ramp, out, act, P->st)
                      : launch_y<float, float>(d, dir, in, tw, ramp, out, act, P->st);
 }
+// the z pass in sixteen values a lane: whether this plan's shape has it, and the pass (launch_zreg)
+template <typename S>
+static bool has_zreg(const fm_plan* P, const Dims& d, int branches) {
+  if (!P->use_tma || !P->tma_z || P->blue[2].n) return false;
+  if constexpr (std::is_same<S, double>::value) return zreg_takes<double, double>(d, branches);
+  else return P->c64 ? zreg_takes<float, double>(d, branches) : zreg_takes<float, float>(d, branches);
+}
+template <typename S>
+static cudaError_t pass_zreg(const fm_plan* P, const Dims& d, int branches, const void* in, const GreenParams& gp,
+                             const void* rz, void* out, const int* act) {
+  int* err = (int*)P->errbuf.p;
+  const void* tw = P->twz16.p;
+  if constexpr (std::is_same<S, double>::value)
+    return launch_zreg<double, double>(d, branches, in, gp, tw, rz, out, act, err, P->sms, P->st);
+  else return P->c64 ? launch_zreg<float, double>(d, branches, in, gp, tw, rz, out, act, err, P->sms, P->st)
+                     : launch_zreg<float, float>(d, branches, in, gp, tw, rz, out, act, err, P->sms, P->st);
+}
 template <typename S>
 static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void* in, const GreenParams& gp,
                            const void* tw, const void* rz, void* out, const int* act) {
@@ -238,6 +255,7 @@ static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void
     else return P->c64 ? launch_bz<float, double>(d, mode, in, gp, P->blue[2], rz, out, act, P->st)
                        : launch_bz<float, float>(d, mode, in, gp, P->blue[2], rz, out, act, P->st);
   }
+  if (mode == ZMODE_ONE && !gp.accumulate && has_zreg<S>(P, d, 1)) return pass_zreg<S>(P, d, 1, in, gp, rz, out, act);
   if (P->use_tma && P->tma_z) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
@@ -250,23 +268,6 @@ static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void
   if constexpr (std::is_same<S, double>::value) return launch_zg<double, double>(d, mode, in, gp, tw, rz, out, act, P->st);
   else return P->c64 ? launch_zg<float, double>(d, mode, in, gp, tw, rz, out, act, P->st)
                      : launch_zg<float, float>(d, mode, in, gp, tw, rz, out, act, P->st);
-}
-// the z pass of a z-only average with both branches in one sweep: whether this plan's shape has it, and the pass
-template <typename S>
-static bool has_zavg(const fm_plan* P, const Dims& d) {
-  if (!P->use_tma || !P->tma_z || !(P->zonly || P->zsplit) || P->blue[2].n) return false;
-  if constexpr (std::is_same<S, double>::value) return zavg_takes<double, double>(d);
-  else return P->c64 ? zavg_takes<float, double>(d) : zavg_takes<float, float>(d);
-}
-template <typename S>
-static cudaError_t pass_zavg(const fm_plan* P, const Dims& d, const void* in, const GreenParams& gp, void* out,
-                             const int* act) {
-  const void* rz = P->zonly ? P->rz.p : P->rzp.p;
-  int* err = (int*)P->errbuf.p;
-  if constexpr (std::is_same<S, double>::value)
-    return launch_zavg<double, double>(d, in, gp, P->twz16.p, rz, out, act, err, P->sms, P->st);
-  else return P->c64 ? launch_zavg<float, double>(d, in, gp, P->twz16.p, rz, out, act, err, P->sms, P->st)
-                     : launch_zavg<float, float>(d, in, gp, P->twz16.p, rz, out, act, err, P->sms, P->st);
 }
 template <typename S>
 static cudaError_t pass_xi(const fm_plan* P, const Dims& d, int epi, const void* in, const void* V, const void* xv,
@@ -320,7 +321,7 @@ static fm_status init_tables(fm_plan* P) {
     BlueAxis& g = P->blue[a];
     g.n = t.n;
     g.m = t.m;
-    FM_CK(upload_cplx<R>(P->gtw[a], twiddles<R>(t.m), P->st));
+    FM_CK(upload_cplx<R>(P->gtw[a], t.m == 512 ? twiddles16(t.m) : twiddles<R>(t.m), P->st));
     g.tw = P->gtw[a].p;
     for (int dir = 0; dir < 2; ++dir) {
       FM_CK(upload_cplx<R>(P->gch[a][dir], t.chirp[dir], P->st));
@@ -329,7 +330,7 @@ static fm_status init_tables(fm_plan* P) {
       g.kern[dir] = P->gkn[a][dir].p;
     }
   }
-  if (P->zonly || P->zsplit) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
+  if (!P->blue[2].n) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
   if (P->zonly) {
     FM_CK(upload_cplx<R>(P->twz2, twiddles<R>(2 * P->dims.nz), P->st));
     FM_CK(upload_cplx<R>(P->rz, ramp(P->dims.nz, P->shift[2], -1.0), P->st));

@@ -60,9 +60,9 @@ inline std::vector<cd_t> twiddles(int L) {
 
 // the same pair for the plans of sixteen values a lane (Plan16); empty for other lengths
 inline std::vector<cd_t> twiddles16(int L) {
-  std::vector<int> r{16, L == 256 ? 16 : 8};
+  std::vector<int> r{16, L == 256 ? 16 : L == 64 ? 4 : 8};
   if (L == 512) r.push_back(4);
-  else if (L != 128 && L != 256) return {};
+  else if (L != 64 && L != 128 && L != 256) return {};
   std::vector<cd_t> t(2 * (size_t)L, cd_t(1.0, 0.0));
   stage_table(t, 0, r);
   std::vector<int> rr(r.rbegin(), r.rend());
