@@ -7,12 +7,15 @@
 // Fourier transform", 1970): with c_n = exp(DIR i pi n^2 / N),
 //    X_k = c_k * sum_n (x_n c_n) conj(c_{k-n}),
 // a circular convolution evaluated with a power-of-two FFT of length M >= 2N - 1.  N <= M/2, so the upper half of the
-// first transform's input is zero and the upper half of the second one's output is not needed.
+// first transform's input is zero and the upper half of the second one's output is not needed.  What stands between
+// the forward and the inverse transform of an axis is diagonal in k, and the two directions' c_k are conjugates of
+// modulus one, so the factor c_k of the forward result and c_k of the inverse input cancel: both are left out, and a
+// pass multiplies once, by c_n times the axis's ramp (forward) or the conjugate of that (inverse).
 //
-// About 160 FP64 instructions per value and transform at N = 201 (M = 512): bound by the FP64 pipe, not by HBM.  The
-// strided passes stage the tile of a CTA in shared memory so that global rows are read and written coalesced.
-// Measured on the 201 x 201 x 197 grid in FP64: one operator application 6.2 ms, against 14.8 ms as nine plain passes
-// per branch with strided accesses (prologue, three DFTs, Green, three DFTs, epilogue).
+// Bound by shared memory and the FP64 pipe (about 150 FP64 instructions per value and transform at N = 201, M = 512),
+// not by HBM.  The strided passes stage the tile of a CTA in shared memory so that global rows are read and written
+// coalesced.  Measured on the 201 x 201 x 197 grid in FP64: one operator application 5.4 ms, against 14.8 ms as nine
+// plain passes per branch with strided accesses (prologue, three DFTs, Green, three DFTs, epilogue).
 #pragma once
 #include "fm_passes.cuh"
 
@@ -22,8 +25,8 @@ namespace fm {
 struct BlueAxis {
   int n = 0;                  // axis length (0: the axis has fused passes)
   int m = 0;                  // FFT length, a power of two >= 2n - 1
-  const void* tw = nullptr;   // [forward-order | reversed-order] stage twiddles of length m (fm_tables.h)
-  const void* chirp[2] = {nullptr, nullptr};  // [forward, inverse]: n values c_k = exp(-/+ i pi k^2 / n)
+  const void* tw = nullptr;   // forward-order stage twiddles of length m (fm_tables.h)
+  const void* chirp = nullptr;                // n values c_k = exp(-i pi k^2 / n): the factor of an axis without a ramp
   const void* kern[2] = {nullptr, nullptr};   // [forward, inverse]: m values FFT_m(conj(c) wrapped) / m
 };
 
@@ -38,47 +41,52 @@ template <typename R> struct BluePlan<512, R> : Plan16<512> {
   static constexpr bool IS16 = true;
 };
 
-// One transform of a pencil: v[e] holds x_i at i = lay_idx<R0>(t, e) < N (zero elsewhere) and returns X_i there.
+// v from the layout of the last radix to the order of the elements (v[i] at t + TP*i), in which every plan here starts
+// (R0 = E): a renaming of registers, so the inverse transform runs the same radix order and table as the forward one.
 template <typename P_, typename T>
-__device__ __forceinline__ void blue_dft(T (&v)[P_::E], T* sm, const T* tw, const T* ch, const T* kk, int N, int t) {
-  constexpr int M = P_::L, E = P_::E, R0 = P_::R0;
+__device__ __forceinline__ void blue_order(T (&v)[P_::E]) {
+  static_assert(P_::R0 == P_::E, "the first radix takes all values of a lane");
+  constexpr int E = P_::E, RL = P_::RL;
+  T w[E];
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = lay_idx<M, E, R0>(t, e);
-    if (e % R0 < R0 / 2 && i < N) v[e] = cmul(v[e], ch[i]);
-  }
+  for (int e = 0; e < E; ++e) w[e / RL + (e % RL) * (E / RL)] = v[e];
+#pragma unroll
+  for (int e = 0; e < E; ++e) v[e] = w[e];
+}
+
+// The convolution of one pencil: v[i], i < E/2, holds x_n c_n at n = t + TP*i (zero from N on), and returns X_n / c_n.
+template <typename P_, typename T>
+__device__ __forceinline__ void blue_conv(T (&v)[P_::E], T* sm, const T* tw, const T* kk, int t) {
+  constexpr int E = P_::E, TP = P_::TP;
   if constexpr (P_::IS16) fft16_fwd<-1, P_, true>(v, sm, tw, t);
   else fft_fwd_plan<-1, P_, true>(v, sm, tw, t);
+  blue_order<P_>(v);
 #pragma unroll
-  for (int e = 0; e < E; ++e) v[e] = cmul(v[e], kk[lay_idx<M, E, P_::RL>(t, e)]);
+  for (int e = 0; e < E; ++e) v[e] = cmul(v[e], kk[t + TP * e]);
   __syncwarp();
-  if constexpr (P_::IS16) fft16_rev<+1, P_>(v, sm, tw + M, t);
-  else fft_rev_plan<+1, P_>(v, sm, tw + M, t);
+  if constexpr (P_::IS16) fft16_fwd<+1, P_>(v, sm, tw, t);
+  else fft_fwd_plan<+1, P_>(v, sm, tw, t);
+  blue_order<P_>(v);
   __syncwarp();
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int i = lay_idx<M, E, R0>(t, e);
-    if (e % R0 < R0 / 2 && i < N) v[e] = cmul(v[e], ch[i]);
-  }
 }
 
 // ---- x rows ------------------------------------------------------------------------------------------------------
-constexpr int BX_WARPS = 4;
+constexpr int BX_WARPS = 4;  // four CTAs an SM, 128 registers (k_bxi at 512 points: 591 us, 811 with 172 registers)
 
-// forward: out = DFT_x(in [.* V [* rs[b]]] [* rampx])   (PRO_COPY / PRO_V / PRO_V_SCALE as in k_xf)
+// forward: out = DFT_x(in [.* V [* rs[b]]] [* ramp]) / c_k   (PRO_COPY / PRO_V / PRO_V_SCALE as in k_xf); f: c_n [* ramp]
 template <typename S, typename R, int M>
-__global__ void __launch_bounds__(32 * BX_WARPS) k_bxf(Dims d, int pro, const cplx<S>* __restrict__ in,
+__global__ void __launch_bounds__(32 * BX_WARPS, 4) k_bxf(Dims d, int pro, const cplx<S>* __restrict__ in,
                                                        const cplx<S>* __restrict__ V,
                                                        const double* __restrict__ rhs_scale, BlueAxis ax,
-                                                       const cplx<R>* __restrict__ rampx, cplx<S>* __restrict__ out,
+                                                       const cplx<R>* __restrict__ f, cplx<S>* __restrict__ out,
                                                        const int* __restrict__ active, VecTab vt) {
   using T = cplx<R>;
   using P_ = BluePlan<M, R>;
-  constexpr int E = P_::E, TP = P_::TP, PW = 32 / TP, R0 = P_::R0;
+  constexpr int H = P_::E / 2, TP = P_::TP, PW = 32 / TP;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* tw = reinterpret_cast<T*>(smraw);
-  T* ex = tw + 2 * M;
-  load_table(tw, (const T*)ax.tw, 2 * M);
+  T* ex = tw + M;
+  load_table(tw, (const T*)ax.tw, M);
   __syncthreads();
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane / TP, t = lane % TP;
@@ -90,7 +98,6 @@ __global__ void __launch_bounds__(32 * BX_WARPS) k_bxf(Dims d, int pro, const cp
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * plane;
   T* sm = warp_smem<T, P_::STRIDE>(ex, wic, PW, p);
-  const T* ch = (const T*)ax.chirp[0];
   const T* kk = (const T*)ax.kern[0];
   const R s = pro == PRO_V_SCALE ? (R)rhs_scale[b] : R(1);
   const cplx<S>* inb = vt.in ? (const cplx<S>*)vt.in[b] : in + (long long)b * 3 * d.n;
@@ -99,43 +106,41 @@ __global__ void __launch_bounds__(32 * BX_WARPS) k_bxf(Dims d, int pro, const cp
   for (int c = 0; c < 3; ++c) {
     const long long base = ((long long)(c + 3 * b) * plane + yz) * N;
     const long long rbase = ((long long)c * plane + yz) * N;
-    T v[E];
+    T v[P_::E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int x = lay_idx<M, E, R0>(t, e);
+    for (int e = 0; e < H; ++e) {
+      const int x = t + TP * e;
       T a = czero<T>();
-      if (e % R0 < R0 / 2 && x < N) {
+      if (x < N) {
         a = cv<T>(inb[rbase + x]);
         if (pro != PRO_COPY) a = cmul(a, cv<T>(Vrow[x]));
         if (pro == PRO_V_SCALE) a = cscale(a, s);
-        if (rampx) a = cmul(a, rampx[x]);
+        a = cmul(a, f[x]);
       }
       v[e] = a;
     }
-    blue_dft<P_>(v, sm, tw, ch, kk, N, t);
+    blue_conv<P_>(v, sm, tw, kk, t);
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int x = lay_idx<M, E, R0>(t, e);
-      if (e % R0 < R0 / 2 && x < N) out[base + x] = cv<cplx<S>>(v[e]);
-    }
+    for (int e = 0; e < H; ++e)
+      if (t + TP * e < N) out[base + t + TP * e] = cv<cplx<S>>(v[e]);
   }
 }
 
-// inverse and epilogue: g = DFT_x^{-1}(in) [* conj(rampx)] [+ ep.gadd], then EPI (fm_passes.cuh, epi_element)
+// inverse and epilogue: g = DFT_x^{-1}(in c_k) [* conj(ramp)] [+ ep.gadd], then EPI (fm_passes.cuh, epi_element)
 template <typename S, typename R, int M, int EPI>
-__global__ void __launch_bounds__(32 * BX_WARPS) k_bxi(Dims d, const cplx<S>* __restrict__ in,
+__global__ void __launch_bounds__(32 * BX_WARPS, 4) k_bxi(Dims d, const cplx<S>* __restrict__ in,
                                                        const cplx<S>* __restrict__ V, const cplx<S>* __restrict__ xv,
                                                        const cplx<S>* __restrict__ bv,
                                                        const double* __restrict__ rhs_scale, EpiParams ep, BlueAxis ax,
-                                                       const cplx<R>* __restrict__ rampx, cplx<S>* __restrict__ out,
+                                                       const cplx<R>* __restrict__ f, cplx<S>* __restrict__ out,
                                                        const int* __restrict__ active, VecTab vt) {
   using T = cplx<R>;
   using P_ = BluePlan<M, R>;
-  constexpr int E = P_::E, TP = P_::TP, PW = 32 / TP, R0 = P_::R0;
+  constexpr int H = P_::E / 2, TP = P_::TP, PW = 32 / TP;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* tw = reinterpret_cast<T*>(smraw);
-  T* ex = tw + 2 * M;
-  load_table(tw, (const T*)ax.tw, 2 * M);
+  T* ex = tw + M;
+  load_table(tw, (const T*)ax.tw, M);
   __syncthreads();
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane / TP, t = lane % TP;
@@ -147,7 +152,6 @@ __global__ void __launch_bounds__(32 * BX_WARPS) k_bxi(Dims d, const cplx<S>* __
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * plane;
   T* sm = warp_smem<T, P_::STRIDE>(ex, wic, PW, p);
-  const T* ch = (const T*)ax.chirp[1];
   const T* kk = (const T*)ax.kern[1];
   const R ie = (EPI == EPI_PREC_OP || EPI == EPI_PREC_RES) ? (ep.inv_eps_b ? (R)ep.inv_eps_b[b] : (R)ep.inv_eps) : R(0);
   const T shf = (EPI == EPI_PREC_OP && ep.shift_b) ? mk((R)ep.shift_b[b].x, (R)ep.shift_b[b].y) : czero<T>();
@@ -161,20 +165,16 @@ __global__ void __launch_bounds__(32 * BX_WARPS) k_bxi(Dims d, const cplx<S>* __
   for (int c = 0; c < 3; ++c) {
     const long long base = ((long long)(c + 3 * b) * plane + yz) * N;
     const long long rbase = ((long long)c * plane + yz) * N;
-    T v[E];
+    T v[P_::E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int x = lay_idx<M, E, R0>(t, e);
-      v[e] = e % R0 < R0 / 2 && x < N ? cv<T>(in[base + x]) : czero<T>();
-    }
-    blue_dft<P_>(v, sm, tw, ch, kk, N, t);
+    for (int e = 0; e < H; ++e) v[e] = t + TP * e < N ? cv<T>(in[base + t + TP * e]) : czero<T>();
+    blue_conv<P_>(v, sm, tw, kk, t);
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int x = lay_idx<M, E, R0>(t, e);
-      if (e % R0 < R0 / 2 && x < N) {
+    for (int e = 0; e < H; ++e) {
+      const int x = t + TP * e;
+      if (x < N) {
         const long long ix = rbase + x;
-        T g = v[e];
-        if (rampx) g = cmul(g, cconj(rampx[x]));
+        T g = cmul(v[e], cconj(f[x]));
         if (ep.gadd) g = cadd(g, cv<T>(reinterpret_cast<const cplx<S>*>(ep.gadd)[(long long)b * 3 * d.n + ix]));
         outb[ix] = cv<cplx<S>>(epi_element<EPI, S, T, R>(g, ix, xvb, bvb, outb, Vrow + x, ie, s, al, be, ep, shf));
       }
@@ -183,121 +183,121 @@ __global__ void __launch_bounds__(32 * BX_WARPS) k_bxi(Dims d, const cplx<S>* __
 }
 
 // ---- y and z pencils ---------------------------------------------------------------------------------------------
-// A CTA takes XT x-consecutive pencils and stages them in shared memory in the arithmetic type (rows of XT values,
-// pencil slots swizzled with the row so that the lanes of a pencil, on consecutive rows, hit distinct banks).  Rows are
-// 128 bytes, and 64 at M = 512: there several CTAs of four warps share an SM, and one's loads overlap another's
-// transforms, where a CTA of eight would be alone (up to 166 KB of shared memory in the z pass).
-template <typename R, int M>
+// A CTA takes XT x-consecutive pencils and stages them in shared memory in the arithmetic type, pencil after pencil:
+// the lanes of a pencil read consecutive slots at constant offsets.  Global rows are 128 bytes; at M = 512 64 in the y
+// pass and 32 in the z pass, which holds three components: narrow tiles let several CTAs share an SM, and one's loads
+// overlap another's transforms (z pass of 201 x 201 x 197, one branch: 1558 us at 64 bytes, 1425 at 32 in FP64, 716 and
+// 628 in FP32; the rows that neighbouring CTAs split meet in L2).
+template <typename R, int M, bool Z>
 struct BlueTile {
   using T = cplx<R>;
   static constexpr int TP = BluePlan<M, R>::TP, PW = 32 / TP;
-  static constexpr int XT = (M == 512 ? 64 : 128) / (int)sizeof(T);
+  static constexpr int XT = (M < 512 ? 128 : Z ? 32 : 64) / (int)sizeof(T);
   static constexpr int W = XT / PW > 0 ? (XT / PW < 8 ? XT / PW : 8) : 1;
   static constexpr int ROUNDS = (XT + W * PW - 1) / (W * PW);
-  static constexpr int SH = XT * (int)sizeof(T) == 128 ? 0 : 1;
   static constexpr int STRIDE = BluePlan<M, R>::STRIDE;
-  __device__ static __forceinline__ int at(int r, int g) { return r * XT + (g ^ ((r >> SH) & (XT - 1))); }
-  static size_t smem(int n, int comps) {
-    return (size_t)(2 * M + W * PW * STRIDE + comps * n * XT) * sizeof(T);
+  // slots per pencil: a residue that puts the XT pencils of a wavefront's rows on disjoint slots in the copies
+  __host__ __device__ static constexpr int pencil(int rows) {
+    constexpr int units = 128 / (int)sizeof(T), want = units / XT > 0 ? units / XT : 1;
+    return rows + ((want - rows % units) % units + units) % units;
   }
+  static size_t smem(int rows) { return (size_t)(M + W * PW * STRIDE + XT * pencil(rows)) * sizeof(T); }
 };
 
+// DIR = -1: DFT_y(in * f) / c_k; +1: DFT_y^{-1}(in c_k) * conj(f); f: c_n [* ramp].  In place or not.
 template <typename S, typename R, int M, int DIR>
-__global__ void __launch_bounds__(32 * BlueTile<R, M>::W) k_by(Dims d, const cplx<S>* in, cplx<S>* out,
-                                                                      BlueAxis ax, const cplx<R>* __restrict__ rampy,
-                                                                      const int* __restrict__ active) {
+__global__ void __launch_bounds__(32 * BlueTile<R, M, false>::W) k_by(Dims d, const cplx<S>* in, cplx<S>* out, BlueAxis ax,
+                                                               const cplx<R>* __restrict__ f,
+                                                               const int* __restrict__ active) {
   using T = cplx<R>;
   using P_ = BluePlan<M, R>;
-  using C = BlueTile<R, M>;
-  constexpr int E = P_::E, TP = P_::TP, R0 = P_::R0, XT = C::XT;
+  using C = BlueTile<R, M, false>;
+  constexpr int H = P_::E / 2, TP = P_::TP, XT = C::XT;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* tw = reinterpret_cast<T*>(smraw);
-  T* ex = tw + 2 * M;
+  T* ex = tw + M;
   T* tile = ex + C::W * C::PW * C::STRIDE;
   const int xtiles = (d.nx + XT - 1) / XT;
   const int x0 = (int)(blockIdx.x % xtiles) * XT;
   const long long zcb = blockIdx.x / xtiles;  // z + nz*(c + 3b)
   const int b = (int)(zcb / (3LL * d.nz));
   if (active && !active[b]) return;
-  const int N = ax.n, w = min(XT, d.nx - x0);
+  const int N = ax.n, w = min(XT, d.nx - x0), PS = C::pencil(N);
   const long long base = zcb * (long long)N * d.nx + x0;
-  load_table(tw, (const T*)ax.tw, 2 * M);
+  load_table(tw, (const T*)ax.tw, M);
   for (int i = threadIdx.x; i < N * XT; i += blockDim.x) {
     const int g = i % XT, r = i / XT;
     T a = czero<T>();
     if (g < w) {
       a = cv<T>(in[base + (long long)r * d.nx + g]);
-      if (DIR < 0 && rampy) a = cmul(a, rampy[r]);
+      if (DIR < 0) a = cmul(a, f[r]);
     }
-    tile[C::at(r, g)] = a;
+    tile[g * PS + r] = a;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane / TP, t = lane % TP;
   T* sm = warp_smem<T, C::STRIDE>(ex, wic, C::PW, p);
-  const T* ch = (const T*)ax.chirp[DIR < 0 ? 0 : 1];
   const T* kk = (const T*)ax.kern[DIR < 0 ? 0 : 1];
 #pragma unroll 1
   for (int rd = 0; rd < C::ROUNDS; ++rd) {
-    const int g = (rd * C::W + wic) * C::PW + p;
-    T v[E];
+    T* pen = tile + ((rd * C::W + wic) * C::PW + p) * PS + t;
+    T v[P_::E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int y = lay_idx<M, E, R0>(t, e);
-      v[e] = e % R0 < R0 / 2 && y < N ? tile[C::at(y, g)] : czero<T>();
-    }
-    blue_dft<P_>(v, sm, tw, ch, kk, N, t);
+    for (int e = 0; e < H; ++e) v[e] = t + TP * e < N ? pen[TP * e] : czero<T>();
+    blue_conv<P_>(v, sm, tw, kk, t);
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int y = lay_idx<M, E, R0>(t, e);
-      if (e % R0 < R0 / 2 && y < N) tile[C::at(y, g)] = v[e];
-    }
+    for (int e = 0; e < H; ++e)
+      if (t + TP * e < N) pen[TP * e] = v[e];
   }
   __syncthreads();
   for (int i = threadIdx.x; i < N * XT; i += blockDim.x) {
     const int g = i % XT, r = i / XT;
     if (g < w) {
-      T a = tile[C::at(r, g)];
-      if (DIR > 0 && rampy) a = cmul(a, cconj(rampy[r]));
+      T a = tile[g * PS + r];
+      if (DIR > 0) a = cmul(a, cconj(f[r]));
       out[base + (long long)r * d.nx + g] = cv<cplx<S>>(a);
     }
   }
 }
 
 // z pass: forward DFT of the three components, the Green of one branch (ZMODE_ONE) or the curl (ZMODE_CURL) per bin,
-// inverse DFT; gp.accumulate adds the result to out.
+// inverse DFT; f: c_n [* the branch's ramp]; gp.accumulate adds the result to out.
 template <typename S, typename R, int M, int MODE>
-__global__ void __launch_bounds__(32 * BlueTile<R, M>::W) k_bz(Dims d, const cplx<S>* __restrict__ in,
-                                                                     GreenParams gp, BlueAxis ax,
-                                                                     const cplx<R>* __restrict__ rz,
-                                                                     cplx<S>* __restrict__ out,
-                                                                     const int* __restrict__ active) {
+__global__ void __launch_bounds__(32 * BlueTile<R, M, true>::W) k_bz(Dims d, const cplx<S>* __restrict__ in, GreenParams gp,
+                                                               BlueAxis ax, const cplx<R>* __restrict__ f,
+                                                               cplx<S>* __restrict__ out,
+                                                               const int* __restrict__ active) {
   using T = cplx<R>;
   using P_ = BluePlan<M, R>;
-  using C = BlueTile<R, M>;
-  constexpr int E = P_::E, TP = P_::TP, R0 = P_::R0, XT = C::XT;
+  using C = BlueTile<R, M, true>;
+  constexpr int H = P_::E / 2, TP = P_::TP, XT = C::XT;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* tw = reinterpret_cast<T*>(smraw);
-  T* ex = tw + 2 * M;
+  T* ex = tw + M;
   T* tile = ex + C::W * C::PW * C::STRIDE;
   const int xtiles = (d.nx + XT - 1) / XT;
   const int x0 = (int)(blockIdx.x % xtiles) * XT;
   const long long yb = blockIdx.x / xtiles;
   const int y = (int)(yb % d.ny), b = (int)(yb / d.ny);
   if (active && !active[b]) return;
-  const int N = ax.n, w = min(XT, d.nx - x0);
+  const int N = ax.n, w = min(XT, d.nx - x0), PS = C::pencil(3 * N);
   const long long plane = (long long)d.nx * d.ny;
   const long long base = (long long)b * 3 * d.n + (long long)y * d.nx + x0;
-  load_table(tw, (const T*)ax.tw, 2 * M);
-  for (int i = threadIdx.x; i < 3 * N * XT; i += blockDim.x) {
-    const int g = i % XT, r = i / XT, c = r / N, z = r - c * N;
-    T a = czero<T>();
-    if (g < w) {
-      a = cv<T>(in[base + (long long)r * plane + g]);  // components follow each other every N planes
-      if (MODE == ZMODE_ONE && rz) a = cmul(a, rz[z]);
+  load_table(tw, (const T*)ax.tw, M);
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c)
+#pragma unroll 4
+    for (int i = threadIdx.x; i < N * XT; i += blockDim.x) {
+      const int g = i % XT, z = i / XT;
+      T a = czero<T>();
+      if (g < w) {
+        const long long o = base + c * d.n + z * plane + g;
+        if (gp.accumulate) prefetch_l2(out + o);  // wanted after the transforms
+        a = cmul(cv<T>(in[o]), f[z]);
+      }
+      tile[g * PS + c * N + z] = a;
     }
-    tile[C::at(r, g)] = a;
-  }
   __syncthreads();
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane / TP, t = lane % TP;
@@ -306,24 +306,19 @@ __global__ void __launch_bounds__(32 * BlueTile<R, M>::W) k_bz(Dims d, const cpl
 #pragma unroll 1
   for (int rd = 0; rd < C::ROUNDS; ++rd) {
     const int g = (rd * C::W + wic) * C::PW + p, x = x0 + g;
+    T* pen = tile + g * PS + t;
 #pragma unroll 1
     for (int dir = 0; dir < 2; ++dir) {
-      const T* ch = (const T*)ax.chirp[dir];
       const T* kk = (const T*)ax.kern[dir];
 #pragma unroll 1
       for (int c = 0; c < 3; ++c) {
-        T v[E];
+        T v[P_::E];
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const int z = lay_idx<M, E, R0>(t, e);
-          v[e] = e % R0 < R0 / 2 && z < N ? tile[C::at(c * N + z, g)] : czero<T>();
-        }
-        blue_dft<P_>(v, sm, tw, ch, kk, N, t);
+        for (int e = 0; e < H; ++e) v[e] = t + TP * e < N ? pen[c * N + TP * e] : czero<T>();
+        blue_conv<P_>(v, sm, tw, kk, t);
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const int z = lay_idx<M, E, R0>(t, e);
-          if (e % R0 < R0 / 2 && z < N) tile[C::at(c * N + z, g)] = v[e];
-        }
+        for (int e = 0; e < H; ++e)
+          if (t + TP * e < N) pen[c * N + TP * e] = v[e];
       }
       __syncwarp();
       if (dir == 0) {
@@ -331,30 +326,29 @@ __global__ void __launch_bounds__(32 * BlueTile<R, M>::W) k_bz(Dims d, const cpl
                                         : (R)gp.dk[0] * (kidx_green<R>(x, d.nx) + (R)gp.shift[0]);
         const R ky = MODE == ZMODE_CURL ? (R)gp.dk[1] * kidx_curl<R>(y, d.ny)
                                         : (R)gp.dk[1] * (kidx_green<R>(y, d.ny) + (R)gp.shift[1]);
-        for (int k = t; k < N; k += TP) {
-          const R kz = MODE == ZMODE_CURL ? (R)gp.dk[2] * kidx_curl<R>(k, N)
-                                          : (R)gp.dk[2] * (kidx_green<R>(k, N) + (R)gp.shift[2]);
-          T& e1 = tile[C::at(k, g)];
-          T& e2 = tile[C::at(N + k, g)];
-          T& e3 = tile[C::at(2 * N + k, g)];
-          if constexpr (MODE == ZMODE_CURL) gb.curl(e1, e2, e3, kx, ky, kz);
-          else gb.green(e1, e2, e3, kx, ky, kz);
+        for (int k = 0; t + k < N; k += TP) {
+          const R kz = MODE == ZMODE_CURL ? (R)gp.dk[2] * kidx_curl<R>(t + k, N)
+                                          : (R)gp.dk[2] * (kidx_green<R>(t + k, N) + (R)gp.shift[2]);
+          if constexpr (MODE == ZMODE_CURL) gb.curl(pen[k], pen[N + k], pen[2 * N + k], kx, ky, kz);
+          else gb.green(pen[k], pen[N + k], pen[2 * N + k], kx, ky, kz);
         }
         __syncwarp();
       }
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 3 * N * XT; i += blockDim.x) {
-    const int g = i % XT, r = i / XT, z = r % N;
-    if (g < w) {
-      T a = tile[C::at(r, g)];
-      if (MODE == ZMODE_ONE && rz) a = cmul(a, cconj(rz[z]));
-      cplx<S>* o = out + base + (long long)r * plane + g;
-      if (gp.accumulate) a = cadd(a, cv<T>(*o));
-      *o = cv<cplx<S>>(a);
+#pragma unroll 1
+  for (int c = 0; c < 3; ++c)
+#pragma unroll 4
+    for (int i = threadIdx.x; i < N * XT; i += blockDim.x) {
+      const int g = i % XT, z = i / XT;
+      if (g < w) {
+        T a = cmul(tile[g * PS + c * N + z], cconj(f[z]));
+        cplx<S>* o = out + base + c * d.n + z * plane + g;
+        if (gp.accumulate) a = cadd(a, cv<T>(*o));
+        *o = cv<cplx<S>>(a);
+      }
     }
-  }
 }
 
 }  // namespace fm

@@ -19,7 +19,7 @@ inline int blue_fft_length(int n) {
   return m;
 }
 
-// FP64 host tables of one axis: the chirps and the transformed convolution kernels of both directions (BlueAxis).
+// FP64 host tables of one axis: the chirps of both directions and the transformed convolution kernels (BlueAxis).
 // The stage twiddles of length m: twiddles16(512), and by the arithmetic type's radix split below that,
 // twiddles<R>(m).
 struct BlueAxisTables {
@@ -28,19 +28,20 @@ struct BlueAxisTables {
 };
 BlueAxisTables blue_axis_tables(int n);
 
-// The same arguments as launch_xf, launch_xi, launch_y and launch_zg, with the axis tables in place of the twiddles.
+// The same arguments as launch_xf, launch_xi, launch_y and launch_zg, with the axis tables in place of the twiddles and
+// f = c_n [* ramp] in place of the ramp.
 template <typename S, typename R>
 cudaError_t launch_bxf(const Dims& d, int pro, const void* in, const void* V, const double* rs, const BlueAxis& ax,
-                       const void* ramp, void* out, const int* act, cudaStream_t st, VecTab vt);
+                       const void* f, void* out, const int* act, cudaStream_t st, VecTab vt);
 template <typename S, typename R>
 cudaError_t launch_bxi(const Dims& d, int epi, const void* in, const void* V, const void* xv, const void* bv,
-                       const double* rs, const EpiParams& ep, const BlueAxis& ax, const void* ramp, void* out,
+                       const double* rs, const EpiParams& ep, const BlueAxis& ax, const void* f, void* out,
                        const int* act, cudaStream_t st, VecTab vt);
 template <typename S, typename R>
-cudaError_t launch_by(const Dims& d, int dir, const void* in, const BlueAxis& ax, const void* ramp, void* out,
+cudaError_t launch_by(const Dims& d, int dir, const void* in, const BlueAxis& ax, const void* f, void* out,
                       const int* act, cudaStream_t st);
 template <typename S, typename R>
 cudaError_t launch_bz(const Dims& d, int mode, const void* in, const GreenParams& gp, const BlueAxis& ax,
-                      const void* rz, void* out, const int* act, cudaStream_t st);
+                      const void* f, void* out, const int* act, cudaStream_t st);
 
 }  // namespace fm

@@ -29,69 +29,69 @@ struct BlueRows {
     return (unsigned)(((long long)d.ny * d.nz * d.nb + BX_WARPS * PW - 1) / (BX_WARPS * PW));
   }
   static constexpr size_t smem =
-      (size_t)(2 * M + BX_WARPS * PW * BluePlan<M, R>::STRIDE) * sizeof(cplx<R>);
+      (size_t)(M + BX_WARPS * PW * BluePlan<M, R>::STRIDE) * sizeof(cplx<R>);
 };
 
 template <typename S, typename R, int M>
 static cudaError_t bxf_M(const Dims& d, int pro, const void* in, const void* V, const double* rs, const BlueAxis& ax,
-                         const void* ramp, void* out, const int* act, cudaStream_t st, VecTab vt) {
+                         const void* f, void* out, const int* act, cudaStream_t st, VecTab vt) {
   using C = BlueRows<R, M>;
   blue_allow_smem(k_bxf<S, R, M>, C::smem);
   k_bxf<S, R, M><<<C::blocks(d), 32 * BX_WARPS, C::smem, st>>>(d, pro, (const cplx<S>*)in, (const cplx<S>*)V, rs, ax,
-                                                               (const cplx<R>*)ramp, (cplx<S>*)out, act, vt);
+                                                               (const cplx<R>*)f, (cplx<S>*)out, act, vt);
   return cudaGetLastError();
 }
 
 template <typename S, typename R, int M, int EPI>
 static cudaError_t bxi_M(const Dims& d, const void* in, const void* V, const void* xv, const void* bv, const double* rs,
-                         const EpiParams& ep, const BlueAxis& ax, const void* ramp, void* out, const int* act,
+                         const EpiParams& ep, const BlueAxis& ax, const void* f, void* out, const int* act,
                          cudaStream_t st, VecTab vt) {
   using C = BlueRows<R, M>;
   using TS = cplx<S>;
   blue_allow_smem(k_bxi<S, R, M, EPI>, C::smem);
   k_bxi<S, R, M, EPI><<<C::blocks(d), 32 * BX_WARPS, C::smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv,
-                                                                    (const TS*)bv, rs, ep, ax, (const cplx<R>*)ramp,
+                                                                    (const TS*)bv, rs, ep, ax, (const cplx<R>*)f,
                                                                     (TS*)out, act, vt);
   return cudaGetLastError();
 }
 
 template <typename S, typename R, int M, int DIR>
-static cudaError_t by_M(const Dims& d, const void* in, const BlueAxis& ax, const void* ramp, void* out, const int* act,
+static cudaError_t by_M(const Dims& d, const void* in, const BlueAxis& ax, const void* f, void* out, const int* act,
                         cudaStream_t st) {
-  using C = BlueTile<R, M>;
-  const size_t smem = C::smem(ax.n, 1);
+  using C = BlueTile<R, M, false>;
+  const size_t smem = C::smem(ax.n);
   const unsigned blocks = (unsigned)((long long)((d.nx + C::XT - 1) / C::XT) * d.nz * 3 * d.nb);
   blue_allow_smem(k_by<S, R, M, DIR>, smem);
-  k_by<S, R, M, DIR><<<blocks, 32 * C::W, smem, st>>>(d, (const cplx<S>*)in, (cplx<S>*)out, ax, (const cplx<R>*)ramp,
+  k_by<S, R, M, DIR><<<blocks, 32 * C::W, smem, st>>>(d, (const cplx<S>*)in, (cplx<S>*)out, ax, (const cplx<R>*)f,
                                                       act);
   return cudaGetLastError();
 }
 
 template <typename S, typename R, int M, int MODE>
-static cudaError_t bz_M(const Dims& d, const void* in, const GreenParams& gp, const BlueAxis& ax, const void* rz,
+static cudaError_t bz_M(const Dims& d, const void* in, const GreenParams& gp, const BlueAxis& ax, const void* f,
                         void* out, const int* act, cudaStream_t st) {
-  using C = BlueTile<R, M>;
-  const size_t smem = C::smem(ax.n, 3);
+  using C = BlueTile<R, M, true>;
+  const size_t smem = C::smem(3 * ax.n);
   const unsigned blocks = (unsigned)((long long)((d.nx + C::XT - 1) / C::XT) * d.ny * d.nb);
   blue_allow_smem(k_bz<S, R, M, MODE>, smem);
-  k_bz<S, R, M, MODE><<<blocks, 32 * C::W, smem, st>>>(d, (const cplx<S>*)in, gp, ax, (const cplx<R>*)rz, (cplx<S>*)out,
+  k_bz<S, R, M, MODE><<<blocks, 32 * C::W, smem, st>>>(d, (const cplx<S>*)in, gp, ax, (const cplx<R>*)f, (cplx<S>*)out,
                                                        act);
   return cudaGetLastError();
 }
 
 template <typename S, typename R>
 cudaError_t launch_bxf(const Dims& d, int pro, const void* in, const void* V, const double* rs, const BlueAxis& ax,
-                       const void* ramp, void* out, const int* act, cudaStream_t st, VecTab vt) {
-#define BX(MM) bxf_M<S, R, MM>(d, pro, in, V, rs, ax, ramp, out, act, st, vt)
+                       const void* f, void* out, const int* act, cudaStream_t st, VecTab vt) {
+#define BX(MM) bxf_M<S, R, MM>(d, pro, in, V, rs, ax, f, out, act, st, vt)
   FM_BLUE_SWITCH(BX)
 #undef BX
 }
 
 template <typename S, typename R>
 cudaError_t launch_bxi(const Dims& d, int epi, const void* in, const void* V, const void* xv, const void* bv,
-                       const double* rs, const EpiParams& ep, const BlueAxis& ax, const void* ramp, void* out,
+                       const double* rs, const EpiParams& ep, const BlueAxis& ax, const void* f, void* out,
                        const int* act, cudaStream_t st, VecTab vt) {
-#define BI(MM, EE) bxi_M<S, R, MM, EE>(d, in, V, xv, bv, rs, ep, ax, ramp, out, act, st, vt)
+#define BI(MM, EE) bxi_M<S, R, MM, EE>(d, in, V, xv, bv, rs, ep, ax, f, out, act, st, vt)
 #define BI0(MM) BI(MM, EPI_STORE)
 #define BI1(MM) BI(MM, EPI_OP)
 #define BI2(MM) BI(MM, EPI_PREC_OP)
@@ -108,10 +108,10 @@ cudaError_t launch_bxi(const Dims& d, int epi, const void* in, const void* V, co
 }
 
 template <typename S, typename R>
-cudaError_t launch_by(const Dims& d, int dir, const void* in, const BlueAxis& ax, const void* ramp, void* out,
+cudaError_t launch_by(const Dims& d, int dir, const void* in, const BlueAxis& ax, const void* f, void* out,
                       const int* act, cudaStream_t st) {
-#define BYF(MM) by_M<S, R, MM, -1>(d, in, ax, ramp, out, act, st)
-#define BYI(MM) by_M<S, R, MM, +1>(d, in, ax, ramp, out, act, st)
+#define BYF(MM) by_M<S, R, MM, -1>(d, in, ax, f, out, act, st)
+#define BYI(MM) by_M<S, R, MM, +1>(d, in, ax, f, out, act, st)
   if (dir < 0) { FM_BLUE_SWITCH(BYF) }
   FM_BLUE_SWITCH(BYI)
 #undef BYF
@@ -120,9 +120,9 @@ cudaError_t launch_by(const Dims& d, int dir, const void* in, const BlueAxis& ax
 
 template <typename S, typename R>
 cudaError_t launch_bz(const Dims& d, int mode, const void* in, const GreenParams& gp, const BlueAxis& ax,
-                      const void* rz, void* out, const int* act, cudaStream_t st) {
-#define BZO(MM) bz_M<S, R, MM, ZMODE_ONE>(d, in, gp, ax, rz, out, act, st)
-#define BZC(MM) bz_M<S, R, MM, ZMODE_CURL>(d, in, gp, ax, rz, out, act, st)
+                      const void* f, void* out, const int* act, cudaStream_t st) {
+#define BZO(MM) bz_M<S, R, MM, ZMODE_ONE>(d, in, gp, ax, f, out, act, st)
+#define BZC(MM) bz_M<S, R, MM, ZMODE_CURL>(d, in, gp, ax, f, out, act, st)
   if (mode == ZMODE_ONE) { FM_BLUE_SWITCH(BZO) }
   if (mode == ZMODE_CURL) { FM_BLUE_SWITCH(BZC) }
   return cudaErrorInvalidValue;

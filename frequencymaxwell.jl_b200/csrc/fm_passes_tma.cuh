@@ -355,7 +355,7 @@ struct ZRegCfg {
   static constexpr int W = WMAX < 4 ? WMAX : 4, THREADS = 32 * W;
   static constexpr int GROUPS = THREADS / (BR * P::TP);  // pencils in flight
   static constexpr int ROUNDS = TX / GROUPS;
-  static constexpr int CTAS = (F64 ? 8 : 16) / W;  // per SM: 255 or 128 registers
+  static constexpr int CTAS = (F64 ? 8 : 12) / W;  // per SM: 255 or 168 registers
   static_assert(W >= 1 && TX % GROUPS == 0 && ROUNDS >= 1, "tile rows hold whole rounds");
   static constexpr int BZ = L > 256 ? 256 : L;  // z extent of one copy
   static constexpr int TILE = 3 * L * ROWB;

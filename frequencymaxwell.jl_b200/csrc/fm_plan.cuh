@@ -92,7 +92,7 @@ struct fm_plan {
   bool zonly = false;   // shifts only on z -> single pass with the length-2L transform
   bool zsplit = false;  // shifts only on z, padded z of a length the length-2L pass does not take: two z passes
   BlueAxis blue[3];     // axes without a fused pass (blue[a].n > 0): tables of their Bluestein passes (fm_generic.cuh)
-  DevBuf gtw[3], gch[3][2], gkn[3][2];
+  DevBuf gtw[3], gch[3], gkn[3][2];
   double shift[3] = {0, 0, 0};
   // potential / physics
   bool have_pot = false;
@@ -193,14 +193,16 @@ inline void tk_end(const Tk& t) {
 // ---------------------------------------------------------------------------
 // pass dispatch: storage type S, arithmetic double when the plan asks for it
 // ---------------------------------------------------------------------------
+// factor of a Bluestein axis: its chirp, which the ramp tables of such an axis hold already (init_tables)
+inline const void* blue_factor(const fm_plan* P, int axis, const void* ramp) { return ramp ? ramp : P->blue[axis].chirp; }
 template <typename S>
 static cudaError_t pass_xf(const fm_plan* P, const Dims& d, int pro, const void* in, const void* V, const double* rs,
                            const void* tw, const void* ramp, void* out, const int* act, VecTab vt = VecTab{}) {
   if (P->blue[0].n) {
     if constexpr (std::is_same<S, double>::value)
-      return launch_bxf<double, double>(d, pro, in, V, rs, P->blue[0], ramp, out, act, P->st, vt);
-    else return P->c64 ? launch_bxf<float, double>(d, pro, in, V, rs, P->blue[0], ramp, out, act, P->st, vt)
-                       : launch_bxf<float, float>(d, pro, in, V, rs, P->blue[0], ramp, out, act, P->st, vt);
+      return launch_bxf<double, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
+    else return P->c64 ? launch_bxf<float, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt)
+                       : launch_bxf<float, float>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
   }
   if constexpr (std::is_same<S, double>::value)
     return launch_xf<double, double>(d, pro, in, V, rs, tw, ramp, out, act, P->st, vt);
@@ -212,9 +214,9 @@ static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* 
                           void* out, const int* act) {
   if (P->blue[1].n) {
     if constexpr (std::is_same<S, double>::value)
-      return launch_by<double, double>(d, dir, in, P->blue[1], ramp, out, act, P->st);
-    else return P->c64 ? launch_by<float, double>(d, dir, in, P->blue[1], ramp, out, act, P->st)
-                       : launch_by<float, float>(d, dir, in, P->blue[1], ramp, out, act, P->st);
+      return launch_by<double, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
+    else return P->c64 ? launch_by<float, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st)
+                       : launch_by<float, float>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
   }
   if (P->use_tma && P->tma_y) {
     cudaError_t e;
@@ -251,9 +253,9 @@ static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void
                            const void* tw, const void* rz, void* out, const int* act) {
   if (P->blue[2].n) {
     if constexpr (std::is_same<S, double>::value)
-      return launch_bz<double, double>(d, mode, in, gp, P->blue[2], rz, out, act, P->st);
-    else return P->c64 ? launch_bz<float, double>(d, mode, in, gp, P->blue[2], rz, out, act, P->st)
-                       : launch_bz<float, float>(d, mode, in, gp, P->blue[2], rz, out, act, P->st);
+      return launch_bz<double, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
+    else return P->c64 ? launch_bz<float, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st)
+                       : launch_bz<float, float>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
   }
   if (mode == ZMODE_ONE && !gp.accumulate && has_zreg<S>(P, d, 1)) return pass_zreg<S>(P, d, 1, in, gp, rz, out, act);
   if (P->use_tma && P->tma_z) {
@@ -275,9 +277,9 @@ static cudaError_t pass_xi(const fm_plan* P, const Dims& d, int epi, const void*
                            void* out, const int* act, VecTab vt = VecTab{}) {
   if (P->blue[0].n) {
     if constexpr (std::is_same<S, double>::value)
-      return launch_bxi<double, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], ramp, out, act, P->st, vt);
-    else return P->c64 ? launch_bxi<float, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], ramp, out, act, P->st, vt)
-                       : launch_bxi<float, float>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], ramp, out, act, P->st, vt);
+      return launch_bxi<double, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
+    else return P->c64 ? launch_bxi<float, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt)
+                       : launch_bxi<float, float>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
   }
   if constexpr (std::is_same<S, double>::value)
     return launch_xi<double, double>(d, epi, in, V, xv, bv, rs, ep, tw, ramp, out, act, P->st, vt);
@@ -312,6 +314,7 @@ template <typename R>
 static fm_status init_tables(fm_plan* P) {
   const int n3[3] = {P->dims.nx, P->dims.ny, P->dims.nz};
   DevBuf* tw[3] = {&P->twx, &P->twy, &P->twz};
+  std::vector<cd> chirp[3];
   for (int a = 0; a < 3; ++a) {
     if (axis_supported(n3[a])) {
       FM_CK(upload_cplx<R>(*tw[a], twiddles<R>(n3[a]), P->st));
@@ -323,27 +326,34 @@ static fm_status init_tables(fm_plan* P) {
     g.m = t.m;
     FM_CK(upload_cplx<R>(P->gtw[a], t.m == 512 ? twiddles16(t.m) : twiddles<R>(t.m), P->st));
     g.tw = P->gtw[a].p;
+    FM_CK(upload_cplx<R>(P->gch[a], t.chirp[0], P->st));
+    g.chirp = P->gch[a].p;
+    chirp[a] = t.chirp[0];
     for (int dir = 0; dir < 2; ++dir) {
-      FM_CK(upload_cplx<R>(P->gch[a][dir], t.chirp[dir], P->st));
       FM_CK(upload_cplx<R>(P->gkn[a][dir], t.kern[dir], P->st));
-      g.chirp[dir] = P->gch[a][dir].p;
       g.kern[dir] = P->gkn[a][dir].p;
     }
   }
+  // ramps; on a Bluestein axis times its chirp
+  auto ramp = [&](int a, double sgn) {
+    std::vector<cd> r = fm::ramp(n3[a], P->shift[a], sgn);
+    for (size_t i = 0; i < chirp[a].size(); ++i) r[i] *= chirp[a][i];
+    return r;
+  };
   if (!P->blue[2].n) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
   if (P->zonly) {
     FM_CK(upload_cplx<R>(P->twz2, twiddles<R>(2 * P->dims.nz), P->st));
-    FM_CK(upload_cplx<R>(P->rz, ramp(P->dims.nz, P->shift[2], -1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rz, ramp(2, -1.0), P->st));
   } else if (P->zsplit) {
-    FM_CK(upload_cplx<R>(P->rzp, ramp(P->dims.nz, P->shift[2], -1.0), P->st));
-    FM_CK(upload_cplx<R>(P->rzm, ramp(P->dims.nz, P->shift[2], +1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rzp, ramp(2, -1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rzm, ramp(2, +1.0), P->st));
   } else if (P->avg) {
-    FM_CK(upload_cplx<R>(P->rxp, ramp(P->dims.nx, P->shift[0], -1.0), P->st));
-    FM_CK(upload_cplx<R>(P->rxm, ramp(P->dims.nx, P->shift[0], +1.0), P->st));
-    FM_CK(upload_cplx<R>(P->ryp, ramp(P->dims.ny, P->shift[1], -1.0), P->st));
-    FM_CK(upload_cplx<R>(P->rym, ramp(P->dims.ny, P->shift[1], +1.0), P->st));
-    FM_CK(upload_cplx<R>(P->rzp, ramp(P->dims.nz, P->shift[2], -1.0), P->st));
-    FM_CK(upload_cplx<R>(P->rzm, ramp(P->dims.nz, P->shift[2], +1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rxp, ramp(0, -1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rxm, ramp(0, +1.0), P->st));
+    FM_CK(upload_cplx<R>(P->ryp, ramp(1, -1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rym, ramp(1, +1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rzp, ramp(2, -1.0), P->st));
+    FM_CK(upload_cplx<R>(P->rzm, ramp(2, +1.0), P->st));
   }
   return FM_OK;
 }
