@@ -116,6 +116,38 @@ __device__ __forceinline__ double warp_transpose_sum(double (&v)[NV]) {
   return s;
 }
 
+// sums[o] = sum over the blocks of part[o*nblk + block], TB values per warp and turn: the partials come from L2, and a
+// few values at once keep more of them in flight (no branches between the loads: values past the end repeat the last).
+// A sweep over one right-hand side of 64^3 with 50 vectors takes 104.5 us, 109.0 with a value at a time (MGS, with the
+// same in the products by T, 129.2 and 135.0); few values do better with a warp each.
+template <int TB>
+__device__ __forceinline__ void gs_grid_sums(const double2* part, int n, int nblk, double2* sums) {
+  const int lane = threadIdx.x & 31;
+  for (int o0 = (threadIdx.x >> 5) * TB; o0 < n; o0 += KV_WARPS * TB) {
+    double2 s[TB];
+    const double2* p[TB];
+#pragma unroll
+    for (int q = 0; q < TB; ++q) {
+      s[q] = make_double2(0.0, 0.0);
+      p[q] = part + (size_t)min(o0 + q, n - 1) * nblk;
+    }
+#pragma unroll 2
+    for (int k = lane; k < nblk; k += 32) {
+#pragma unroll
+      for (int q = 0; q < TB; ++q) {
+        const double2 v = __ldcg(p[q] + k);
+        s[q].x += v.x;
+        s[q].y += v.y;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < TB; ++q) {
+      s[q] = warp_sum(s[q]);
+      if (lane == 0 && o0 + q < n) sums[o0 + q] = s[q];
+    }
+  }
+}
+
 // Modified Gram-Schmidt of the newest vector from one sweep of inner products.  MGS applies
 // (I - v_j v_j^H) ... (I - v_0 v_0^H) to w; its coefficients h solve (I + L) h = V^H w with the strictly lower
 // triangular L_ik = <v_i, v_k> (A. Bjorck, "Numerics of Gram-Schmidt orthogonalization", 1994, section 3; used for
@@ -241,21 +273,11 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // grid sums: a warp per value (fixed order, so the result does not depend on the schedule)
   double2* rs = reinterpret_cast<double2*>(&acc[0][0]);
-  for (int o = wi; o < NO; o += KV_WARPS) {
-    double2 s = make_double2(0.0, 0.0);
-    for (int k = lane; k < nblk; k += 32) {
-      const double2 v = __ldcg(&part[((size_t)b * NO + o) * nblk + k]);
-      s.x += v.x;
-      s.y += v.y;
-    }
-    s = warp_sum(s);
-    if (lane == 0) {
-      if constexpr (MGS) rs[o] = s;
-      else out[(size_t)b * NO + o] = s;
-    }
-  }
+  // (fixed order, so the result does not depend on the schedule)
+  double2* const sums = MGS ? rs : out + (size_t)b * NO;
+  if (NO > 2 * KV_WARPS) gs_grid_sums<4>(part + (size_t)b * NO * nblk, NO, nblk, sums);
+  else gs_grid_sums<1>(part + (size_t)b * NO * nblk, NO, nblk, sums);
   if (threadIdx.x == 0) counter[b] = 0;
   if constexpr (MGS) {
     // rs[2m] = <U_m, w>, rs[2m+1] = <U_m, U_j>, j = K - 1.  L_jm = <v_j, v_m>;  T_j = e_j - L_j T;  h = T V^H w.
@@ -279,7 +301,7 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int
       const int k = threadIdx.x & (KV_KMAX - 1), half = threadIdx.x / KV_KMAX;
       double2 s = make_double2(0.0, 0.0);
       if (k < j) {
-#pragma unroll 4
+#pragma unroll 8
         for (int m = k + half; m < j; m += 2) {
           const double2 l = rs[m], t = __ldcg(&Tb[(size_t)m * KV_KMAX + k]);
           s.x = fma(-l.x, t.x, fma(l.y, t.y, s.x));
@@ -297,15 +319,29 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int
       Tb[(size_t)j * KV_KMAX + threadIdx.x] = t;
     }
     __syncthreads();
-    for (int i = wi; i < K; i += KV_WARPS) {
-      double2 s = make_double2(0.0, 0.0);
-      for (int k = lane; k <= i; k += 32) {
-        const double2 t = i == j ? trow[0][k] : __ldcg(&Tb[(size_t)i * KV_KMAX + k]);
-        s.x = fma(t.x, r[k].x, fma(-t.y, r[k].y, s.x));
-        s.y = fma(t.x, r[k].y, fma(t.y, r[k].x, s.y));
+    constexpr int TB = 4;
+    for (int i0 = wi * TB; i0 < K; i0 += KV_WARPS * TB) {
+      double2 s[TB];
+#pragma unroll
+      for (int q = 0; q < TB; ++q) s[q] = make_double2(0.0, 0.0);
+      for (int k = lane; k < min(K, i0 + TB); k += 32) {
+        double2 t[TB];
+#pragma unroll
+        for (int q = 0; q < TB; ++q) t[q] = __ldcg(&Tb[(size_t)min(i0 + q, max(j - 1, 0)) * KV_KMAX + k]);
+        const double2 rk = r[k], tj = trow[0][k];
+#pragma unroll
+        for (int q = 0; q < TB; ++q) {
+          if (i0 + q == j) t[q] = tj;
+          if (k > i0 + q) t[q] = make_double2(0.0, 0.0);  // T is lower triangular
+          s[q].x = fma(t[q].x, rk.x, fma(-t[q].y, rk.y, s[q].x));
+          s[q].y = fma(t[q].x, rk.y, fma(t[q].y, rk.x, s[q].y));
+        }
       }
-      s = warp_sum(s);
-      if (lane == 0) mt.h[(size_t)b * mt.hs + i] = s;
+#pragma unroll
+      for (int q = 0; q < TB; ++q) {
+        s[q] = warp_sum(s[q]);
+        if (lane == 0 && i0 + q < K) mt.h[(size_t)b * mt.hs + i0 + q] = s[q];
+      }
     }
   }
 }
