@@ -190,7 +190,7 @@ void fm_plan_destroy(fm_plan* P) {
   if (!P) return;
   cudaSetDevice(P->desc.device);
   if (P->st) cudaStreamSynchronize(P->st);
-  DevBuf* bufs[] = {&P->twx, &P->twy, &P->twz, &P->twz2, &P->twz16, &P->rz, &P->rxp, &P->rxm, &P->ryp, &P->rym, &P->rzp,
+  DevBuf* bufs[] = {&P->twx, &P->twy, &P->twz, &P->twz2, &P->twz16, &P->twyt, &P->rz, &P->rxp, &P->rxm, &P->ryp, &P->rym, &P->rzp,
                     &P->rzm, &P->V, &P->t1, &P->t2, &P->t3, &P->bbuf, &P->xbuf, &P->ebuf, &P->sbuf, &P->basis,
                     &P->gbuf2, &P->red_part, &P->red_out, &P->red_cnt, &P->active, &P->scale, &P->coef,
                     &P->hbuf, &P->mgsT, &P->eps_dev, &P->fx, &P->fy, &P->fz, &P->maxpart, &P->maxout, &P->wt_x,

@@ -456,4 +456,25 @@ __device__ __forceinline__ void fft16_rev(T (&v)[16], T* sm, const T* tw_rev, in
   else fft16_run<DIR, P::L, P::R2, P::R1, P::R0>(v, sm, tw_rev, t);
 }
 
+// ---- plans of the x rows and of the y tiles: in FP64 sixteen values a lane at 512 points, and in the y tiles at 256
+// (k_y_tma 256^3, FP32 storage, 64-byte rows: 220 us with eight values, 191 with sixteen; the x rows, whose CTAs hold no
+// tile, run faster with eight values and more warps: k_xf 223 against 240, k_xi 331 against 374).  Plan elsewhere. ----
+template <int L, typename R> struct RowPlan : Plan<L, R> {
+  static constexpr bool IS16 = false;
+  static constexpr int STRIDE = PencilStride<L, typename CT<R>::T, Plan<L, R>::TP, true>::v;
+};
+template <> struct RowPlan<512, double> : Plan16<512> { static constexpr bool IS16 = true; };
+template <int L, typename R> struct YTilePlan : RowPlan<L, R> {};
+template <> struct YTilePlan<256, double> : Plan16<256> { static constexpr bool IS16 = true; };
+template <int DIR, typename P, typename T>
+__device__ __forceinline__ void long_fwd(T (&v)[P::E], T* sm, const T* tw_fwd, int t) {
+  if constexpr (P::IS16) fft16_fwd<DIR, P>(v, sm, tw_fwd, t);
+  else fft_fwd_plan<DIR, P>(v, sm, tw_fwd, t);
+}
+template <int DIR, typename P, typename T>
+__device__ __forceinline__ void long_rev(T (&v)[P::E], T* sm, const T* tw_rev, int t) {
+  if constexpr (P::IS16) fft16_rev<DIR, P>(v, sm, tw_rev, t);
+  else fft_rev_plan<DIR, P>(v, sm, tw_rev, t);
+}
+
 }  // namespace fm

@@ -20,13 +20,13 @@ static cudaError_t xf_L(const Dims& d, const void* in, const void* V, const doub
                         void* out, const int* act, cudaStream_t st, const VecTab& vt) {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P_ = Plan<L, R>;
+  using P_ = RowPlan<L, R>;
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
   const long long rows = (long long)d.ny * d.nz * d.nb;
   const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
-  const size_t smem = (size_t)(L + W * PW * PencilStride<L, T, P_::TP, true>::v) * sizeof(T);
+  const size_t smem = (size_t)(L + W * PW * P_::STRIDE) * sizeof(T);
   allow_smem(k_xf<S, R, L, PRO>, smem);
   k_xf<S, R, L, PRO><<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, rs, (const T*)tw,
                                                          (const T*)ramp, (TS*)out, act, vt);
@@ -39,13 +39,13 @@ static cudaError_t xi_L(const Dims& d, const void* in, const void* V, const void
                         cudaStream_t st, const VecTab& vt) {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P_ = Plan<L, R>;
+  using P_ = RowPlan<L, R>;
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
   const long long rows = (long long)d.ny * d.nz * d.nb;
   const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
-  const size_t smem = (size_t)(L + W * PW * PencilStride<L, T, P_::TP, true>::v) * sizeof(T);
+  const size_t smem = (size_t)(L + W * PW * P_::STRIDE) * sizeof(T);
   allow_smem(k_xi<S, R, L, EPI>, smem);
   k_xi<S, R, L, EPI><<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv, (const TS*)bv,
                                                          rs, ep, (const T*)tw, (const T*)ramp, (TS*)out, act, vt);
@@ -57,13 +57,13 @@ static cudaError_t xi_xf_L(const Dims& d, const void* in, const void* V, const v
                            const void* tw, void* out, void* out2, const int* act, cudaStream_t st) {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P_ = Plan<L, R>;
+  using P_ = RowPlan<L, R>;
   constexpr int PW = 32 / P_::TP;
   const int W = row_threads(d) / 32;
   const long long rows = (long long)d.ny * d.nz * d.nb;
   const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
-  const size_t smem = (size_t)(2 * L + W * PW * PencilStride<L, T, P_::TP, true>::v) * sizeof(T);
+  const size_t smem = (size_t)(2 * L + W * PW * P_::STRIDE) * sizeof(T);
   allow_smem(k_xi_xf<S, R, L>, smem);
   k_xi_xf<S, R, L><<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv, ep, (const T*)tw,
                                                  (TS*)out, (TS*)out2, act);

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cpl
                                             const int* __restrict__ active, VecTab vt) {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P_ = Plan<L, R>;
+  using P_ = RowPlan<L, R>;
   constexpr int E = P_::E, TP = P_::TP, PW = 32 / TP;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* tw = reinterpret_cast<T*>(smraw);
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cpl
   const int b = (int)(row / ((long long)d.ny * d.nz));
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * d.ny * d.nz;
-  T* sm = warp_smem<T, PencilStride<L, T, TP, true>::v>(ex, wic, PW, p);
+  T* sm = warp_smem<T, P_::STRIDE>(ex, wic, PW, p);
   // V is held across the three components, except at the long lengths: there the registers it would take decide how
   // many CTAs fit on an SM, and it is read per component (an L1 hit after the first)
   constexpr bool HOLD = PRO != PRO_COPY && L <= 128;
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cpl
       v[e] = a;
     }
     if (ahead && c < 2) prefetch_row<TP>(inb + rbase + (long long)d.ny * d.nz * L, L, t);
-    fft_fwd_plan<-1, P_>(v, sm, tw, t);
+    long_fwd<-1, P_>(v, sm, tw, t);
 #pragma unroll
     for (int e = 0; e < E; ++e) out[base + lay_idx<L, E, P_::RL>(t, e)] = cv<TS>(v[e]);
     __syncwarp();
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cpl
                                             cplx<S>* __restrict__ out, const int* __restrict__ active, VecTab vt) {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P_ = Plan<L, R>;
+  using P_ = RowPlan<L, R>;
   constexpr int E = P_::E, TP = P_::TP, PW = 32 / TP;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* tw = reinterpret_cast<T*>(smraw);
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cpl
   const int b = (int)(row / ((long long)d.ny * d.nz));
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * d.ny * d.nz;
-  T* sm = warp_smem<T, PencilStride<L, T, TP, true>::v>(ex, wic, PW, p);
+  T* sm = warp_smem<T, P_::STRIDE>(ex, wic, PW, p);
   // (i/eps) V is formed per component from V (an L1 hit after the first component) rather than held across
   // the three components: the registers it would take decide how many CTAs fit on an SM
   const R ie = (EPI == EPI_PREC_OP || EPI == EPI_PREC_RES) ? (ep.inv_eps_b ? (R)ep.inv_eps_b[b] : (R)ep.inv_eps) : R(0);
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cpl
       if ((EPI == EPI_PREC_OP || EPI == EPI_PREC_RES) && c == 0) prefetch_row<TP>(Vrow, L, t);
       if (c < 2) prefetch_row<TP>(in + base + cstride, L, t);
     }
-    fft_rev_plan<+1, P_>(v, sm, tw, t);
+    long_rev<+1, P_>(v, sm, tw, t);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int x = lay_idx<L, E, P_::R0>(t, e);
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
                                                                           const int* __restrict__ active) {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P_ = Plan<L, R>;
+  using P_ = RowPlan<L, R>;
   constexpr int E = P_::E, TP = P_::TP, PW = 32 / TP;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* twf = reinterpret_cast<T*>(smraw);  // forward-order stage twiddles
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
   const int b = (int)(row / ((long long)d.ny * d.nz));
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * d.ny * d.nz;
-  T* sm = warp_smem<T, PencilStride<L, T, TP, true>::v>(ex, wic, PW, p);
+  T* sm = warp_smem<T, P_::STRIDE>(ex, wic, PW, p);
   const R ie = ep.inv_eps_b ? (R)ep.inv_eps_b[b] : (R)ep.inv_eps;
   const cplx<S>* Vrow = V + b * d.vstride + yz * L;
   const T shf = ep.shift_b ? mk((R)ep.shift_b[b].x, (R)ep.shift_b[b].y) : czero<T>();
@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
       if (c == 0) prefetch_row<TP>(Vrow, L, t);
       if (c < 2) prefetch_row<TP>(in + base + cstride, L, t);
     }
-    fft_rev_plan<+1, P_>(v, sm, twr, t);
+    long_rev<+1, P_>(v, sm, twr, t);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int x = lay_idx<L, E, P_::R0>(t, e);
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
       v[e] = cmul(cv<T>(rs), cv<T>(Vrow[x]));  // PRO_V of the next application on the stored value
     }
     __syncwarp();
-    fft_fwd_plan<-1, P_>(v, sm, twf, t);
+    long_fwd<-1, P_>(v, sm, twf, t);
 #pragma unroll
     for (int e = 0; e < E; ++e) out2[base + lay_idx<L, E, P_::RL>(t, e)] = cv<TS>(v[e]);
     __syncwarp();

@@ -29,15 +29,17 @@ template <typename S, typename R, int L>
 struct YTmaCfg {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P = Plan<L, R>;
-  static constexpr int ROWB = L == 512 ? 64 : 128;  // bytes of a tile row
+  using P = YTilePlan<L, R>;
+  // bytes of a tile row: at 256 points and FP32 storage 64-byte rows run four CTAs an SM (4.2 TB/s, 3.8 with 128), in
+  // FP64 storage whole lines are better (5.9, 5.2 with 64)
+  static constexpr int ROWB = L == 512 || (L == 256 && sizeof(S) == 4) ? 64 : 128;
   static constexpr int TX = ROWB / (int)sizeof(TS);
   static constexpr int PW = 32 / P::TP;
   static constexpr int CW = (TX / PW) < 4 ? (TX / PW) : 4;
   static constexpr int ROUNDS = TX / (CW * PW);
   static constexpr int TILE = L * ROWB;
   static constexpr int NST = L <= 128 ? 3 : 2;  // three stages leave room for three CTAs per SM
-  static constexpr int STRIDE = PencilStride<L, T, P::TP, true>::v;
+  static constexpr int STRIDE = P::STRIDE;
   using SM = TmaSmem<TILE, NST, CW * PW * STRIDE * (int)sizeof(T), L * (int)sizeof(T)>;
   static constexpr int THREADS = CW * 32;
 };
@@ -118,14 +120,14 @@ __global__ void __launch_bounds__(YTmaCfg<S, R, L>::THREADS)
           if (rampy) a = cmul(a, rampy[y]);
           v[e] = a;
         }
-        fft_fwd_plan<-1, P_>(v, sm, tw, t);
+        long_fwd<-1, P_>(v, sm, tw, t);
         __syncwarp();
 #pragma unroll
         for (int e = 0; e < E; ++e) *tile_at<TS, C::ROWB>(tl, lay_idx<L, E, P_::RL>(t, e), xl) = cv<TS>(v[e]);
       } else {
 #pragma unroll
         for (int e = 0; e < E; ++e) v[e] = cv<T>(*tile_at<TS, C::ROWB>(tl, lay_idx<L, E, P_::RL>(t, e), xl));
-        fft_rev_plan<+1, P_>(v, sm, tw, t);
+        long_rev<+1, P_>(v, sm, tw, t);
         __syncwarp();
 #pragma unroll
         for (int e = 0; e < E; ++e) {

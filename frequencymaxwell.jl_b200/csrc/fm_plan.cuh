@@ -99,7 +99,7 @@ struct fm_plan {
   double k_bg = 0, eps_imag = 0, wavelength = 0, kref2 = 1;
   int bornmax = 0;
   // tables (plan precision)
-  DevBuf twx, twy, twz, twz2, twz16, rz, rxp, rxm, ryp, rym, rzp, rzm;
+  DevBuf twx, twy, twz, twz2, twz16, twyt, rz, rxp, rxm, ryp, rym, rzp, rzm;
   DevBuf V;
   // workspace
   DevBuf t1, t2, t3, bbuf, xbuf, ebuf, sbuf, basis, gbuf2;  // t3: first branch of a two-branch average
@@ -221,10 +221,10 @@ static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* 
   if (P->use_tma && P->tma_y) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
-      e = launch_y_tma<double, double>(d, dir, in, tw, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
+      e = launch_y_tma<double, double>(d, dir, in, P->twyt.p, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
     else
-      e = P->c64 ? launch_y_tma<float, double>(d, dir, in, tw, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st)
-                 : launch_y_tma<float, float>(d, dir, in, tw, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
+      e = P->c64 ? launch_y_tma<float, double>(d, dir, in, P->twyt.p, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st)
+                 : launch_y_tma<float, float>(d, dir, in, P->twyt.p, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
     if (e != cudaErrorNotSupported) return e;
   }
   if constexpr (std::is_same<S, double>::value) return launch_y<double, double>(d, dir, in, tw, ramp, out, act, P->st);
@@ -318,6 +318,7 @@ static fm_status init_tables(fm_plan* P) {
   for (int a = 0; a < 3; ++a) {
     if (axis_supported(n3[a])) {
       FM_CK(upload_cplx<R>(*tw[a], twiddles<R>(n3[a]), P->st));
+      if (a == 1) FM_CK(upload_cplx<R>(P->twyt, ytile_twiddles<R>(n3[a]), P->st));
       continue;
     }
     const BlueAxisTables t = blue_axis_tables(n3[a]);

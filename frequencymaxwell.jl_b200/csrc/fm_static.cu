@@ -103,7 +103,7 @@ fm_status run(const fm_plan_desc& dsc, double k_bg, double eps_imag, int nrhs, c
   // tables (FP64 on the host, cast to the arithmetic type)
   if ((e = cudaMemsetAsync(err, 0, sizeof(int), st)) != cudaSuccess ||
       (e = put_table<CR>(sc + o_tx, twiddles<R>(n3[0]), st)) != cudaSuccess ||
-      (e = put_table<CR>(sc + o_ty, twiddles<R>(n3[1]), st)) != cudaSuccess ||
+      (e = put_table<CR>(sc + o_ty, ytile_twiddles<R>(n3[1]), st)) != cudaSuccess ||
       (e = put_table<CR>(sc + o_tz, twiddles<R>(lz), st)) != cudaSuccess ||
       (e = put_table<CR>(sc + o_rz, ramp(n3[2], zonly ? 0.25 : 0.0, -1.0), st)) != cudaSuccess)
     return noalloc_fail(FM_ERR_CUDA, std::string("table upload: ") + cudaGetErrorString(e));

@@ -70,6 +70,12 @@ inline std::vector<cd_t> twiddles16(int L) {
   return t;
 }
 
+// the pair for the y tiles (YTilePlan)
+template <typename R>
+inline std::vector<cd_t> ytile_twiddles(int L) {
+  return std::is_same<R, double>::value && L == 256 ? twiddles16(L) : twiddles<R>(L);  // (512: the radices agree)
+}
+
 // exp(sgn * 2 pi i * idx * s / L)
 inline std::vector<cd_t> ramp(int L, double s, double sgn) {
   std::vector<cd_t> t(L);
