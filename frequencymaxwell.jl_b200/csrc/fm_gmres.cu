@@ -158,13 +158,37 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
                           P->st));
     return FM_OK;
   };
-  // r0 = M^{-1}(b - A x) into U[0]
-  auto residual_into_U0 = [&](const int* a) -> fm_status {
-    return green_op<R>(P, nb, P->xbuf.p, PRO_V, nullptr, EPI_PREC_RES, P->xbuf.p, P->bbuf.p, ep, U, a);
+  // r0 = M^{-1}(b - A x) into U[0].  At a restart of the FP32-storage form with FP64 arithmetic the passes run on FP64
+  // copies, which the dead basis vectors U[1..mem] hold: an error of this residual is one of the right-hand side that no
+  // later cycle sees, and rounding its four pass temporaries to FP32 was most of the error of the fields (64-bit study,
+  // 512 x 64 x 512, GMRES(20): fields off by 6.3e-6 with it, 1.8e-6 without).  It costs three FP32 applications per cycle.
+  const size_t widef = (2 * fbytes + 255) / 256 * 256;  // one FP64 field of the batch
+  const bool branches = P->avg && !P->zonly && !P->zsplit;
+  const bool wide = P->c64 && sizeof(T) == 8 &&
+                    (branches ? 5 : 4) * widef + (size_t)P->n * sizeof(double2) + 256 <= (size_t)mem * fbytes;
+  auto residual_into_U0 = [&](const int* a, bool restart) -> fm_status {
+    if (!wide || !restart)
+      return green_op<R>(P, nb, P->xbuf.p, PRO_V, nullptr, EPI_PREC_RES, P->xbuf.p, P->bbuf.p, ep, U, a);
+    char* w = (char*)(((uintptr_t)(U + nb * fe) + 255) & ~(uintptr_t)255);
+    void *x = w, *b = w + widef;
+    RhsCtx rc;
+    for (int i = 0; i < (branches ? 3 : 2); ++i) rc.tmp[i] = w + (2 + i) * widef;
+    double2* V = (double2*)(w + (branches ? 5 : 4) * widef);
+    rc.V = V;
+    const double cb = (double)fbytes * 3;
+    FM_TRACK(P, KC_SETUP, (double)P->n * 24, (k_to_f64<R><<<8 * P->sms, 256, 0, P->st>>>(P->n, (const T*)P->V.p, 1.0, V)));
+    FM_TRACK(P, KC_SETUP, cb, (k_to_f64<R><<<8 * P->sms, 256, 0, P->st>>>(nb * P->M, (const T*)P->xbuf.p, 1.0, (double2*)x)));
+    FM_TRACK(P, KC_SETUP, cb, (k_to_f64<R><<<8 * P->sms, 256, 0, P->st>>>(nb * P->M, (const T*)P->bbuf.p, 1.0, (double2*)b)));
+    FM_CK(cudaGetLastError());
+    // the last pass reads tmp[1] and may write tmp[0]
+    FM_TRY(green_op<double>(P, nb, x, PRO_V, nullptr, EPI_PREC_RES, x, b, ep, rc.tmp[0], a, -1, &rc));
+    FM_TRACK(P, KC_SETUP, cb, (k_from_f64<R><<<8 * P->sms, 256, 0, P->st>>>(nb * P->M, (const double2*)rc.tmp[0], 1.0, U)));
+    FM_CK(cudaGetLastError());
+    return FM_OK;
   };
 
   FM_TRY(upload_active());
-  FM_TRY(residual_into_U0(act));
+  FM_TRY(residual_into_U0(act, false));
   std::vector<double2> hv;
   FM_TRY(multidot<R>(P, nb, 0, U, U, true, act, hv));
   int iter = 0;
@@ -334,6 +358,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
       }
       for (int i = 0; i < n_in; ++i) yh[(size_t)b * (KV_KMAX + 1) + i] = make_double2(y[i].real(), y[i].imag());
       Kmax = std::max(Kmax, n_in);
+      acth[b] = n_in;
       r.inner = 0;
     }
     if (Kmax > 0) {
@@ -341,7 +366,9 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
       FM_CK(cudaMemcpyAsync(P->coef.p, yh.data(), yh.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
       FM_CK(cudaMemcpyAsync(sc, sch.data(), (size_t)(KV_KMAX + 1) * nb * sizeof(double), cudaMemcpyHostToDevice, P->st));
       Coef cf{(const double2*)P->coef.p, KV_KMAX + 1, sc, nb, 1.0, 1};
-      FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, nullptr, nb)));
+      // each right-hand side reads the vectors of this pass alone: the rest of U may hold anything (residual_into_U0)
+      FM_TRY(upload_active());
+      FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, act, nb, nullptr, act)));
     }
     any = false;
     for (int b = 0; b < nb; ++b) {
@@ -351,7 +378,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
     if (any && iter < itmax) {
       // restart: new residual for the RHS still running
       FM_TRY(upload_active());
-      FM_TRY(residual_into_U0(act));
+      FM_TRY(residual_into_U0(act, true));
       FM_TRY(multidot<R>(P, nb, 0, U, U, true, act, hv));
       for (int b = 0; b < nb; ++b)
         if (S[b].active) S[b].beta = std::sqrt(hv[b].x);

@@ -32,8 +32,13 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
   Dims d = P->dims;
   d.nb = nb;
   const size_t fbytes = (size_t)nb * P->M * sizeof(T);
-  FM_CK(P->t1.ensure(fbytes));
-  FM_CK(P->t2.ensure(fbytes));
+  const bool own = !(rc && rc->tmp[0]);
+  if (own) {
+    FM_CK(P->t1.ensure(fbytes));
+    FM_CK(P->t2.ensure(fbytes));
+  }
+  void* const t1 = own ? P->t1.p : rc->tmp[0];
+  void* const t2 = own ? P->t2.p : rc->tmp[1];
   GreenParams gp{};
   const double kr = std::sqrt(P->kref2);
   for (int a = 0; a < 3; ++a) gp.dk[a] = 2.0 * M_PI / ((double)(a == 0 ? d.nx : a == 1 ? d.ny : d.nz) * P->desc.resolution[a]) / kr;
@@ -52,41 +57,41 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
     cudaError_t e;
     if (!(chain & GREEN_CHAIN_HAVE_XF)) {
       FM_TRACK(P, KC_XF, 2 * fbA + (pro != PRO_COPY ? vb : 0.0),
-               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, nullptr, P->t1.p, act, vt));
+               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, nullptr, t1, act, vt));
       FM_CK(e);
     }
-    FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, P->t1.p, P->twy.p, nullptr, P->t2.p, act));
+    FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, t1, P->twy.p, nullptr, t2, act));
     FM_CK(e);
     if (P->avg && has_zreg<R>(P, d, 2)) {
       gp.shift[2] = P->shift[2];
       gp.scale_re = 1.0 / ((double)P->n * 2.0);
-      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zreg<R>(P, d, 2, P->t2.p, gp, P->zonly ? P->rz.p : P->rzp.p, P->t1.p, act));
+      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zreg<R>(P, d, 2, t2, gp, P->zonly ? P->rz.p : P->rzp.p, t1, act));
       FM_CK(e);
     } else if (P->zsplit) {
       // the two z branches (+s, -s) as two length-L z passes with their phase ramps; the second adds to the first
       gp.scale_re = 1.0 / ((double)P->n * 2.0);
       gp.shift[2] = P->shift[2];
       gp.accumulate = 0;
-      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, P->t2.p, gp, P->twz.p, P->rzp.p, P->t1.p, act));
+      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, t2, gp, P->twz.p, P->rzp.p, t1, act));
       FM_CK(e);
       gp.shift[2] = -P->shift[2];
       gp.accumulate = 1;
-      FM_TRACK(P, KC_ZG, 3 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, P->t2.p, gp, P->twz.p, P->rzm.p, P->t1.p, act));
+      FM_TRACK(P, KC_ZG, 3 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, t2, gp, P->twz.p, P->rzm.p, t1, act));
       FM_CK(e);
     } else {
       gp.shift[2] = P->zonly ? P->shift[2] : 0.0;
       gp.scale_re = 1.0 / ((double)P->n * (P->zonly ? 2.0 : 1.0));
       FM_TRACK(P, KC_ZG, 2 * fbA,
-               e = pass_zg<R>(P, d, P->zonly ? ZMODE_AVG2 : ZMODE_ONE, P->t2.p, gp, P->zonly ? P->twz2.p : P->twz.p,
-                              P->zonly ? P->rz.p : nullptr, P->t1.p, act));
+               e = pass_zg<R>(P, d, P->zonly ? ZMODE_AVG2 : ZMODE_ONE, t2, gp, P->zonly ? P->twz2.p : P->twz.p,
+                              P->zonly ? P->rz.p : nullptr, t1, act));
       FM_CK(e);
     }
-    FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, P->t1.p, P->twy.p, nullptr, P->t2.p, act));
+    FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, t1, P->twy.p, nullptr, t2, act));
     FM_CK(e);
     if (chain & GREEN_CHAIN_NEXT_XF)
-      FM_TRACK(P, KC_XI, xib + fbA, e = pass_xi_xf<R>(P, d, P->t2.p, V, xv, ep, P->twx.p, out, P->t1.p, act));
+      FM_TRACK(P, KC_XI, xib + fbA, e = pass_xi_xf<R>(P, d, t2, V, xv, ep, P->twx.p, out, t1, act));
     else
-      FM_TRACK(P, KC_XI, xib, e = pass_xi<R>(P, d, epi, P->t2.p, V, xv, bv, rs, ep, P->twx.p, nullptr, out, act, vt));
+      FM_TRACK(P, KC_XI, xib, e = pass_xi<R>(P, d, epi, t2, V, xv, bv, rs, ep, P->twx.p, nullptr, out, act, vt));
     FM_CK(e);
     return FM_OK;
   }
@@ -96,7 +101,8 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
   // shifted k (dyadic_green.jl:189-221).  Branch + stores half of G(+s) psi in t3; branch - adds it to half of
   // G(-s) psi in the XI pass, before the epilogue.
   {
-    FM_CK(P->t3.ensure(fbytes));
+    if (own) FM_CK(P->t3.ensure(fbytes));
+    void* const t3 = own ? P->t3.p : rc->tmp[2];
     gp.scale_re = 1.0 / ((double)P->n * 2.0);
     cudaError_t e;
     for (int br = 0; br < 2; ++br) {
@@ -106,24 +112,24 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
       const void* ry = P->shift[1] != 0.0 ? (br == 0 ? P->ryp.p : P->rym.p) : nullptr;
       const void* rzt = P->shift[2] != 0.0 ? (br == 0 ? P->rzp.p : P->rzm.p) : nullptr;
       FM_TRACK(P, KC_XF, 2 * fbA + (pro != PRO_COPY ? vb : 0.0),
-               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, rx, P->t1.p, act, vt));
+               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, rx, t1, act, vt));
       FM_CK(e);
-      FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, P->t1.p, P->twy.p, ry, P->t2.p, act));
+      FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, t1, P->twy.p, ry, t2, act));
       FM_CK(e);
-      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, P->t2.p, gp, P->twz.p, rzt, P->t1.p, act));
+      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, t2, gp, P->twz.p, rzt, t1, act));
       FM_CK(e);
-      FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, P->t1.p, P->twy.p, ry, P->t2.p, act));
+      FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, t1, P->twy.p, ry, t2, act));
       FM_CK(e);
       if (br == 0) {
         EpiParams e0{};
         FM_TRACK(P, KC_XI, 2 * fbA,
-                 e = pass_xi<R>(P, d, EPI_STORE, P->t2.p, V, nullptr, nullptr, nullptr, e0, P->twx.p, rx, P->t3.p,
+                 e = pass_xi<R>(P, d, EPI_STORE, t2, V, nullptr, nullptr, nullptr, e0, P->twx.p, rx, t3,
                                 act));
       } else {
         EpiParams e1 = ep;
-        e1.gadd = P->t3.p;
+        e1.gadd = t3;
         FM_TRACK(P, KC_XI, xib + fbA,
-                 e = pass_xi<R>(P, d, epi, P->t2.p, V, xv, bv, rs, e1, P->twx.p, rx, out, act, vt));
+                 e = pass_xi<R>(P, d, epi, t2, V, xv, bv, rs, e1, P->twx.p, rx, out, act, vt));
       }
       FM_CK(e);
     }

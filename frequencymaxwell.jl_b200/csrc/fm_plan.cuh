@@ -410,6 +410,7 @@ struct RhsCtx {
   const double* ksq_im_b = nullptr;   // eps_imag / k_ref^2 per RHS
   const double* inv_eps_b = nullptr;  // k_ref^2 / eps_imag per RHS
   VecTab vt;
+  void* tmp[3] = {nullptr, nullptr, nullptr};  // pass temporaries, nb fields each, in place of the plan's t1, t2, t3
 };
 
 // ---- operator drivers (fm_ops.cu) ----
