@@ -63,11 +63,60 @@ cudaError_t scratch_address(int dev, void** out) {
   return cudaSuccess;
 }
 
-template <typename C>
-cudaError_t put_table(unsigned char* dst, const std::vector<cd_t>& v, cudaStream_t st) {
-  std::vector<C> h(v.size());
-  for (size_t i = 0; i < v.size(); ++i) h[i] = mk((typename RealOf<C>::R)v[i].real(), (typename RealOf<C>::R)v[i].imag());
-  return cudaMemcpyAsync(dst, h.data(), h.size() * sizeof(C), cudaMemcpyHostToDevice, st);
+// The tables of one call, written where they are used by one launch that also clears the error flag.  A call pays for
+// its tables every time, and built on the host they were four copies from pageable memory, each of which the stream
+// waited for (128^3 FP32, with the z pass of launch_zreg: 218 us a call before both, 179 with them).
+struct PairJob {
+  unsigned off;  // bytes into the scratch
+  int L, r[3];   // length, radices in forward order (1: no such stage)
+};
+struct TableJobs {
+  PairJob pair[3];
+  unsigned ramp_off;
+  int ramp_L;
+  double ramp_s;  // exp(-2 pi i k s / L)
+};
+
+PairJob pair_job(size_t off, int L, const std::vector<int>& r) {
+  return {(unsigned)off, L, {r[0], r.size() > 1 ? r[1] : 1, r.size() > 2 ? r[2] : 1}};
+}
+
+// entry j of the stage table of radices r0, r1, r2 (stage_table in fm_tables.h)
+__device__ double2 stage_entry(int j, int r0, int r1, int r2) {
+  int ns = r0, q = r1;
+  if (j >= r0 * r1 - 1) {
+    ns = r0 * r1;
+    q = r2;
+  }
+  const int m = j - (ns - 1);
+  if (m < 0 || m >= (q - 1) * ns) return make_double2(1.0, 0.0);
+  double sn, cs;
+  sincospi(-2.0 * (double)((m % ns) * (m / ns + 1)) / (double)(ns * q), &sn, &cs);
+  return make_double2(cs, sn);
+}
+
+template <typename R>
+__global__ void k_tables(unsigned char* sc, int* err, TableJobs jobs) {
+  using T = cplx<R>;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && err) *err = 0;
+  int at = i;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const PairJob& p = jobs.pair[a];
+    if (at >= 0 && at < 2 * p.L) {
+      const double2 v = at < p.L ? stage_entry(at, p.r[0], p.r[1], p.r[2])
+                        : p.r[2] > 1 ? stage_entry(at - p.L, p.r[2], p.r[1], p.r[0])
+                                     : stage_entry(at - p.L, p.r[1], p.r[0], 1);
+      reinterpret_cast<T*>(sc + p.off)[at] = mk((R)v.x, (R)v.y);
+    }
+    at -= 2 * p.L;
+  }
+  if (at >= 0 && at < jobs.ramp_L) {
+    double sn, cs;
+    sincospi(-2.0 * (double)at * jobs.ramp_s / (double)jobs.ramp_L, &sn, &cs);
+    reinterpret_cast<T*>(sc + jobs.ramp_off)[at] = mk((R)cs, (R)sn);
+  }
 }
 
 bool pow2_in(int n, int lo, int hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; }
@@ -100,13 +149,19 @@ fm_status run(const fm_plan_desc& dsc, double k_bg, double eps_imag, int nrhs, c
   if (e != cudaSuccess) return noalloc_fail(FM_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
   unsigned char* sc = (unsigned char*)base;
   int* err = (int*)(sc + o_err);
-  // tables (FP64 on the host, cast to the arithmetic type)
-  if ((e = cudaMemsetAsync(err, 0, sizeof(int), st)) != cudaSuccess ||
-      (e = put_table<CR>(sc + o_tx, twiddles<R>(n3[0]), st)) != cudaSuccess ||
-      (e = put_table<CR>(sc + o_ty, ytile_twiddles<R>(n3[1]), st)) != cudaSuccess ||
-      (e = put_table<CR>(sc + o_tz, twiddles<R>(lz), st)) != cudaSuccess ||
-      (e = put_table<CR>(sc + o_rz, ramp(n3[2], zonly ? 0.25 : 0.0, -1.0), st)) != cudaSuccess)
-    return noalloc_fail(FM_ERR_CUDA, std::string("table upload: ") + cudaGetErrorString(e));
+  // the z pass in sixteen values a lane where the size has it (launch_zreg), else the passes of fm_passes*.cuh
+  const bool zreg = zreg_takes<S, R>(d, zonly ? 2 : 1);
+  const int lt = zreg ? n3[2] : lz;
+  TableJobs jobs{{pair_job(o_tx, n3[0], radices<R>(n3[0])), pair_job(o_ty, n3[1], ytile_radices<R>(n3[1])),
+                  pair_job(o_tz, lt, zreg ? radices16(lt) : radices<R>(lt))},
+                 (unsigned)o_rz, n3[2], zonly ? 0.25 : 0.0};
+  auto tables = [&](int* clear) {
+    const int entries = 2 * (n3[0] + n3[1] + jobs.pair[2].L) + n3[2];
+    k_tables<R><<<(entries + 127) / 128, 128, 0, st>>>(sc, clear, jobs);
+    return cudaGetLastError();
+  };
+  if ((e = tables(err)) != cudaSuccess)
+    return noalloc_fail(FM_ERR_CUDA, std::string("tables: ") + cudaGetErrorString(e));
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
   // k in units of k_bg (as the plans compute it), so |k|^2 - k_square stays O(1) in FP32 arithmetic:
@@ -125,15 +180,25 @@ fm_status run(const fm_plan_desc& dsc, double k_bg, double eps_imag, int nrhs, c
   // x -> y (x FFT) -> tmp (y FFT) -> y (z FFT, Green, inverse z FFT) -> tmp (inverse y FFT) -> y (inverse x FFT)
   auto ytma = [&](int dir, const void* in, void* out) -> cudaError_t {
     cudaError_t r = launch_y_tma<S, R>(d, dir, in, sc + o_ty, nullptr, out, nullptr, err, sms, st);
-    if (r == cudaErrorNotSupported) r = launch_y<S, R>(d, dir, in, sc + o_ty, nullptr, out, nullptr, st);
-    return r;
+    if (r != cudaErrorNotSupported) return r;
+    // no tiles (a narrow x, or buffers off the tensor maps' 16 bytes): the register pass, on its plan's table
+    if (ytile_radices<R>(n3[1]) != radices<R>(n3[1])) {
+      jobs.pair[1] = pair_job(o_ty, n3[1], radices<R>(n3[1]));
+      if ((r = tables(nullptr)) != cudaSuccess) return r;
+    }
+    return launch_y<S, R>(d, dir, in, sc + o_ty, nullptr, out, nullptr, st);
   };
   if ((e = launch_xf<S, R>(d, PRO_COPY, x, nullptr, nullptr, sc + o_tx, nullptr, y, nullptr, st)) != cudaSuccess ||
       (e = ytma(-1, y, tmp)) != cudaSuccess)
     return noalloc_fail(FM_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
-  e = launch_zg_tma<S, R>(d, mode, tmp, gp, sc + o_tz, zonly ? (const void*)(sc + o_rz) : nullptr, y, nullptr, err, sms, st);
-  if (e == cudaErrorNotSupported)
-    e = launch_zg<S, R>(d, mode, tmp, gp, sc + o_tz, zonly ? (const void*)(sc + o_rz) : nullptr, y, nullptr, st);
+  const void* rz = zonly ? (const void*)(sc + o_rz) : nullptr;
+  e = zreg ? launch_zreg<S, R>(d, zonly ? 2 : 1, tmp, gp, sc + o_tz, rz, y, nullptr, err, sms, st)
+           : launch_zg_tma<S, R>(d, mode, tmp, gp, sc + o_tz, rz, y, nullptr, err, sms, st);
+  if (e == cudaErrorNotSupported) {
+    jobs.pair[2] = pair_job(o_tz, lz, radices<R>(lz));
+    e = zreg ? tables(nullptr) : cudaSuccess;
+    if (e == cudaSuccess) e = launch_zg<S, R>(d, mode, tmp, gp, sc + o_tz, rz, y, nullptr, st);
+  }
   if (e != cudaSuccess || (e = ytma(+1, y, tmp)) != cudaSuccess ||
       (e = launch_xi<S, R>(d, EPI_STORE, tmp, nullptr, nullptr, nullptr, nullptr, ep, sc + o_tx, nullptr, y, nullptr,
                            st)) != cudaSuccess)

@@ -36,45 +36,44 @@ inline std::vector<int> radices_of() {
   return r;
 }
 
-// [forward-order table | reversed-order table] for an FFT of length L in arithmetic type R
+// radices of Plan<L, R>, and of the plans of sixteen values a lane (Plan16; empty for other lengths)
 template <typename R>
-inline std::vector<cd_t> twiddles(int L) {
-  std::vector<int> r;
+inline std::vector<int> radices(int L) {
   switch (L) {
-    case 8: r = radices_of<8, R>(); break;
-    case 16: r = radices_of<16, R>(); break;
-    case 32: r = radices_of<32, R>(); break;
-    case 64: r = radices_of<64, R>(); break;
-    case 128: r = radices_of<128, R>(); break;
-    case 256: r = radices_of<256, R>(); break;
-    case 512: r = radices_of<512, R>(); break;
-    case 96: r = radices_of<96, R>(); break;
-    default: break;
+    case 8: return radices_of<8, R>();
+    case 16: return radices_of<16, R>();
+    case 32: return radices_of<32, R>();
+    case 64: return radices_of<64, R>();
+    case 128: return radices_of<128, R>();
+    case 256: return radices_of<256, R>();
+    case 512: return radices_of<512, R>();
+    case 96: return radices_of<96, R>();
+    default: return {};
   }
-  std::vector<cd_t> t(2 * (size_t)L, cd_t(1.0, 0.0));
-  stage_table(t, 0, r);
-  std::vector<int> rr(r.rbegin(), r.rend());
-  stage_table(t, L, rr);
-  return t;
 }
-
-// the same pair for the plans of sixteen values a lane (Plan16); empty for other lengths
-inline std::vector<cd_t> twiddles16(int L) {
-  std::vector<int> r{16, L == 256 ? 16 : L == 64 ? 4 : 8};
-  if (L == 512) r.push_back(4);
-  else if (L != 64 && L != 128 && L != 256) return {};
-  std::vector<cd_t> t(2 * (size_t)L, cd_t(1.0, 0.0));
-  stage_table(t, 0, r);
-  std::vector<int> rr(r.rbegin(), r.rend());
-  stage_table(t, L, rr);
-  return t;
+inline std::vector<int> radices16(int L) {
+  return L == 64 ? std::vector<int>{16, 4} : L == 128 ? std::vector<int>{16, 8} : L == 256 ? std::vector<int>{16, 16}
+         : L == 512 ? std::vector<int>{16, 8, 4} : std::vector<int>{};
 }
-
-// the pair for the y tiles (YTilePlan)
+// of the y tiles (YTilePlan; at 512 the radices agree)
 template <typename R>
-inline std::vector<cd_t> ytile_twiddles(int L) {
-  return std::is_same<R, double>::value && L == 256 ? twiddles16(L) : twiddles<R>(L);  // (512: the radices agree)
+inline std::vector<int> ytile_radices(int L) {
+  return std::is_same<R, double>::value && L == 256 ? radices16(L) : radices<R>(L);
 }
+
+// [forward-order table | reversed-order table] of an FFT of length L
+inline std::vector<cd_t> twiddle_pair(int L, const std::vector<int>& r) {
+  if (r.empty()) return {};
+  std::vector<cd_t> t(2 * (size_t)L, cd_t(1.0, 0.0));
+  stage_table(t, 0, r);
+  stage_table(t, L, std::vector<int>(r.rbegin(), r.rend()));
+  return t;
+}
+template <typename R>
+inline std::vector<cd_t> twiddles(int L) { return twiddle_pair(L, radices<R>(L)); }
+inline std::vector<cd_t> twiddles16(int L) { return twiddle_pair(L, radices16(L)); }
+template <typename R>
+inline std::vector<cd_t> ytile_twiddles(int L) { return twiddle_pair(L, ytile_radices<R>(L)); }
 
 // exp(sgn * 2 pi i * idx * s / L)
 inline std::vector<cd_t> ramp(int L, double s, double sgn) {
