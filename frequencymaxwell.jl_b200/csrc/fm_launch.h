@@ -52,7 +52,7 @@ template <typename S, typename R>
 cudaError_t launch_zreg(const Dims& d, int branches, const void* in, const GreenParams& gp, const void* twz,
                         const void* rz, void* out, const int* active, int* err, int sms, cudaStream_t st);
 
-// pencils that share one warp for an axis of length L (y/z passes need nx to be a multiple)
+// pencils that share one warp for an axis of length L (fm_green_apply_noalloc takes an nx that is a multiple)
 template <typename R>
 int pencils_per_warp(int L);
 

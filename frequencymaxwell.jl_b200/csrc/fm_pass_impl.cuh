@@ -344,21 +344,14 @@ template <typename S, typename R>
 cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenParams& gp, const void* tw,
                           const void* rz, void* out, const int* act, int* err, int sms, cudaStream_t st) {
 #define ZT(LL, M) zg_tma_L<S, R, LL, M>(d, in, gp, tw, rz, out, act, err, sms, st)
+  // the Green pass where launch_zreg does not take it (zreg_takes), and the curl
+  if (mode == ZMODE_ONE) return d.nz == 32 ? ZT(32, ZMODE_ONE) : cudaErrorNotSupported;
   if (mode == ZMODE_AVG2) {
-    switch (d.nz) {
-      case 32: return ZT(32, ZMODE_AVG2);
-      case 64: return ZT(64, ZMODE_AVG2);
-      case 128: return ZT(128, ZMODE_AVG2);
-      default: return cudaErrorNotSupported;
+    if (d.nz == 32) return ZT(32, ZMODE_AVG2);
+    if constexpr (sizeof(R) == 4) {
+      if (d.nz == 64) return ZT(64, ZMODE_AVG2);
     }
-  }
-  if (mode == ZMODE_ONE) {
-    switch (d.nz) {
-      case 32: return ZT(32, ZMODE_ONE);
-      case 64: return ZT(64, ZMODE_ONE);
-      case 128: return ZT(128, ZMODE_ONE);
-      default: return cudaErrorNotSupported;
-    }
+    return cudaErrorNotSupported;
   }
   switch (d.nz) {
     case 32: return ZT(32, ZMODE_CURL);

@@ -1,5 +1,5 @@
-// Tensor-map x coordinates count 8-byte words: a tile row is 16 words (128 bytes) whatever the
-// storage type, so tile xt starts at word 16*xt.
+// Tensor-map x coordinates count 8-byte words: a tile row is ROWB/8 words (128, 64 or 32 bytes) whatever the
+// storage type, so tile xt starts at word xt*ROWB/8, a multiple of 16 bytes.
 // TMA-staged versions of the strided passes (y pencils; z pencils with the dyadic Green or the curl).
 // Same arithmetic as k_y / k_zg in fm_passes.cuh; the data path goes through swizzled shared-memory
 // tiles loaded and stored by the tensor memory accelerator (see fm_tma.cuh).
@@ -30,8 +30,9 @@ struct YTmaCfg {
   using T = cplx<R>;
   using TS = cplx<S>;
   using P = YTilePlan<L, R>;
-  // bytes of a tile row: at 256 points and FP32 storage 64-byte rows run four CTAs an SM (4.2 TB/s, 3.8 with 128), in
-  // FP64 storage whole lines are better (5.9, 5.2 with 64)
+  // bytes of a tile row: at 512 points two stages of whole lines leave no room for a second CTA; at 256 points and FP32
+  // storage 64-byte rows run four CTAs an SM (4.2 TB/s, 3.8 with 128), in FP64 storage whole lines are better (5.9, 5.2
+  // with 64)
   static constexpr int ROWB = L == 512 || (L == 256 && sizeof(S) == 4) ? 64 : 128;
   static constexpr int TX = ROWB / (int)sizeof(TS);
   static constexpr int PW = 32 / P::TP;
@@ -179,10 +180,7 @@ struct ZTmaCfg {
   static constexpr int TILE = 3 * L * 128;
   static constexpr int NST = TILE <= 32768 ? 3 : 2;
   static constexpr int STRIDE = PencilStride<LF, T, P::TP, true>::v;
-  // exchange buffers per pencil: the three components of a length-256 transform run stage by stage together
-  // (their exchanges overlap), each with its own buffer; shorter transforms run one component at a time
-  static constexpr int NCX = LF >= 256 ? 3 : 1;
-  using SM = TmaSmem<TILE, NST, CW * PW * NCX * STRIDE * (int)sizeof(T), (2 * LF + L) * (int)sizeof(T)>;
+  using SM = TmaSmem<TILE, NST, CW * PW * STRIDE * (int)sizeof(T), (2 * LF + L) * (int)sizeof(T)>;
   static constexpr int THREADS = CW * 32;
 };
 
@@ -233,8 +231,7 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
     }
   }
   const int p = lane / TP, t = lane % TP;
-  constexpr int NCX = C::NCX, SMS = C::STRIDE;
-  T* sm = ex + (warp * PW + p) * NCX * SMS;
+  T* sm = ex + (warp * PW + p) * C::STRIDE;
   int it = 0;
   bool ok = true;
   for (long long tile = next_active(blockIdx.x, ntiles, per_rhs, active); tile < ntiles;
@@ -264,13 +261,7 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
           }
           v[c][e] = a;
         }
-        if constexpr (NCX == 1) {
-          fft_fwd_plan<-1, P_, MODE == ZMODE_AVG2>(v[c], sm, tw, t);
-          __syncwarp();
-        }
-      }
-      if constexpr (NCX == 3) {
-        fft_fwd_plan_n<-1, P_, 3, SMS, MODE == ZMODE_AVG2>(v, sm, tw, t);
+        fft_fwd_plan<-1, P_, MODE == ZMODE_AVG2>(v[c], sm, tw, t);
         __syncwarp();
       }
       R kx, ky;
@@ -287,16 +278,10 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
         if constexpr (MODE == ZMODE_CURL) gb.curl(v[0][e], v[1][e], v[2][e], kx, ky, kz);
         else gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
       }
-      if constexpr (NCX == 3) {
-        fft_rev_plan_n<+1, P_, 3, SMS>(v, sm, twr, t);
-        __syncwarp();
-      }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        if constexpr (NCX == 1) {
-          fft_rev_plan<+1, P_>(v[c], sm, twr, t);
-          __syncwarp();
-        }
+        fft_rev_plan<+1, P_>(v[c], sm, twr, t);
+        __syncwarp();
 #pragma unroll
         for (int e = 0; e < E; ++e) {
           const int z = lay_idx<LF, E, P_::R0>(t, e);
