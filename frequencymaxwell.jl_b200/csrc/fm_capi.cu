@@ -138,14 +138,20 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   const int prec = desc->precision == FM_PREC_F64 ? FM_PREC_F64 : FM_PREC_F32;  // storage
   const bool c64 = desc->precision != FM_PREC_F32;                                   // arithmetic
   // Fused passes take an axis of 96 or a power of two in [8, 512]; any other length up to 256 runs Bluestein passes
-  // on that axis (fm_generic.cuh).
+  // on that axis (fm_generic.cuh), and in FP32 arithmetic the whole grid runs the passes of fm_general32.cuh.
   for (int a = 0; a < 3; ++a)
     if (!axis_supported(n3[a]) && !blue_axis_supported(n3[a]))
       return fail(FM_ERR_UNSUPPORTED, "padded axis sizes must be at most 256, or powers of two up to 512");
   // shifts on z only: both branches in one length-2L z pass where the length has one, else two z passes (the second
   // adds to the first)
   const bool avg2 = axis_supported(n3[2]) && n3[2] <= AXIS_MAX_AVG2 && (n3[2] & (n3[2] - 1)) == 0;
-  const bool zsplit = zonly && !avg2;
+  bool general32 = false;
+  if (!c64) {
+    const int pwy = pencils_per_warp<float>(n3[1]), pwz = pencils_per_warp<float>(zonly && avg2 ? 2 * n3[2] : n3[2]);
+    for (int a = 0; a < 3; ++a) general32 |= !axis_supported(n3[a]);
+    general32 |= (zonly && (n3[2] & (n3[2] - 1)) != 0) || pwy <= 0 || pwz <= 0 || n3[0] % pwy || n3[0] % pwz;
+  }
+  const bool zsplit = zonly && !avg2 && !general32;
   if (cudaSetDevice(desc->device) != cudaSuccess) return fail(FM_ERR_CUDA, "cudaSetDevice failed");
   fm_plan* P = new fm_plan();
   P->desc = *desc;
@@ -158,8 +164,9 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   P->M = 3 * P->n;
   P->pi = PadInfo{desc->grid[0], desc->grid[1], desc->grid[2], desc->pad[0], desc->pad[1], desc->pad[2], n3[0], n3[1], n3[2]};
   P->avg = avg;
-  P->zonly = zonly && !zsplit;
+  P->zonly = zonly && !zsplit && !general32;
   P->zsplit = zsplit;
+  P->general32 = general32;
   for (int a = 0; a < 3; ++a) P->shift[a] = desc->absorbing[a] ? 0.25 : 0.0;
   {
     cudaDeviceProp prop;

@@ -22,6 +22,10 @@ template <typename T> __host__ __device__ __forceinline__ T csub(T a, T b) { ret
 template <typename T> __host__ __device__ __forceinline__ T cmul(T a, T b) {
   return mk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// cmul with its fused multiply-adds written out: the same bits wherever it is used
+template <typename T> __device__ __forceinline__ T cmul_fixed(T a, T b) {
+  return mk(fma(a.x, b.x, -(a.y * b.y)), fma(a.y, b.x, a.x * b.y));
+}
 // a * conj(b)
 template <typename T> __host__ __device__ __forceinline__ T cmulc(T a, T b) {
   return mk(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
@@ -59,10 +63,8 @@ __device__ __forceinline__ double widen(float x) {
   return __hiloint2double((i >> 3) & 0x8fffffff, i << 29);
 }
 __device__ __forceinline__ double2 widen(float2 a) { return make_double2(widen(a.x), widen(a.y)); }
-__device__ __forceinline__ double2 widen(double2 a) { return a; }
 // accumulates zero for finite values and NaN otherwise
 __device__ __forceinline__ void nonfinite_mark(float& t, float2 a) { t = fmaf(a.x, 0.0f, fmaf(a.y, 0.0f, t)); }
-__device__ __forceinline__ void nonfinite_mark(float&, double2) {}
 // the mark as a double: 0 or NaN (the hardware's NaN result is 0x7fffffff, whose bits are a double's NaN too)
 __device__ __forceinline__ double mark_d(float t) { return __hiloint2double(__float_as_int(t), 0); }
 

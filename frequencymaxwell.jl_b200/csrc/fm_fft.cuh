@@ -233,6 +233,76 @@ __device__ __forceinline__ void fft_run(T (&v)[E], T* sm, const T* tw, int t) {
   }
 }
 
+// ---- NC pencils of one lane group run stage by stage together ----
+// Pencil c exchanges through its own buffer sm + c*SMS, so between two __syncwarp the loads and butterflies of
+// all NC pencils are independent and one pencil's exchange latency overlaps the others' arithmetic.  The stage
+// twiddles are loaded once, before any store of the stage, and shared by the NC pencils.
+template <int DIR, int L, int E, int RAD, int NS, bool LAST, int NC, int SMS, typename T>
+__device__ __forceinline__ void fft_stage_n(T (&v)[NC][E], T* sm, const T* tw, int t) {
+  constexpr int TP = L / E;
+  constexpr int NB = E / RAD;
+  static_assert(E % RAD == 0, "radix must divide E");
+  T w[NB][RAD - 1];
+  if constexpr (NS > 1) {
+#pragma unroll
+    for (int m = 0; m < NB; ++m)
+#pragma unroll
+      for (int q = 1; q < RAD; ++q) {
+        T a = tw[(NS - 1) + (q - 1) * NS + (t + TP * m) % NS];
+        if constexpr (DIR > 0) a = cconj(a);
+        w[m][q - 1] = a;
+      }
+  }
+#pragma unroll
+  for (int m = 0; m < NB; ++m) {
+    const int j = t + TP * m;
+    const int k = j % NS;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      if constexpr (NS > 1) {
+#pragma unroll
+        for (int q = 1; q < RAD; ++q) v[c][m * RAD + q] = cmul(v[c][m * RAD + q], w[m][q - 1]);
+      }
+      bfly<DIR, RAD>(&v[c][m * RAD]);
+      if constexpr (!LAST) {
+        const int base = (j / NS) * NS * RAD + k;
+#pragma unroll
+        for (int q = 0; q < RAD; ++q) sm[c * SMS + sm_phys<T>(base + q * NS)] = v[c][m * RAD + q];
+      }
+    }
+  }
+}
+
+template <int L, int E, int RAD, int NC, int SMS, typename T>
+__device__ __forceinline__ void fft_gather_n(T (&v)[NC][E], const T* sm, int t) {
+#pragma unroll
+  for (int c = 0; c < NC; ++c) fft_gather<L, E, RAD>(v[c], sm + c * SMS, t);
+}
+
+template <int DIR, int L, int E, int R0, int R1, int R2, int NC, int SMS, typename T>
+__device__ __forceinline__ void fft_run_n(T (&v)[NC][E], T* sm, const T* tw, int t) {
+  static_assert(R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) == L, "radices must multiply to L");
+  if constexpr (R1 == 0) {
+    fft_stage_n<DIR, L, E, R0, 1, true, NC, SMS>(v, sm, tw, t);
+  } else if constexpr (R2 == 0) {
+    fft_stage_n<DIR, L, E, R0, 1, false, NC, SMS>(v, sm, tw, t);
+    __syncwarp();
+    fft_gather_n<L, E, R1, NC, SMS>(v, sm, t);
+    __syncwarp();
+    fft_stage_n<DIR, L, E, R1, R0, true, NC, SMS>(v, sm, tw, t);
+  } else {
+    fft_stage_n<DIR, L, E, R0, 1, false, NC, SMS>(v, sm, tw, t);
+    __syncwarp();
+    fft_gather_n<L, E, R1, NC, SMS>(v, sm, t);
+    __syncwarp();
+    fft_stage_n<DIR, L, E, R1, R0, false, NC, SMS>(v, sm, tw, t);
+    __syncwarp();
+    fft_gather_n<L, E, R2, NC, SMS>(v, sm, t);
+    __syncwarp();
+    fft_stage_n<DIR, L, E, R2, R0 * R1, true, NC, SMS>(v, sm, tw, t);
+  }
+}
+
 // ---- per-length plans ----
 // E elements per lane and the forward radix sequence; TP = L/E lanes per pencil, 4 <= TP <= 32
 // (so at most 8 pencils share a warp and every axis of >= 8 points tiles a warp).
@@ -275,6 +345,18 @@ __device__ __forceinline__ void fft_rev_plan(T (&v)[P::E], T* sm, const T* tw_re
   else fft_run<DIR, P::L, P::E, P::R2, P::R1, P::R0>(v, sm, tw_rev, t);
 }
 
+// NC pencils at once (exchange buffers SMS elements apart)
+template <int DIR, typename P, int NC, int SMS, typename T>
+__device__ __forceinline__ void fft_fwd_plan_n(T (&v)[NC][P::E], T* sm, const T* tw_fwd, int t) {
+  fft_run_n<DIR, P::L, P::E, P::R0, P::R1, P::R2, NC, SMS>(v, sm, tw_fwd, t);
+}
+template <int DIR, typename P, int NC, int SMS, typename T>
+__device__ __forceinline__ void fft_rev_plan_n(T (&v)[NC][P::E], T* sm, const T* tw_rev, int t) {
+  if constexpr (P::R1 == 0) fft_run_n<DIR, P::L, P::E, P::R0, 0, 0, NC, SMS>(v, sm, tw_rev, t);
+  else if constexpr (P::R2 == 0) fft_run_n<DIR, P::L, P::E, P::R1, P::R0, 0, NC, SMS>(v, sm, tw_rev, t);
+  else fft_run_n<DIR, P::L, P::E, P::R2, P::R1, P::R0, NC, SMS>(v, sm, tw_rev, t);
+}
+
 // Padded pencil stride in the exchange buffer.  A shared-memory wavefront serves
 // 128 bytes: 16 lanes of 8-byte or 8 lanes of 16-byte elements.  With lanes
 // t-fastest (x rows) a wavefront spans 128/size/TP pencils, each using TP
@@ -308,6 +390,12 @@ template <int L_> struct Plan16 {
   // slots per pencil: the padded length; pencils that share a wavefront (L = 64, and 128 in FP32) on disjoint slots
   static constexpr int STRIDE = L_ == 64 ? 84 : L_ + L_ / 8 + (L_ == 128 ? 8 : 0);
 };
+
+// whether Plan16 splits L as Plan does in arithmetic R: then the transforms agree bit for bit
+template <int L, typename R>
+constexpr bool same_radices() {
+  return Plan<L, R>::R0 == Plan16<L>::R0 && Plan<L, R>::R1 == Plan16<L>::R1 && Plan<L, R>::R2 == Plan16<L>::R2;
+}
 
 template <int DIR, int L, int RAD, int NS, bool LAST, int PS, bool LO, typename T>
 __device__ __forceinline__ void fft16_stage(T (&v)[16], T* sm, const T* tw, int t) {
@@ -373,16 +461,17 @@ __device__ __forceinline__ void fft16_rev(T (&v)[16], T* sm, const T* tw_rev, in
   else fft16_run<DIR, P::L, P::R2, P::R1, P::R0>(v, sm, tw_rev, t);
 }
 
-// ---- plans of the x rows and of the y tiles: in FP64 sixteen values a lane at 512 points, and in the y tiles at 256
-// (k_y_tma 256^3, FP32 storage, 64-byte rows: 220 us with eight values, 191 with sixteen; the x rows, whose CTAs hold no
-// tile, run faster with eight values and more warps: k_xf 223 against 240, k_xi 331 against 374).  Plan elsewhere. ----
+// ---- plans of the x rows and of the y tiles: in FP64 sixteen values a lane at 512 points (Plan's radices), and in the y
+// tiles of FP64 storage at 256 (FP32 storage keeps Plan's radices, see k_dot32: k_y_tma 256^3, 64-byte rows, 223 us
+// where sixteen values would take 191; the x rows, whose CTAs hold no tile, run faster with eight values and more warps:
+// k_xf 223 against 240, k_xi 331 against 374).  Plan elsewhere. ----
 template <int L, typename R> struct RowPlan : Plan<L, R> {
   static constexpr bool IS16 = false;
   static constexpr int STRIDE = PencilStride<L, typename CT<R>::T, Plan<L, R>::TP, true>::v;
 };
 template <> struct RowPlan<512, double> : Plan16<512> { static constexpr bool IS16 = true; };
-template <int L, typename R> struct YTilePlan : RowPlan<L, R> {};
-template <> struct YTilePlan<256, double> : Plan16<256> { static constexpr bool IS16 = true; };
+template <int L, typename S, typename R> struct YTilePlan : RowPlan<L, R> {};
+template <> struct YTilePlan<256, double, double> : Plan16<256> { static constexpr bool IS16 = true; };
 template <int DIR, typename P, typename T>
 __device__ __forceinline__ void long_fwd(T (&v)[P::E], T* sm, const T* tw_fwd, int t) {
   if constexpr (P::IS16) fft16_fwd<DIR, P>(v, sm, tw_fwd, t);

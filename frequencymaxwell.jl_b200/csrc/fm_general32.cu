@@ -1,0 +1,90 @@
+// Launchers of the general-length passes in FP32 arithmetic (fm_general32.cuh).
+#include <algorithm>
+
+#include "fm_general32.h"
+
+namespace fm {
+
+template <typename K>
+static void gen_allow_smem(K kern, size_t bytes) {
+  if (bytes > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+static unsigned gen_blocks(long long work) {
+  return (unsigned)std::max<long long>(1, std::min<long long>((work + 255) / 256, 148LL * 32));
+}
+
+template <int M, int DIR>
+static cudaError_t gen_axis_M(const Dims& d, int axis, const void* in, void* out, const GenAxis& ax, const int* act,
+                              cudaStream_t st) {
+  using P_ = Plan<M, float>;
+  constexpr int PW = 32 / P_::TP;
+  constexpr int W = 8;
+  const long long pencils = d.n / ax.n * 3 * d.nb;
+  const long long warps = (pencils + PW - 1) / PW;
+  const unsigned blocks = (unsigned)((warps + W - 1) / W);
+  const size_t smem = (size_t)(2 * M + W * PW * PencilStride<M, float2, P_::TP, true>::v) * sizeof(float2);
+  gen_allow_smem(k_gen_axis<M, DIR>, smem);
+  k_gen_axis<M, DIR><<<blocks, W * 32, smem, st>>>(d, axis, (const float2*)in, (float2*)out, ax, act);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_gen_axis(const Dims& d, int axis, int dir, const void* in, void* out, const GenAxis& ax,
+                            const int* act, cudaStream_t st) {
+#define FM_GEN_AXIS(MM)                                                               \
+  case MM:                                                                            \
+    return dir < 0 ? gen_axis_M<MM, -1>(d, axis, in, out, ax, act, st)          \
+                   : gen_axis_M<MM, +1>(d, axis, in, out, ax, act, st);
+  switch (ax.m) {
+    FM_GEN_AXIS(8)
+    FM_GEN_AXIS(16)
+    FM_GEN_AXIS(32)
+    FM_GEN_AXIS(64)
+    FM_GEN_AXIS(128)
+    FM_GEN_AXIS(256)
+    FM_GEN_AXIS(512)
+    default:
+      return cudaErrorNotSupported;
+  }
+#undef FM_GEN_AXIS
+}
+
+cudaError_t launch_gen_pre(const Dims& d, int pro, const void* in, const void* V, const double* rs, const GenRamps& rp,
+                           void* out, const int* act, cudaStream_t st, VecTab vt) {
+  const unsigned bl = gen_blocks(3 * d.n * d.nb);
+  if (pro == PRO_COPY)
+    k_gen_pre<PRO_COPY><<<bl, 256, 0, st>>>(d, (const float2*)in, (const float2*)V, rs, rp, (float2*)out, act, vt);
+  else if (pro == PRO_V)
+    k_gen_pre<PRO_V><<<bl, 256, 0, st>>>(d, (const float2*)in, (const float2*)V, rs, rp, (float2*)out, act, vt);
+  else
+    k_gen_pre<PRO_V_SCALE><<<bl, 256, 0, st>>>(d, (const float2*)in, (const float2*)V, rs, rp, (float2*)out, act,
+                                                     vt);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_gen_kspace(const Dims& d, int mode, void* f, const GreenParams& gp, const int* act, cudaStream_t st) {
+  const unsigned bl = gen_blocks(d.n * d.nb);
+  if (mode == ZMODE_CURL) k_gen_kspace<ZMODE_CURL><<<bl, 256, 0, st>>>(d, (float2*)f, gp, act);
+  else k_gen_kspace<ZMODE_ONE><<<bl, 256, 0, st>>>(d, (float2*)f, gp, act);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_gen_post(const Dims& d, int epi, const void* in, const void* V, const void* xv, const void* bv,
+                            const double* rs, const EpiParams& ep, const GenRamps& rp, void* out, const int* act,
+                            cudaStream_t st, VecTab vt) {
+  const unsigned bl = gen_blocks(3 * d.n * d.nb);
+#define FM_GEN_POST(EE)                                                                                          \
+  k_gen_post<EE><<<bl, 256, 0, st>>>(d, (const float2*)in, (const float2*)V, (const float2*)xv, (const float2*)bv, rs, ep, rp, \
+                                           (float2*)out, act, vt)
+  switch (epi) {
+    case EPI_STORE: FM_GEN_POST(EPI_STORE); break;
+    case EPI_OP: FM_GEN_POST(EPI_OP); break;
+    case EPI_PREC_OP: FM_GEN_POST(EPI_PREC_OP); break;
+    case EPI_PREC_RES: FM_GEN_POST(EPI_PREC_RES); break;
+    default: return cudaErrorInvalidValue;
+  }
+#undef FM_GEN_POST
+  return cudaGetLastError();
+}
+
+}  // namespace fm

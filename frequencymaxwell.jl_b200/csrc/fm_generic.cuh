@@ -1,5 +1,5 @@
-// Axis passes for lengths without a fused pass (odd lengths, other non-powers of two, e.g. the 201 x 201 x 197 padded
-// grid of the reference's two-beam example).  They take the places of k_xf, k_y, k_zg and k_xi (fm_passes.cuh) axis by
+// Axis passes in FP64 arithmetic for lengths without a fused pass (odd lengths, other non-powers of two, e.g. the
+// 201 x 201 x 197 padded grid of the reference's two-beam example; FP32 arithmetic: fm_general32.cuh).  They take the places of k_xf, k_y, k_zg and k_xi (fm_passes.cuh) axis by
 // axis, so a grid pays for Bluestein's algorithm only on the axes that need it, and the two sub-pixel-shifted branches
 // of a z-only boundary share the x and y passes.
 //
@@ -31,8 +31,8 @@ struct BlueAxis {
 };
 
 // FFT of length M inside the transform.  At 512 the sixteen-value plan's padding keeps the strided writes off each
-// other's banks (201 x 201 x 197, k_bxf: 606 -> 529 us in FP64, 418 -> 315 in FP32); at 256 eight values a lane and twice
-// the warps are faster (100 points, FP64: 56 us against 64)
+// other's banks (201 x 201 x 197, k_bxf: 606 -> 529 us); at 256 eight values a lane and twice the warps are faster
+// (100 points: 56 us against 64)
 template <int M, typename R> struct BluePlan : Plan<M, R> {
   static constexpr bool IS16 = false;
   static constexpr int STRIDE = PencilStride<M, cplx<R>, Plan<M, R>::TP, true>::v;
@@ -186,8 +186,7 @@ __global__ void __launch_bounds__(32 * BX_WARPS, 4) k_bxi(Dims d, const cplx<S>*
 // A CTA takes XT x-consecutive pencils and stages them in shared memory in the arithmetic type, pencil after pencil:
 // the lanes of a pencil read consecutive slots at constant offsets.  Global rows are 128 bytes; at M = 512 64 in the y
 // pass and 32 in the z pass, which holds three components: narrow tiles let several CTAs share an SM, and one's loads
-// overlap another's transforms (z pass of 201 x 201 x 197, one branch: 1558 us at 64 bytes, 1425 at 32 in FP64, 716 and
-// 628 in FP32; the rows that neighbouring CTAs split meet in L2).
+// overlap another's transforms (z pass of 201 x 201 x 197, one branch: 1558 us at 64 bytes, 1425 at 32; the rows that neighbouring CTAs split meet in L2).
 template <typename R, int M, bool Z>
 struct BlueTile {
   using T = cplx<R>;

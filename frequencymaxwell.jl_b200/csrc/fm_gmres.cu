@@ -11,11 +11,20 @@ template <typename R>
 cudaError_t gs_dot(fm_plan* P, int nb, int K, const void* U, const void* w, bool wnorm, const int* act, int nact,
                    const void* const* wtab, const int* Kb) {
   using T = cplx<R>;
-  auto kern = wnorm ? k_gsdot<R, true, false> : k_gsdot<R, false, false>;
-  FM_TRACK(P, KC_DOT, (double)(K + 1) * nact * P->M * sizeof(T),
-           (kern<<<dim3(gs_blocks<R>(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
-               P->M, nb, K, (const T*)U, (const T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
-               (unsigned*)P->red_cnt.p, act, (const T* const*)wtab, Kb, MgsTail{})));
+  const double bytes = (double)(K + 1) * nact * P->M * sizeof(T);
+  if constexpr (sizeof(R) == 4) {
+    auto kern = wnorm ? k_dot32<true> : k_dot32<false>;
+    FM_TRACK(P, KC_DOT, bytes,
+             (kern<<<dim3(s32_blocks(P, nb), nb), S32_THREADS, 0, P->st>>>(
+                 P->M, nb, K, (const T*)U, (const T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
+                 (unsigned*)P->red_cnt.p, act, (const T* const*)wtab, Kb)));
+  } else {
+    auto kern = wnorm ? k_gsdot<true, false> : k_gsdot<false, false>;
+    FM_TRACK(P, KC_DOT, bytes,
+             (kern<<<dim3(gs_blocks(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
+                 P->M, nb, K, (const T*)U, (const T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
+                 (unsigned*)P->red_cnt.p, act, (const T* const*)wtab, Kb, MgsTail{})));
+  }
   return cudaGetLastError();
 }
 
@@ -23,11 +32,18 @@ template <typename R>
 cudaError_t gs_update(fm_plan* P, int nb, int K, const void* U, const Coef& cf, void* w, bool norm, const int* act,
                       int nact, void* const* wtab, const int* Kb) {
   using T = cplx<R>;
-  auto kern = norm ? k_gsupdate<R, true> : k_gsupdate<R, false>;
-  FM_TRACK(P, KC_UPD, (double)(K + 2) * nact * P->M * sizeof(T),
-           (kern<<<dim3(gs_blocks<R>(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
-               P->M, nb, K, (const T*)U, cf, (T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
-               (unsigned*)P->red_cnt.p, act, (T* const*)wtab, Kb)));
+  auto launch = [&](auto kern, int nblk, int threads) {
+    FM_TRACK(P, KC_UPD, (double)(K + 2) * nact * P->M * sizeof(T),
+             (kern<<<dim3(nblk, nb), threads, 0, P->st>>>(
+                 P->M, nb, K, (const T*)U, cf, (T*)w, (double2*)P->red_part.p, (double2*)P->red_out.p,
+                 (unsigned*)P->red_cnt.p, act, (T* const*)wtab, Kb)));
+  };
+  if constexpr (sizeof(R) == 4) {
+    launch(norm ? k_update32<true> : k_update32<false>, s32_blocks(P, nb), S32_THREADS);
+  } else {
+    auto kern = norm ? k_gsupdate<true> : k_gsupdate<false>;
+    launch(kern, gs_blocks(P, kern, nb), KV_THREADS);
+  }
   return cudaGetLastError();
 }
 
@@ -118,6 +134,87 @@ double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
+// One step of modified Gram-Schmidt as Krylov.jl runs it (sc[i*ss + b] scales U_i), FP32 storage:
+//   if i > 0:  w -= h_{i-1} * v_{i-1}        (h read from device, v = sc*U)
+//   if i < K:  h_i = <v_i, w>                (reduced into hout[b*hs + i])
+//   else:      hout[b*hs + K] = ||w||^2
+// w is rounded to storage after every vector, which the one sweep of k_gsdot has no place for.
+constexpr int MGS32_CTAS = 6;  // CTAs an SM: with the chunk, what fixes the blocks
+static __global__ void __launch_bounds__(KV_THREADS, MGS32_CTAS)
+    k_mgs32(long long M, int B, int i, int K, const float2* __restrict__ U, const double* __restrict__ sc, int ss,
+            float2* __restrict__ w, double2* __restrict__ hout, int hs, double2* __restrict__ part,
+            unsigned* __restrict__ counter, const int* __restrict__ active) {
+  __shared__ double2 red[KV_WARPS];
+  const int b = blockIdx.y, nblk = gridDim.x;
+  if (active && !active[b]) return;
+  const long long chunk = (long long)KV_THREADS * KV_EPT;
+  const long long per = ((M + nblk - 1) / nblk + chunk - 1) / chunk * chunk;
+  const long long lo = (long long)blockIdx.x * per, hi = min(M, lo + per);
+  float2* wb = w + (size_t)b * M;
+  double2 cprev = make_double2(0.0, 0.0);
+  const float2* up = nullptr;
+  if (i > 0) {
+    double2 h = hout[(size_t)b * hs + (i - 1)];
+    double s = sc ? sc[(size_t)(i - 1) * ss + b] : 1.0;
+    cprev = make_double2(-h.x * s, -h.y * s);
+    up = U + ((size_t)(i - 1) * B + b) * M;
+  }
+  const float2* ui = (i < K) ? U + ((size_t)i * B + b) * M : nullptr;
+  const double si = (i < K && sc) ? sc[(size_t)i * ss + b] : 1.0;
+  double2 acc = make_double2(0.0, 0.0);
+  for (long long c0 = lo; c0 < hi; c0 += chunk) {
+#pragma unroll
+    for (int k = 0; k < KV_EPT; ++k) {
+      long long e = c0 + (long long)k * KV_THREADS + threadIdx.x;
+      if (e < hi) {
+        double2 wv = to_d(wb[e]);
+        if (up) {
+          double2 u = to_d(up[e]);
+          wv.x = fma(cprev.x, u.x, fma(-cprev.y, u.y, wv.x));
+          wv.y = fma(cprev.x, u.y, fma(cprev.y, u.x, wv.y));
+          float2 r = from_d<float2>(wv);
+          wb[e] = r;
+          wv = to_d(r);
+        }
+        if (ui) {
+          double2 u = to_d(ui[e]);
+          acc.x = fma(u.x, wv.x, fma(u.y, wv.y, acc.x));
+          acc.y = fma(u.x, wv.y, fma(-u.y, wv.x, acc.y));
+        } else {
+          acc.x = fma(wv.x, wv.x, fma(wv.y, wv.y, acc.x));
+        }
+      }
+    }
+  }
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double2 t = make_double2(0.0, 0.0);
+    for (int q = 0; q < KV_WARPS; ++q) { t.x += red[q].x; t.y += red[q].y; }
+    if (ui) { t.x *= si; t.y *= si; }
+    part[(size_t)b * nblk + blockIdx.x] = t;
+  }
+  // reduce into hout[b*hs + i]
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = (atomicAdd(&counter[b], 1u) == (unsigned)(nblk - 1));
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) {
+    double2 s = make_double2(0.0, 0.0);
+    for (int k = 0; k < nblk; ++k) {
+      double2 v = __ldcg(&part[(size_t)b * nblk + k]);
+      s.x += v.x;
+      s.y += v.y;
+    }
+    hout[(size_t)b * hs + i] = s;
+    counter[b] = 0;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // GMRES (Krylov.jl semantics) on a batch of nb RHS; b in P->bbuf, x (warm
 // start u0 = b) in P->xbuf.  Basis vectors are kept unnormalised with their
@@ -135,7 +232,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
   FM_CK(P->scale.ensure((size_t)(KV_KMAX + 1) * nb * sizeof(double)));
   if (o.ortho == FM_ORTHO_MGS) {
     FM_CK(P->hbuf.ensure((size_t)nb * (KV_KMAX + 2) * sizeof(double2)));
-    FM_CK(P->mgsT.ensure((size_t)nb * KV_KMAX * KV_KMAX * sizeof(double2)));
+    if (sizeof(R) == 8) FM_CK(P->mgsT.ensure((size_t)nb * KV_KMAX * KV_KMAX * sizeof(double2)));
   }
   FM_CK(P->active.ensure((size_t)nb * sizeof(int)));
   FM_TRY(ensure_reduce(P, nb, mem + 1));
@@ -158,37 +255,13 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
                           P->st));
     return FM_OK;
   };
-  // r0 = M^{-1}(b - A x) into U[0].  At a restart of the FP32-storage form with FP64 arithmetic the passes run on FP64
-  // copies, which the dead basis vectors U[1..mem] hold: an error of this residual is one of the right-hand side that no
-  // later cycle sees, and rounding its four pass temporaries to FP32 was most of the error of the fields (64-bit study,
-  // 512 x 64 x 512, GMRES(20): fields off by 6.3e-6 with it, 1.8e-6 without).  It costs three FP32 applications per cycle.
-  const size_t widef = (2 * fbytes + 255) / 256 * 256;  // one FP64 field of the batch
-  const bool branches = P->avg && !P->zonly && !P->zsplit;
-  const bool wide = P->c64 && sizeof(T) == 8 &&
-                    (branches ? 5 : 4) * widef + (size_t)P->n * sizeof(double2) + 256 <= (size_t)mem * fbytes;
-  auto residual_into_U0 = [&](const int* a, bool restart) -> fm_status {
-    if (!wide || !restart)
-      return green_op<R>(P, nb, P->xbuf.p, PRO_V, nullptr, EPI_PREC_RES, P->xbuf.p, P->bbuf.p, ep, U, a);
-    char* w = (char*)(((uintptr_t)(U + nb * fe) + 255) & ~(uintptr_t)255);
-    void *x = w, *b = w + widef;
-    RhsCtx rc;
-    for (int i = 0; i < (branches ? 3 : 2); ++i) rc.tmp[i] = w + (2 + i) * widef;
-    double2* V = (double2*)(w + (branches ? 5 : 4) * widef);
-    rc.V = V;
-    const double cb = (double)fbytes * 3;
-    FM_TRACK(P, KC_SETUP, (double)P->n * 24, (k_to_f64<R><<<8 * P->sms, 256, 0, P->st>>>(P->n, (const T*)P->V.p, 1.0, V)));
-    FM_TRACK(P, KC_SETUP, cb, (k_to_f64<R><<<8 * P->sms, 256, 0, P->st>>>(nb * P->M, (const T*)P->xbuf.p, 1.0, (double2*)x)));
-    FM_TRACK(P, KC_SETUP, cb, (k_to_f64<R><<<8 * P->sms, 256, 0, P->st>>>(nb * P->M, (const T*)P->bbuf.p, 1.0, (double2*)b)));
-    FM_CK(cudaGetLastError());
-    // the last pass reads tmp[1] and may write tmp[0]
-    FM_TRY(green_op<double>(P, nb, x, PRO_V, nullptr, EPI_PREC_RES, x, b, ep, rc.tmp[0], a, -1, &rc));
-    FM_TRACK(P, KC_SETUP, cb, (k_from_f64<R><<<8 * P->sms, 256, 0, P->st>>>(nb * P->M, (const double2*)rc.tmp[0], 1.0, U)));
-    FM_CK(cudaGetLastError());
-    return FM_OK;
+  // r0 = M^{-1}(b - A x) into U[0]
+  auto residual_into_U0 = [&](const int* a) -> fm_status {
+    return green_op<R>(P, nb, P->xbuf.p, PRO_V, nullptr, EPI_PREC_RES, P->xbuf.p, P->bbuf.p, ep, U, a);
   };
 
   FM_TRY(upload_active());
-  FM_TRY(residual_into_U0(act, false));
+  FM_TRY(residual_into_U0(act));
   std::vector<double2> hv;
   FM_TRY(multidot<R>(P, nb, 0, U, U, true, act, hv));
   int iter = 0;
@@ -233,25 +306,36 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
       const int K = j + 1;
       std::vector<double2> hcol((size_t)nb * (K + 1));
       if (o.ortho == FM_ORTHO_MGS) {
-        // one sweep for the coefficients (k_gsdot's MGS tail leaves them on the device), one for the subtraction:
-        // two reads of the basis per iteration, where projecting vector by vector reads it twice and w K times
         double2* hd = (double2*)P->hbuf.p;
         const int hs = KV_KMAX + 2;
-        auto kern = k_gsdot<R, false, true>;
-        FM_TRACK(P, KC_DOT, (K + 1) * fbA,
-                 (kern<<<dim3(gs_blocks<R>(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
-                     P->M, nb, K, U, Uw, (double2*)P->red_part.p, nullptr, (unsigned*)P->red_cnt.p, act, nullptr,
-                     nullptr, MgsTail{(double2*)P->mgsT.p, sc, nb, hd, hs})));
-        FM_CK(cudaGetLastError());
-        FM_CK((gs_update<R>(P, nb, K, U, Coef{hd, hs, sc, nb, -1.0, 1}, Uw, true, act, nact)));
         std::vector<double2> hh((size_t)nb * hs), nn(nb);
+        if constexpr (sizeof(R) == 4) {
+          const dim3 g(s32_blocks(P, nb, MGS32_CTAS), nb);
+          for (int i = 0; i <= K; ++i) {
+            const double mb = fbA * ((i > 0 ? 1 : 0) + (i < K ? 1 : 0) + 1 + (i > 0 ? 1 : 0));
+            FM_TRACK(P, KC_MGS, mb,
+                     (k_mgs32<<<g, KV_THREADS, 0, P->st>>>(P->M, nb, i, K, U, sc, nb, Uw, hd, hs,
+                                                           (double2*)P->red_part.p, (unsigned*)P->red_cnt.p, act)));
+          }
+          FM_CK(cudaGetLastError());
+        } else {
+          // one sweep for the coefficients (k_gsdot's MGS tail leaves them on the device), one for the subtraction:
+          // two reads of the basis per iteration, where projecting vector by vector reads it twice and w K times
+          auto kern = k_gsdot<false, true>;
+          FM_TRACK(P, KC_DOT, (K + 1) * fbA,
+                   (kern<<<dim3(gs_blocks(P, kern, nb), nb), KV_THREADS, 0, P->st>>>(
+                       P->M, nb, K, U, Uw, (double2*)P->red_part.p, nullptr, (unsigned*)P->red_cnt.p, act, nullptr,
+                       nullptr, MgsTail{(double2*)P->mgsT.p, sc, nb, hd, hs})));
+          FM_CK(cudaGetLastError());
+          FM_CK((gs_update<R>(P, nb, K, U, Coef{hd, hs, sc, nb, -1.0, 1}, Uw, true, act, nact)));
+          FM_CK(cudaMemcpyAsync(nn.data(), P->red_out.p, nb * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
+        }
         FM_CK(cudaMemcpyAsync(hh.data(), hd, hh.size() * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
-        FM_CK(cudaMemcpyAsync(nn.data(), P->red_out.p, nb * sizeof(double2), cudaMemcpyDeviceToHost, P->st));
         FM_CK(cudaStreamSynchronize(P->st));
         tk_resolve(P);
         for (int b = 0; b < nb; ++b) {
           for (int i = 0; i < K; ++i) hcol[(size_t)b * (K + 1) + i] = hh[(size_t)b * hs + i];
-          hcol[(size_t)b * (K + 1) + K] = nn[b];
+          hcol[(size_t)b * (K + 1) + K] = sizeof(R) == 4 ? hh[(size_t)b * hs + K] : nn[b];
         }
       } else {
         // classical Gram-Schmidt (optionally twice), FP64 coefficients
@@ -366,7 +450,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
       FM_CK(cudaMemcpyAsync(P->coef.p, yh.data(), yh.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
       FM_CK(cudaMemcpyAsync(sc, sch.data(), (size_t)(KV_KMAX + 1) * nb * sizeof(double), cudaMemcpyHostToDevice, P->st));
       Coef cf{(const double2*)P->coef.p, KV_KMAX + 1, sc, nb, 1.0, 1};
-      // each right-hand side reads the vectors of this pass alone: the rest of U may hold anything (residual_into_U0)
+      // each right-hand side reads the vectors of this pass alone: the rest of U may hold anything
       FM_TRY(upload_active());
       FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, act, nb, nullptr, act)));
     }
@@ -378,7 +462,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
     if (any && iter < itmax) {
       // restart: new residual for the RHS still running
       FM_TRY(upload_active());
-      FM_TRY(residual_into_U0(act, true));
+      FM_TRY(residual_into_U0(act));
       FM_TRY(multidot<R>(P, nb, 0, U, U, true, act, hv));
       for (int b = 0; b < nb; ++b)
         if (S[b].active) S[b].beta = std::sqrt(hv[b].x);

@@ -50,15 +50,38 @@ __device__ __forceinline__ void finish_reduce(double2* part, double2* out, unsig
   if (threadIdx.x == 0) counter[b] = 0;
 }
 
-// The same tail for one real value per block (part[b*nblk + blk].x): the first warp sums the partials.
+// The same tail for one real value per block (part[b*nblk + blk].x).  SEQ: in block order, as finish_reduce adds them,
+// by one thread from shared memory; else the first warp sums the partials.
+template <bool SEQ>
 __device__ __forceinline__ void finish_norm(double2* part, double2* out, unsigned* counter, int nblk, int b) {
   __shared__ bool last;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(&counter[b], 1u) == (unsigned)(nblk - 1);
   __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
+  if (!last) return;
   __threadfence();
+  if constexpr (SEQ) {
+    __shared__ double stage[KV_THREADS];
+    double t = 0.0;
+    for (int k0 = 0; k0 < nblk; k0 += blockDim.x) {
+      const int k = k0 + (int)threadIdx.x;
+      if (k < nblk) stage[threadIdx.x] = __ldcg(&part[(size_t)b * nblk + k]).x;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        const int n = min((int)blockDim.x, nblk - k0);
+#pragma unroll 8
+        for (int q = 0; q < n; ++q) t += stage[q];
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      out[b] = make_double2(t, 0.0);
+      counter[b] = 0;
+    }
+    return;
+  }
+  if (threadIdx.x >= 32) return;
   double2 s = make_double2(0.0, 0.0);
   for (int k = threadIdx.x; k < nblk; k += 32) s.x += __ldcg(&part[(size_t)b * nblk + k]).x;
   s = warp_sum(s);
@@ -69,25 +92,20 @@ __device__ __forceinline__ void finish_norm(double2* part, double2* out, unsigne
 }
 
 // ---------------------------------------------------------------------------
-// Gram-Schmidt passes against a stored basis: k_gsdot (inner products) and k_gsupdate (combination).
+// Gram-Schmidt passes against a stored basis, FP64 storage: k_gsdot (inner products) and k_gsupdate (combination).
 //
 // Both stream the basis once from HBM and do little with each value, so bytes in flight decide.  A warp owns one
-// contiguous range of elements and takes GS_GROUP basis vectors at a time, GsCfg::EPT elements a lane from each (192
-// or 256 bytes in flight per thread, no prefetch registers, two CTAs of 8 warps an SM).  k_gsupdate walks its ranges
-// backwards, so its first reads are the elements that k_gsdot read last and L2 still holds.
+// contiguous range of elements and takes GS_GROUP basis vectors at a time, GS_EPT elements a lane from each (256 bytes
+// in flight per thread, no prefetch registers, two CTAs of 8 warps an SM).  k_gsupdate walks its ranges backwards, so its
+// first reads are the elements that k_gsdot read last and L2 still holds.
 //
-// Measured on 50 basis vectors of one 128^3 right-hand side (3 x 128^3 values): FP64 6.6 (dot) and 6.5 TB/s (update);
-// FP32 6.2 and 6.2 TB/s with widen(), 4.2 and 4.8 TB/s at best with the conversion instruction.  Smaller groups, fewer
-// elements a lane, or three CTAs an SM with spills were 5-30 % slower in FP32 (EPT 4: 5.6, 8: 5.9, 6 in pairs: 5.6).
+// Measured on 50 basis vectors of one 128^3 right-hand side (3 x 128^3 values): 6.6 (dot) and 6.5 TB/s (update).
 // ---------------------------------------------------------------------------
 constexpr int GS_GROUP = 4;
-template <typename R> struct GsCfg {
-  static constexpr bool F32 = sizeof(R) == 4;  // basis values go through widen() (fm_complex.cuh)
-  static constexpr int EPT = F32 ? 6 : 4;
-  static constexpr int STEP = 32 * EPT;  // elements of one warp step
-};
+constexpr int GS_EPT = 4;
+constexpr int GS_STEP = 32 * GS_EPT;  // elements of one warp step
 
-// element range [lo, hi) of this warp (multiples of 4, so FP32 ranges start on 32-byte sectors)
+// element range [lo, hi) of this warp
 __device__ __forceinline__ void gs_range(long long M, int nblk, long long& lo, long long& hi) {
   const long long nw = (long long)nblk * KV_WARPS;
   const long long per = ((M + nw - 1) / nw + 3) / 4 * 4;
@@ -166,19 +184,17 @@ struct MgsTail {
 // Optional per-RHS arguments: wtab[b] replaces w + b*M, Kb[b] (<= K) the number of basis vectors.
 // MGS: U_{K-1} is the newest basis vector; mt.h gets the modified Gram-Schmidt coefficients of w against
 // v_0 .. v_{K-1} and row K-1 of mt.T is formed (no `out`).
-// Bound by HBM (MGS in FP64 6.4 TB/s at the size above; in FP32 4.9, where twice the sums per value bind it).
+// Bound by HBM (MGS 6.4 TB/s at the size above).
 // Against one launch per basis vector (three field accesses each, 3.8 TB/s), the MGS form and k_gsupdate took one
 // FP64 solve of 100 iterations on 128^3 from 574 to 220 ms, and on 64^3 from 154 to 38 ms.
-template <typename R, bool WNORM, bool MGS>
-__global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int K, const cplx<R>* __restrict__ U,
-                                                      const cplx<R>* __restrict__ w, double2* __restrict__ part,
+template <bool WNORM, bool MGS>
+__global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int K, const double2* __restrict__ U,
+                                                      const double2* __restrict__ w, double2* __restrict__ part,
                                                       double2* __restrict__ out, unsigned* __restrict__ counter,
                                                       const int* __restrict__ active,
-                                                      const cplx<R>* const* __restrict__ wtab,
+                                                      const double2* const* __restrict__ wtab,
                                                       const int* __restrict__ Kb, MgsTail mt) {
-  using T = cplx<R>;
-  constexpr int EPT = GsCfg<R>::EPT, G = GS_GROUP, NV = MGS ? 2 : 1;  // NV right-hand vectors: w (and U_{K-1})
-  constexpr bool F32 = GsCfg<R>::F32;
+  constexpr int EPT = GS_EPT, G = GS_GROUP, NV = MGS ? 2 : 1;  // NV right-hand vectors: w (and U_{K-1})
   constexpr int NQ = G * NV * 2;
   static_assert(!(WNORM && MGS), "the norm belongs to the plain dot");
   __shared__ double acc[KV_WARPS][(KV_KMAX + G) * NV * 2];
@@ -191,34 +207,29 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int
   __syncwarp();
   long long lo, hi;
   gs_range(M, nblk, lo, hi);
-  const T* wb = wtab ? wtab[b] : w + (size_t)b * M;
+  const double2* wb = wtab ? wtab[b] : w + (size_t)b * M;
   const int Kr = Kb ? Kb[b] : K;
   const size_t us = (size_t)B * M;
-  const T* ub = U + (size_t)b * M;
+  const double2* ub = U + (size_t)b * M;
   double nrm = 0.0;
-  for (long long c0 = lo; c0 < hi; c0 += GsCfg<R>::STEP) {
+  for (long long c0 = lo; c0 < hi; c0 += GS_STEP) {
     double2 wv[NV][EPT];
     bool in[EPT];
 #pragma unroll
     for (int k = 0; k < EPT; ++k) {
       const long long e = c0 + 32 * k + lane;
       in[k] = e < hi;
-      wv[0][k] = in[k] ? to_d(wb[e]) : make_double2(0.0, 0.0);
-      if constexpr (MGS) wv[1][k] = in[k] ? to_d(ub[(size_t)(K - 1) * us + e]) : make_double2(0.0, 0.0);
+      wv[0][k] = in[k] ? wb[e] : make_double2(0.0, 0.0);
+      if constexpr (MGS) wv[1][k] = in[k] ? ub[(size_t)(K - 1) * us + e] : make_double2(0.0, 0.0);
       if constexpr (WNORM) nrm = fma(wv[0][k].x, wv[0][k].x, fma(wv[0][k].y, wv[0][k].y, nrm));
-      if constexpr (F32) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) wv[v][k] = cscale(wv[v][k], WIDEN_HALF);
-      }
     }
     for (int i0 = 0; i0 < Kr; i0 += G) {
-      T u[G][EPT];
+      double2 u[G][EPT];
 #pragma unroll
       for (int g = 0; g < G; ++g)
 #pragma unroll
         for (int k = 0; k < EPT; ++k) {
-          u[g][k].x = 0;
-          u[g][k].y = 0;
+          u[g][k] = make_double2(0.0, 0.0);
           if (i0 + g < Kr && in[k]) u[g][k] = ub[(size_t)(i0 + g) * us + c0 + 32 * k + lane];
         }
       double s[NQ];
@@ -227,15 +238,9 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
           double sx = 0.0, sy = 0.0;
-          if constexpr (F32) {
-            float bad = 0.0f;
-#pragma unroll
-            for (int k = 0; k < EPT; ++k) nonfinite_mark(bad, u[g][k]);
-            sx = mark_d(bad);
-          }
 #pragma unroll
           for (int k = 0; k < EPT; ++k) {
-            const double2 x = widen(u[g][k]);
+            const double2 x = u[g][k];
             sx = fma(x.x, wv[v][k].x, fma(x.y, wv[v][k].y, sx));
             sy = fma(x.x, wv[v][k].y, fma(-x.y, wv[v][k].x, sy));
           }
@@ -264,7 +269,6 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsdot(long long M, int B, int
         s.y += acc[q][2 * o + 1];
       }
     }
-    if (F32 && !(WNORM && o == K)) s = cscale(s, WIDEN_HALF);
     part[((size_t)b * NO + o) * nblk + blockIdx.x] = s;
   }
   __threadfence();
@@ -368,31 +372,28 @@ struct Coef {
   }
 };
 
-// w[b] += sum_i coef(b,i) * U_i[b]   (FP64 accumulation); optional out[b] = ||w'||^2 (of the stored values).
-// Optional per-RHS arguments as in k_gsdot.
-template <typename R, bool NORM>
-__global__ void __launch_bounds__(KV_THREADS, 2) k_gsupdate(long long M, int B, int K, const cplx<R>* __restrict__ U,
-                                                         Coef cf, cplx<R>* __restrict__ w,
+// w[b] += sum_i coef(b,i) * U_i[b]; optional out[b] = ||w'||^2.  FP64 storage; optional per-RHS arguments as in k_gsdot.
+template <bool NORM>
+__global__ void __launch_bounds__(KV_THREADS, 2) k_gsupdate(long long M, int B, int K, const double2* __restrict__ U,
+                                                         Coef cf, double2* __restrict__ w,
                                                          double2* __restrict__ part, double2* __restrict__ out,
                                                          unsigned* __restrict__ counter, const int* __restrict__ active,
-                                                         cplx<R>* const* __restrict__ wtab,
+                                                         double2* const* __restrict__ wtab,
                                                          const int* __restrict__ Kb) {
-  using T = cplx<R>;
-  constexpr int EPT = GsCfg<R>::EPT, G = GS_GROUP, STEP = GsCfg<R>::STEP;
-  constexpr bool F32 = GsCfg<R>::F32;
+  constexpr int EPT = GS_EPT, G = GS_GROUP, STEP = GS_STEP;
   __shared__ double2 cs[KV_KMAX + G];
   __shared__ double red[KV_WARPS];
   const int b = blockIdx.y, nblk = gridDim.x;
   if (active && !active[b]) return;
   const int Kr = Kb ? Kb[b] : K;
-  for (int i = threadIdx.x; i < Kr; i += blockDim.x) cs[i] = F32 ? cscale(cf.get(b, i), WIDEN_HALF) : cf.get(b, i);
+  for (int i = threadIdx.x; i < Kr; i += blockDim.x) cs[i] = cf.get(b, i);
   __syncthreads();
   const int lane = threadIdx.x & 31;
   long long lo, hi;
   gs_range(M, nblk, lo, hi);
   const size_t us = (size_t)B * M;
-  const T* ub = U + (size_t)b * M;
-  T* wb = wtab ? wtab[b] : w + (size_t)b * M;
+  const double2* ub = U + (size_t)b * M;
+  double2* wb = wtab ? wtab[b] : w + (size_t)b * M;
   double nrm = 0.0;
   if (lo < hi) {
     for (long long c0 = lo + (hi - lo - 1) / STEP * STEP; c0 >= lo; c0 -= STEP) {
@@ -402,20 +403,15 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsupdate(long long M, int B, 
       for (int k = 0; k < EPT; ++k) {
         const long long e = c0 + 32 * k + lane;
         in[k] = e < hi;
-        acc[k] = in[k] ? to_d(wb[e]) : make_double2(0.0, 0.0);
-        if constexpr (F32) acc[k] = cscale(acc[k], 1.0 / WIDEN_HALF);
+        acc[k] = in[k] ? wb[e] : make_double2(0.0, 0.0);
       }
-      float bad[EPT];
-#pragma unroll
-      for (int k = 0; k < EPT; ++k) bad[k] = 0.0f;
       for (int i0 = 0; i0 < Kr; i0 += G) {
-        T u[G][EPT];
+        double2 u[G][EPT];
 #pragma unroll
         for (int g = 0; g < G; ++g)
 #pragma unroll
           for (int k = 0; k < EPT; ++k) {
-            u[g][k].x = 0;
-            u[g][k].y = 0;
+            u[g][k] = make_double2(0.0, 0.0);
             if (i0 + g < Kr && in[k]) u[g][k] = ub[(size_t)(i0 + g) * us + c0 + 32 * k + lane];
           }
 #pragma unroll
@@ -424,24 +420,16 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsupdate(long long M, int B, 
           const double2 c = cs[i0 + g];
 #pragma unroll
           for (int k = 0; k < EPT; ++k) {
-            nonfinite_mark(bad[k], u[g][k]);
-            const double2 x = widen(u[g][k]);
-            acc[k].x = fma(c.x, x.x, fma(-c.y, x.y, acc[k].x));
-            acc[k].y = fma(c.x, x.y, fma(c.y, x.x, acc[k].y));
+            acc[k].x = fma(c.x, u[g][k].x, fma(-c.y, u[g][k].y, acc[k].x));
+            acc[k].y = fma(c.x, u[g][k].y, fma(c.y, u[g][k].x, acc[k].y));
           }
         }
       }
 #pragma unroll
       for (int k = 0; k < EPT; ++k) {
         if (in[k]) {
-          if constexpr (F32) acc[k] = make_double2(fma(acc[k].x, WIDEN_HALF, mark_d(bad[k])),
-                                                   fma(acc[k].y, WIDEN_HALF, mark_d(bad[k])));
-          const T r = from_d<T>(acc[k]);
-          wb[c0 + 32 * k + lane] = r;
-          if constexpr (NORM) {
-            const double2 rd = to_d(r);
-            nrm = fma(rd.x, rd.x, fma(rd.y, rd.y, nrm));
-          }
+          wb[c0 + 32 * k + lane] = acc[k];
+          if constexpr (NORM) nrm = fma(acc[k].x, acc[k].x, fma(acc[k].y, acc[k].y, nrm));
         }
       }
     }
@@ -455,7 +443,242 @@ __global__ void __launch_bounds__(KV_THREADS, 2) k_gsupdate(long long M, int B, 
       for (int q = 0; q < KV_WARPS; ++q) t += red[q];
       part[(size_t)b * nblk + blockIdx.x] = make_double2(t, 0.0);
     }
-    finish_norm(part, out, counter, nblk, b);
+    finish_norm<false>(part, out, counter, nblk, b);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// FP32 storage: k_dot32 and k_update32, the same sums with a fixed order.
+//
+// A solve that stores its vectors in FP32 rounds every value of every pass, and which way a value near a tie falls
+// hangs on the last bits of the FP64 number before it.  One different bit there changes one stored value, the next
+// transform carries that to all of them, and after four applications the whole rounding noise is another one: two
+// orders of arithmetic gave GMRES(20) fields on 512 x 64 x 512 that are 2.4e-5 apart, each 1.6e-5 from the exact ones.
+// So the order of these sums belongs to the result: blocks of whole chunks of KV_THREADS * KV_EPT elements, as many as
+// three CTAs an SM hold; within a chunk eight elements a thread, a stride of KV_THREADS apart, then the warp's tree,
+// then the chunks, the warps and the blocks one after another.
+//
+// Values go through widen() (exact, so it is no part of the order).  Bound by HBM as k_gsdot.  A block's eight warps of
+// elements are run by four warps, two each: three CTAs an SM then have 168 registers a thread, for four vectors at a
+// time: 5.9 TB/s the dot and 6.2 the update on 128^3 with 100 vectors, 5.8 and 6.1 on 256^3 with 20 (eight warps and 80
+// registers: two vectors at a time, spills, 5.0 and 5.2; with the conversion instruction 4.7 and 5.0).
+// ---------------------------------------------------------------------------
+constexpr int S32_CTAS = 3;      // CTAs an SM: with the chunk, what fixes the blocks
+constexpr int S32_THREADS = 128;
+constexpr int S32_GROUP = 4;     // basis vectors at a time
+
+// out[b][i] = sum_e conj(U_i[b][e]) * w[b][e] (i < K), plus out[b][K] = ||w||^2 when WNORM; arguments as k_gsdot
+template <bool WNORM>
+__global__ void __launch_bounds__(S32_THREADS, S32_CTAS) k_dot32(long long M, int B, int K, const float2* __restrict__ U,
+                                                              const float2* __restrict__ w, double2* __restrict__ part,
+                                                              double2* __restrict__ out, unsigned* __restrict__ counter,
+                                                              const int* __restrict__ active,
+                                                              const float2* const* __restrict__ wtab,
+                                                              const int* __restrict__ Kb) {
+  constexpr int EPT = KV_EPT, G = S32_GROUP;
+  __shared__ double acc[KV_WARPS][(KV_KMAX + G) * 2];  // times 1 / WIDEN_HALF
+  __shared__ double nacc[KV_WARPS];
+  __shared__ bool last;
+  const int b = blockIdx.y, nblk = gridDim.x;
+  const int KK = K + (WNORM ? 1 : 0);
+  if (active && !active[b]) return;  // uniform per block; no reduction is issued for inactive RHS
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x; i < KV_WARPS * (KV_KMAX + G) * 2; i += S32_THREADS) (&acc[0][0])[i] = 0.0;
+  if (threadIdx.x < KV_WARPS) nacc[threadIdx.x] = 0.0;
+  __syncthreads();
+  const long long chunk = (long long)KV_THREADS * EPT;
+  const long long per = ((M + nblk - 1) / nblk + chunk - 1) / chunk * chunk;
+  const long long lo = (long long)blockIdx.x * per, hi = min(M, lo + per);
+  const float2* wb = wtab ? wtab[b] : w + (size_t)b * M;
+  const int Kr = Kb ? Kb[b] : K;
+  const size_t us = (size_t)B * M;
+  const float2* ub = U + (size_t)b * M;
+  for (long long c0 = lo; c0 < hi; c0 += chunk)
+#pragma unroll 1
+    for (int t0 = threadIdx.x; t0 < KV_THREADS; t0 += S32_THREADS) {
+      const int wi = t0 >> 5;
+      const long long e0 = c0 + t0;
+      const int nk = (int)min((long long)EPT, (hi - e0 + KV_THREADS - 1) / KV_THREADS);  // elements of this lane (<= 0: none)
+      double2 wv[EPT];
+#pragma unroll
+      for (int k = 0; k < EPT; ++k) wv[k] = k < nk ? to_d(wb[e0 + k * KV_THREADS]) : make_double2(0.0, 0.0);
+      if constexpr (WNORM) {
+        double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < EPT; ++k) s.x = fma(wv[k].x, wv[k].x, fma(wv[k].y, wv[k].y, s.x));
+        s = warp_sum(s);
+        if (lane == 0) nacc[wi] += s.x;
+      }
+#pragma unroll
+      for (int k = 0; k < EPT; ++k) wv[k] = cscale(wv[k], WIDEN_HALF);
+      for (int i0 = 0; i0 < Kr; i0 += G) {
+        float2 u[G][EPT];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const float2* p = ub + (size_t)(i0 + g) * us + e0;
+          const int n = i0 + g < Kr ? nk : 0;
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            u[g][k] = make_float2(0.0f, 0.0f);
+            if (k < n) u[g][k] = p[k * KV_THREADS];
+          }
+        }
+        double s[2 * G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          float bad = 0.0f;
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) nonfinite_mark(bad, u[g][k]);
+          double sx = mark_d(bad), sy = 0.0;
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            const double2 x = widen(u[g][k]);
+            sx = fma(x.x, wv[k].x, fma(x.y, wv[k].y, sx));
+            sy = fma(x.x, wv[k].y, fma(-x.y, wv[k].x, sy));
+          }
+          s[2 * g] = sx;
+          s[2 * g + 1] = sy;
+        }
+        const double t = warp_transpose_sum<2 * G>(s);  // the sums of warp_sum, bit for bit
+        constexpr int LPV = 32 / (2 * G);               // lanes per value
+        if ((lane & (LPV - 1)) == 0) acc[wi][2 * i0 + lane / LPV] += t;
+      }
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < KK; i += S32_THREADS) {
+    double2 s = make_double2(0.0, 0.0);
+    for (int q = 0; q < KV_WARPS; ++q) {
+      if (WNORM && i == K) {
+        s.x += nacc[q];
+      } else {
+        s.x += acc[q][2 * i];
+        s.y += acc[q][2 * i + 1];
+      }
+    }
+    if (!(WNORM && i == K)) s = cscale(s, WIDEN_HALF);
+    part[((size_t)b * nblk + blockIdx.x) * KK + i] = s;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&counter[b], 1u) == (unsigned)(nblk - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // the blocks one after another, a value a thread; the loads of sixteen blocks are in flight at a time
+  for (int i = threadIdx.x; i < KK; i += S32_THREADS) {
+    double2 s = make_double2(0.0, 0.0);
+    const double2* p = part + (size_t)b * nblk * KK + i;
+#pragma unroll 16
+    for (int k = 0; k < nblk; ++k) {
+      const double2 v = __ldcg(p + (size_t)k * KK);
+      s.x += v.x;
+      s.y += v.y;
+    }
+    out[(size_t)b * KK + i] = s;
+  }
+  if (threadIdx.x == 0) counter[b] = 0;
+}
+
+// w[b] += sum_i coef(b,i) * U_i[b], optional out[b] = ||w'||^2 (of the stored values); arguments as k_gsupdate
+template <bool NORM>
+__global__ void __launch_bounds__(S32_THREADS, S32_CTAS) k_update32(long long M, int B, int K, const float2* __restrict__ U,
+                                                                 Coef cf, float2* __restrict__ w,
+                                                                 double2* __restrict__ part, double2* __restrict__ out,
+                                                                 unsigned* __restrict__ counter,
+                                                                 const int* __restrict__ active,
+                                                                 float2* const* __restrict__ wtab,
+                                                                 const int* __restrict__ Kb) {
+  constexpr int EPT = KV_EPT, G = S32_GROUP, HALVES = KV_THREADS / S32_THREADS;
+  __shared__ double2 cs[KV_KMAX + G];  // times WIDEN_HALF
+  __shared__ double red[KV_WARPS];
+  const int b = blockIdx.y, nblk = gridDim.x;
+  if (active && !active[b]) return;
+  const int Kr = Kb ? Kb[b] : K;
+  for (int i = threadIdx.x; i < Kr; i += S32_THREADS) cs[i] = cscale(cf.get(b, i), WIDEN_HALF);
+  __syncthreads();
+  const long long chunk = (long long)KV_THREADS * EPT;
+  const long long per = ((M + nblk - 1) / nblk + chunk - 1) / chunk * chunk;
+  const long long lo = (long long)blockIdx.x * per, hi = min(M, lo + per);
+  const size_t us = (size_t)B * M;
+  const float2* ub = U + (size_t)b * M;
+  float2* wb = wtab ? wtab[b] : w + (size_t)b * M;
+  double nrm[HALVES] = {};
+  for (long long c0 = lo; c0 < hi; c0 += chunk)
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) {
+      const long long e0 = c0 + h * S32_THREADS + threadIdx.x;
+      const int nk = (int)min((long long)EPT, (hi - e0 + KV_THREADS - 1) / KV_THREADS);
+      double2 acc[EPT];
+#pragma unroll
+      for (int k = 0; k < EPT; ++k)
+        acc[k] = k < nk ? cscale(to_d(wb[e0 + k * KV_THREADS]), 1.0 / WIDEN_HALF) : make_double2(0.0, 0.0);
+      float bad = 0.0f;
+      for (int i0 = 0; i0 < Kr; i0 += G) {
+        float2 u[G][EPT];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const float2* p = ub + (size_t)(i0 + g) * us + e0;
+          const int n = i0 + g < Kr ? nk : 0;
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            u[g][k] = make_float2(0.0f, 0.0f);
+            if (k < n) u[g][k] = p[k * KV_THREADS];
+          }
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          if (i0 + g >= Kr) break;  // uniform
+          const double2 c = cs[i0 + g];
+#pragma unroll
+          for (int k = 0; k < EPT; ++k) {
+            nonfinite_mark(bad, u[g][k]);
+            const double2 x = widen(u[g][k]);
+            acc[k].x = fma(c.x, x.x, fma(-c.y, x.y, acc[k].x));
+            acc[k].y = fma(c.x, x.y, fma(c.y, x.x, acc[k].y));
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < EPT; ++k) acc[k] = cscale(acc[k], WIDEN_HALF);
+      if (bad != 0.0f) {  // an infinity or a NaN among the vectors: these elements again by conversion
+#pragma unroll
+        for (int k = 0; k < EPT; ++k) {
+          if (k >= nk) break;
+          double2 a = to_d(wb[e0 + k * KV_THREADS]);
+#pragma unroll 1
+          for (int i = 0; i < Kr; ++i) {
+            const double2 c = cscale(cs[i], 1.0 / WIDEN_HALF), x = to_d(ub[(size_t)i * us + e0 + k * KV_THREADS]);
+            a.x = fma(c.x, x.x, fma(-c.y, x.y, a.x));
+            a.y = fma(c.x, x.y, fma(c.y, x.x, a.y));
+          }
+          acc[k] = a;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < EPT; ++k) {
+        if (k < nk) {
+          const float2 r = from_d<float2>(acc[k]);
+          wb[e0 + k * KV_THREADS] = r;
+          if constexpr (NORM) {
+            const double2 rd = to_d(r);
+            nrm[h] = fma(rd.x, rd.x, fma(rd.y, rd.y, nrm[h]));
+          }
+        }
+      }
+    }
+  if constexpr (NORM) {
+#pragma unroll
+    for (int h = 0; h < HALVES; ++h) {
+      const double2 s = warp_sum(make_double2(nrm[h], 0.0));
+      if ((threadIdx.x & 31) == 0) red[(h * S32_THREADS + threadIdx.x) >> 5] = s.x;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int q = 0; q < KV_WARPS; ++q) t += red[q];
+      part[(size_t)b * nblk + blockIdx.x] = make_double2(t, 0.0);
+    }
+    finish_norm<true>(part, out, counter, nblk, b);
   }
 }
 
@@ -986,7 +1209,7 @@ __global__ void __launch_bounds__(KV_THREADS) k_axpby3(long long M, const cplx<R
       for (int q = 0; q < KV_WARPS; ++q) t += red[q];
       part[(size_t)b * nblk + blockIdx.x] = make_double2(t, 0.0);
     }
-    finish_norm(part, out, counter, nblk, b);
+    finish_norm<sizeof(R) == 4>(part, out, counter, nblk, b);
   }
 }
 

@@ -43,11 +43,12 @@ template <typename S, typename R>
 cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenParams& gp, const void* twz,
                           const void* rz, void* out, const int* active, int* err, int sms, cudaStream_t st);
 
-// z pass in sixteen values a lane (k_zreg): nz 64, 128, 256 or 512, nx a multiple of the tile (zreg_takes).
-// branches 2: the z-only average in one sweep, rz = exp(-2 pi i z/(4 nz)) and gp.shift[2] = 1/4; branches 1: one branch
-// as ZMODE_ONE (rz null without a shift).  twz: the table of twiddles16(nz).
+// z pass in sixteen values a lane (k_zreg), nx a multiple of the tile.  branches 2: the z-only average in one sweep,
+// rz = exp(-2 pi i z/(4 nz)) and gp.shift[2] = 1/4; branches 1: one branch as ZMODE_ONE (rz null without a shift).
+// zreg_length: the length n of its transforms, nz or 2 nz, where it takes the shape, else 0.  twz: the table of
+// twiddles16(n).
 template <typename S, typename R>
-bool zreg_takes(const Dims& d, int branches);
+int zreg_length(const Dims& d, int branches);
 template <typename S, typename R>
 cudaError_t launch_zreg(const Dims& d, int branches, const void* in, const GreenParams& gp, const void* twz,
                         const void* rz, void* out, const int* active, int* err, int sms, cudaStream_t st);

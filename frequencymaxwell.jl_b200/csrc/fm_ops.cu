@@ -10,6 +10,80 @@
 //   epi : EPI_* epilogue applied to g = G_avg(psi)
 // ---------------------------------------------------------------------------
 
+// The Green application / CBS operator of green_op on a plan of the FP32-arithmetic general passes.  Per branch:
+// PRE (potential, forward ramps) -> forward DFT along x, y, z -> Green of the branch -> inverse DFT along z, y,
+// x -> POST (reverse ramps, epilogue).  With an absorbing axis the +s branch stores half its result in t3 and
+// the -s branch adds it before the epilogue (dyadic_green.jl:127-152).
+static fm_status gen_green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs, int epi, const void* xv,
+                              const void* bv, const EpiParams& ep_in, void* out, const int* act, int nact,
+                              const RhsCtx* rc) {
+  using T = float2;
+  if (nact < 0) nact = nb;
+  EpiParams ep = ep_in;
+  if (rc) ep.inv_eps_b = rc->inv_eps_b;
+  Dims d = P->dims;
+  d.nb = nb;
+  const size_t fbytes = (size_t)nb * P->M * sizeof(T);
+  const double fbA = (double)nact * P->M * sizeof(T), vb = (double)nact * P->n * sizeof(T);
+  FM_CK(P->t1.ensure(fbytes));
+  const int nbr = P->avg ? 2 : 1;
+  if (nbr == 2) FM_CK(P->t3.ensure(fbytes));
+  GreenParams gp{};
+  const double kr = std::sqrt(P->kref2);
+  for (int a = 0; a < 3; ++a) gp.dk[a] = 2.0 * M_PI / ((double)(a == 0 ? d.nx : a == 1 ? d.ny : d.nz) * P->desc.resolution[a]) / kr;
+  gp.ksq_re = P->k_bg * P->k_bg / P->kref2;
+  gp.ksq_im = P->eps_imag / P->kref2;
+  gp.scale_re = 1.0 / ((double)P->n * nbr);
+  const void* V = P->V.p;
+  VecTab vt{};
+  if (rc) {
+    V = rc->V;
+    d.vstride = rc->vstride;
+    gp.ksq_im_b = rc->ksq_im_b;
+    vt = rc->vt;
+  }
+  double postb = 2 * fbA;
+  if (epi != EPI_STORE) postb += fbA;
+  if (epi == EPI_PREC_RES) postb += fbA;
+  if (epi == EPI_PREC_OP || epi == EPI_PREC_RES) postb += vb;
+  if (epi == EPI_OP && (ep.beta_re != 0.0 || ep.beta_im != 0.0)) postb += fbA;
+  const DevBuf* rpos[3] = {&P->rxp, &P->ryp, &P->rzp};
+  const DevBuf* rneg[3] = {&P->rxm, &P->rym, &P->rzm};
+  cudaError_t e;
+  for (int br = 0; br < nbr; ++br) {
+    GenRamps rp;
+    for (int a = 0; a < 3; ++a) {
+      gp.shift[a] = (br == 0 ? 1.0 : -1.0) * P->shift[a];
+      rp.r[a] = P->shift[a] != 0.0 ? (br == 0 ? rpos[a]->p : rneg[a]->p) : nullptr;
+    }
+    FM_TRACK(P, KC_XF, 2 * fbA + (pro != PRO_COPY ? vb : 0.0),
+             e = launch_gen_pre(d, pro, in, V, rs, rp, P->t1.p, act, P->st, vt));
+    FM_CK(e);
+    for (int a = 0; a < 3; ++a) {
+      FM_TRACK(P, KC_YF, 2 * fbA, e = launch_gen_axis(d, a, -1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+      FM_CK(e);
+    }
+    FM_TRACK(P, KC_ZG, 2 * fbA, e = launch_gen_kspace(d, ZMODE_ONE, P->t1.p, gp, act, P->st));
+    FM_CK(e);
+    for (int a = 2; a >= 0; --a) {
+      FM_TRACK(P, KC_YI, 2 * fbA, e = launch_gen_axis(d, a, +1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+      FM_CK(e);
+    }
+    if (nbr == 2 && br == 0) {
+      EpiParams e0{};
+      FM_TRACK(P, KC_XI, 2 * fbA,
+               e = launch_gen_post(d, EPI_STORE, P->t1.p, V, nullptr, nullptr, nullptr, e0, rp, P->t3.p, act, P->st));
+    } else {
+      EpiParams e1 = ep;
+      if (nbr == 2) e1.gadd = P->t3.p;
+      FM_TRACK(P, KC_XI, postb + (nbr == 2 ? fbA : 0.0),
+               e = launch_gen_post(d, epi, P->t1.p, V, xv, bv, rs, e1, rp, out, act, P->st, vt));
+    }
+    FM_CK(e);
+  }
+  return FM_OK;
+}
+
 template <typename R>
 fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs, int epi, const void* xv,
                    const void* bv, const EpiParams& ep_in, void* out, const int* act, int nact, const RhsCtx* rc,
@@ -20,6 +94,7 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
         ((chain & GREEN_CHAIN_NEXT_XF) && (epi != EPI_PREC_OP || rs || xv != in)))
       return fail(FM_ERR_INVALID, "operator chaining needs the fused passes, PRO_V and EPI_PREC_OP on the input");
   }
+  if (P->general32) return gen_green_op(P, nb, in, pro, rs, epi, xv, bv, ep_in, out, act, nact, rc);
   if (nact < 0) nact = nb;
   EpiParams ep = ep_in;
   if (rc) ep.inv_eps_b = rc->inv_eps_b;
@@ -32,13 +107,8 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
   Dims d = P->dims;
   d.nb = nb;
   const size_t fbytes = (size_t)nb * P->M * sizeof(T);
-  const bool own = !(rc && rc->tmp[0]);
-  if (own) {
-    FM_CK(P->t1.ensure(fbytes));
-    FM_CK(P->t2.ensure(fbytes));
-  }
-  void* const t1 = own ? P->t1.p : rc->tmp[0];
-  void* const t2 = own ? P->t2.p : rc->tmp[1];
+  FM_CK(P->t1.ensure(fbytes));
+  FM_CK(P->t2.ensure(fbytes));
   GreenParams gp{};
   const double kr = std::sqrt(P->kref2);
   for (int a = 0; a < 3; ++a) gp.dk[a] = 2.0 * M_PI / ((double)(a == 0 ? d.nx : a == 1 ? d.ny : d.nz) * P->desc.resolution[a]) / kr;
@@ -57,41 +127,41 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
     cudaError_t e;
     if (!(chain & GREEN_CHAIN_HAVE_XF)) {
       FM_TRACK(P, KC_XF, 2 * fbA + (pro != PRO_COPY ? vb : 0.0),
-               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, nullptr, t1, act, vt));
+               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, nullptr, P->t1.p, act, vt));
       FM_CK(e);
     }
-    FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, t1, P->twy.p, nullptr, t2, act));
+    FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, P->t1.p, P->twy.p, nullptr, P->t2.p, act));
     FM_CK(e);
     if (P->avg && has_zreg<R>(P, d, 2)) {
       gp.shift[2] = P->shift[2];
       gp.scale_re = 1.0 / ((double)P->n * 2.0);
-      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zreg<R>(P, d, 2, t2, gp, P->zonly ? P->rz.p : P->rzp.p, t1, act));
+      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zreg<R>(P, d, 2, P->t2.p, gp, P->zonly ? P->rz.p : P->rzp.p, P->t1.p, act));
       FM_CK(e);
     } else if (P->zsplit) {
       // the two z branches (+s, -s) as two length-L z passes with their phase ramps; the second adds to the first
       gp.scale_re = 1.0 / ((double)P->n * 2.0);
       gp.shift[2] = P->shift[2];
       gp.accumulate = 0;
-      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, t2, gp, P->twz.p, P->rzp.p, t1, act));
+      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, P->t2.p, gp, P->twz.p, P->rzp.p, P->t1.p, act));
       FM_CK(e);
       gp.shift[2] = -P->shift[2];
       gp.accumulate = 1;
-      FM_TRACK(P, KC_ZG, 3 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, t2, gp, P->twz.p, P->rzm.p, t1, act));
+      FM_TRACK(P, KC_ZG, 3 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, P->t2.p, gp, P->twz.p, P->rzm.p, P->t1.p, act));
       FM_CK(e);
     } else {
       gp.shift[2] = P->zonly ? P->shift[2] : 0.0;
       gp.scale_re = 1.0 / ((double)P->n * (P->zonly ? 2.0 : 1.0));
       FM_TRACK(P, KC_ZG, 2 * fbA,
-               e = pass_zg<R>(P, d, P->zonly ? ZMODE_AVG2 : ZMODE_ONE, t2, gp, P->zonly ? P->twz2.p : P->twz.p,
-                              P->zonly ? P->rz.p : nullptr, t1, act));
+               e = pass_zg<R>(P, d, P->zonly ? ZMODE_AVG2 : ZMODE_ONE, P->t2.p, gp, P->zonly ? P->twz2.p : P->twz.p,
+                              P->zonly ? P->rz.p : nullptr, P->t1.p, act));
       FM_CK(e);
     }
-    FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, t1, P->twy.p, nullptr, t2, act));
+    FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, P->t1.p, P->twy.p, nullptr, P->t2.p, act));
     FM_CK(e);
     if (chain & GREEN_CHAIN_NEXT_XF)
-      FM_TRACK(P, KC_XI, xib + fbA, e = pass_xi_xf<R>(P, d, t2, V, xv, ep, P->twx.p, out, t1, act));
+      FM_TRACK(P, KC_XI, xib + fbA, e = pass_xi_xf<R>(P, d, P->t2.p, V, xv, ep, P->twx.p, out, P->t1.p, act));
     else
-      FM_TRACK(P, KC_XI, xib, e = pass_xi<R>(P, d, epi, t2, V, xv, bv, rs, ep, P->twx.p, nullptr, out, act, vt));
+      FM_TRACK(P, KC_XI, xib, e = pass_xi<R>(P, d, epi, P->t2.p, V, xv, bv, rs, ep, P->twx.p, nullptr, out, act, vt));
     FM_CK(e);
     return FM_OK;
   }
@@ -101,8 +171,7 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
   // shifted k (dyadic_green.jl:189-221).  Branch + stores half of G(+s) psi in t3; branch - adds it to half of
   // G(-s) psi in the XI pass, before the epilogue.
   {
-    if (own) FM_CK(P->t3.ensure(fbytes));
-    void* const t3 = own ? P->t3.p : rc->tmp[2];
+    FM_CK(P->t3.ensure(fbytes));
     gp.scale_re = 1.0 / ((double)P->n * 2.0);
     cudaError_t e;
     for (int br = 0; br < 2; ++br) {
@@ -112,24 +181,24 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
       const void* ry = P->shift[1] != 0.0 ? (br == 0 ? P->ryp.p : P->rym.p) : nullptr;
       const void* rzt = P->shift[2] != 0.0 ? (br == 0 ? P->rzp.p : P->rzm.p) : nullptr;
       FM_TRACK(P, KC_XF, 2 * fbA + (pro != PRO_COPY ? vb : 0.0),
-               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, rx, t1, act, vt));
+               e = pass_xf<R>(P, d, pro, in, V, rs, P->twx.p, rx, P->t1.p, act, vt));
       FM_CK(e);
-      FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, t1, P->twy.p, ry, t2, act));
+      FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, P->t1.p, P->twy.p, ry, P->t2.p, act));
       FM_CK(e);
-      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, t2, gp, P->twz.p, rzt, t1, act));
+      FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zg<R>(P, d, ZMODE_ONE, P->t2.p, gp, P->twz.p, rzt, P->t1.p, act));
       FM_CK(e);
-      FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, t1, P->twy.p, ry, t2, act));
+      FM_TRACK(P, KC_YI, 2 * fbA, e = pass_y<R>(P, d, +1, P->t1.p, P->twy.p, ry, P->t2.p, act));
       FM_CK(e);
       if (br == 0) {
         EpiParams e0{};
         FM_TRACK(P, KC_XI, 2 * fbA,
-                 e = pass_xi<R>(P, d, EPI_STORE, t2, V, nullptr, nullptr, nullptr, e0, P->twx.p, rx, t3,
+                 e = pass_xi<R>(P, d, EPI_STORE, P->t2.p, V, nullptr, nullptr, nullptr, e0, P->twx.p, rx, P->t3.p,
                                 act));
       } else {
         EpiParams e1 = ep;
-        e1.gadd = t3;
+        e1.gadd = P->t3.p;
         FM_TRACK(P, KC_XI, xib + fbA,
-                 e = pass_xi<R>(P, d, epi, t2, V, xv, bv, rs, e1, P->twx.p, rx, out, act, vt));
+                 e = pass_xi<R>(P, d, epi, P->t2.p, V, xv, bv, rs, e1, P->twx.p, rx, out, act, vt));
       }
       FM_CK(e);
     }
@@ -155,6 +224,25 @@ fm_status curl_batch(fm_plan* P, int nb, const void* in, void* out, const int* a
   gp.scale_im = -f;
   const double cb = 2.0 * nb * P->M * sizeof(T);
   cudaError_t e;
+  if (P->general32) {
+    GenRamps none;
+    FM_TRACK(P, KC_CURL, cb, e = launch_gen_pre(d, PRO_COPY, in, nullptr, nullptr, none, P->t1.p, act, P->st));
+    FM_CK(e);
+    for (int a = 0; a < 3; ++a) {
+      FM_TRACK(P, KC_CURL, cb, e = launch_gen_axis(d, a, -1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+      FM_CK(e);
+    }
+    FM_TRACK(P, KC_CURL, cb, e = launch_gen_kspace(d, ZMODE_CURL, P->t1.p, gp, act, P->st));
+    FM_CK(e);
+    for (int a = 2; a >= 0; --a) {
+      FM_TRACK(P, KC_CURL, cb, e = launch_gen_axis(d, a, +1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+      FM_CK(e);
+    }
+    FM_TRACK(P, KC_CURL, cb,
+             e = launch_gen_post(d, EPI_STORE, P->t1.p, nullptr, nullptr, nullptr, nullptr, ep, none, out, act, P->st));
+    FM_CK(e);
+    return FM_OK;
+  }
   FM_TRACK(P, KC_CURL, cb, e = pass_xf<R>(P, d, PRO_COPY, in, nullptr, nullptr, P->twx.p, nullptr, P->t1.p, act));
   FM_CK(e);
   FM_TRACK(P, KC_CURL, cb, e = pass_y<R>(P, d, -1, P->t1.p, P->twy.p, nullptr, P->t2.p, act));

@@ -18,7 +18,7 @@ template cudaError_t launch_y_tma<float, float>(const Dims&, int, const void*, c
                                           const int*, int*, int, cudaStream_t);
 template cudaError_t launch_zg_tma<float, float>(const Dims&, int, const void*, const GreenParams&, const void*,
                                           const void*, void*, const int*, int*, int, cudaStream_t);
-template bool zreg_takes<float, float>(const Dims&, int);
+template int zreg_length<float, float>(const Dims&, int);
 template cudaError_t launch_zreg<float, float>(const Dims&, int, const void*, const GreenParams&, const void*, const void*,
                                           void*, const int*, int*, int, cudaStream_t);
 }  // namespace fm

@@ -17,7 +17,7 @@ template cudaError_t launch_y_tma<float, double>(const Dims&, int, const void*, 
                                           const int*, int*, int, cudaStream_t);
 template cudaError_t launch_zg_tma<float, double>(const Dims&, int, const void*, const GreenParams&, const void*,
                                           const void*, void*, const int*, int*, int, cudaStream_t);
-template bool zreg_takes<float, double>(const Dims&, int);
+template int zreg_length<float, double>(const Dims&, int);
 template cudaError_t launch_zreg<float, double>(const Dims&, int, const void*, const GreenParams&, const void*, const void*,
                                           void*, const int*, int*, int, cudaStream_t);
 }  // namespace fm

@@ -18,7 +18,7 @@ template cudaError_t launch_y_tma<double, double>(const Dims&, int, const void*,
                                           const int*, int*, int, cudaStream_t);
 template cudaError_t launch_zg_tma<double, double>(const Dims&, int, const void*, const GreenParams&, const void*,
                                           const void*, void*, const int*, int*, int, cudaStream_t);
-template bool zreg_takes<double, double>(const Dims&, int);
+template int zreg_length<double, double>(const Dims&, int);
 template cudaError_t launch_zreg<double, double>(const Dims&, int, const void*, const GreenParams&, const void*, const void*,
                                           void*, const int*, int*, int, cudaStream_t);
 }  // namespace fm

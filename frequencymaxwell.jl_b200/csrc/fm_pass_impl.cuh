@@ -344,12 +344,15 @@ template <typename S, typename R>
 cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenParams& gp, const void* tw,
                           const void* rz, void* out, const int* act, int* err, int sms, cudaStream_t st) {
 #define ZT(LL, M) zg_tma_L<S, R, LL, M>(d, in, gp, tw, rz, out, act, err, sms, st)
-  // the Green pass where launch_zreg does not take it (zreg_takes), and the curl
-  if (mode == ZMODE_ONE) return d.nz == 32 ? ZT(32, ZMODE_ONE) : cudaErrorNotSupported;
-  if (mode == ZMODE_AVG2) {
-    if (d.nz == 32) return ZT(32, ZMODE_AVG2);
-    if constexpr (sizeof(R) == 4) {
-      if (d.nz == 64) return ZT(64, ZMODE_AVG2);
+  // the Green pass where launch_zreg does not take it (zreg_length), and the curl
+  if (mode != ZMODE_CURL) {
+    if (d.nz == 32) return mode == ZMODE_ONE ? ZT(32, ZMODE_ONE) : ZT(32, ZMODE_AVG2);
+    if constexpr (sizeof(S) == 4) {
+      if (d.nz == 64) return mode == ZMODE_ONE ? ZT(64, ZMODE_ONE) : ZT(64, ZMODE_AVG2);
+      if (d.nz == 128 && mode == ZMODE_AVG2) return ZT(128, ZMODE_AVG2);
+      if constexpr (sizeof(R) == 8) {
+        if (d.nz == 128) return ZT(128, ZMODE_ONE);
+      }
     }
     return cudaErrorNotSupported;
   }
@@ -362,10 +365,10 @@ cudaError_t launch_zg_tma(const Dims& d, int mode, const void* in, const GreenPa
 #undef ZT
 }
 
-template <typename S, typename R, int L, int BR>
+template <typename S, typename R, int L, int MODE>
 static cudaError_t zreg_L(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz,
                           void* out, const int* act, int* err, int sms, cudaStream_t st) {
-  using C = ZRegCfg<S, R, L, BR>;
+  using C = ZRegCfg<S, R, L, MODE>;
   static_assert(2 * (C::SM::total + 1024) <= 233472, "two CTAs at least share the 228 KB of an SM");
   CUtensorMap mi, mo;
   if (!make_map(&mi, const_cast<void*>(in), d, (int)sizeof(cplx<S>), 4, 1, C::BZ, C::ROWB) ||
@@ -373,34 +376,64 @@ static cudaError_t zreg_L(const Dims& d, const void* in, const GreenParams& gp, 
     return cudaErrorNotSupported;
   const long long ntiles = (long long)(d.nx / C::TX) * d.ny * d.nb;
   const size_t smem = C::SM::total;
-  allow_smem(k_zreg<S, R, L, BR>, smem);
-  const unsigned grid = persistent_grid(k_zreg<S, R, L, BR>, C::THREADS, smem, ntiles, sms, d.tma_ctas);
-  k_zreg<S, R, L, BR><<<grid, C::THREADS, smem, st>>>(d, mi, mo, gp, (const cplx<R>*)tw, (const cplx<R>*)rz, act, err);
+  allow_smem(k_zreg<S, R, L, MODE>, smem);
+  const unsigned grid = persistent_grid(k_zreg<S, R, L, MODE>, C::THREADS, smem, ntiles, sms, d.tma_ctas);
+  k_zreg<S, R, L, MODE><<<grid, C::THREADS, smem, st>>>(d, mi, mo, gp, (const cplx<R>*)tw, (const cplx<R>*)rz, act, err);
   return cudaGetLastError();
 }
 
+// Which form of k_zreg a length takes for one branch (BR 1) or the average (BR 2), ZR_NONE if none.
+// FP64 storage: the branches side by side.  FP32 storage: Plan's radices, since with others its results are other ones by
+// more than their rounding (k_dot32): one branch where Plan16 has the same radices, the average at 256 points as one
+// transform of 512, and at 512 points, where that is out of reach, as two transforms, each rounded to storage before
+// their sum.
+template <typename S, typename R, int L, int BR>
+constexpr int zreg_mode() {
+  if constexpr (sizeof(S) == 8) return BR == 2 ? ZR_TWO : ZR_ONE;
+  else if constexpr (BR == 1) return same_radices<L, R>() ? ZR_ONE : ZR_NONE;
+  else if constexpr (L == 512) return ZR_TWO;
+  else return L == 256 ? ZR_PAD : ZR_NONE;
+}
+
 template <typename S, typename R>
-bool zreg_takes(const Dims& d, int branches) {
-  // (in FP32 the length-2L transform of 64 points exchanges once too: 16.7 us against 18.8 on 64^3)
-  if (sizeof(R) == 4 && d.nz == 64 && branches == 2) return false;
-#define ZR(LL) (d.nx % (branches == 2 ? ZRegCfg<S, R, LL, 2>::TX : ZRegCfg<S, R, LL, 1>::TX) == 0)
-  return d.nz == 64 ? ZR(64) : d.nz == 128 ? ZR(128) : d.nz == 256 ? ZR(256) : d.nz == 512 ? ZR(512) : false;
-#undef ZR
+int zreg_length(const Dims& d, int branches) {
+  auto len = [&](auto l) {
+    constexpr int L = decltype(l)::value;
+    auto fits = [&](auto m) {
+      constexpr int MODE = decltype(m)::value;
+      if constexpr (MODE == ZR_NONE) return 0;
+      else return d.nx % ZRegCfg<S, R, L, MODE>::TX == 0 ? ZRegCfg<S, R, L, MODE>::LF : 0;
+    };
+    return branches == 2 ? fits(std::integral_constant<int, zreg_mode<S, R, L, 2>()>{})
+                         : fits(std::integral_constant<int, zreg_mode<S, R, L, 1>()>{});
+  };
+  switch (d.nz) {
+    case 64: return len(std::integral_constant<int, 64>{});
+    case 128: return len(std::integral_constant<int, 128>{});
+    case 256: return len(std::integral_constant<int, 256>{});
+    case 512: return len(std::integral_constant<int, 512>{});
+    default: return 0;
+  }
 }
 
 template <typename S, typename R>
 cudaError_t launch_zreg(const Dims& d, int branches, const void* in, const GreenParams& gp, const void* tw,
                         const void* rz, void* out, const int* act, int* err, int sms, cudaStream_t st) {
-#define ZR(LL) (branches == 2 ? zreg_L<S, R, LL, 2>(d, in, gp, tw, rz, out, act, err, sms, st) \
-                              : zreg_L<S, R, LL, 1>(d, in, gp, tw, rz, out, act, err, sms, st))
+  auto run = [&](auto l, auto br) {
+    constexpr int L = decltype(l)::value, MODE = zreg_mode<S, R, L, decltype(br)::value>();
+    if constexpr (MODE == ZR_NONE) return cudaErrorNotSupported;
+    else return zreg_L<S, R, L, MODE>(d, in, gp, tw, rz, out, act, err, sms, st);
+  };
+  auto len = [&](auto l) {
+    return branches == 2 ? run(l, std::integral_constant<int, 2>{}) : run(l, std::integral_constant<int, 1>{});
+  };
   switch (d.nz) {
-    case 64: return ZR(64);
-    case 128: return ZR(128);
-    case 256: return ZR(256);
-    case 512: return ZR(512);
+    case 64: return len(std::integral_constant<int, 64>{});
+    case 128: return len(std::integral_constant<int, 128>{});
+    case 256: return len(std::integral_constant<int, 256>{});
+    case 512: return len(std::integral_constant<int, 512>{});
     default: return cudaErrorNotSupported;
   }
-#undef ZR
 }
 
 template <typename R>

@@ -285,6 +285,23 @@ struct GreenBin {
     e2 = cmul(csub(e2, cscale(kE, ky)), f);
     e3 = cmul(csub(e3, cscale(kE, kz)), f);
   }
+  // The same with every fused multiply-add written out, in the order in which the compiler forms them for k_zg, so that
+  // k_zreg returns the same bits (DD: which square is fused; in k_zg's FP32 average di's).  The scale is real here.
+  template <bool DD>
+  __device__ __forceinline__ void green_fixed(T& e1, T& e2, T& e3, R kx, R ky, R kz) const {
+    const T k = mk(fma(e3.x, kz, fma(e1.x, kx, e2.x * ky)), fma(e3.y, kz, fma(e1.y, kx, e2.y * ky)));
+    const T kE = mk(fma(k.x, iks.x, -(k.y * iks.y)), fma(k.x, iks.y, k.y * iks.x));
+    const R dr = fma(kz, kz, fma(kx, kx, ky * ky)) - ksr, di = -ksi;
+    const R rdd = R(1) / (DD ? fma(di, di, dr * dr) : fma(dr, dr, di * di));
+    const T f = mk(sc.x * (dr * rdd), sc.x * (-di * rdd));
+    auto out = [&](T e, R c) {
+      const T a = mk(fma(-kE.x, c, e.x), fma(-kE.y, c, e.y));
+      return mk(fma(a.x, f.x, -(a.y * f.y)), fma(a.x, f.y, a.y * f.x));
+    };
+    e1 = out(e1, kx);
+    e2 = out(e2, ky);
+    e3 = out(e3, kz);
+  }
   // i k x E
   __device__ __forceinline__ void curl(T& e1, T& e2, T& e3, R kx, R ky, R kz) const {
     const T isc = cmul_i<1>(sc);
@@ -383,21 +400,54 @@ __global__ void __launch_bounds__(256) k_zg(Dims d, const cplx<S>* __restrict__ 
 
   // per-bin 3x3 operator
   {
-    const GreenBin<R> gb(gp, b);
+    int kxi = x, kyi = y;
     R kx, ky;
     if (MODE == ZMODE_CURL) {
-      kx = (R)gp.dk[0] * kidx_curl<R>(x, d.nx);
-      ky = (R)gp.dk[1] * kidx_curl<R>(y, d.ny);
+      kx = (R)gp.dk[0] * kidx_curl<R>(kxi, d.nx);
+      ky = (R)gp.dk[1] * kidx_curl<R>(kyi, d.ny);
     } else {
-      kx = (R)gp.dk[0] * (kidx_green<R>(x, d.nx) + (R)gp.shift[0]);
-      ky = (R)gp.dk[1] * (kidx_green<R>(y, d.ny) + (R)gp.shift[1]);
+      kx = (R)gp.dk[0] * (kidx_green<R>(kxi, d.nx) + (R)gp.shift[0]);
+      ky = (R)gp.dk[1] * (kidx_green<R>(kyi, d.ny) + (R)gp.shift[1]);
     }
+    const R ksr = (R)gp.ksq_re, ksi = gp.ksq_im_b ? (R)gp.ksq_im_b[b] : (R)gp.ksq_im;
+    const T sc = mk((R)gp.scale_re, (R)gp.scale_im);
+    // 1/k_square
+    const R kden = ksr * ksr + ksi * ksi;
+    const T iks = mk(ksr / kden, -ksi / kden);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int m = lay_idx<LF, E, P_::RL>(t, e);
-      const R kz = z_wavenumber<MODE, L, R>(gp, m);
-      if constexpr (MODE == ZMODE_CURL) gb.curl(v[0][e], v[1][e], v[2][e], kx, ky, kz);
-      else gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+      R kz;
+      if constexpr (MODE == ZMODE_AVG2) {
+        if ((m & 1) == 0) kz = (R)gp.dk[2] * (kidx_green<R>(m >> 1, L) + (R)gp.shift[2]);
+        else kz = (R)gp.dk[2] * (kidx_green<R>(((m + 1) >> 1) % L, L) - (R)gp.shift[2]);
+      } else if constexpr (MODE == ZMODE_ONE) {
+        kz = (R)gp.dk[2] * (kidx_green<R>(m, L) + (R)gp.shift[2]);
+      } else {
+        kz = (R)gp.dk[2] * kidx_curl<R>(m, L);
+      }
+      T e1 = v[0][e], e2 = v[1][e], e3 = v[2][e];
+      if constexpr (MODE == ZMODE_CURL) {
+        // (ik x E) * sc
+        T c1 = csub(cscale(e3, ky), cscale(e2, kz));
+        T c2 = csub(cscale(e1, kz), cscale(e3, kx));
+        T c3 = csub(cscale(e2, kx), cscale(e1, ky));
+        const T isc = cmul_i<1>(sc);
+        v[0][e] = cmul(c1, isc);
+        v[1][e] = cmul(c2, isc);
+        v[2][e] = cmul(c3, isc);
+      } else {
+        T kE = cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz));
+        kE = cmul(kE, iks);
+        const R k2 = kx * kx + ky * ky + kz * kz;
+        const R dr = k2 - ksr, di = -ksi;
+        const R dd = dr * dr + di * di;
+        const R rdd = R(1) / dd;  // one division for both parts of 1 / (k^2 - ks)
+        const T f = cmul(sc, mk(dr * rdd, -di * rdd));
+        v[0][e] = cmul(csub(e1, cscale(kE, kx)), f);
+        v[1][e] = cmul(csub(e2, cscale(kE, ky)), f);
+        v[2][e] = cmul(csub(e3, cscale(kE, kz)), f);
+      }
     }
   }
 

@@ -29,10 +29,10 @@ template <typename S, typename R, int L>
 struct YTmaCfg {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P = YTilePlan<L, R>;
+  using P = YTilePlan<L, S, R>;
   // bytes of a tile row: at 512 points two stages of whole lines leave no room for a second CTA; at 256 points and FP32
-  // storage 64-byte rows run four CTAs an SM (4.2 TB/s, 3.8 with 128), in FP64 storage whole lines are better (5.9, 5.2
-  // with 64)
+  // storage 64-byte rows run more CTAs an SM (k_y_tma 256^3: 223 us, 395 with 128), in FP64 storage whole lines are better
+  // (5.9 TB/s, 5.2 with 64)
   static constexpr int ROWB = L == 512 || (L == 256 && sizeof(S) == 4) ? 64 : 128;
   static constexpr int TX = ROWB / (int)sizeof(TS);
   static constexpr int PW = 32 / P::TP;
@@ -180,7 +180,10 @@ struct ZTmaCfg {
   static constexpr int TILE = 3 * L * 128;
   static constexpr int NST = TILE <= 32768 ? 3 : 2;
   static constexpr int STRIDE = PencilStride<LF, T, P::TP, true>::v;
-  using SM = TmaSmem<TILE, NST, CW * PW * STRIDE * (int)sizeof(T), (2 * LF + L) * (int)sizeof(T)>;
+  // exchange buffers per pencil: the three components of a length-256 transform run stage by stage together
+  // (their exchanges overlap), each with its own buffer; shorter transforms run one component at a time
+  static constexpr int NCX = LF >= 256 ? 3 : 1;
+  using SM = TmaSmem<TILE, NST, CW * PW * NCX * STRIDE * (int)sizeof(T), (2 * LF + L) * (int)sizeof(T)>;
   static constexpr int THREADS = CW * 32;
 };
 
@@ -231,7 +234,10 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
     }
   }
   const int p = lane / TP, t = lane % TP;
-  T* sm = ex + (warp * PW + p) * C::STRIDE;
+  constexpr int NCX = C::NCX, SMS = C::STRIDE;
+  T* sm = ex + (warp * PW + p) * NCX * SMS;
+  const R ksr = (R)gp.ksq_re;
+  const T sc = mk((R)gp.scale_re, (R)gp.scale_im);
   int it = 0;
   bool ok = true;
   for (long long tile = next_active(blockIdx.x, ntiles, per_rhs, active); tile < ntiles;
@@ -243,7 +249,9 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
     const uint32_t ph = (it / NST) & 1;
     if (!mbar_wait(full + s, ph, err, 23)) { ok = false; break; }
     unsigned char* tl = tiles + s * C::TILE;
-    const GreenBin<R> gb(gp, b);
+    const R ksi = gp.ksq_im_b ? (R)gp.ksq_im_b[b] : (R)gp.ksq_im;
+    const R kden = ksr * ksr + ksi * ksi;
+    const T iks = mk(ksr / kden, -ksi / kden);
 #pragma unroll 1
     for (int rd = 0; rd < C::ROUNDS; ++rd) {
       const int xl = rd * CW * PW + warp * PW + p;
@@ -261,7 +269,13 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
           }
           v[c][e] = a;
         }
-        fft_fwd_plan<-1, P_, MODE == ZMODE_AVG2>(v[c], sm, tw, t);
+        if constexpr (NCX == 1) {
+          fft_fwd_plan<-1, P_>(v[c], sm, tw, t);
+          __syncwarp();
+        }
+      }
+      if constexpr (NCX == 3) {
+        fft_fwd_plan_n<-1, P_, 3, SMS>(v, sm, tw, t);
         __syncwarp();
       }
       R kx, ky;
@@ -274,14 +288,44 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
       }
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const R kz = z_wavenumber<MODE, L, R>(gp, lay_idx<LF, E, P_::RL>(t, e));
-        if constexpr (MODE == ZMODE_CURL) gb.curl(v[0][e], v[1][e], v[2][e], kx, ky, kz);
-        else gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+        const int m = lay_idx<LF, E, P_::RL>(t, e);
+        R kz;
+        if constexpr (MODE == ZMODE_AVG2) {
+          if ((m & 1) == 0) kz = (R)gp.dk[2] * (kidx_green<R>(m >> 1, L) + (R)gp.shift[2]);
+          else kz = (R)gp.dk[2] * (kidx_green<R>(((m + 1) >> 1) % L, L) - (R)gp.shift[2]);
+        } else if constexpr (MODE == ZMODE_ONE) {
+          kz = (R)gp.dk[2] * (kidx_green<R>(m, L) + (R)gp.shift[2]);
+        } else {
+          kz = (R)gp.dk[2] * kidx_curl<R>(m, L);
+        }
+        T e1 = v[0][e], e2 = v[1][e], e3 = v[2][e];
+        if constexpr (MODE == ZMODE_CURL) {
+          const T isc = cmul_i<1>(sc);
+          v[0][e] = cmul(csub(cscale(e3, ky), cscale(e2, kz)), isc);
+          v[1][e] = cmul(csub(cscale(e1, kz), cscale(e3, kx)), isc);
+          v[2][e] = cmul(csub(cscale(e2, kx), cscale(e1, ky)), isc);
+        } else {
+          T kE = cmul(cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz)), iks);
+          const R k2 = kx * kx + ky * ky + kz * kz;
+          const R dr = k2 - ksr, di = -ksi;
+          const R dd = dr * dr + di * di;
+          const R rdd = R(1) / dd;  // one division for both parts of 1 / (k^2 - ks)
+          const T f = cmul(sc, mk(dr * rdd, -di * rdd));
+          v[0][e] = cmul(csub(e1, cscale(kE, kx)), f);
+          v[1][e] = cmul(csub(e2, cscale(kE, ky)), f);
+          v[2][e] = cmul(csub(e3, cscale(kE, kz)), f);
+        }
+      }
+      if constexpr (NCX == 3) {
+        fft_rev_plan_n<+1, P_, 3, SMS>(v, sm, twr, t);
+        __syncwarp();
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        fft_rev_plan<+1, P_>(v[c], sm, twr, t);
-        __syncwarp();
+        if constexpr (NCX == 1) {
+          fft_rev_plan<+1, P_>(v[c], sm, twr, t);
+          __syncwarp();
+        }
 #pragma unroll
         for (int e = 0; e < E; ++e) {
           const int z = lay_idx<LF, E, P_::R0>(t, e);
@@ -318,25 +362,30 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
 }
 
 // ---------------------------------------------------------------------------
-// z pass in sixteen values a lane and component, for L = 64, 128, 256, 512: all three components stay in registers
-// from the forward transform through the Green product to the inverse one.  BR = 2 is the averaged Green function
+// z pass in sixteen values a lane and component, for L = 64, 128, 256, 512 (zreg_mode): all three components stay in
+// registers from the forward transform through the Green product to the inverse one.  BR = 2 is the averaged Green function
 // (shift 1/4 on z): the two shifted branches run as two transforms of length L on neighbouring lane groups; branch s
 // multiplies by exp(-/+ 2 pi i z/(4L)), and the groups add their results at the end (a shuffle; for L = 512, where a
 // branch fills a warp, through shared memory).  BR = 1 is one branch with its ramp rz (none when z has no shift).
+// ZR_PAD is the average as one transform of length 2 L of the zero-padded pencil (z_wavenumber): FP32 storage at 256
+// points, whose results have its radices (zreg_mode; 256^3: 943 us, 1170 in k_zg, 829 as two branches).
 //
 // What bounds it is shared memory: per value and branch one exchange (two at L = 512) each way, where the length-2L
 // transform in eight values a lane exchanges twice on twice the values.  In FP64 192 of 255 registers hold the values,
 // so an SM has eight warps, in CTAs of one tile each; one CTA's copies overlap the others' transforms.
 // ---------------------------------------------------------------------------
-template <typename S, typename R, int L, int BR>
+enum { ZR_NONE = 0, ZR_ONE = 1, ZR_TWO = 2, ZR_PAD = 3 };
+
+template <typename S, typename R, int L, int MODE>
 struct ZRegCfg {
   using T = cplx<R>;
   using TS = cplx<S>;
-  using P = Plan16<L>;
+  static constexpr int BR = MODE == ZR_TWO ? 2 : 1, LF = MODE == ZR_PAD ? 2 * L : L;
+  using P = Plan16<LF>;
   static constexpr bool F64 = sizeof(R) == 8;
   // bytes of a tile row: what lets a CTA's lane groups take whole rows, and the SM its CTAs
-  static constexpr int ROWB = L <= 128 ? (F64 && sizeof(TS) == 16 ? 128 : 64)
-                              : L == 256 ? (F64 || BR == 1 ? 64 : 32) : 32;
+  static constexpr int ROWB = LF <= 128 ? (F64 && sizeof(TS) == 16 ? 128 : 64)
+                              : LF == 256 ? (F64 || BR == 1 ? 64 : 32) : 32;
   static constexpr int TX = ROWB / (int)sizeof(TS);  // pencils of a tile
   static constexpr int WMAX = TX * BR * P::TP / 32;  // warps that one round of the tile keeps busy
   static constexpr int W = WMAX < 4 ? WMAX : 4, THREADS = 32 * W;
@@ -347,7 +396,7 @@ struct ZRegCfg {
   static constexpr int BZ = L > 256 ? 256 : L;  // z extent of one copy
   static constexpr int TILE = 3 * L * ROWB;
   static constexpr int EXB = BR * GROUPS * P::STRIDE * (int)sizeof(T);
-  using SM = TmaSmem<TILE, 1, EXB, 3 * L * (int)sizeof(T)>;
+  using SM = TmaSmem<TILE, 1, EXB, (2 * LF + L) * (int)sizeof(T)>;
   // element (component 0, z = t < TP, pencil x) of the tile: rows of ROWB bytes, swizzled by the copy in 16-byte chunks
   static __device__ __forceinline__ unsigned char* at(unsigned char* tile, int t, int x) {
     const int byte = x * (int)sizeof(TS);
@@ -364,28 +413,32 @@ struct ZRegCfg {
   }
 };
 
-template <typename S, typename R, int L, int BR>
-__global__ void __launch_bounds__(ZRegCfg<S, R, L, BR>::THREADS, ZRegCfg<S, R, L, BR>::CTAS)
+template <typename S, typename R, int L, int MODE>
+__global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R, L, MODE>::CTAS)
     k_zreg(Dims d, const __grid_constant__ CUtensorMap tm_in, const __grid_constant__ CUtensorMap tm_out, GreenParams gp,
            const cplx<R>* __restrict__ twz, const cplx<R>* __restrict__ rz, const int* __restrict__ active,
            int* __restrict__ err) {
-  using C = ZRegCfg<S, R, L, BR>;
+  using C = ZRegCfg<S, R, L, MODE>;
   using T = typename C::T;
   using TS = typename C::TS;
   using P_ = typename C::P;
-  constexpr int TP = P_::TP;
+  constexpr int TP = P_::TP, BR = C::BR, LF = C::LF;
+  constexpr int EL = MODE == ZR_PAD ? 8 : 16;  // values of a lane that the pencil has (the padding has the others)
+  static_assert(P_::R0 == 16, "value e of a lane is z = t + e TP");
+  // at 512 points and FP32 storage each branch is rounded to storage before their sum (zreg_mode)
+  constexpr bool ROUND = BR == 2 && sizeof(TS) < sizeof(T);
   extern __shared__ unsigned char smraw_[];
   unsigned char* sm0 = (unsigned char*)(((uintptr_t)smraw_ + 1023) & ~(uintptr_t)1023);
   unsigned char* tl = sm0 + C::SM::tiles;
   T* ex = reinterpret_cast<T*>(sm0 + C::SM::ex);
   T* tw = reinterpret_cast<T*>(sm0 + C::SM::tab);
-  T* twr = tw + L;
-  T* rtab = twr + L;
+  T* twr = tw + LF;
+  T* rtab = twr + LF;
   uint64_t* full = reinterpret_cast<uint64_t*>(sm0 + C::SM::bars);
   const int xtiles = d.nx / C::TX;
   const long long per_rhs = (long long)xtiles * d.ny;
   const long long ntiles = per_rhs * d.nb;
-  load_table(tw, twz, 2 * L);
+  load_table(tw, twz, 2 * LF);
   if (rz) load_table(rtab, rz, L);
   if (threadIdx.x == 0) {
     mbar_init(full, 1);
@@ -426,38 +479,45 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, BR>::THREADS, ZRegCfg<S, R, L
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
+        for (int e = 0; e < EL; ++e) {
           T a = cv<T>(*reinterpret_cast<TS*>((e & 1 ? tp1 : tp0) + C::off(c, e)));
-          if (BR == 2 || rz) {
+          if (MODE != ZR_ONE || rz) {
             T r = rtab[t + e * TP];
             r.y *= sg;
-            a = cmul(a, r);
+            a = cmul_fixed(a, r);
           }
           v[c][e] = a;
         }
-        fft16_fwd<-1, P_>(v[c], sm, tw, t);
+        fft16_fwd<-1, P_, MODE == ZR_PAD>(v[c], sm, tw, t);
         __syncwarp();
       }
       const R kx = (R)gp.dk[0] * (kidx_green<R>(xt * C::TX + xl, d.nx) + (R)gp.shift[0]);
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const R kz = (R)gp.dk[2] * (kidx_green<R>(lay_idx<L, 16, P_::RL>(t, e), L) + sg * (R)gp.shift[2]);
-        gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+        const int m = lay_idx<LF, 16, P_::RL>(t, e);
+        R kz;
+        if constexpr (MODE == ZR_PAD) kz = z_wavenumber<ZMODE_AVG2, L, R>(gp, m);
+        else kz = (R)gp.dk[2] * (kidx_green<R>(m, L) + sg * (R)gp.shift[2]);
+        gb.template green_fixed<MODE == ZR_PAD && !C::F64>(v[0][e], v[1][e], v[2][e], kx, ky, kz);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         fft16_rev<+1, P_>(v[c], sm, twr, t);
-        if (BR == 2 || rz) {
+        if (MODE != ZR_ONE || rz) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
+          for (int e = 0; e < EL; ++e) {
             T r = rtab[t + e * TP];
             r.y *= -sg;
-            v[c][e] = cmul(v[c][e], r);
+            v[c][e] = cmul_fixed(v[c][e], r);
           }
+        }
+        if constexpr (ROUND) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[c][e] = cv<T>(cv<TS>(v[c][e]));
         }
         if constexpr (BR == 1) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) *reinterpret_cast<TS*>((e & 1 ? tp1 : tp0) + C::off(c, e)) = cv<TS>(v[c][e]);
+          for (int e = 0; e < EL; ++e) *reinterpret_cast<TS*>((e & 1 ? tp1 : tp0) + C::off(c, e)) = cv<TS>(v[c][e]);
         } else {
           // sum of the branches: each group keeps half of the values and takes the partner's share of them.  By now
           // both groups of the pencil have read the tile (the exchanges synchronise them): the result may go into it.

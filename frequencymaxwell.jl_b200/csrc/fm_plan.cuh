@@ -22,6 +22,7 @@
 #include "../../include/fmcuda.h"
 #include "fm_blockdot.h"
 #include "fm_krylov.cuh"
+#include "fm_general32.h"
 #include "fm_generic.h"
 #include "fm_launch.h"
 #include "fm_setup.cuh"
@@ -92,6 +93,8 @@ struct fm_plan {
   bool zonly = false;   // shifts only on z -> single pass with the length-2L transform
   bool zsplit = false;  // shifts only on z, padded z of a length the length-2L pass does not take: two z passes
   BlueAxis blue[3];     // axes without a fused pass (blue[a].n > 0): tables of their Bluestein passes (fm_generic.cuh)
+  bool general32 = false;  // FP32 arithmetic and an axis without a fused pass: the passes of fm_general32.cuh
+  GenAxis gax[3];          // their tables
   DevBuf gtw[3], gch[3], gkn[3][2];
   double shift[3] = {0, 0, 0};
   // potential / physics
@@ -201,8 +204,7 @@ static cudaError_t pass_xf(const fm_plan* P, const Dims& d, int pro, const void*
   if (P->blue[0].n) {
     if constexpr (std::is_same<S, double>::value)
       return launch_bxf<double, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
-    else return P->c64 ? launch_bxf<float, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt)
-                       : launch_bxf<float, float>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
+    else return launch_bxf<float, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
   }
   if constexpr (std::is_same<S, double>::value)
     return launch_xf<double, double>(d, pro, in, V, rs, tw, ramp, out, act, P->st, vt);
@@ -215,34 +217,33 @@ static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* 
   if (P->blue[1].n) {
     if constexpr (std::is_same<S, double>::value)
       return launch_by<double, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
-    else return P->c64 ? launch_by<float, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st)
-                       : launch_by<float, float>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
+    else return launch_by<float, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
   }
   if (P->use_tma && P->tma_y) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
       e = launch_y_tma<double, double>(d, dir, in, P->twyt.p, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
     else
-      e = P->c64 ? launch_y_tma<float, double>(d, dir, in, P->twyt.p, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st)
-                 : launch_y_tma<float, float>(d, dir, in, P->twyt.p, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
+      e = P->c64 ? launch_y_tma<float, double>(d, dir, in, tw, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st)
+                 : launch_y_tma<float, float>(d, dir, in, tw, ramp, out, act, (int*)P->errbuf.p, P->sms, P->st);
     if (e != cudaErrorNotSupported) return e;
   }
   if constexpr (std::is_same<S, double>::value) return launch_y<double, double>(d, dir, in, tw, ramp, out, act, P->st);
   else return P->c64 ? launch_y<float, double>(d, dir, in, tw, ramp, out, act, P->st)
                      : launch_y<float, float>(d, dir, in, tw, ramp, out, act, P->st);
 }
-// the z pass in sixteen values a lane: whether this plan's shape has it, and the pass (launch_zreg)
+// the z pass in sixteen values a lane: its transform's length where this plan's shape has it (else 0), and the pass
 template <typename S>
-static bool has_zreg(const fm_plan* P, const Dims& d, int branches) {
-  if (!P->use_tma || !P->tma_z || P->blue[2].n) return false;
-  if constexpr (std::is_same<S, double>::value) return zreg_takes<double, double>(d, branches);
-  else return P->c64 ? zreg_takes<float, double>(d, branches) : zreg_takes<float, float>(d, branches);
+static int has_zreg(const fm_plan* P, const Dims& d, int branches) {
+  if (!P->use_tma || !P->tma_z || P->blue[2].n) return 0;
+  if constexpr (std::is_same<S, double>::value) return zreg_length<double, double>(d, branches);
+  else return P->c64 ? zreg_length<float, double>(d, branches) : zreg_length<float, float>(d, branches);
 }
 template <typename S>
 static cudaError_t pass_zreg(const fm_plan* P, const Dims& d, int branches, const void* in, const GreenParams& gp,
                              const void* rz, void* out, const int* act) {
   int* err = (int*)P->errbuf.p;
-  const void* tw = P->twz16.p;
+  const void* tw = has_zreg<S>(P, d, branches) == d.nz ? P->twz16.p : P->twz2.p;
   if constexpr (std::is_same<S, double>::value)
     return launch_zreg<double, double>(d, branches, in, gp, tw, rz, out, act, err, P->sms, P->st);
   else return P->c64 ? launch_zreg<float, double>(d, branches, in, gp, tw, rz, out, act, err, P->sms, P->st)
@@ -254,8 +255,7 @@ static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void
   if (P->blue[2].n) {
     if constexpr (std::is_same<S, double>::value)
       return launch_bz<double, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
-    else return P->c64 ? launch_bz<float, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st)
-                       : launch_bz<float, float>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
+    else return launch_bz<float, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
   }
   if (mode == ZMODE_ONE && !gp.accumulate && has_zreg<S>(P, d, 1)) return pass_zreg<S>(P, d, 1, in, gp, rz, out, act);
   if (P->use_tma && P->tma_z) {
@@ -278,8 +278,7 @@ static cudaError_t pass_xi(const fm_plan* P, const Dims& d, int epi, const void*
   if (P->blue[0].n) {
     if constexpr (std::is_same<S, double>::value)
       return launch_bxi<double, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
-    else return P->c64 ? launch_bxi<float, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt)
-                       : launch_bxi<float, float>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
+    else return launch_bxi<float, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
   }
   if constexpr (std::is_same<S, double>::value)
     return launch_xi<double, double>(d, epi, in, V, xv, bv, rs, ep, tw, ramp, out, act, P->st, vt);
@@ -316,9 +315,29 @@ static fm_status init_tables(fm_plan* P) {
   DevBuf* tw[3] = {&P->twx, &P->twy, &P->twz};
   std::vector<cd> chirp[3];
   for (int a = 0; a < 3; ++a) {
+    if (P->general32) {
+      GenAxis& g = P->gax[a];
+      g.n = g.m = n3[a];
+      if (!gen_axis_plain(g.n)) {
+        const BlueAxisTables t = blue_axis_tables(g.n);
+        g.m = t.m;
+        std::vector<cd> both = t.chirp[0];
+        both.insert(both.end(), t.chirp[1].begin(), t.chirp[1].end());
+        FM_CK(upload_cplx<R>(P->gch[a], both, P->st));
+        for (int dir = 0; dir < 2; ++dir) {
+          FM_CK(upload_cplx<R>(P->gkn[a][dir], t.kern[dir], P->st));
+          g.chirp[dir] = (const cplx<R>*)P->gch[a].p + dir * g.n;
+          g.kern[dir] = P->gkn[a][dir].p;
+        }
+      }
+      FM_CK(upload_cplx<R>(P->gtw[a], twiddles<R>(g.m), P->st));
+      g.tw = P->gtw[a].p;
+      continue;
+    }
     if (axis_supported(n3[a])) {
       FM_CK(upload_cplx<R>(*tw[a], twiddles<R>(n3[a]), P->st));
-      if (a == 1) FM_CK(upload_cplx<R>(P->twyt, ytile_twiddles<R>(n3[a]), P->st));
+      // (a plan of FP32 storage runs its FP64 block vectors through the tiles of FP64 storage; its own use twy)
+      if (a == 1 && sizeof(R) == 8) FM_CK(upload_cplx<R>(P->twyt, ytile_twiddles<double, R>(n3[a]), P->st));
       continue;
     }
     const BlueAxisTables t = blue_axis_tables(n3[a]);
@@ -341,7 +360,7 @@ static fm_status init_tables(fm_plan* P) {
     for (size_t i = 0; i < chirp[a].size(); ++i) r[i] *= chirp[a][i];
     return r;
   };
-  if (!P->blue[2].n) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
+  if (!P->blue[2].n && !P->general32) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
   if (P->zonly) {
     FM_CK(upload_cplx<R>(P->twz2, twiddles<R>(2 * P->dims.nz), P->st));
     FM_CK(upload_cplx<R>(P->rz, ramp(2, -1.0), P->st));
@@ -375,17 +394,23 @@ static int kv_blocks(const fm_plan* P, Kern kern, int nb) {
   return (int)std::max(1LL, std::min<long long>(maxb, cap / nb));
 }
 // The same for the Gram-Schmidt passes, whose smallest share is one warp step per warp.
-template <typename R, typename Kern>
+template <typename Kern>
 static int gs_blocks(const fm_plan* P, Kern kern, int nb) {
   int bps = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, KV_THREADS, 0) != cudaSuccess || bps < 1) bps = 1;
   const long long cap = (long long)P->sms * std::min(bps, 8);
-  const long long maxb = (P->M + KV_WARPS * GsCfg<R>::STEP - 1) / (KV_WARPS * GsCfg<R>::STEP);
+  const long long maxb = (P->M + KV_WARPS * GS_STEP - 1) / (KV_WARPS * GS_STEP);
   return (int)std::max(1LL, std::min<long long>(maxb, cap / nb));
 }
+// Blocks per RHS of k_dot32 and k_update32 (S32_CTAS an SM), and of k_mgs32 (MGS32_CTAS): a function of the size alone,
+// since it orders their sums.
+inline int s32_blocks(const fm_plan* P, int nb, int ctas = S32_CTAS) {
+  const long long chunk = (long long)KV_THREADS * KV_EPT, maxb = (P->M + chunk - 1) / chunk;
+  return (int)std::max(1LL, std::min<long long>(maxb, (long long)P->sms * ctas / nb));
+}
 inline int red_blocks_max(const fm_plan* P, int nb) {
-  // upper bound of kv_blocks and gs_blocks over all kernels (at most 8 blocks of 256 threads per SM)
-  const long long chunk = KV_WARPS * GsCfg<double>::STEP;
+  // upper bound of kv_blocks, gs_blocks and s32_blocks over all kernels (at most 8 blocks of 256 threads per SM)
+  const long long chunk = KV_WARPS * GS_STEP;
   const long long maxb = (P->M + chunk - 1) / chunk;
   return (int)std::max(1LL, std::min<long long>(maxb, (long long)P->sms * 8 / nb));
 }
@@ -410,7 +435,6 @@ struct RhsCtx {
   const double* ksq_im_b = nullptr;   // eps_imag / k_ref^2 per RHS
   const double* inv_eps_b = nullptr;  // k_ref^2 / eps_imag per RHS
   VecTab vt;
-  void* tmp[3] = {nullptr, nullptr, nullptr};  // pass temporaries, nb fields each, in place of the plan's t1, t2, t3
 };
 
 // ---- operator drivers (fm_ops.cu) ----
@@ -427,7 +451,7 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
 // one sweep of the passes (no shift, or z-only shifts), fused x passes, contiguous batches: where green_op can
 // chain applications
 inline bool green_chain_ok(const fm_plan* P, const RhsCtx* rc) {
-  return !P->blue[0].n && (!P->avg || P->zonly || P->zsplit) && !(rc && (rc->vt.in || rc->vt.out));
+  return !P->blue[0].n && !P->general32 && (!P->avg || P->zonly || P->zsplit) && !(rc && (rc->vt.in || rc->vt.out));
 }
 // H = -i lambda/(2 pi 377) curl(E) for nb fields (in -> out, contiguous batches; act masks RHS)
 template <typename R>

@@ -150,9 +150,9 @@ fm_status run(const fm_plan_desc& dsc, double k_bg, double eps_imag, int nrhs, c
   unsigned char* sc = (unsigned char*)base;
   int* err = (int*)(sc + o_err);
   // the z pass in sixteen values a lane where the size has it (launch_zreg), else the passes of fm_passes*.cuh
-  const bool zreg = zreg_takes<S, R>(d, zonly ? 2 : 1);
-  const int lt = zreg ? n3[2] : lz;
-  TableJobs jobs{{pair_job(o_tx, n3[0], radices<R>(n3[0])), pair_job(o_ty, n3[1], ytile_radices<R>(n3[1])),
+  const int zreg = zreg_length<S, R>(d, zonly ? 2 : 1);
+  const int lt = zreg ? zreg : lz;
+  TableJobs jobs{{pair_job(o_tx, n3[0], radices<R>(n3[0])), pair_job(o_ty, n3[1], ytile_radices<S, R>(n3[1])),
                   pair_job(o_tz, lt, zreg ? radices16(lt) : radices<R>(lt))},
                  (unsigned)o_rz, n3[2], zonly ? 0.25 : 0.0};
   auto tables = [&](int* clear) {
@@ -182,7 +182,7 @@ fm_status run(const fm_plan_desc& dsc, double k_bg, double eps_imag, int nrhs, c
     cudaError_t r = launch_y_tma<S, R>(d, dir, in, sc + o_ty, nullptr, out, nullptr, err, sms, st);
     if (r != cudaErrorNotSupported) return r;
     // no tiles (a narrow x, or buffers off the tensor maps' 16 bytes): the register pass, on its plan's table
-    if (ytile_radices<R>(n3[1]) != radices<R>(n3[1])) {
+    if (ytile_radices<S, R>(n3[1]) != radices<R>(n3[1])) {
       jobs.pair[1] = pair_job(o_ty, n3[1], radices<R>(n3[1]));
       if ((r = tables(nullptr)) != cudaSuccess) return r;
     }

@@ -55,10 +55,10 @@ inline std::vector<int> radices16(int L) {
   return L == 64 ? std::vector<int>{16, 4} : L == 128 ? std::vector<int>{16, 8} : L == 256 ? std::vector<int>{16, 16}
          : L == 512 ? std::vector<int>{16, 8, 4} : std::vector<int>{};
 }
-// of the y tiles (YTilePlan; at 512 the radices agree)
-template <typename R>
+// of the y tiles (YTilePlan: Plan but for FP64 storage at 256)
+template <typename S, typename R>
 inline std::vector<int> ytile_radices(int L) {
-  return std::is_same<R, double>::value && L == 256 ? radices16(L) : radices<R>(L);
+  return std::is_same<S, double>::value && L == 256 ? radices16(L) : radices<R>(L);
 }
 
 // [forward-order table | reversed-order table] of an FFT of length L
@@ -72,8 +72,8 @@ inline std::vector<cd_t> twiddle_pair(int L, const std::vector<int>& r) {
 template <typename R>
 inline std::vector<cd_t> twiddles(int L) { return twiddle_pair(L, radices<R>(L)); }
 inline std::vector<cd_t> twiddles16(int L) { return twiddle_pair(L, radices16(L)); }
-template <typename R>
-inline std::vector<cd_t> ytile_twiddles(int L) { return twiddle_pair(L, ytile_radices<R>(L)); }
+template <typename S, typename R>
+inline std::vector<cd_t> ytile_twiddles(int L) { return twiddle_pair(L, ytile_radices<S, R>(L)); }
 
 // exp(sgn * 2 pi i * idx * s / L)
 inline std::vector<cd_t> ramp(int L, double s, double sgn) {
