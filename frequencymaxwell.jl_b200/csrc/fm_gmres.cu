@@ -795,11 +795,16 @@ static fm_status gmres_block(fm_plan* P, int nb, const fm_solve_opts& o, std::ve
   // ---- x += V y = X Rf^{-1} y ----
   std::vector<double2> yh((size_t)nb * KV_KMAX, make_double2(0, 0));
   int Kmax = 0;
-  for (int b = 0; b < nb; ++b) Kmax = std::max(Kmax, blk_solution(St[b], yh.data() + (size_t)b * KV_KMAX));
+  for (int b = 0; b < nb; ++b) {
+    acth[b] = blk_solution(St[b], yh.data() + (size_t)b * KV_KMAX);
+    Kmax = std::max(Kmax, acth[b]);
+  }
   if (Kmax > 0) {
     FM_CK(cudaMemcpyAsync(P->coef.p, yh.data(), yh.size() * sizeof(double2), cudaMemcpyHostToDevice, P->st));
     Coef cf{(const double2*)P->coef.p, KV_KMAX, nullptr, nb, 1.0, 1};
-    FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, nullptr, nb)));
+    // each right-hand side reads its own vectors alone: beyond them U holds what an earlier solve left
+    FM_CK(cudaMemcpyAsync(act, acth.data(), nb * sizeof(int), cudaMemcpyHostToDevice, P->st));
+    FM_CK((gs_update<R>(P, nb, Kmax, U, cf, P->xbuf.p, false, act, nb, nullptr, act)));
   }
   for (int b = 0; b < nb; ++b) {
     info[b].iterations = St[b].iters;
