@@ -132,10 +132,13 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
     }
     FM_TRACK(P, KC_YF, 2 * fbA, e = pass_y<R>(P, d, -1, P->t1.p, P->twy.p, nullptr, P->t2.p, act));
     FM_CK(e);
+    e = cudaErrorNotSupported;
     if (P->avg && has_zreg<R>(P, d, 2)) {
       gp.shift[2] = P->shift[2];
       gp.scale_re = 1.0 / ((double)P->n * 2.0);
       FM_TRACK(P, KC_ZG, 2 * fbA, e = pass_zreg<R>(P, d, 2, P->t2.p, gp, P->zonly ? P->rz.p : P->rzp.p, P->t1.p, act));
+    }
+    if (e != cudaErrorNotSupported) {
       FM_CK(e);
     } else if (P->zsplit) {
       // the two z branches (+s, -s) as two length-L z passes with their phase ramps; the second adds to the first

@@ -83,7 +83,8 @@ struct fm_plan {
   long long n = 0, M = 0;  // voxels, elements per field (3n)
   cudaStream_t st = nullptr;
   int sms = 148;
-  bool use_tma = true;  // TMA-staged y/z passes (FMCUDA_NO_TMA=1 selects the register-only passes)
+  bool use_tma = true;  // TMA-staged y/z passes (FMCUDA_NO_TMA=1 selects the register-only passes; 2 does too, by way of
+                        // launchers that find no tensor maps)
   bool tma_y = true, tma_z = true;  // tuning: TMA-staged y / z passes where the size has one
   bool bd_bulk = false;             // tuning: bulk-copy pipelined block dot where the shape has one
   bool bd_wide = false;             // tuning: register block dot with four basis groups per warp (5 <= s <= 8)
@@ -257,7 +258,10 @@ static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void
       return launch_bz<double, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
     else return launch_bz<float, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
   }
-  if (mode == ZMODE_ONE && !gp.accumulate && has_zreg<S>(P, d, 1)) return pass_zreg<S>(P, d, 1, in, gp, rz, out, act);
+  if (mode == ZMODE_ONE && !gp.accumulate && has_zreg<S>(P, d, 1)) {
+    const cudaError_t e = pass_zreg<S>(P, d, 1, in, gp, rz, out, act);
+    if (e != cudaErrorNotSupported) return e;
+  }
   if (P->use_tma && P->tma_z) {
     cudaError_t e;
     if constexpr (std::is_same<S, double>::value)
