@@ -77,6 +77,7 @@ static fm_status plan_wave_size(fm_plan* P, int nrhs, const fm_solve_opts& o, in
   }
   else if (o.method == FM_METHOD_BICGSTAB) vecs = 6;
   else vecs = 1;
+  if (o.method == FM_METHOD_GMRES && o.ortho == FM_ORTHO_MGS && sizeof(R) == 8) extra = MGS_T_BYTES;
   // basis + b + x + s + e + t1 + t2 + fp64 staging and outputs
   // (the output term also covers the second output slot of host-output solves: 2 * 3g * 16 <= 2 * M * 16)
   // (+ t3 when the Green average runs as two branches: absorbing x or y)
@@ -84,7 +85,7 @@ static fm_status plan_wave_size(fm_plan* P, int nrhs, const fm_solve_opts& o, in
   const size_t per = fb * (size_t)(vecs + 6 + two_branch) + (size_t)P->M * sizeof(double2) * 5 + extra;
   const size_t held = P->basis.cap + P->bbuf.cap + P->xbuf.cap + P->sbuf.cap + P->ebuf.cap + P->t1.cap + P->t2.cap +
                       P->t3.cap +
-                      P->gbuf2.cap + P->Eo.cap + P->Ho.cap + P->yblk.cap;
+                      P->gbuf2.cap + P->Eo.cap + P->Ho.cap + P->yblk.cap + P->mgsT.cap;
   const size_t avail = (size_t)((freeb + held) * 0.92);
   wave = (int)std::max<size_t>(1, std::min<size_t>((size_t)nrhs, avail / per));
   wave = std::min(wave, std::max(1, P->desc.max_rhs));
@@ -114,9 +115,9 @@ long long fm_plan_bytes(const fm_plan_desc* d, int nrhs, int basis) {
   for (int a = 0; a < 3; ++a) n *= (long long)(d->grid[a] + 2 * d->pad[a]);
   const long long fb = 3 * n * (d->precision == FM_PREC_F64 ? 16 : 8);
   // basis + six work fields per right-hand side, the potential, and the FP64 E/H outputs in two slots (host
-  // outputs are copied from one slot while the next wave fills the other)
+  // outputs are copied from one slot while the next wave fills the other), and in FP64 the table of modified Gram-Schmidt
   return fb * (long long)nrhs * (basis + 6) + n * (d->precision == FM_PREC_F64 ? 16 : 8) +
-         4LL * 3 * n * 16 * nrhs;
+         4LL * 3 * n * 16 * nrhs + (d->precision == FM_PREC_F64 ? (long long)MGS_T_BYTES * nrhs : 0);
 }
 
 fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {

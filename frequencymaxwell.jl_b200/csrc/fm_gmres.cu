@@ -232,7 +232,7 @@ static fm_status gmres(fm_plan* P, int nb, const fm_solve_opts& o, std::vector<f
   FM_CK(P->scale.ensure((size_t)(KV_KMAX + 1) * nb * sizeof(double)));
   if (o.ortho == FM_ORTHO_MGS) {
     FM_CK(P->hbuf.ensure((size_t)nb * (KV_KMAX + 2) * sizeof(double2)));
-    if (sizeof(R) == 8) FM_CK(P->mgsT.ensure((size_t)nb * KV_KMAX * KV_KMAX * sizeof(double2)));
+    if (sizeof(R) == 8) FM_CK(P->mgsT.ensure(nb * MGS_T_BYTES));
   }
   FM_CK(P->active.ensure((size_t)nb * sizeof(int)));
   FM_TRY(ensure_reduce(P, nb, mem + 1));

@@ -180,6 +180,8 @@ struct MgsTail {
   int hs;
 };
 
+constexpr size_t MGS_T_BYTES = (size_t)KV_KMAX * KV_KMAX * sizeof(double2);  // T of one right-hand side
+
 // out[b][i] = sum_e conj(U_i[b][e]) * w[b][e]   (i < K), plus out[b][K] = ||w||^2 when WNORM.
 // Optional per-RHS arguments: wtab[b] replaces w + b*M, Kb[b] (<= K) the number of basis vectors.
 // MGS: U_{K-1} is the newest basis vector; mt.h gets the modified Gram-Schmidt coefficients of w against
