@@ -98,7 +98,9 @@ __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cpl
   const int p = lane / TP, t = lane % TP;
   const long long rows = (long long)d.ny * d.nz * d.nb;
   const long long row = ((long long)blockIdx.x * (blockDim.x >> 5) + wic) * PW + p;
-  if (row >= rows) return;  // whole pencils exit together (rows is a multiple of PW)
+  // whole pencils leave; where ny*nz*nb is no multiple of PW the last warp goes on with some of its lanes, so what
+  // follows has no shuffles (__syncwarp does not wait for lanes that have left)
+  if (row >= rows) return;
   const int b = (int)(row / ((long long)d.ny * d.nz));
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * d.ny * d.nz;
@@ -625,7 +627,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
   const int p = lane / TP, t = lane % TP;
   const long long rows = (long long)d.ny * d.nz * d.nb;
   const long long row = ((long long)blockIdx.x * (blockDim.x >> 5) + wic) * PW + p;
-  if (row >= rows) return;  // whole pencils exit together (rows is a multiple of PW)
+  if (row >= rows) return;  // as in k_xf
   const int b = (int)(row / ((long long)d.ny * d.nz));
   if (active && !active[b]) return;
   const long long yz = row - (long long)b * d.ny * d.nz;
