@@ -427,6 +427,7 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
   static_assert(P_::R0 == 16, "value e of a lane is z = t + e TP");
   // at 512 points and FP32 storage each branch is rounded to storage before their sum (zreg_mode)
   constexpr bool ROUND = BR == 2 && sizeof(TS) < sizeof(T);
+  constexpr bool FIXED = sizeof(TS) == 8;  // FP32 storage: the multiply-adds as in k_zg (GreenBin::green_fixed)
   extern __shared__ unsigned char smraw_[];
   unsigned char* sm0 = (unsigned char*)(((uintptr_t)smraw_ + 1023) & ~(uintptr_t)1023);
   unsigned char* tl = sm0 + C::SM::tiles;
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
           if (MODE != ZR_ONE || rz) {
             T r = rtab[t + e * TP];
             r.y *= sg;
-            a = cmul_fixed(a, r);
+            a = FIXED ? cmul_fixed(a, r) : cmul(a, r);
           }
           v[c][e] = a;
         }
@@ -498,7 +499,8 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
         R kz;
         if constexpr (MODE == ZR_PAD) kz = z_wavenumber<ZMODE_AVG2, L, R>(gp, m);
         else kz = (R)gp.dk[2] * (kidx_green<R>(m, L) + sg * (R)gp.shift[2]);
-        gb.template green_fixed<MODE == ZR_PAD && !C::F64>(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+        if constexpr (FIXED) gb.template green_fixed<MODE == ZR_PAD && !C::F64>(v[0][e], v[1][e], v[2][e], kx, ky, kz);
+        else gb.green(v[0][e], v[1][e], v[2][e], kx, ky, kz);
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -508,7 +510,7 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
           for (int e = 0; e < EL; ++e) {
             T r = rtab[t + e * TP];
             r.y *= -sg;
-            v[c][e] = cmul_fixed(v[c][e], r);
+            v[c][e] = FIXED ? cmul_fixed(v[c][e], r) : cmul(v[c][e], r);
           }
         }
         if constexpr (ROUND) {
