@@ -373,7 +373,6 @@ template <typename S, typename R, int L, int MODE>
 static cudaError_t zreg_L(const Dims& d, const void* in, const GreenParams& gp, const void* tw, const void* rz,
                           void* out, const int* act, int* err, int sms, cudaStream_t st) {
   using C = ZRegCfg<S, R, L, MODE>;
-  static_assert(2 * (C::SM::total + 1024) <= 233472, "two CTAs at least share the 228 KB of an SM");
   CUtensorMap mi, mo;
   if (!make_map(&mi, const_cast<void*>(in), d, (int)sizeof(cplx<S>), 4, 1, C::BZ, C::ROWB) ||
       !make_map(&mo, out, d, (int)sizeof(cplx<S>), 4, 1, C::BZ, C::ROWB))

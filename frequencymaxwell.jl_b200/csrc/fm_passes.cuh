@@ -77,7 +77,8 @@ enum { PRO_COPY = 0, PRO_V = 1, PRO_V_SCALE = 2 };
 
 // CTAs of 256 threads per SM that a row pass is compiled for, by its length.  At 256 one CTA an SM (no bound on the
 // registers) ran the FP32-storage passes of 256^3 at 2.6 (k_xf) and 1.6 TB/s (k_xi); two and three run them at
-// 3.9 and 3.2; k_xf with three spills (3.5).  At 512 (16 values a lane) two fit.
+// 3.9 and 3.2; k_xf with three spills (3.5).  At 512 (16 values a lane) two fit, k_xf with V in FP64 only by spilling 224
+// to 248 bytes a thread.
 constexpr int row_ctas(int L, int small, int at256) { return L == 96 ? 1 : L <= 128 ? small : L == 256 ? at256 : 2; }
 
 template <typename S, typename R, int L, int PRO>

@@ -372,7 +372,9 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
 //
 // What bounds it is shared memory: per value and branch one exchange (two at L = 512) each way, where the length-2L
 // transform in eight values a lane exchanges twice on twice the values.  In FP64 192 of 255 registers hold the values,
-// so an SM has eight warps, in CTAs of one tile each; one CTA's copies overlap the others' transforms.
+// so an SM has eight warps at most, in CTAs of one tile each (one branch of FP64 storage: shared memory holds four to six);
+// one CTA's copies overlap the others' transforms.  The rest of the registers is too few for the compiler: in FP64 it
+// spills 56 to 320 bytes a thread (128 points, both branches: 120 stored, 204 loaded).
 // ---------------------------------------------------------------------------
 enum { ZR_NONE = 0, ZR_ONE = 1, ZR_TWO = 2, ZR_PAD = 3 };
 
@@ -391,12 +393,15 @@ struct ZRegCfg {
   static constexpr int W = WMAX < 4 ? WMAX : 4, THREADS = 32 * W;
   static constexpr int GROUPS = THREADS / (BR * P::TP);  // pencils in flight
   static constexpr int ROUNDS = TX / GROUPS;
-  static constexpr int CTAS = (F64 ? 8 : 12) / W;  // per SM: 255 or 168 registers
   static_assert(W >= 1 && TX % GROUPS == 0 && ROUNDS >= 1, "tile rows hold whole rounds");
   static constexpr int BZ = L > 256 ? 256 : L;  // z extent of one copy
   static constexpr int TILE = 3 * L * ROWB;
   static constexpr int EXB = BR * GROUPS * P::STRIDE * (int)sizeof(T);
   using SM = TmaSmem<TILE, 1, EXB, (2 * LF + L) * (int)sizeof(T)>;
+  // CTAs per SM: what 255 (FP32 arithmetic: 168) registers a thread and the 228 KB of shared memory hold
+  static constexpr int BYREG = (F64 ? 8 : 12) / W, BYMEM = 233472 / (SM::total + 1024);
+  static constexpr int CTAS = BYREG < BYMEM ? BYREG : BYMEM;
+  static_assert(CTAS >= 2, "one CTA's copies overlap another's transforms");
   // element (component 0, z = t < TP, pencil x) of the tile: rows of ROWB bytes, swizzled by the copy in 16-byte chunks
   static __device__ __forceinline__ unsigned char* at(unsigned char* tile, int t, int x) {
     const int byte = x * (int)sizeof(TS);
@@ -427,7 +432,9 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
   static_assert(P_::R0 == 16, "value e of a lane is z = t + e TP");
   // at 512 points and FP32 storage each branch is rounded to storage before their sum (zreg_mode)
   constexpr bool ROUND = BR == 2 && sizeof(TS) < sizeof(T);
-  constexpr bool FIXED = sizeof(TS) == 8;  // FP32 storage: the multiply-adds as in k_zg (GreenBin::green_fixed)
+  // the multiply-adds as in k_zg (GreenBin::green_fixed): FP32 storage, and one branch, which is faster with them (128^3,
+  // FP64, two right-hand sides: 150 us, 174 with the compiler's; the average is not: 645 and 634 us for six)
+  constexpr bool FIXED = sizeof(TS) == 8 || MODE == ZR_ONE;
   extern __shared__ unsigned char smraw_[];
   unsigned char* sm0 = (unsigned char*)(((uintptr_t)smraw_ + 1023) & ~(uintptr_t)1023);
   unsigned char* tl = sm0 + C::SM::tiles;
