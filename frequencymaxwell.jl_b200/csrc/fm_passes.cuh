@@ -47,8 +47,9 @@ __device__ __forceinline__ T* warp_smem(T* base, int warp_in_cta, int pencils_pe
 // Starts bringing n consecutive values at p to L2 (lanes t of TP, one 128-byte line each at a time).  The row passes ask
 // for the operands of their epilogue and of the next component this way before a transform: a load would need
 // registers until then, and after the transform's synchronisations it would wait for HBM.
-// Only for batches beyond PREFETCH_BYTES a field: smaller ones are in L2 already, and the instructions cost more than
-// they save (64^3 in FP64, 12.6 MB a field: k_xi 16.0 -> 17.7 us with them; 128^3, 100 MB: 92 -> 84).
+// Only for batches beyond PREFETCH_BYTES a field: smaller ones are in L2 already, and the instructions cost as much as
+// they save.  k_xi with and without them, FP64: 1.6 MB a field 1.04, 12.6 MB 0.99-1.00, 25 MB 0.88, 50 MB 0.83, 100 MB and
+// more 0.87-0.97; FP32: 12.6 MB 1.00, 21 MB 0.99, 25 MB 0.88, 50 MB 0.83 (64^3 in batches, 96^3, 128^3).
 constexpr long long PREFETCH_BYTES = 24ll << 20;
 template <typename TS>
 __device__ __forceinline__ bool prefetch_pays(const Dims& d) {
