@@ -12,10 +12,11 @@
 // modulus one, so the factor c_k of the forward result and c_k of the inverse input cancel: both are left out, and a
 // pass multiplies once, by c_n times the axis's ramp (forward) or the conjugate of that (inverse).
 //
-// Bound by shared memory and the FP64 pipe (about 150 FP64 instructions per value and transform at N = 201, M = 512),
-// not by HBM.  The strided passes stage the tile of a CTA in shared memory so that global rows are read and written
-// coalesced.  Measured on the 201 x 201 x 197 grid in FP64: one operator application 5.4 ms, against 14.8 ms as nine
-// plain passes per branch with strided accesses (prologue, three DFTs, Green, three DFTs, epilogue).
+// Bound by latency: registers and shared memory hold 8 (z) to 16 (x) warps an SM, which wait for their loads and for the
+// exchanges.  On the 201 x 201 x 197 grid the FP64 pipe is 26-41 % busy (about 150 FP64 instructions per value and
+// transform at N = 201, M = 512), shared memory and L1 55-78 %, DRAM 7-24 %.  The strided passes stage the tile of a CTA in
+// shared memory so that global rows are read and written coalesced.  One operator application there takes 5.4 ms, against
+// 14.8 ms as nine plain passes per branch with strided accesses (prologue, three DFTs, Green, three DFTs, epilogue).
 #pragma once
 #include "fm_passes.cuh"
 

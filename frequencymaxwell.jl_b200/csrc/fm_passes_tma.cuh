@@ -1,5 +1,3 @@
-// Tensor-map x coordinates count 8-byte words: a tile row is ROWB/8 words (128, 64 or 32 bytes) whatever the
-// storage type, so tile xt starts at word xt*ROWB/8, a multiple of 16 bytes.
 // TMA-staged versions of the strided passes (y pencils; z pencils with the dyadic Green or the curl).
 // Same arithmetic as k_y / k_zg in fm_passes.cuh; the data path goes through swizzled shared-memory
 // tiles loaded and stored by the tensor memory accelerator (see fm_tma.cuh).
@@ -9,6 +7,9 @@
 // from stage s (and the store has read the stage) it issues the load of tile i + NST into stage s.
 // Every consumer warp waits on the stage's "full" barrier; each warp arrives on the stage's "done"
 // barrier after writing its pencils back, and thread 0 waits on "done" before storing.
+//
+// Tensor-map x coordinates count 8-byte words: a tile row is ROWB/8 words (128, 64 or 32 bytes) whatever the
+// storage type, so tile xt starts at word xt*ROWB/8, a multiple of 16 bytes.
 #pragma once
 #include "fm_passes.cuh"
 #include "fm_tma.cuh"
