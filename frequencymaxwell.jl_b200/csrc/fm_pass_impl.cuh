@@ -29,8 +29,9 @@ static cudaError_t xf_L(const Dims& d, const void* in, const void* V, const doub
   const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(L + W * PW * P_::STRIDE) * sizeof(T);
-  allow_smem(k_xf<S, R, L, PRO>, smem);
-  k_xf<S, R, L, PRO><<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, rs, (const T*)tw,
+  auto kern = prefetch_pays<TS>(d) ? k_xf<S, R, L, PRO, true> : k_xf<S, R, L, PRO, false>;
+  allow_smem(kern, smem);
+  kern<<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, rs, (const T*)tw,
                                                          (const T*)ramp, (TS*)out, act, vt);
   return cudaGetLastError();
 }
@@ -48,8 +49,9 @@ static cudaError_t xi_L(const Dims& d, const void* in, const void* V, const void
   const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(L + W * PW * P_::STRIDE) * sizeof(T);
-  allow_smem(k_xi<S, R, L, EPI>, smem);
-  k_xi<S, R, L, EPI><<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv, (const TS*)bv,
+  auto kern = prefetch_pays<TS>(d) ? k_xi<S, R, L, EPI, true> : k_xi<S, R, L, EPI, false>;
+  allow_smem(kern, smem);
+  kern<<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv, (const TS*)bv,
                                                          rs, ep, (const T*)tw, (const T*)ramp, (TS*)out, act, vt);
   return cudaGetLastError();
 }
@@ -66,8 +68,9 @@ static cudaError_t xi_xf_L(const Dims& d, const void* in, const void* V, const v
   const long long warps = (rows + PW - 1) / PW;
   const unsigned blocks = (unsigned)((warps + W - 1) / W);
   const size_t smem = (size_t)(2 * L + W * PW * P_::STRIDE) * sizeof(T);
-  allow_smem(k_xi_xf<S, R, L>, smem);
-  k_xi_xf<S, R, L><<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv, ep, (const T*)tw,
+  auto kern = prefetch_pays<TS>(d) ? k_xi_xf<S, R, L, true> : k_xi_xf<S, R, L, false>;
+  allow_smem(kern, smem);
+  kern<<<blocks, W * 32, smem, st>>>(d, (const TS*)in, (const TS*)V, (const TS*)xv, ep, (const T*)tw,
                                                  (TS*)out, (TS*)out2, act);
   return cudaGetLastError();
 }

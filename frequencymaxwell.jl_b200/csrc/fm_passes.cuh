@@ -51,8 +51,10 @@ __device__ __forceinline__ T* warp_smem(T* base, int warp_in_cta, int pencils_pe
 // they save.  k_xi with and without them, FP64: 1.6 MB a field 1.04, 12.6 MB 0.99-1.00, 25 MB 0.88, 50 MB 0.83, 100 MB and
 // more 0.87-0.97; FP32: 12.6 MB 1.00, 21 MB 0.99, 25 MB 0.88, 50 MB 0.83 (64^3 in batches, 96^3, 128^3).
 constexpr long long PREFETCH_BYTES = 24ll << 20;
+// (AHEAD of the row passes: compiled in for those alone, since the code costs small fields 5-14 % of k_xi even where it is
+// skipped: 64^3 15.4 us, 17.5 with it)
 template <typename TS>
-__device__ __forceinline__ bool prefetch_pays(const Dims& d) {
+inline bool prefetch_pays(const Dims& d) {
   return 3 * d.n * d.nb * (long long)sizeof(TS) > PREFETCH_BYTES;
 }
 template <int TP, typename TS>
@@ -82,7 +84,7 @@ enum { PRO_COPY = 0, PRO_V = 1, PRO_V_SCALE = 2 };
 // to 248 bytes a thread.
 constexpr int row_ctas(int L, int small, int at256) { return L == 96 ? 1 : L <= 128 ? small : L == 256 ? at256 : 2; }
 
-template <typename S, typename R, int L, int PRO>
+template <typename S, typename R, int L, int PRO, bool AHEAD>
 __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cplx<S>* __restrict__ in, const cplx<S>* __restrict__ V,
                                             const double* __restrict__ rhs_scale, const cplx<R>* __restrict__ twx,
                                             const cplx<R>* __restrict__ rampx, cplx<S>* __restrict__ out,
@@ -119,7 +121,6 @@ __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cpl
   R s = R(1);
   if constexpr (PRO == PRO_V_SCALE) s = (R)rhs_scale[b];
   const cplx<S>* inb = vt.in ? (const cplx<S>*)vt.in[b] : in + (long long)b * 3 * d.n;
-  const bool ahead = prefetch_pays<TS>(d);
 #pragma unroll 1
   for (int c = 0; c < 3; ++c) {
     const long long base = ((long long)(c + 3 * b) * d.ny * d.nz + yz) * L;
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 2, 2)) k_xf(Dims d, const cpl
       if (rampx) a = cmul(a, rampx[x]);
       v[e] = a;
     }
-    if (ahead && c < 2) prefetch_row<TP>(inb + rbase + (long long)d.ny * d.nz * L, L, t);
+    if (AHEAD && c < 2) prefetch_row<TP>(inb + rbase + (long long)d.ny * d.nz * L, L, t);
     long_fwd<-1, P_>(v, sm, tw, t);
 #pragma unroll
     for (int e = 0; e < E; ++e) out[base + lay_idx<L, E, P_::RL>(t, e)] = cv<TS>(v[e]);
@@ -535,7 +536,7 @@ __device__ __forceinline__ T epi_element(T g, long long ix, const cplx<S>* xvb, 
   }
 }
 
-template <typename S, typename R, int L, int EPI>
+template <typename S, typename R, int L, int EPI, bool AHEAD>
 __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cplx<S>* __restrict__ in, const cplx<S>* __restrict__ V,
                                             const cplx<S>* __restrict__ xv, const cplx<S>* __restrict__ bv,
                                             const double* __restrict__ rhs_scale, EpiParams ep,
@@ -571,7 +572,6 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cpl
   cplx<S>* outb = vt.out ? (cplx<S>*)vt.out[b] : out + (long long)b * 3 * d.n;
   const cplx<S>* bvb = bv + (long long)b * 3 * d.n;
   const long long cstride = (long long)d.ny * d.nz * L;  // from one component's row to the next one's
-  const bool ahead = prefetch_pays<TS>(d);
 #pragma unroll 1
   for (int c = 0; c < 3; ++c) {
     const long long base = ((long long)(c + 3 * b) * d.ny * d.nz + yz) * L;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cpl
     T v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = cv<T>(in[base + lay_idx<L, E, P_::RL>(t, e)]);
-    if (ahead) {
+    if constexpr (AHEAD) {
       if constexpr (EPI != EPI_STORE) prefetch_row<TP>(xvb + rbase, L, t);
       if constexpr (EPI == EPI_PREC_RES) prefetch_row<TP>(bvb + rbase, L, t);
       if ((EPI == EPI_PREC_OP || EPI == EPI_PREC_RES) && c == 0) prefetch_row<TP>(Vrow, L, t);
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi(Dims d, const cpl
 // Each row's result is still in registers in the R0 layout that the forward transform takes, so the next
 // application's x pass neither reads `out` nor V again.  The forward input is the stored (storage-typed) value,
 // so out2 equals k_xf's output bit for bit.  Contiguous batches and no x ramp (the z-only and periodic plans).
-template <typename S, typename R, int L>
+template <typename S, typename R, int L, bool AHEAD>
 __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const cplx<S>* __restrict__ in,
                                                                           const cplx<S>* __restrict__ V,
                                                                           const cplx<S>* __restrict__ xv,
@@ -641,7 +641,6 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
   const cplx<S>* xvb = xv + (long long)b * 3 * d.n;
   cplx<S>* outb = out + (long long)b * 3 * d.n;
   const long long cstride = (long long)d.ny * d.nz * L;  // from one component's row to the next one's
-  const bool ahead = prefetch_pays<TS>(d);
 #pragma unroll 1
   for (int c = 0; c < 3; ++c) {
     const long long base = ((long long)(c + 3 * b) * d.ny * d.nz + yz) * L;
@@ -649,7 +648,7 @@ __global__ void __launch_bounds__(256, row_ctas(L, 3, 3)) k_xi_xf(Dims d, const 
     T v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = cv<T>(in[base + lay_idx<L, E, P_::RL>(t, e)]);
-    if (ahead) {
+    if constexpr (AHEAD) {
       prefetch_row<TP>(xvb + rbase, L, t);
       if (c == 0) prefetch_row<TP>(Vrow, L, t);
       if (c < 2) prefetch_row<TP>(in + base + cstride, L, t);
