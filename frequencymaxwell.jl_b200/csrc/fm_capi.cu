@@ -81,7 +81,7 @@ static fm_status plan_wave_size(fm_plan* P, int nrhs, const fm_solve_opts& o, in
   // basis + b + x + s + e + t1 + t2 + fp64 staging and outputs
   // (the output term also covers the second output slot of host-output solves: 2 * 3g * 16 <= 2 * M * 16)
   // (+ t3 when the Green average runs as two branches: absorbing x or y)
-  const size_t two_branch = (P->avg && !P->zonly && !P->zsplit) ? 1 : 0;
+  const size_t two_branch = (P->avg && (P->general32 || (!P->zonly && !P->zsplit))) ? 1 : 0;
   const size_t per = fb * (size_t)(vecs + 6 + two_branch) + (size_t)P->M * sizeof(double2) * 5 + extra;
   const size_t held = P->basis.cap + P->bbuf.cap + P->xbuf.cap + P->sbuf.cap + P->ebuf.cap + P->t1.cap + P->t2.cap +
                       P->t3.cap +
@@ -139,7 +139,7 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   const int prec = desc->precision == FM_PREC_F64 ? FM_PREC_F64 : FM_PREC_F32;  // storage
   const bool c64 = desc->precision != FM_PREC_F32;                                   // arithmetic
   // Fused passes take an axis of 96 or a power of two in [8, 512]; any other length up to 256 runs Bluestein passes
-  // on that axis (fm_generic.cuh), and in FP32 arithmetic the whole grid runs the passes of fm_general32.cuh.
+  // on that axis (fm_generic.cuh), and fields in FP32 storage the passes of fm_general32.cuh on the whole grid.
   for (int a = 0; a < 3; ++a)
     if (!axis_supported(n3[a]) && !blue_axis_supported(n3[a]))
       return fail(FM_ERR_UNSUPPORTED, "padded axis sizes must be at most 256, or powers of two up to 512");
@@ -147,12 +147,11 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   // adds to the first)
   const bool avg2 = axis_supported(n3[2]) && n3[2] <= AXIS_MAX_AVG2 && (n3[2] & (n3[2] - 1)) == 0;
   bool general32 = false;
-  if (!c64) {
-    const int pwy = pencils_per_warp<float>(n3[1]), pwz = pencils_per_warp<float>(zonly && avg2 ? 2 * n3[2] : n3[2]);
+  if (prec == FM_PREC_F32) {
     for (int a = 0; a < 3; ++a) general32 |= !axis_supported(n3[a]);
-    general32 |= (zonly && (n3[2] & (n3[2] - 1)) != 0) || pwy <= 0 || pwz <= 0 || n3[0] % pwy || n3[0] % pwz;
+    general32 |= zonly && (n3[2] & (n3[2] - 1)) != 0;
   }
-  const bool zsplit = zonly && !avg2 && !general32;
+  const bool zsplit = zonly && !avg2;
   if (cudaSetDevice(desc->device) != cudaSuccess) return fail(FM_ERR_CUDA, "cudaSetDevice failed");
   fm_plan* P = new fm_plan();
   P->desc = *desc;
@@ -165,7 +164,7 @@ fm_status fm_plan_create(const fm_plan_desc* desc, fm_plan** out) {
   P->M = 3 * P->n;
   P->pi = PadInfo{desc->grid[0], desc->grid[1], desc->grid[2], desc->pad[0], desc->pad[1], desc->pad[2], n3[0], n3[1], n3[2]};
   P->avg = avg;
-  P->zonly = zonly && !zsplit && !general32;
+  P->zonly = zonly && !zsplit;
   P->zsplit = zsplit;
   P->general32 = general32;
   for (int a = 0; a < 3; ++a) P->shift[a] = desc->absorbing[a] ? 0.25 : 0.0;
@@ -206,6 +205,14 @@ void fm_plan_destroy(fm_plan* P) {
                     &P->shifts, &P->yblk, &P->V64, &P->gtw[0], &P->gtw[1], &P->gtw[2], &P->gch[0],
                     &P->gch[1], &P->gch[2], &P->gkn[0][0],
                     &P->gkn[0][1], &P->gkn[1][0], &P->gkn[1][1], &P->gkn[2][0], &P->gkn[2][1], &P->shapes};
+  for (int a = 0; a < 3; ++a) {
+    P->gentw[a].release();
+    P->genchirp[a].release();
+    for (int i = 0; i < 2; ++i) {
+      P->genkern[a][i].release();
+      P->genramp[a][i].release();
+    }
+  }
   for (DevBuf* b : bufs) b->release();
   tk_resolve(P);
   for (cudaEvent_t e : P->evpool) cudaEventDestroy(e);

@@ -1,5 +1,5 @@
-// General axis lengths in FP32 arithmetic: the Green application and the curl on grids with a padded axis that has no
-// fused pass, and the two sub-pixel-shifted branches on any set of axes.
+// General axis lengths on FP32 storage, in either arithmetic: the Green application and the curl on grids with a padded
+// axis that has no fused pass, and the two sub-pixel-shifted branches on any set of axes.
 //
 // The work is split into plain passes over the batch, each reading and writing it once:
 //   PRE   psi = V.*x [* scale] * ramp_x(x) ramp_y(y) ramp_z(z)       (dyadic_green.jl:243-266, forward ramp)
@@ -11,16 +11,16 @@
 //   POST  g = result * conj(ramps) [+ the stored first branch], then the XI epilogue (operator, preconditioner,
 //         residual; fm_passes.cuh)
 //
-// The passes of fm_generic.cuh are faster (one application of 84 x 59 x 127: 260 us, 463 here), but in FP32 arithmetic
-// their results are other ones: a solve at the iteration limit amplifies the rounding of its transforms, and GMRES on
-// 51 x 85 x 51 came out 6.8e-5 from the fields of these passes, on 41 x 73 x 58 2.7e-5.  A faster pass is not to move a
-// result by more than FP32 resolves.
+// The passes of fm_generic.cuh are faster (one application of 84 x 59 x 127 in FP32 arithmetic: 260 us, 463 here), but
+// round elsewhere, and a solve at the iteration limit amplifies its rounding (k_dot32): in FP32 arithmetic GMRES on
+// 51 x 85 x 51 came out 6.8e-5 from the fields of these passes, on 41 x 73 x 58 2.7e-5; in FP64 arithmetic GMRES(20) on
+// 96 x 82 x 175 1.1e-5.  A faster pass is not to move a result by more than FP32 resolves.
 #pragma once
 #include "fm_passes.cuh"
 
 namespace fm {
 
-// Tables of one axis for the AXIS pass (device pointers).
+// Tables of one axis for the AXIS pass (arithmetic type R, device pointers).
 struct GenAxis {
   int n = 0;                  // axis length
   int m = 0;                  // FFT length: n (a power of two) or the Bluestein length (a power of two >= 2n - 1)
@@ -35,16 +35,17 @@ struct GenRamps {
 
 // AXIS: DIR = -1 forward DFT, +1 inverse (unnormalised), along `axis` of a batch of 3-component fields.  A lane
 // group reads its whole pencil before it writes, and pencils do not overlap, so the pass may run in place.
-template <int M, int DIR>
+template <typename R, int M, int DIR>
 __global__ void __launch_bounds__(256) k_gen_axis(Dims d, int axis, const float2* in, float2* out, GenAxis ax,
                                                   const int* __restrict__ active) {  // in may equal out
-  using P_ = Plan<M, float>;
+  using T = cplx<R>;
+  using P_ = Plan<M, R>;
   constexpr int E = P_::E, TP = P_::TP, PW = 32 / TP;
   extern __shared__ __align__(16) unsigned char smraw[];
-  float2* tw = reinterpret_cast<float2*>(smraw);
-  float2* twr = tw + M;
-  float2* ex = twr + M;
-  load_table(tw, (const float2*)ax.tw, 2 * M);
+  T* tw = reinterpret_cast<T*>(smraw);
+  T* twr = tw + M;
+  T* ex = twr + M;
+  load_table(tw, (const T*)ax.tw, 2 * M);
   __syncthreads();
   const int lane = threadIdx.x & 31, wic = threadIdx.x >> 5;
   const int p = lane / TP, t = lane % TP;
@@ -69,16 +70,16 @@ __global__ void __launch_bounds__(256) k_gen_axis(Dims d, int axis, const float2
   }
   const int b = on ? (int)(base / (3 * d.n)) : 0;
   const bool live = on && !(active && !active[b]);
-  float2* sm = warp_smem<float2, PencilStride<M, float2, TP, true>::v>(ex, wic, PW, p);
+  T* sm = warp_smem<T, PencilStride<M, T, TP, true>::v>(ex, wic, PW, p);
   const bool blue = N != M;
-  const float2* ch = blue ? (const float2*)ax.chirp[DIR < 0 ? 0 : 1] : nullptr;
-  float2 v[E];
+  const T* ch = blue ? (const T*)ax.chirp[DIR < 0 ? 0 : 1] : nullptr;
+  T v[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int i = lay_idx<M, E, P_::R0>(t, e);
-    float2 a = czero<float2>();
+    T a = czero<T>();
     if (live && i < N) {
-      a = in[base + (long long)i * stride];
+      a = cv<T>(in[base + (long long)i * stride]);
       if (blue) a = cmul(a, ch[i]);
     }
     v[e] = a;
@@ -87,12 +88,12 @@ __global__ void __launch_bounds__(256) k_gen_axis(Dims d, int axis, const float2
     fft_fwd_plan<DIR, P_>(v, sm, tw, t);
     if (live) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) out[base + (long long)lay_idx<M, E, P_::RL>(t, e) * stride] = v[e];
+      for (int e = 0; e < E; ++e) out[base + (long long)lay_idx<M, E, P_::RL>(t, e) * stride] = cv<float2>(v[e]);
     }
     return;
   }
   fft_fwd_plan<-1, P_>(v, sm, tw, t);
-  const float2* kk = (const float2*)ax.kern[DIR < 0 ? 0 : 1];
+  const T* kk = (const T*)ax.kern[DIR < 0 ? 0 : 1];
 #pragma unroll
   for (int e = 0; e < E; ++e) v[e] = cmul(v[e], kk[lay_idx<M, E, P_::RL>(t, e)]);
   __syncwarp();
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(256) k_gen_axis(Dims d, int axis, const float2
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       const int k = lay_idx<M, E, P_::R0>(t, e);
-      if (k < N) out[base + (long long)k * stride] = cmul(v[e], ch[k]);
+      if (k < N) out[base + (long long)k * stride] = cv<float2>(cmul(v[e], ch[k]));
     }
   }
 }
@@ -124,39 +125,43 @@ __device__ __forceinline__ GenIdx gen_idx(const Dims& d, long long i) {
   return g;
 }
 
-__device__ __forceinline__ float2 ramp3(const GenRamps& rp, const GenIdx& g) {
-  float2 w = mk(1.0f, 0.0f);
-  if (rp.r[0]) w = cmul(w, ((const float2*)rp.r[0])[g.x]);
-  if (rp.r[1]) w = cmul(w, ((const float2*)rp.r[1])[g.y]);
-  if (rp.r[2]) w = cmul(w, ((const float2*)rp.r[2])[g.z]);
+template <typename R>
+__device__ __forceinline__ cplx<R> ramp3(const GenRamps& rp, const GenIdx& g) {
+  using T = cplx<R>;
+  T w = mk(R(1), R(0));
+  if (rp.r[0]) w = cmul(w, ((const T*)rp.r[0])[g.x]);
+  if (rp.r[1]) w = cmul(w, ((const T*)rp.r[1])[g.y]);
+  if (rp.r[2]) w = cmul(w, ((const T*)rp.r[2])[g.z]);
   return w;
 }
 
 // PRE: out = in [.* V [* rs[b]]] * ramps  (PRO_COPY / PRO_V / PRO_V_SCALE as in k_xf)
-template <int PRO>
+template <typename R, int PRO>
 __global__ void __launch_bounds__(256) k_gen_pre(Dims d, const float2* __restrict__ in, const float2* __restrict__ V,
                                                  const double* __restrict__ rhs_scale, GenRamps rp,
                                                  float2* __restrict__ out, const int* __restrict__ active, VecTab vt) {
+  using T = cplx<R>;
   const long long total = 3 * d.n * d.nb;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const GenIdx g = gen_idx(d, i);
     if (active && !active[g.b]) continue;
     const float2* inb = vt.in ? (const float2*)vt.in[g.b] : in + (long long)g.b * 3 * d.n;
-    float2 a = inb[g.ix];
-    if constexpr (PRO != PRO_COPY) a = cmul(a, V[g.b * d.vstride + g.xyz]);
-    if constexpr (PRO == PRO_V_SCALE) a = cscale(a, (float)rhs_scale[g.b]);
-    a = cmul(a, ramp3(rp, g));
-    out[i] = a;
+    T a = cv<T>(inb[g.ix]);
+    if constexpr (PRO != PRO_COPY) a = cmul(a, cv<T>(V[g.b * d.vstride + g.xyz]));
+    if constexpr (PRO == PRO_V_SCALE) a = cscale(a, (R)rhs_scale[g.b]);
+    a = cmul(a, ramp3<R>(rp, g));
+    out[i] = cv<float2>(a);
   }
 }
 
 // KSPACE: in place.  ZMODE_ONE: the Green of one branch (shifts in gp.shift); ZMODE_CURL: i k x E.
 // Both scaled by gp.scale.
-template <int MODE>
+template <typename R, int MODE>
 __global__ void __launch_bounds__(256) k_gen_kspace(Dims d, float2* __restrict__ f, GreenParams gp,
                                                     const int* __restrict__ active) {
+  using T = cplx<R>;
   const long long total = d.n * d.nb;
-  const float2 sc = mk((float)gp.scale_re, (float)gp.scale_im);
+  const T sc = mk((R)gp.scale_re, (R)gp.scale_im);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int b = (int)(i / d.n);
     if (active && !active[b]) continue;
@@ -165,61 +170,59 @@ __global__ void __launch_bounds__(256) k_gen_kspace(Dims d, float2* __restrict__
     const long long r = xyz / d.nx;
     const int y = (int)(r % d.ny), z = (int)(r / d.ny);
     float2* fb = f + (long long)b * 3 * d.n + xyz;
-    const float2 e1 = fb[0], e2 = fb[d.n], e3 = fb[2 * d.n];
-    float2 o1, o2, o3;
+    const T e1 = cv<T>(fb[0]), e2 = cv<T>(fb[d.n]), e3 = cv<T>(fb[2 * d.n]);
+    T o1, o2, o3;
     if constexpr (MODE == ZMODE_CURL) {
-      const float kx = (float)gp.dk[0] * kidx_curl<float>(x, d.nx), ky = (float)gp.dk[1] * kidx_curl<float>(y, d.ny),
-                  kz = (float)gp.dk[2] * kidx_curl<float>(z, d.nz);
-      const float2 isc = cmul_i<1>(sc);
+      const R kx = (R)gp.dk[0] * kidx_curl<R>(x, d.nx), ky = (R)gp.dk[1] * kidx_curl<R>(y, d.ny),
+              kz = (R)gp.dk[2] * kidx_curl<R>(z, d.nz);
+      const T isc = cmul_i<1>(sc);
       o1 = cmul(csub(cscale(e3, ky), cscale(e2, kz)), isc);
       o2 = cmul(csub(cscale(e1, kz), cscale(e3, kx)), isc);
       o3 = cmul(csub(cscale(e2, kx), cscale(e1, ky)), isc);
     } else {
-      const float kx = (float)gp.dk[0] * (kidx_green<float>(x, d.nx) + (float)gp.shift[0]);
-      const float ky = (float)gp.dk[1] * (kidx_green<float>(y, d.ny) + (float)gp.shift[1]);
-      const float kz = (float)gp.dk[2] * (kidx_green<float>(z, d.nz) + (float)gp.shift[2]);
-      const float ksr = (float)gp.ksq_re, ksi = gp.ksq_im_b ? (float)gp.ksq_im_b[b] : (float)gp.ksq_im;
-      const float kden = ksr * ksr + ksi * ksi;
-      const float2 iks = mk(ksr / kden, -ksi / kden);
-      const float2 kE = cmul(cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz)), iks);
-      const float dr = kx * kx + ky * ky + kz * kz - ksr, di = -ksi;
-      const float rdd = 1.0f / (dr * dr + di * di);
-      const float2 fac = cmul(sc, mk(dr * rdd, -di * rdd));
+      const R kx = (R)gp.dk[0] * (kidx_green<R>(x, d.nx) + (R)gp.shift[0]);
+      const R ky = (R)gp.dk[1] * (kidx_green<R>(y, d.ny) + (R)gp.shift[1]);
+      const R kz = (R)gp.dk[2] * (kidx_green<R>(z, d.nz) + (R)gp.shift[2]);
+      const R ksr = (R)gp.ksq_re, ksi = gp.ksq_im_b ? (R)gp.ksq_im_b[b] : (R)gp.ksq_im;
+      const R kden = ksr * ksr + ksi * ksi;
+      const T iks = mk(ksr / kden, -ksi / kden);
+      const T kE = cmul(cadd(cadd(cscale(e1, kx), cscale(e2, ky)), cscale(e3, kz)), iks);
+      const R dr = kx * kx + ky * ky + kz * kz - ksr, di = -ksi;
+      const R rdd = R(1) / (dr * dr + di * di);
+      const T fac = cmul(sc, mk(dr * rdd, -di * rdd));
       o1 = cmul(csub(e1, cscale(kE, kx)), fac);
       o2 = cmul(csub(e2, cscale(kE, ky)), fac);
       o3 = cmul(csub(e3, cscale(kE, kz)), fac);
     }
-    fb[0] = o1;
-    fb[d.n] = o2;
-    fb[2 * d.n] = o3;
+    fb[0] = cv<float2>(o1);
+    fb[d.n] = cv<float2>(o2);
+    fb[2 * d.n] = cv<float2>(o3);
   }
 }
 
 // POST: g = in * conj(ramps) [+ ep.gadd], then the epilogue EPI (fm_passes.cuh, epi_element) into out.
-template <int EPI>
+template <typename R, int EPI>
 __global__ void __launch_bounds__(256) k_gen_post(Dims d, const float2* __restrict__ in, const float2* __restrict__ V,
                                                   const float2* __restrict__ xv, const float2* __restrict__ bv,
                                                   const double* __restrict__ rhs_scale, EpiParams ep, GenRamps rp,
                                                   float2* __restrict__ out, const int* __restrict__ active, VecTab vt) {
+  using T = cplx<R>;
   const long long total = 3 * d.n * d.nb;
-  const float2 al = mk((float)ep.alpha_re, (float)ep.alpha_im), be = mk((float)ep.beta_re, (float)ep.beta_im);
+  const T al = mk((R)ep.alpha_re, (R)ep.alpha_im), be = mk((R)ep.beta_re, (R)ep.beta_im);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const GenIdx g = gen_idx(d, i);
     const int b = g.b;
     if (active && !active[b]) continue;
-    float2 gv = cmul(in[i], cconj(ramp3(rp, g)));
-    if (ep.gadd) gv = cadd(gv, reinterpret_cast<const float2*>(ep.gadd)[i]);
-    const float ie = (EPI == EPI_PREC_OP || EPI == EPI_PREC_RES)
-                         ? (ep.inv_eps_b ? (float)ep.inv_eps_b[b] : (float)ep.inv_eps) : 0.0f;
-    const float2 shf = (EPI == EPI_PREC_OP && ep.shift_b) ? mk((float)ep.shift_b[b].x, (float)ep.shift_b[b].y)
-                                                          : czero<float2>();
-    const float s = rhs_scale ? (float)rhs_scale[b] : 1.0f;
+    T gv = cmul(cv<T>(in[i]), cconj(ramp3<R>(rp, g)));
+    if (ep.gadd) gv = cadd(gv, cv<T>(reinterpret_cast<const float2*>(ep.gadd)[i]));
+    const R ie = (EPI == EPI_PREC_OP || EPI == EPI_PREC_RES) ? (ep.inv_eps_b ? (R)ep.inv_eps_b[b] : (R)ep.inv_eps) : R(0);
+    const T shf = (EPI == EPI_PREC_OP && ep.shift_b) ? mk((R)ep.shift_b[b].x, (R)ep.shift_b[b].y) : czero<T>();
+    const R s = rhs_scale ? (R)rhs_scale[b] : R(1);
     const float2* xvb = vt.in ? (const float2*)vt.in[b] : xv + (long long)b * 3 * d.n;
     float2* outb = vt.out ? (float2*)vt.out[b] : out + (long long)b * 3 * d.n;
     const float2* bvb = bv + (long long)b * 3 * d.n;
-    const float2 r = epi_element<EPI, float, float2, float>(gv, g.ix, xvb, bvb, outb, V + b * d.vstride + g.xyz, ie, s, al,
-                                                            be, ep, shf);
-    outb[g.ix] = r;
+    const T r = epi_element<EPI, float, T, R>(gv, g.ix, xvb, bvb, outb, V + b * d.vstride + g.xyz, ie, s, al, be, ep, shf);
+    outb[g.ix] = cv<float2>(r);
   }
 }
 

@@ -1,5 +1,5 @@
-// Axis passes in FP64 arithmetic for lengths without a fused pass (odd lengths, other non-powers of two, e.g. the
-// 201 x 201 x 197 padded grid of the reference's two-beam example; FP32 arithmetic: fm_general32.cuh).  They take the places of k_xf, k_y, k_zg and k_xi (fm_passes.cuh) axis by
+// Axis passes on FP64 storage for lengths without a fused pass (odd lengths, other non-powers of two, e.g. the
+// 201 x 201 x 197 padded grid of the reference's two-beam example; FP32 storage: fm_general32.cuh).  They take the places of k_xf, k_y, k_zg and k_xi (fm_passes.cuh) axis by
 // axis, so a grid pays for Bluestein's algorithm only on the axes that need it, and the two sub-pixel-shifted branches
 // of a z-only boundary share the x and y passes.
 //

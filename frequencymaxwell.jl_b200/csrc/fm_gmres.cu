@@ -743,7 +743,7 @@ static fm_status gmres_block(fm_plan* P, int nb, const fm_solve_opts& o, std::ve
     }
     // Y_t = M^{-1}A Y_{t-1} - theta_t Y_{t-1}, t = 1..S; on the fused passes the x pass of application t+1 runs
     // inside the last pass of application t (GREEN_CHAIN_*), so Y_t and V are not read back for it
-    const bool chainable = green_chain_ok(P, &rcY);
+    const bool chainable = green_chain_ok<YR>(P, &rcY);
     std::vector<double2> th(nb);
     for (int t = 1; t <= S; ++t) {
       for (int b = 0; b < nb; ++b) th[b] = make_double2(St[b].theta[t - 1].real(), St[b].theta[t - 1].imag());

@@ -10,10 +10,11 @@
 //   epi : EPI_* epilogue applied to g = G_avg(psi)
 // ---------------------------------------------------------------------------
 
-// The Green application / CBS operator of green_op on a plan of the FP32-arithmetic general passes.  Per branch:
+// The Green application / CBS operator of green_op on FP32 storage and a grid of the general passes.  Per branch:
 // PRE (potential, forward ramps) -> forward DFT along x, y, z -> Green of the branch -> inverse DFT along z, y,
 // x -> POST (reverse ramps, epilogue).  With an absorbing axis the +s branch stores half its result in t3 and
 // the -s branch adds it before the epilogue (dyadic_green.jl:127-152).
+template <typename R>
 static fm_status gen_green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs, int epi, const void* xv,
                               const void* bv, const EpiParams& ep_in, void* out, const int* act, int nact,
                               const RhsCtx* rc) {
@@ -47,37 +48,35 @@ static fm_status gen_green_op(fm_plan* P, int nb, const void* in, int pro, const
   if (epi == EPI_PREC_RES) postb += fbA;
   if (epi == EPI_PREC_OP || epi == EPI_PREC_RES) postb += vb;
   if (epi == EPI_OP && (ep.beta_re != 0.0 || ep.beta_im != 0.0)) postb += fbA;
-  const DevBuf* rpos[3] = {&P->rxp, &P->ryp, &P->rzp};
-  const DevBuf* rneg[3] = {&P->rxm, &P->rym, &P->rzm};
   cudaError_t e;
   for (int br = 0; br < nbr; ++br) {
     GenRamps rp;
     for (int a = 0; a < 3; ++a) {
       gp.shift[a] = (br == 0 ? 1.0 : -1.0) * P->shift[a];
-      rp.r[a] = P->shift[a] != 0.0 ? (br == 0 ? rpos[a]->p : rneg[a]->p) : nullptr;
+      rp.r[a] = P->genramp[a][br].p;
     }
     FM_TRACK(P, KC_XF, 2 * fbA + (pro != PRO_COPY ? vb : 0.0),
-             e = launch_gen_pre(d, pro, in, V, rs, rp, P->t1.p, act, P->st, vt));
+             e = launch_gen_pre<R>(d, pro, in, V, rs, rp, P->t1.p, act, P->st, vt));
     FM_CK(e);
     for (int a = 0; a < 3; ++a) {
-      FM_TRACK(P, KC_YF, 2 * fbA, e = launch_gen_axis(d, a, -1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+      FM_TRACK(P, KC_YF, 2 * fbA, e = launch_gen_axis<R>(d, a, -1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
       FM_CK(e);
     }
-    FM_TRACK(P, KC_ZG, 2 * fbA, e = launch_gen_kspace(d, ZMODE_ONE, P->t1.p, gp, act, P->st));
+    FM_TRACK(P, KC_ZG, 2 * fbA, e = launch_gen_kspace<R>(d, ZMODE_ONE, P->t1.p, gp, act, P->st));
     FM_CK(e);
     for (int a = 2; a >= 0; --a) {
-      FM_TRACK(P, KC_YI, 2 * fbA, e = launch_gen_axis(d, a, +1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+      FM_TRACK(P, KC_YI, 2 * fbA, e = launch_gen_axis<R>(d, a, +1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
       FM_CK(e);
     }
     if (nbr == 2 && br == 0) {
       EpiParams e0{};
       FM_TRACK(P, KC_XI, 2 * fbA,
-               e = launch_gen_post(d, EPI_STORE, P->t1.p, V, nullptr, nullptr, nullptr, e0, rp, P->t3.p, act, P->st));
+               e = launch_gen_post<R>(d, EPI_STORE, P->t1.p, V, nullptr, nullptr, nullptr, e0, rp, P->t3.p, act, P->st));
     } else {
       EpiParams e1 = ep;
       if (nbr == 2) e1.gadd = P->t3.p;
       FM_TRACK(P, KC_XI, postb + (nbr == 2 ? fbA : 0.0),
-               e = launch_gen_post(d, epi, P->t1.p, V, xv, bv, rs, e1, rp, out, act, P->st, vt));
+               e = launch_gen_post<R>(d, epi, P->t1.p, V, xv, bv, rs, e1, rp, out, act, P->st, vt));
     }
     FM_CK(e);
   }
@@ -90,11 +89,15 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
                    int chain) {
   using T = cplx<R>;
   if (chain) {
-    if (!green_chain_ok(P, rc) || ((chain & GREEN_CHAIN_HAVE_XF) && pro != PRO_V) ||
+    if (!green_chain_ok<R>(P, rc) || ((chain & GREEN_CHAIN_HAVE_XF) && pro != PRO_V) ||
         ((chain & GREEN_CHAIN_NEXT_XF) && (epi != EPI_PREC_OP || rs || xv != in)))
       return fail(FM_ERR_INVALID, "operator chaining needs the fused passes, PRO_V and EPI_PREC_OP on the input");
   }
-  if (P->general32) return gen_green_op(P, nb, in, pro, rs, epi, xv, bv, ep_in, out, act, nact, rc);
+  if constexpr (sizeof(R) == 4) {
+    if (P->general32)
+      return P->c64 ? gen_green_op<double>(P, nb, in, pro, rs, epi, xv, bv, ep_in, out, act, nact, rc)
+                    : gen_green_op<float>(P, nb, in, pro, rs, epi, xv, bv, ep_in, out, act, nact, rc);
+  }
   if (nact < 0) nact = nb;
   EpiParams ep = ep_in;
   if (rc) ep.inv_eps_b = rc->inv_eps_b;
@@ -209,6 +212,30 @@ fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs
   }
 }
 
+// the curl of curl_batch on such a grid
+template <typename R>
+static fm_status gen_curl(fm_plan* P, const Dims& d, double cb, const void* in, void* out, const GreenParams& gp,
+                          const EpiParams& ep, const int* act) {
+  cudaError_t e;
+  const GenRamps none;
+  FM_TRACK(P, KC_CURL, cb, e = launch_gen_pre<R>(d, PRO_COPY, in, nullptr, nullptr, none, P->t1.p, act, P->st));
+  FM_CK(e);
+  for (int a = 0; a < 3; ++a) {
+    FM_TRACK(P, KC_CURL, cb, e = launch_gen_axis<R>(d, a, -1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+    FM_CK(e);
+  }
+  FM_TRACK(P, KC_CURL, cb, e = launch_gen_kspace<R>(d, ZMODE_CURL, P->t1.p, gp, act, P->st));
+  FM_CK(e);
+  for (int a = 2; a >= 0; --a) {
+    FM_TRACK(P, KC_CURL, cb, e = launch_gen_axis<R>(d, a, +1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
+    FM_CK(e);
+  }
+  FM_TRACK(P, KC_CURL, cb,
+           e = launch_gen_post<R>(d, EPI_STORE, P->t1.p, nullptr, nullptr, nullptr, nullptr, ep, none, out, act, P->st));
+  FM_CK(e);
+  return FM_OK;
+}
+
 // H = -i lambda/(2 pi 377) curl(E) for nb fields (in -> out, both contiguous batches; act masks RHS)
 template <typename R>
 fm_status curl_batch(fm_plan* P, int nb, const void* in, void* out, const int* act) {
@@ -227,24 +254,9 @@ fm_status curl_batch(fm_plan* P, int nb, const void* in, void* out, const int* a
   gp.scale_im = -f;
   const double cb = 2.0 * nb * P->M * sizeof(T);
   cudaError_t e;
-  if (P->general32) {
-    GenRamps none;
-    FM_TRACK(P, KC_CURL, cb, e = launch_gen_pre(d, PRO_COPY, in, nullptr, nullptr, none, P->t1.p, act, P->st));
-    FM_CK(e);
-    for (int a = 0; a < 3; ++a) {
-      FM_TRACK(P, KC_CURL, cb, e = launch_gen_axis(d, a, -1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
-      FM_CK(e);
-    }
-    FM_TRACK(P, KC_CURL, cb, e = launch_gen_kspace(d, ZMODE_CURL, P->t1.p, gp, act, P->st));
-    FM_CK(e);
-    for (int a = 2; a >= 0; --a) {
-      FM_TRACK(P, KC_CURL, cb, e = launch_gen_axis(d, a, +1, P->t1.p, P->t1.p, P->gax[a], act, P->st));
-      FM_CK(e);
-    }
-    FM_TRACK(P, KC_CURL, cb,
-             e = launch_gen_post(d, EPI_STORE, P->t1.p, nullptr, nullptr, nullptr, nullptr, ep, none, out, act, P->st));
-    FM_CK(e);
-    return FM_OK;
+  if constexpr (sizeof(R) == 4) {
+    if (P->general32)
+      return P->c64 ? gen_curl<double>(P, d, cb, in, out, gp, ep, act) : gen_curl<float>(P, d, cb, in, out, gp, ep, act);
   }
   FM_TRACK(P, KC_CURL, cb, e = pass_xf<R>(P, d, PRO_COPY, in, nullptr, nullptr, P->twx.p, nullptr, P->t1.p, act));
   FM_CK(e);

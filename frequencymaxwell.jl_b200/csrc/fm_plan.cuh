@@ -94,8 +94,11 @@ struct fm_plan {
   bool zonly = false;   // shifts only on z -> single pass with the length-2L transform
   bool zsplit = false;  // shifts only on z, padded z of a length the length-2L pass does not take: two z passes
   BlueAxis blue[3];     // axes without a fused pass (blue[a].n > 0): tables of their Bluestein passes (fm_generic.cuh)
-  bool general32 = false;  // FP32 arithmetic and an axis without a fused pass: the passes of fm_general32.cuh
-  GenAxis gax[3];          // their tables
+  // FP32 storage and an axis without a fused pass: fields in storage run the passes of fm_general32.cuh (the FP64 block
+  // vectors of such a plan the others), with their tables and per-axis ramps of the branches
+  bool general32 = false;
+  GenAxis gax[3];
+  DevBuf gentw[3], genchirp[3], genkern[3][2], genramp[3][2];
   DevBuf gtw[3], gch[3], gkn[3][2];
   double shift[3] = {0, 0, 0};
   // potential / physics
@@ -203,9 +206,9 @@ template <typename S>
 static cudaError_t pass_xf(const fm_plan* P, const Dims& d, int pro, const void* in, const void* V, const double* rs,
                            const void* tw, const void* ramp, void* out, const int* act, VecTab vt = VecTab{}) {
   if (P->blue[0].n) {
-    if constexpr (std::is_same<S, double>::value)
+    if constexpr (std::is_same<S, double>::value)  // (FP32 storage: fm_general32.cuh)
       return launch_bxf<double, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
-    else return launch_bxf<float, double>(d, pro, in, V, rs, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
+    else return cudaErrorNotSupported;
   }
   if constexpr (std::is_same<S, double>::value)
     return launch_xf<double, double>(d, pro, in, V, rs, tw, ramp, out, act, P->st, vt);
@@ -216,9 +219,9 @@ template <typename S>
 static cudaError_t pass_y(const fm_plan* P, const Dims& d, int dir, const void* in, const void* tw, const void* ramp,
                           void* out, const int* act) {
   if (P->blue[1].n) {
-    if constexpr (std::is_same<S, double>::value)
+    if constexpr (std::is_same<S, double>::value)  // (FP32 storage: fm_general32.cuh)
       return launch_by<double, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
-    else return launch_by<float, double>(d, dir, in, P->blue[1], blue_factor(P, 1, ramp), out, act, P->st);
+    else return cudaErrorNotSupported;
   }
   if (P->use_tma && P->tma_y) {
     cudaError_t e;
@@ -254,9 +257,9 @@ template <typename S>
 static cudaError_t pass_zg(const fm_plan* P, const Dims& d, int mode, const void* in, const GreenParams& gp,
                            const void* tw, const void* rz, void* out, const int* act) {
   if (P->blue[2].n) {
-    if constexpr (std::is_same<S, double>::value)
+    if constexpr (std::is_same<S, double>::value)  // (FP32 storage: fm_general32.cuh)
       return launch_bz<double, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
-    else return launch_bz<float, double>(d, mode, in, gp, P->blue[2], blue_factor(P, 2, rz), out, act, P->st);
+    else return cudaErrorNotSupported;
   }
   if (mode == ZMODE_ONE && !gp.accumulate && has_zreg<S>(P, d, 1)) {
     const cudaError_t e = pass_zreg<S>(P, d, 1, in, gp, rz, out, act);
@@ -280,9 +283,9 @@ static cudaError_t pass_xi(const fm_plan* P, const Dims& d, int epi, const void*
                            const void* bv, const double* rs, const EpiParams& ep, const void* tw, const void* ramp,
                            void* out, const int* act, VecTab vt = VecTab{}) {
   if (P->blue[0].n) {
-    if constexpr (std::is_same<S, double>::value)
+    if constexpr (std::is_same<S, double>::value)  // (FP32 storage: fm_general32.cuh)
       return launch_bxi<double, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
-    else return launch_bxi<float, double>(d, epi, in, V, xv, bv, rs, ep, P->blue[0], blue_factor(P, 0, ramp), out, act, P->st, vt);
+    else return cudaErrorNotSupported;
   }
   if constexpr (std::is_same<S, double>::value)
     return launch_xi<double, double>(d, epi, in, V, xv, bv, rs, ep, tw, ramp, out, act, P->st, vt);
@@ -327,16 +330,19 @@ static fm_status init_tables(fm_plan* P) {
         g.m = t.m;
         std::vector<cd> both = t.chirp[0];
         both.insert(both.end(), t.chirp[1].begin(), t.chirp[1].end());
-        FM_CK(upload_cplx<R>(P->gch[a], both, P->st));
+        FM_CK(upload_cplx<R>(P->genchirp[a], both, P->st));
         for (int dir = 0; dir < 2; ++dir) {
-          FM_CK(upload_cplx<R>(P->gkn[a][dir], t.kern[dir], P->st));
-          g.chirp[dir] = (const cplx<R>*)P->gch[a].p + dir * g.n;
-          g.kern[dir] = P->gkn[a][dir].p;
+          FM_CK(upload_cplx<R>(P->genkern[a][dir], t.kern[dir], P->st));
+          g.chirp[dir] = (const cplx<R>*)P->genchirp[a].p + dir * g.n;
+          g.kern[dir] = P->genkern[a][dir].p;
         }
       }
-      FM_CK(upload_cplx<R>(P->gtw[a], twiddles<R>(g.m), P->st));
-      g.tw = P->gtw[a].p;
-      continue;
+      FM_CK(upload_cplx<R>(P->gentw[a], twiddles<R>(g.m), P->st));
+      g.tw = P->gentw[a].p;
+      if (P->shift[a] != 0.0)
+        for (int br = 0; br < 2; ++br)
+          FM_CK(upload_cplx<R>(P->genramp[a][br], fm::ramp(n3[a], P->shift[a], br == 0 ? -1.0 : 1.0), P->st));
+      if (!P->c64) continue;  // (no FP64 block vectors)
     }
     if (axis_supported(n3[a])) {
       FM_CK(upload_cplx<R>(*tw[a], twiddles<R>(n3[a]), P->st));
@@ -364,7 +370,8 @@ static fm_status init_tables(fm_plan* P) {
     for (size_t i = 0; i < chirp[a].size(); ++i) r[i] *= chirp[a][i];
     return r;
   };
-  if (!P->blue[2].n && !P->general32) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
+  if (P->general32 && !P->c64) return FM_OK;
+  if (!P->blue[2].n) FM_CK(upload_cplx<R>(P->twz16, twiddles16(P->dims.nz), P->st));
   if (P->zonly) {
     FM_CK(upload_cplx<R>(P->twz2, twiddles<R>(2 * P->dims.nz), P->st));
     FM_CK(upload_cplx<R>(P->rz, ramp(2, -1.0), P->st));
@@ -452,10 +459,11 @@ template <typename R>
 fm_status green_op(fm_plan* P, int nb, const void* in, int pro, const double* rs, int epi, const void* xv,
                    const void* bv, const EpiParams& ep_in, void* out, const int* act, int nact = -1,
                    const RhsCtx* rc = nullptr, int chain = 0);
-// one sweep of the passes (no shift, or z-only shifts), fused x passes, contiguous batches: where green_op can
+// one sweep of the passes (no shift, or z-only shifts), fused x passes, contiguous batches: where green_op<R> can
 // chain applications
+template <typename R>
 inline bool green_chain_ok(const fm_plan* P, const RhsCtx* rc) {
-  return !P->blue[0].n && !P->general32 && (!P->avg || P->zonly || P->zsplit) && !(rc && (rc->vt.in || rc->vt.out));
+  return !P->blue[0].n && !(P->general32 && sizeof(R) == 4) && (!P->avg || P->zonly || P->zsplit) && !(rc && (rc->vt.in || rc->vt.out));
 }
 // H = -i lambda/(2 pi 377) curl(E) for nb fields (in -> out, contiguous batches; act masks RHS)
 template <typename R>

@@ -45,6 +45,10 @@ CASES = {  # grid, layer of voxels per side that absorbs (z; a negative number: 
     "single_41x73x58": ((41, 73, 50), 4, "float32", GMRES),
     "single_51x85x51": ((51, 85, 43), 4, "float32", GMRES),
     "single_open_general": ((30, 33, 25), -5, "float32", GMRES),
+    "general_66x90x99": ((66, 90, 59), 20, "float32-math64", GMRES20),
+    "general_128x96x101": ((128, 96, 61), 20, "float32-math64", GMRES20),
+    "general_open": ((30, 33, 25), -5, "float32-math64", GMRES),
+    "general_z96": ((32, 32, 64), 16, "float32-math64", GMRES),
     "single_z96": ((32, 32, 64), 16, "float32", GMRES),
 }
 
