@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(ZTmaCfg<S, R, L, MODE>::THREADS)
 // transform in eight values a lane exchanges twice on twice the values.  In FP64 192 of 255 registers hold the values,
 // so an SM has eight warps at most, in CTAs of one tile each (one branch of FP64 storage: shared memory holds four to six);
 // one CTA's copies overlap the others' transforms.  The rest of the registers is too few for the compiler: in FP64 it
-// spills 56 to 320 bytes a thread (128 points, both branches: 120 stored, 204 loaded).
+// spills 56 to 320 bytes a thread (128 points, both branches: 120 stored, 208 loaded).
 // ---------------------------------------------------------------------------
 enum { ZR_NONE = 0, ZR_ONE = 1, ZR_TWO = 2, ZR_PAD = 3 };
 
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
     const long long yb = tile / xtiles;
     const int y = (int)(yb % d.ny), b = (int)(yb / d.ny);
     const bool ok = mbar_wait(full, ph, err, 33);
-    if (__syncthreads_or(!ok)) break;  // timed out: nothing of this CTA is in flight but the load that did not come
+    if (__syncthreads_or(!ok)) break;  // timed out
     const GreenBin<R> gb(gp, b);
     const R ky = (R)gp.dk[1] * (kidx_green<R>(y, d.ny) + (R)gp.shift[1]);
 #pragma unroll 1
@@ -567,7 +567,10 @@ __global__ void __launch_bounds__(ZRegCfg<S, R, L, MODE>::THREADS, ZRegCfg<S, R,
     }
     tile = next;
   }
-  if (threadIdx.x == 0) bulk_wait0();
+  if (threadIdx.x == 0) {
+    if (tile < ntiles) mbar_wait(full, ph, err, 34);  // timed out: once more (bounded) for the load in flight
+    bulk_wait0();
+  }
 }
 
 }  // namespace fm
